@@ -65,8 +65,8 @@ class DecoderModel:
         lw, s = self.w.layers[i], self.spec
         if s.qk_norm:
             qkv = ops.linear(n, lw.wqkv)
-            self._qk_norm(qkv, lw)
-            ops.rope_kv_paged(qkv, b.positions, b.slots, kv.k[i], kv.v[i], self.hq, self.hkv, self.d, s.rope_theta)
+            ops.rope_kv_paged(qkv, b.positions, b.slots, kv.k[i], kv.v[i], self.hq, self.hkv, self.d, s.rope_theta,
+                              q_norm=lw.q_norm, k_norm=lw.k_norm, eps=s.rms_eps)
         else:
             qkv = ops.linear_rope_kv(n, lw.wqkv, b.positions, b.slots, kv.k[i], kv.v[i], self.hq, self.hkv, self.d,
                                      s.rope_theta, cos_sin=self._rope_cs)
@@ -83,15 +83,6 @@ class DecoderModel:
         if self.trace is not None:
             self.trace.record(f"layer.{i}.attn", a)
         return self.comm.row_linear(a, lw.wo)
-
-    def _qk_norm(self, qkv: torch.Tensor, lw) -> None:
-        rows = qkv.shape[0]
-        q = qkv[:, : self.hq * self.d].reshape(rows * self.hq, self.d)
-        k = qkv[:, self.hq * self.d: (self.hq + self.hkv) * self.d].reshape(rows * self.hkv, self.d)
-        qn = ops.rmsnorm(q.contiguous(), lw.q_norm, self.spec.rms_eps)
-        kn = ops.rmsnorm(k.contiguous(), lw.k_norm, self.spec.rms_eps)
-        qkv[:, : self.hq * self.d] = qn.view(rows, -1)
-        qkv[:, self.hq * self.d: (self.hq + self.hkv) * self.d] = kn.view(rows, -1)
 
     def _ffn(self, i: int, n: torch.Tensor) -> torch.Tensor:
         lw = self.w.layers[i]

@@ -43,7 +43,6 @@ class FlintModel(DecoderModel):
         glob = self.is_global(i)
         window = 0 if glob else self.window
         qkv = ops.linear(n, lw.wqkv)
-        self._qk_norm(qkv, lw)
         if glob:
             # no positional encoding: the rotary kernel at position 0 is the identity and still writes K / V
             if self._zero_pos is None or self._zero_pos.numel() < b.positions.numel():
@@ -51,7 +50,8 @@ class FlintModel(DecoderModel):
             pos = self._zero_pos[: b.positions.numel()]
         else:
             pos = b.positions
-        ops.rope_kv_paged(qkv, pos, b.slots, kv.k[i], kv.v[i], self.hq, self.hkv, self.d, s.rope_theta)
+        ops.rope_kv_paged(qkv, pos, b.slots, kv.k[i], kv.v[i], self.hq, self.hkv, self.d, s.rope_theta,
+                          q_norm=lw.q_norm, k_norm=lw.k_norm, eps=s.rms_eps)
         if b.is_decode:
             assert b.tree_mask is None, "tree verification is not available with a learnable soft-max"
             a = ops.attn_decode(qkv, kv.k[i], kv.v[i], b.block_table, b.ctx_lens, self.hq, self.hkv, self.d, self.scale,

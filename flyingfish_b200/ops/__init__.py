@@ -413,8 +413,17 @@ def residual_add(res: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
 # ------------------------------------------------------------------------------------------
 def rope_kv_paged(qkv: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, kcache: torch.Tensor,
                   vcache: torch.Tensor, hq: int, hkv: int, dim: int, theta: float, rot_dim: int | None = None,
-                  inv_freq: torch.Tensor | None = None) -> None:
-    """In place on ``qkv`` ([rows, (hq+2*hkv)*dim], Q and K rotated) and the paged cache."""
+                  inv_freq: torch.Tensor | None = None, q_norm: torch.Tensor | None = None,
+                  k_norm: torch.Tensor | None = None, eps: float = 0.0) -> None:
+    """In place on ``qkv`` ([rows, (hq+2*hkv)*dim], Q and K rotated) and the paged cache. ``q_norm`` / ``k_norm`` ([dim], given
+    together): every Q and K head is RMS-normed with them and ``eps`` first."""
+    _require((q_norm is None) == (k_norm is None), "rope_kv_paged: both head norms or none")
+    if q_norm is not None and (not _is_cuda(qkv) or dim != 128):
+        rows = qkv.shape[0]
+        for lo, heads, w in ((0, hq, q_norm), (hq, hkv, k_norm)):
+            part = qkv[:, lo * dim: (lo + heads) * dim]
+            part.copy_(rmsnorm(part.reshape(rows * heads, dim), w, eps).view(rows, -1))
+        q_norm = k_norm = None
     if not _is_cuda(qkv):
         ref.rope_kv_paged(qkv, positions, slots, kcache, vcache, hq, hkv, dim, theta, rot_dim, inv_freq)
         return
@@ -424,9 +433,13 @@ def rope_kv_paged(qkv: torch.Tensor, positions: torch.Tensor, slots: torch.Tenso
     _require(kcache.is_contiguous() and vcache.is_contiguous() and kcache.dim() == 4, "rope_kv_paged: cache layout")
     nb, ch, bs, cd = kcache.shape
     _require(ch == hkv and cd == dim, "rope_kv_paged: cache geometry differs from the heads")
-    rc = kernels().ff_rope_kv_paged(ptr(qkv), ptr(positions), ptr(slots), ptr(kcache), ptr(vcache), ptr(inv_freq),
-                                    rows, hq, hkv, dim, rot_dim or dim, bs, nb, c_float(theta), ld,
-                                    ptr(status_tensor(qkv.device)), stream_ptr())
+    form = (rows, hq, hkv, dim, rot_dim or dim, bs, nb, c_float(theta), ld, ptr(status_tensor(qkv.device)), stream_ptr())
+    where = (ptr(qkv), ptr(positions), ptr(slots), ptr(kcache), ptr(vcache), ptr(inv_freq))
+    if q_norm is None:
+        rc = kernels().ff_rope_kv_paged(*where, *form)
+    else:
+        _require(all(w.dtype == BF16 and w.numel() == dim and w.is_contiguous() for w in (q_norm, k_norm)), "rope_kv_paged: head norms")
+        rc = kernels().ff_norm_rope_kv_paged(*where, ptr(q_norm), ptr(k_norm), c_float(eps), *form)
     check(rc, "ff_rope_kv_paged")
     _count()
 

@@ -14,75 +14,124 @@ namespace ff {
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
-// One thread = one 16-byte vector pair (8 dims of the first half + the matching 8 dims of the
-// second half) of one head of one row.
-__global__ void rope_kv_paged_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
-                                     const int* __restrict__ slots, __nv_bfloat16* __restrict__ kcache,
-                                     __nv_bfloat16* __restrict__ vcache, const float* __restrict__ inv_freq_tab,
-                                     int rows, int hq, int hkv, int dim, int rot_dim, int block_size, int num_blocks,
-                                     float theta, int ldqkv, int* status, const float2* __restrict__ cos_sin) {
+// Rotation, optional RMS norm of the q and k heads before it, and the paged K / V write in one pass over the packed rows. A CTA
+// owns R rows: its threads make the rows' (cos, sin) once in shared memory -- sine, cosine and power of every element of every head
+// are what a thread-per-vector form spends its time on -- and then walk the rows' vector pairs (8 elements of a head's first half
+// and the 8 they turn with), UNROLL of them in flight. NORM: heads of 128 elements are 8 neighbouring lanes, whose sums of squares
+// meet by shuffles; the normed value is rounded to BF16 before it is turned, as a norm kernel of its own would.
+// Bound by DRAM. 8192 rows of 32 + 16 heads of 128: 186 us with angles per vector, 63 us now (216 MB); 2039 rows of
+// 64 + 8 heads: norms, copies and rotation 398 us, 36 us now.
+constexpr int ROPE_THREADS = 256, ROPE_UNROLL = 3;
+
+template <bool NORM>
+__global__ void __launch_bounds__(ROPE_THREADS)
+rope_kv_paged_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions, const int* __restrict__ slots,
+                     __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache, const float* __restrict__ inv_freq_tab,
+                     int rows, int hq, int hkv, int dim, int rot_dim, int block_size, int num_blocks, float theta, int ldqkv,
+                     int* status, const float2* __restrict__ cos_sin, const __nv_bfloat16* __restrict__ q_weight,
+                     const __nv_bfloat16* __restrict__ k_weight, float eps, int R) {
+  extern __shared__ float2 s_cs[];                     // [R][rhalf]
   pdl_trigger();
   if (threadIdx.x == 0) FF_TL(status, KID_ROPE_KV, 0);
   pdl_wait();
   if (threadIdx.x == 0) FF_TL(status, KID_ROPE_KV, 1);
-  const int vec_per_head = dim >> 4;                 // pairs of uint4
-  const int heads = hq + 2 * hkv;
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)rows * heads * vec_per_head;
-  if (gid >= total) return;
-  const int c = (int)(gid % vec_per_head);
-  const int head = (int)((gid / vec_per_head) % heads);
-  const int row = (int)(gid / ((long long)vec_per_head * heads));
-  __nv_bfloat16* base = qkv + (size_t)row * ldqkv + (size_t)head * dim;
-  const int half = dim >> 1;
-  uint4 lo = reinterpret_cast<uint4*>(base)[c];
-  uint4 hi = reinterpret_cast<uint4*>(base + half)[c];
-  const bool is_v = head >= hq + hkv;
-  if (!is_v) {
-    const int pos = cos_sin ? 0 : positions[row];
-    uint32_t* lp = reinterpret_cast<uint32_t*>(&lo);
-    uint32_t* hp = reinterpret_cast<uint32_t*>(&hi);
-    const int rhalf = rot_dim >> 1;
+  const int row0 = blockIdx.x * R, nrow = min(R, rows - row0);
+  const int vph = dim >> 4, rhalf = rot_dim >> 1, half = dim >> 1;
+  const int per_row = (hq + 2 * hkv) * vph, n = nrow * per_row;
+  for (int i = threadIdx.x; i < nrow * rhalf; i += ROPE_THREADS) {
+    const int r = i / rhalf, j = i - r * rhalf;
+    if (cos_sin) {                                     // per-row table (2-D / multi-axis rotary): already BF16-rounded
+      s_cs[i] = cos_sin[(size_t)(row0 + r) * rhalf + j];
+    } else {
+      const float inv = inv_freq_tab ? inv_freq_tab[j] : 1.0f / powf(theta, (float)(2 * j) / (float)rot_dim);
+      float sn, cs;
+      sincosf((float)positions[row0 + r] * inv, &sn, &cs);
+      s_cs[i] = make_float2(bf16r(cs), bf16r(sn));     // cos/sin rounded to BF16
+    }
+  }
+  __syncthreads();
+  for (int base = threadIdx.x; base - (int)threadIdx.x < n; base += ROPE_THREADS * ROPE_UNROLL) {
+    uint4 lo[ROPE_UNROLL], hi[ROPE_UNROLL];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 a = unpack_bf16x2(lp[j]), b = unpack_bf16x2(hp[j]);
-      float ao[2] = {a.x, a.y}, bo[2] = {b.x, b.y};
+    for (int u = 0; u < ROPE_UNROLL; ++u) {
+      const int i = base + u * ROPE_THREADS;
+      lo[u] = hi[u] = make_uint4(0, 0, 0, 0);
+      if (i < n) {
+        const int r = i / per_row, v = i - r * per_row, head = v / vph, c = v - head * vph;
+        const __nv_bfloat16* src = qkv + (size_t)(row0 + r) * ldqkv + (size_t)head * dim;
+        lo[u] = reinterpret_cast<const uint4*>(src)[c];
+        hi[u] = reinterpret_cast<const uint4*>(src + half)[c];
+      }
+    }
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int i = c * 8 + j * 2 + e;               // index inside the half
-        if (i < rhalf) {
-          float sn, cs;
-          if (cos_sin) {                                // per-row table (2-D / multi-axis rotary): already BF16-rounded
-            const float2 t = cos_sin[(size_t)row * rhalf + i];
-            cs = t.x; sn = t.y;
-          } else {
-            const float inv = inv_freq_tab ? inv_freq_tab[i] : 1.0f / powf(theta, (float)(2 * i) / (float)rot_dim);
-            sincosf((float)pos * inv, &sn, &cs);
-            cs = bf16r(cs); sn = bf16r(sn);             // cos/sin rounded to BF16
+    for (int u = 0; u < ROPE_UNROLL; ++u) {
+      const int i = min(base + u * ROPE_THREADS, n - 1);
+      const bool live = base + u * ROPE_THREADS < n;
+      const int r = i / per_row, v = i - r * per_row, head = v / vph, c = v - head * vph;
+      const int row = row0 + r;
+      const bool is_v = head >= hq + hkv;
+      uint32_t* lp = reinterpret_cast<uint32_t*>(&lo[u]);
+      uint32_t* hp = reinterpret_cast<uint32_t*>(&hi[u]);
+      if (NORM) {                                      // every lane takes part: per_row and ROPE_THREADS are multiples of 8
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 a = unpack_bf16x2(lp[j]), b = unpack_bf16x2(hp[j]);
+          ss += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
+        }
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1); ss += __shfl_xor_sync(0xffffffffu, ss, 2); ss += __shfl_xor_sync(0xffffffffu, ss, 4);
+        if (!is_v) {
+          const float rstd = rsqrtf(ss / (float)dim + eps);
+          const __nv_bfloat16* w = head < hq ? q_weight : k_weight;
+          const uint4 wl = __ldg(reinterpret_cast<const uint4*>(w) + c), wh = __ldg(reinterpret_cast<const uint4*>(w + half) + c);
+          const uint32_t* wlp = reinterpret_cast<const uint32_t*>(&wl);
+          const uint32_t* whp = reinterpret_cast<const uint32_t*>(&wh);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 a = unpack_bf16x2(lp[j]), b = unpack_bf16x2(hp[j]), ga = unpack_bf16x2(wlp[j]), gb = unpack_bf16x2(whp[j]);
+            lp[j] = pack_bf16x2(a.x * rstd * ga.x, a.y * rstd * ga.y);
+            hp[j] = pack_bf16x2(b.x * rstd * gb.x, b.y * rstd * gb.y);
           }
-          const float x1 = ao[e], x2 = bo[e];
-          // BF16 arithmetic: every product and the final sum/difference round to BF16
-          ao[e] = bf16r(bf16r(x1 * cs) - bf16r(x2 * sn));
-          bo[e] = bf16r(bf16r(x2 * cs) + bf16r(x1 * sn));
         }
       }
-      lp[j] = pack_bf16x2(ao[0], ao[1]);
-      hp[j] = pack_bf16x2(bo[0], bo[1]);
+      if (!live) continue;
+      if (!is_v) {
+        const float2* cs = s_cs + r * rhalf;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 a = unpack_bf16x2(lp[j]), b = unpack_bf16x2(hp[j]);
+          float ao[2] = {a.x, a.y}, bo[2] = {b.x, b.y};
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int k = c * 8 + j * 2 + e;           // index inside the half
+            if (k < rhalf) {
+              const float2 t = cs[k];
+              const float x1 = ao[e], x2 = bo[e];
+              // BF16 arithmetic: every product and the final sum/difference round to BF16
+              ao[e] = bf16r(bf16r(x1 * t.x) - bf16r(x2 * t.y));
+              bo[e] = bf16r(bf16r(x2 * t.x) + bf16r(x1 * t.y));
+            }
+          }
+          lp[j] = pack_bf16x2(ao[0], ao[1]);
+          hp[j] = pack_bf16x2(bo[0], bo[1]);
+        }
+        __nv_bfloat16* dst = qkv + (size_t)row * ldqkv + (size_t)head * dim;
+        reinterpret_cast<uint4*>(dst)[c] = lo[u];
+        reinterpret_cast<uint4*>(dst + half)[c] = hi[u];
+      }
+      if (head >= hq) {
+        const int slot = slots[row];
+        if (slot < 0) continue;                        // padding row: nothing cached
+        const int blk = slot / block_size, off = slot - blk * block_size;
+        if (blk >= num_blocks) { set_status(status, KID_ROPE_KV, FF_ERR_BOUNDS, row, slot); continue; }
+        const int kvh = is_v ? head - hq - hkv : head - hq;
+        if (c == 0) dbg_write_once(status, KID_ROPE_KV, is_v ? DBG_KV_V : DBG_KV_K, (long long)slot * hkv + kvh);
+        FF_DBG_CHECK(off >= 0 && off < block_size && kvh >= 0 && kvh < hkv, status, KID_ROPE_KV, row, kvh);
+        __nv_bfloat16* dst = (is_v ? vcache : kcache) + (((size_t)blk * hkv + kvh) * block_size + off) * dim;
+        reinterpret_cast<uint4*>(dst)[c] = lo[u];
+        reinterpret_cast<uint4*>(dst + half)[c] = hi[u];
+      }
     }
-    reinterpret_cast<uint4*>(base)[c] = lo;
-    reinterpret_cast<uint4*>(base + half)[c] = hi;
-  }
-  if (head >= hq) {
-    const int slot = slots[row];
-    if (slot < 0) return;                               // padding row: nothing cached
-    const int blk = slot / block_size, off = slot - blk * block_size;
-    if (blk >= num_blocks) { set_status(status, KID_ROPE_KV, FF_ERR_BOUNDS, row, slot); return; }
-    const int kvh = is_v ? head - hq - hkv : head - hq;
-    if (c == 0) dbg_write_once(status, KID_ROPE_KV, is_v ? DBG_KV_V : DBG_KV_K, (long long)slot * hkv + kvh);
-    FF_DBG_CHECK(off >= 0 && off < block_size && kvh >= 0 && kvh < hkv, status, KID_ROPE_KV, row, kvh);
-    __nv_bfloat16* dst = (is_v ? vcache : kcache) + (((size_t)blk * hkv + kvh) * block_size + off) * dim;
-    reinterpret_cast<uint4*>(dst)[c] = lo;
-    reinterpret_cast<uint4*>(dst + half)[c] = hi;
   }
 }
 
@@ -420,15 +469,38 @@ sample_rows_kernel(const float* __restrict__ logits, int* __restrict__ out_ids, 
 }  // namespace ff
 using namespace ff;
 
+// Rows per CTA: four where that still leaves several CTAs per SM (fewer angles made twice, three vectors of a thread in flight), one
+// for decode batches.
+static int rope_launch(void* qkv, const int* positions, const int* slots, void* kcache, void* vcache, const float* inv_freq, int rows, int hq,
+                       int hkv, int dim, int rot_dim, int block_size, int num_blocks, float theta, int ldqkv, int* status, const float* cos_sin,
+                       const void* q_weight, const void* k_weight, float eps, cudaStream_t s) {
+  if (rows <= 0 || dim % 16 || rot_dim > dim || rot_dim % 2 || ldqkv % 8) return FF_HOST_BAD_SHAPE;
+  const int R = rows >= 4 * 4 * 148 && rot_dim <= 1024 ? 4 : 1;
+  const size_t smem = (size_t)R * (rot_dim / 2) * sizeof(float2);
+  auto kern = q_weight ? rope_kv_paged_kernel<true> : rope_kv_paged_kernel<false>;
+  if (smem > 48 * 1024)
+    if (int r = opt_in_smem(kern, (int)smem)) return r;
+  if (int lr_ = launch_pdl(kern, dim3((unsigned)((rows + R - 1) / R)), dim3(ROPE_THREADS), smem, s, 0, (__nv_bfloat16*)qkv, positions, slots,
+      (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, inv_freq, rows, hq, hkv, dim, rot_dim, block_size, num_blocks, theta, ldqkv, status,
+      reinterpret_cast<const float2*>(cos_sin), (const __nv_bfloat16*)q_weight, (const __nv_bfloat16*)k_weight, eps, R)) return lr_;
+  return launch_result();
+}
+
 FF_EXPORT int ff_rope_kv_paged(void* qkv, const int* positions, const int* slots, void* kcache, void* vcache,
                                const float* inv_freq, int rows, int hq, int hkv, int dim, int rot_dim, int block_size,
                                int num_blocks, float theta, int ldqkv, int* status, cudaStream_t s) {
-  if (rows <= 0 || dim % 16 || rot_dim > dim || rot_dim % 2 || ldqkv % 8) return FF_HOST_BAD_SHAPE;
-  const long long total = (long long)rows * (hq + 2 * hkv) * (dim / 16);
-  if (int lr_ = launch_pdl(rope_kv_paged_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, 0, (__nv_bfloat16*)qkv, positions, slots,
-      (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, inv_freq, rows, hq, hkv, dim, rot_dim, block_size, num_blocks,
-      theta, ldqkv, status, (const float2*)nullptr)) return lr_;
-  return launch_result();
+  return rope_launch(qkv, positions, slots, kcache, vcache, inv_freq, rows, hq, hkv, dim, rot_dim, block_size, num_blocks, theta, ldqkv, status,
+                     nullptr, nullptr, nullptr, 0.f, s);
+}
+
+// The same with an RMS norm per q and k head (weights of 128 elements) before the rotation.
+FF_EXPORT int ff_norm_rope_kv_paged(void* qkv, const int* positions, const int* slots, void* kcache, void* vcache, const float* inv_freq,
+                                    const void* q_weight, const void* k_weight, float eps, int rows, int hq, int hkv, int dim, int rot_dim,
+                                    int block_size, int num_blocks, float theta, int ldqkv, int* status, cudaStream_t s) {
+  if (dim != 128 || !q_weight || !k_weight) return FF_HOST_BAD_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(q_weight) & 15) || (reinterpret_cast<uintptr_t>(k_weight) & 15)) return FF_HOST_BAD_ALIGN;
+  return rope_launch(qkv, positions, slots, kcache, vcache, inv_freq, rows, hq, hkv, dim, rot_dim, block_size, num_blocks, theta, ldqkv, status,
+                     nullptr, q_weight, k_weight, eps, s);
 }
 
 // Same with the angles given as a table: cos_sin [rows, rot_dim/2] (cos, sin) FP32 holding BF16-rounded values.
@@ -437,12 +509,9 @@ FF_EXPORT int ff_rope_kv_paged(void* qkv, const int* positions, const int* slots
 FF_EXPORT int ff_rope_kv_paged_table(void* qkv, const float* cos_sin, const int* slots, void* kcache, void* vcache,
                                      int rows, int hq, int hkv, int dim, int rot_dim, int block_size, int num_blocks,
                                      int ldqkv, int* status, cudaStream_t s) {
-  if (rows <= 0 || dim % 16 || rot_dim > dim || rot_dim % 2 || ldqkv % 8 || !cos_sin) return FF_HOST_BAD_SHAPE;
-  const long long total = (long long)rows * (hq + 2 * hkv) * (dim / 16);
-  if (int lr_ = launch_pdl(rope_kv_paged_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, 0, (__nv_bfloat16*)qkv,
-      (const int*)nullptr, slots, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, (const float*)nullptr, rows, hq, hkv, dim,
-      rot_dim, block_size, num_blocks, 1.0f, ldqkv, status, reinterpret_cast<const float2*>(cos_sin))) return lr_;
-  return launch_result();
+  if (!cos_sin) return FF_HOST_BAD_SHAPE;
+  return rope_launch(qkv, nullptr, slots, kcache, vcache, nullptr, rows, hq, hkv, dim, rot_dim, block_size, num_blocks, 1.0f, ldqkv, status,
+                     cos_sin, nullptr, nullptr, 0.f, s);
 }
 
 // out: float2 [rows, rot_dim/2]
