@@ -21,6 +21,9 @@ from .decoder import DecoderModel
 from .weights import LayerWeights, ModelWeights, TPInfo, build_decoder_weights
 
 
+EXPAND_MAX_BYTES = 2 << 30       # most memory that a layer's expanded keys and values take
+
+
 @dataclass
 class MlaWeights:
     q_a: torch.Tensor | None        # [q_lora, h]
@@ -29,8 +32,12 @@ class MlaWeights:
     kv_a: torch.Tensor              # [kv_lora + rope, h]
     kv_a_ln: torch.Tensor
     w_uk_t: torch.Tensor            # [heads, kv_lora, nope]   (absorb: q_lat = q_nope @ W_UK)
-    w_uv: torch.Tensor              # [heads, v, kv_lora]
+    w_kv: torch.Tensor              # [heads * nope | heads * v, kv_lora]: all key matrices, then all value matrices
     wo: torch.Tensor                # [h, heads*v]
+
+    def w_uv(self, heads: int) -> torch.Tensor:
+        """[heads, v, kv_lora]"""
+        return self.w_kv[heads * self.w_uk_t.shape[2]:].view(heads, -1, self.w_kv.shape[1])
 
 
 def build_deepseek_weights(spec: ModelSpec, source, device, tp: TPInfo | None = None, ep: TPInfo | None = None
@@ -70,7 +77,7 @@ def build_deepseek_weights(spec: ModelSpec, source, device, tp: TPInfo | None = 
         kv_b = source(p + "kv_b_proj.weight", (heads * (a.qk_nope_dim + a.v_head_dim), a.kv_lora_rank))
         kv_b = kv_b.view(heads, a.qk_nope_dim + a.v_head_dim, a.kv_lora_rank)
         w_uk = kv_b[:, : a.qk_nope_dim]                         # [heads, nope, kv_lora]
-        w_uv = kv_b[:, a.qk_nope_dim:].contiguous()             # [heads, v, kv_lora]
+        w_kv = torch.cat([w_uk.reshape(-1, a.kv_lora_rank), kv_b[:, a.qk_nope_dim:].reshape(-1, a.kv_lora_rank)])
         wo = source(p + "o_proj.weight", (h, heads * a.v_head_dim))
         w_uk_t = w_uk.transpose(1, 2).contiguous()
         if fp8:
@@ -79,7 +86,7 @@ def build_deepseek_weights(spec: ModelSpec, source, device, tp: TPInfo | None = 
             from ..ops.quant_ops import Fp8Weight
             q_a = Fp8Weight.from_dense(q_a) if q_a is not None else None
             q_b, kv_a, wo = Fp8Weight.from_dense(q_b), Fp8Weight.from_dense(kv_a), Fp8Weight.from_dense(wo)
-        lw.extra["mla"] = MlaWeights(q_a, q_a_ln, q_b, kv_a, kv_a_ln, w_uk_t, w_uv, wo)
+        lw.extra["mla"] = MlaWeights(q_a, q_a_ln, q_b, kv_a, kv_a_ln, w_uk_t, w_kv, wo)
         lw.wo = wo
     return w
 
@@ -112,8 +119,55 @@ class DeepseekModel(DecoderModel):
             q = ops.linear(qa, m.q_b)
         else:
             q = ops.linear(n, m.q_b)
-        q = q.view(rows, heads, a.qk_nope_dim + a.qk_rope_dim)
         kva = ops.linear(n, m.kv_a)
+        if n.is_cuda:
+            o = self._attend(i, q, kva, m, b, kv)
+        else:
+            o = self._attend_oracle(i, q, kva, m, b, kv)
+        if self.trace is not None:
+            self.trace.record(f"layer.{i}.attn", o.view(rows, heads, a.v_head_dim))
+        return self.comm.row_linear(o, m.wo)
+
+    def _attend(self, i: int, q: torch.Tensor, kva: torch.Tensor, m: MlaWeights, b, kv) -> torch.Tensor:
+        """[rows, heads * v] on the GPU. Portions of prompts expand the visible latents to keys and values; decoded tokens, short
+        portions and contexts beyond the expansion's memory go through the latent space."""
+        s, a, heads, rows = self.spec, self.mla, self.spec.heads, q.shape[0]
+        cache, nope, dv = kv.k[i], a.qk_nope_dim, a.v_head_dim
+        form = (kva, m.kv_a_ln, b.positions, b.slots, cache, heads, nope, s.rope_theta, s.rms_eps)
+        pages = None
+        if not b.is_decode and mla_ops.expands(q, self.latent_dim, nope, a.qk_rope_dim, dv, b.max_q_len):
+            pages = self._key_pages(b, kv)
+        if pages is not None:
+            mla_ops.norm_rope_cache(q, *form)
+            out = torch.empty(rows, heads * dv, dtype=q.dtype, device=q.device)
+            return mla_ops.expanded_attention(q, q.view(rows, heads, -1), cache, m.w_kv, pages, b.block_table, b.q_start, b.q_lens, b.ctx_lens,
+                                              b.max_q_len, nope, dv, a.kv_lora_rank, self.scale, 0, None, out)
+        q_full = torch.empty(rows, heads, self.latent_dim, dtype=q.dtype, device=q.device)
+        mla_ops.norm_rope_cache(q, *form, q_full)
+        ops.head_linear(q, m.w_uk_t, out=q_full.view(rows, -1), x_cols=nope + a.qk_rope_dim, out_cols=self.latent_dim)
+        lat = mla_ops.attention(q_full, cache, b.block_table, b.q_start, b.q_lens, b.ctx_lens, b.nq if b.is_decode else b.max_q_len, b.max_ctx,
+                                self.scale, a.kv_lora_rank)
+        return ops.head_linear(lat.view(rows, -1), m.w_uv(heads))
+
+    def hidden_states(self, b, kv, inputs_embeds=None):
+        self._pages = None                      # pages the portions of this step can see, listed by its first layer
+        return super().hidden_states(b, kv, inputs_embeds)
+
+    def _key_pages(self, b, kv):
+        """The pages of a step's portions, or None where keys and values of all heads would take over ``EXPAND_MAX_BYTES``."""
+        if self._pages is None:
+            L, h, n = b.layout, b.host, b.batch
+            table = h[L.block_table: L.block_table + L.max_batch * L.max_blocks].view(L.max_batch, L.max_blocks)[:n]
+            ctx = h[L.ctx_lens: L.ctx_lens + n].tolist()
+            keys = sum((c + kv.block_size - 1) // kv.block_size for c in ctx) * kv.block_size
+            fits = 2 * keys * self.spec.heads * (self.mla.qk_nope_dim + self.mla.v_head_dim) <= EXPAND_MAX_BYTES
+            self._pages = (mla_ops.KeyPages.of(h[L.q_lens: L.q_lens + n].tolist(), ctx, table, 0, kv.block_size, b.device) if fits else None,)
+        return self._pages[0]
+
+    def _attend_oracle(self, i: int, q: torch.Tensor, kva: torch.Tensor, m: MlaWeights, b, kv) -> torch.Tensor:
+        """[rows, heads * v] through the latent space, operator by operator (CPU)."""
+        s, a, heads, rows = self.spec, self.mla, self.spec.heads, q.shape[0]
+        q = q.view(rows, heads, a.qk_nope_dim + a.qk_rope_dim)
         c = ops.rmsnorm(kva[:, : a.kv_lora_rank], m.kv_a_ln, s.rms_eps)
         k_rope = kva[:, a.kv_lora_rank:].contiguous()
         q_rope = q[:, :, a.qk_nope_dim:].reshape(rows, heads * a.qk_rope_dim).contiguous()
@@ -122,16 +176,6 @@ class DeepseekModel(DecoderModel):
         mla_ops.cache_write(c, k_rope, b.slots, kv.k[i])
         q_lat = mla_ops.per_head_linear(q[:, :, : a.qk_nope_dim].contiguous(), m.w_uk_t)      # [rows, heads, kv_lora]
         q_full = torch.cat([q_lat, q_rope.view(rows, heads, a.qk_rope_dim)], dim=2).contiguous()
-        if b.is_decode:
-            batch = b.batch
-            q_start = b.q_start
-            q_lens = b.q_lens
-            max_q = b.nq
-        else:
-            q_start, q_lens, max_q = b.q_start, b.q_lens, b.max_q_len
-        out_lat = mla_ops.attention(q_full, kv.k[i], b.block_table, q_start, q_lens, b.ctx_lens, max_q,
-                                    b.max_ctx, self.scale, a.kv_lora_rank)
-        o = mla_ops.per_head_linear(out_lat, m.w_uv)                                          # [rows, heads, v]
-        if self.trace is not None:
-            self.trace.record(f"layer.{i}.attn", o)
-        return self.comm.row_linear(o.reshape(rows, heads * a.v_head_dim), m.wo)
+        lat = mla_ops.attention(q_full, kv.k[i], b.block_table, b.q_start, b.q_lens, b.ctx_lens, b.nq if b.is_decode else b.max_q_len, b.max_ctx,
+                                self.scale, a.kv_lora_rank)
+        return mla_ops.per_head_linear(lat, m.w_uv(heads)).reshape(rows, heads * a.v_head_dim)

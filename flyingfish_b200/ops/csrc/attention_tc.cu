@@ -377,7 +377,7 @@ struct PrefillForm {
   // sequence b is at key row (exp_off[b] + t) * 64. The last dr elements of queries and keys come from maps of their own: tmG, rows with
   // head h at column h * qr_pitch + qr_col, and tmR, the cache's rows, at column kr_col.
   const int* exp_off;
-  int dr, qr_pitch, qr_col, kr_col;
+  int dr, q_pitch, qr_pitch, qr_col, kr_col;
 };
 
 // Capped scores. N raw products of a thread become tanh(y), y = s cap_in; the cap is the factor of the exponent. Where all |y| of the
@@ -504,9 +504,10 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(&bars.q_full, (k_hi ? TC_Q_BYTES : TC_Q_BYTES / 2) + (LAT ? 16384 : 0));
-      tma_load_2d(sQ, &tmQ, &bars.q_full, h * dk, qs + r0);
+      const int qx = h * (LAT ? f.q_pitch : dk);
+      tma_load_2d(sQ, &tmQ, &bars.q_full, qx, qs + r0);
       if (LAT) tma_load_2d(sQ + 2 * TC_BM * 128, &tmG, &bars.q_full, h * f.qr_pitch + f.qr_col, qs + r0);
-      if (k_hi) tma_load_2d(sQ + TC_BM * 128, &tmQ, &bars.q_full, h * dk + 64, qs + r0);
+      if (k_hi) tma_load_2d(sQ + TC_BM * 128, &tmQ, &bars.q_full, qx + 64, qs + r0);
       bool ok = true, bad = false;
       const int nblk = (ctx + TC_PAGE - 1) / TC_PAGE;
       auto tile_row = [&](int j) -> int {
@@ -776,7 +777,7 @@ FF_EXPORT int ff_attn_prefill_tc(const void* q, const void* kcache, const void* 
   const float scale_log2 = (softcap > 0.f ? softcap : scale) * 1.4426950408889634f;
   dim3 grid((max_q_len + TC_BM - 1) / TC_BM, hq, batch);
   const PrefillForm f = {window < 0 ? 0 : window, chunk, window < 0 ? 0 : 1, dk, dv, gate != nullptr ? 1 : 0, window > 0 ? keep : 0,
-                         softcap > 0.f ? scale / softcap : 0.f, (const __nv_bfloat16*)head_gate, ldhg, nullptr, 0, 0, 0, 0};
+                         softcap > 0.f ? scale / softcap : 0.f, (const __nv_bfloat16*)head_gate, ldhg, nullptr, 0, 0, 0, 0, 0};
   CUtensorMap tmG = tmQ;
   if (gate != nullptr)
     if (int r = make_tmap_2d(&tmG, gate, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)hq * dv, (uint64_t)total_rows, (uint64_t)ldg * 2, 64, TC_BM)) return r;
@@ -809,21 +810,21 @@ FF_EXPORT int ff_attn_prefill_tc(const void* q, const void* kcache, const void* 
 
 // Latent attention over keys and values expanded from the latents (prefill; one product of all heads' matrices with the rows the queries
 // can see): head h's key is [expanded key (dk) | rotated key of the cache row (dr)]. q: rows [rows, ldq] with head h's unrotated part at
-// column h * dk; q_rot: rows of heads * qr_pitch columns with its rotated part at h * qr_pitch + qr_col; expanded: [exp_rows, lde], head
+// column h * q_pitch; q_rot: rows of heads * qr_pitch columns with its rotated part at h * qr_pitch + qr_col; expanded: [exp_rows, lde], head
 // h's key at column h * dk and its value at hq * dk + h * dv; page t of sequence b starts at row (exp_off[b] + t) * 64; cache:
 // [num_blocks, 1, 64, cache_width] with the rotated key at column kr_col. out [rows, ldo]. dk, dv multiples of 16 up to 128, dr up to 64.
 FF_EXPORT int ff_attn_prefill_latent(const void* q, const void* q_rot, const void* expanded, const void* cache, const int* block_table,
                                      const int* q_start, const int* q_lens, const int* ctx_lens, const int* exp_off, void* out, int batch,
-                                     int total_rows, int max_q_len, int hq, int dk, int dr, int dv, int ldq, int qr_pitch, int qr_col, int lde,
+                                     int total_rows, int max_q_len, int hq, int dk, int dr, int dv, int ldq, int q_pitch, int qr_pitch, int qr_col, int lde,
                                      int exp_rows, int cache_width, int kr_col, int ldo, int max_blocks, int num_blocks, float scale, int window,
                                      const void* head_gate, int ldhg, int* status, cudaStream_t s) {
   if (batch <= 0 || max_q_len <= 0 || hq <= 0 || total_rows <= 0 || exp_rows <= 0 || window < 0 || !(scale > 0.f)) return FF_HOST_BAD_SHAPE;
   if (dk < 16 || dk > TC_HD || dk % 16 || dv < 16 || dv > TC_HD || dv % 16 || dr < 16 || dr > 64 || dr % 16) return FF_HOST_BAD_SHAPE;
-  if (ldq < hq * dk || lde < hq * (dk + dv) || qr_pitch < qr_col + dr || cache_width < kr_col + dr || exp_off == nullptr) return FF_HOST_BAD_SHAPE;
-  if (ldq % 8 || lde % 8 || qr_pitch % 8 || qr_col % 8 || cache_width % 8 || kr_col % 8 || ldo % 8 || (reinterpret_cast<uintptr_t>(out) & 15)) return FF_HOST_BAD_ALIGN;
+  if (q_pitch < dk || ldq < (hq - 1) * q_pitch + dk || lde < hq * (dk + dv) || qr_pitch < qr_col + dr || cache_width < kr_col + dr || exp_off == nullptr) return FF_HOST_BAD_SHAPE;
+  if (ldq % 8 || lde % 8 || q_pitch % 8 || qr_pitch % 8 || qr_col % 8 || cache_width % 8 || kr_col % 8 || ldo % 8 || (reinterpret_cast<uintptr_t>(out) & 15)) return FF_HOST_BAD_ALIGN;
   constexpr auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap tmQ, tmG, tmK, tmV, tmR;
-  if (int r = make_tmap_2d(&tmQ, q, BF, 2, (uint64_t)hq * dk, total_rows, (uint64_t)ldq * 2, 64, TC_BM)) return r;
+  if (int r = make_tmap_2d(&tmQ, q, BF, 2, (uint64_t)(hq - 1) * q_pitch + dk, total_rows, (uint64_t)ldq * 2, 64, TC_BM)) return r;
   if (int r = make_tmap_2d(&tmG, q_rot, BF, 2, (uint64_t)hq * qr_pitch, total_rows, (uint64_t)hq * qr_pitch * 2, 64, TC_BM)) return r;
   if (int r = make_tmap_2d(&tmK, expanded, BF, 2, (uint64_t)hq * dk, exp_rows, (uint64_t)lde * 2, 64, TC_PAGE)) return r;
   const __nv_bfloat16* values = (const __nv_bfloat16*)expanded + (size_t)hq * dk;
@@ -831,7 +832,7 @@ FF_EXPORT int ff_attn_prefill_latent(const void* q, const void* q_rot, const voi
   if (int r = make_tmap_2d(&tmR, cache, BF, 2, cache_width, (uint64_t)num_blocks * TC_PAGE, (uint64_t)cache_width * 2, 64, TC_PAGE)) return r;
   PrefillForm f = {};
   f.window = window; f.causal = 1; f.dk = dk; f.dv = dv; f.head_gate = (const __nv_bfloat16*)head_gate; f.ldhg = ldhg;
-  f.exp_off = exp_off; f.dr = dr; f.qr_pitch = qr_pitch; f.qr_col = qr_col; f.kr_col = kr_col;
+  f.exp_off = exp_off; f.dr = dr; f.q_pitch = q_pitch; f.qr_pitch = qr_pitch; f.qr_col = qr_col; f.kr_col = kr_col;
   auto kern = dk == TC_HD && dv == TC_HD ? attn_prefill_tc2_kernel<2, true, true, false, true> : attn_prefill_tc2_kernel<2, false, true, false, true>;
   if (int r = opt_in_smem(kern, LAT_SMEM)) return r;
   kern<<<dim3((max_q_len + TC_BM - 1) / TC_BM, hq, batch), 320, LAT_SMEM, s>>>(tmQ, tmK, tmV, tmG, tmR, block_table, q_start, q_lens, ctx_lens,

@@ -287,6 +287,86 @@ __global__ void mla_cache_write_kernel(const __nv_bfloat16* __restrict__ c, cons
   }
 }
 
+// What stands between the projections and the attention of a layer, in one pass: the rotary part of every query head is turned (to
+// `q_rot` where given, in place otherwise), the latent is RMS-normed and goes with the turned key part to the row's cache slot. Halves
+// turn against each other in BF16 arithmetic, as the rotary kernel does. A CTA owns a row. One launch of 4 us (64 rows) for a norm, two
+// copies, two rotations and a cache write of 30 us together; at 1594 rows 15 us for 120 us.
+// q: head h's rotary part at column h * q_pitch + q_col; q_rot: [rows, heads, rot_pitch], the turned part in its last 64 columns.
+__global__ void __launch_bounds__(256)
+mla_norm_rope_cache_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kva, const __nv_bfloat16* __restrict__ weight,
+                           const int* __restrict__ positions, const int* __restrict__ slots, __nv_bfloat16* __restrict__ cache,
+                           __nv_bfloat16* __restrict__ q_rot, int heads, int ldq, int q_pitch, int q_col, int rot_pitch, int ldkva,
+                           int num_blocks, float theta, float eps, int* status) {
+  constexpr int ROT = LD - LV, RH = ROT / 2;             // 64 rotary elements, 32 pairs
+  __shared__ float2 cs[RH];
+  __shared__ float red[2];
+  pdl_trigger();
+  pdl_wait();
+  const int row = blockIdx.x, tid = threadIdx.x;
+  const __nv_bfloat16* src = kva + (size_t)row * ldkva;
+  uint4 lat = make_uint4(0, 0, 0, 0);
+  if (tid < LV / 8) {                                    // warps 0 and 1: the latent, 8 elements per thread
+    lat = reinterpret_cast<const uint4*>(src)[tid];
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(&lat);
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { const float2 f = unpack_bf16x2(w[j]); ss += f.x * f.x + f.y * f.y; }
+    ss = warp_sum(ss);
+    if ((tid & 31) == 0) red[tid >> 5] = ss;
+  } else if (tid < LV / 8 + RH) {
+    const int i = tid - LV / 8;
+    const float inv = 1.0f / powf(theta, (float)(2 * i) / (float)ROT);
+    float sn, c;
+    sincosf((float)positions[row] * inv, &sn, &c);
+    cs[i] = make_float2(__bfloat162float(__float2bfloat16(c)), __bfloat162float(__float2bfloat16(sn)));
+  }
+  __syncthreads();
+  auto turn = [&](uint4& lo, uint4& hi, int c) {
+    uint32_t* lp = reinterpret_cast<uint32_t*>(&lo);
+    uint32_t* hp = reinterpret_cast<uint32_t*>(&hi);
+    auto r = [](float x) { return __bfloat162float(__float2bfloat16(x)); };
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 a = unpack_bf16x2(lp[j]), b = unpack_bf16x2(hp[j]), t0 = cs[c * 8 + 2 * j], t1 = cs[c * 8 + 2 * j + 1];
+      lp[j] = pack_bf16x2(r(a.x * t0.x) - r(b.x * t0.y), r(a.y * t1.x) - r(b.y * t1.y));
+      hp[j] = pack_bf16x2(r(b.x * t0.x) + r(a.x * t0.y), r(b.y * t1.x) + r(a.y * t1.y));
+    }
+  };
+  constexpr int VPH = RH / 8;                            // vector pairs of a head
+  for (int i = tid; i < heads * VPH; i += 256) {
+    const int h = i / VPH, c = i % VPH;
+    __nv_bfloat16* p = q + (size_t)row * ldq + (size_t)h * q_pitch + q_col;
+    uint4 lo = reinterpret_cast<const uint4*>(p)[c], hi = reinterpret_cast<const uint4*>(p + RH)[c];
+    turn(lo, hi, c);
+    __nv_bfloat16* d = q_rot ? q_rot + ((size_t)row * heads + h) * rot_pitch + rot_pitch - ROT : p;
+    reinterpret_cast<uint4*>(d)[c] = lo;
+    reinterpret_cast<uint4*>(d + RH)[c] = hi;
+  }
+  const int slot = slots[row];
+  if (slot < 0) return;
+  if (slot >= num_blocks * PAGE) { if (tid == 0) set_status(status, KID_MLA, FF_ERR_BOUNDS, row, slot); return; }
+  __nv_bfloat16* dst = cache + (size_t)slot * LD;
+  if (tid < LV / 8) {
+    const float rstd = rsqrtf((red[0] + red[1]) / (float)LV + eps);
+    const uint4 wv = reinterpret_cast<const uint4*>(weight)[tid];
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(&lat);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(&wv);
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_bf16x2(a[j]), g = unpack_bf16x2(w[j]);
+      o[j] = pack_bf16x2(f.x * rstd * g.x, f.y * rstd * g.y);
+    }
+    reinterpret_cast<uint4*>(dst)[tid] = make_uint4(o[0], o[1], o[2], o[3]);
+  } else if (tid < LV / 8 + VPH) {
+    const int c = tid - LV / 8;
+    uint4 lo = reinterpret_cast<const uint4*>(src + LV)[c], hi = reinterpret_cast<const uint4*>(src + LV + RH)[c];
+    turn(lo, hi, c);
+    reinterpret_cast<uint4*>(dst + LV)[c] = lo;
+    reinterpret_cast<uint4*>(dst + LV + RH)[c] = hi;
+  }
+}
+
 }  // namespace mla
 }  // namespace ff
 using namespace ff;
@@ -349,5 +429,22 @@ FF_EXPORT int ff_mla_cache_write(const void* c, const void* k_rope, const int* s
   if (rows <= 0 || ldc % 8 || ldk % 8) return FF_HOST_BAD_SHAPE;
   mla::mla_cache_write_kernel<<<rows, 96, 0, s>>>((const __nv_bfloat16*)c, (const __nv_bfloat16*)k_rope, slots,
                                                   (__nv_bfloat16*)cache, rows, ldc, ldk, num_blocks, status);
+  return launch_result();
+}
+
+// q rows of pitch ldq with head h's rotary part (64 elements) at column h * q_pitch + q_col; kva rows of pitch ldkva: latent (512), rotary
+// key part (64); weight [512]; cache [num_blocks, 1, 64, 576]; q_rot: null, or [rows, heads, rot_pitch].
+FF_EXPORT int ff_mla_norm_rope_cache(void* q, const void* kva, const void* weight, const int* positions, const int* slots, void* cache, void* q_rot,
+                                     int rows, int heads, int ldq, int q_pitch, int q_col, int rot_pitch, int ldkva, int num_blocks, float theta,
+                                     float eps, int* status, cudaStream_t s) {
+  constexpr int ROT = mla::LD - mla::LV;
+  if (rows <= 0 || heads <= 0 || num_blocks <= 0 || q_pitch < q_col + ROT || ldq < (heads - 1) * q_pitch + q_col + ROT || ldkva < mla::LD) return FF_HOST_BAD_SHAPE;
+  if (q_rot && rot_pitch < ROT) return FF_HOST_BAD_SHAPE;
+  if (ldq % 8 || q_pitch % 8 || q_col % 8 || rot_pitch % 8 || ldkva % 8) return FF_HOST_BAD_ALIGN;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kva) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(cache) |
+       reinterpret_cast<uintptr_t>(q_rot)) & 15) return FF_HOST_BAD_ALIGN;
+  if (int r = launch_pdl(mla::mla_norm_rope_cache_kernel, dim3(rows), dim3(256), 0, s, 0, (__nv_bfloat16*)q, (const __nv_bfloat16*)kva,
+                         (const __nv_bfloat16*)weight, positions, slots, (__nv_bfloat16*)cache, (__nv_bfloat16*)q_rot, heads, ldq, q_pitch, q_col,
+                         rot_pitch, ldkva, num_blocks, theta, eps, status)) return r;
   return launch_result();
 }

@@ -32,6 +32,24 @@ def cache_write(c: torch.Tensor, k_rope: torch.Tensor, slots: torch.Tensor, cach
     _count()
 
 
+def norm_rope_cache(q: torch.Tensor, kva: torch.Tensor, weight: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, cache: torch.Tensor,
+                    heads: int, nope: int, theta: float, eps: float, q_full: torch.Tensor | None = None) -> None:
+    """The steps between the projections and the attention, one kernel (CUDA): the rotary part of every query head of ``q`` ([rows, heads *
+    (nope + 64)]) is turned, in place or into the last columns of ``q_full`` ([rows, heads, width]); the latent of ``kva`` ([rows, 512 + 64])
+    is normed with ``weight`` and goes with the turned key part to ``slots`` of ``cache``."""
+    nb, one, bs, d = cache.shape
+    rows = q.shape[0]
+    _require(one == 1 and bs == 64 and d == 576 and cache.is_contiguous() and weight.numel() == 512, "MLA kernel: kv_lora 512 + rope 64")
+    _require(q.stride(1) == 1 and kva.stride(1) == 1 and kva.shape == (rows, 576) and q.shape[1] == heads * (nope + 64), "norm_rope_cache: rows")
+    _require(all(t.dtype == torch.bfloat16 for t in (q, kva, weight, cache)) and positions.dtype == slots.dtype == torch.int32, "norm_rope_cache: types")
+    _require(q_full is None or (q_full.is_contiguous() and q_full.shape[:2] == (rows, heads) and q_full.dtype == q.dtype), "norm_rope_cache: q_full")
+    rc = kernels().ff_mla_norm_rope_cache(ptr(q), ptr(kva), ptr(weight), ptr(positions), ptr(slots), ptr(cache), ptr(q_full), rows, heads, q.stride(0),
+                                          nope + 64, nope, 0 if q_full is None else q_full.shape[2], kva.stride(0), nb, c_float(theta), c_float(eps),
+                                          ptr(status_tensor(q.device)), stream_ptr())
+    check(rc, "ff_mla_norm_rope_cache")
+    _count()
+
+
 def attention(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, q_start: torch.Tensor,
               q_lens: torch.Tensor, ctx_lens: torch.Tensor, max_q: int, max_ctx: int, scale: float, kv_lora: int,
               window: int = 0, head_gate: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -197,18 +215,21 @@ def expanded_attention(q: torch.Tensor, q_full: torch.Tensor, cache: torch.Tenso
     """Prefill attention with every visible latent expanded once: ``w_kv`` ([heads * (dim + vdim), rank], all key matrices, then all value
     matrices) makes keys and values of the pages, then the tcgen05 prefill kernel reads them beside the cache's rotated key parts.
     q: rows with the heads' unrotated parts (``dim`` each); ``q_full`` [rows, heads, rank + rot] holds the rotated ones behind
-    ``rank`` columns. out: [rows, heads * vdim]."""
+    ``rank`` columns, or is ``q`` itself, whose heads are then dim + rot wide. out: [rows, heads * vdim]."""
     rows, heads, width = q_full.shape
     nb, one, bs, cw = cache.shape
-    _require(one == 1 and bs == 64 and cw == width and cache.is_contiguous() and q_full.is_contiguous() and q.stride(1) == 1 and out.is_contiguous(),
+    rot = cw - rank
+    packed = q_full.data_ptr() == q.data_ptr()
+    q_pitch = width if packed else dim
+    _require(one == 1 and bs == 64 and width == (dim + rot if packed else cw) and cache.is_contiguous() and q_full.is_contiguous() and q.stride(1) == 1 and out.is_contiguous(),
              "expanded_attention: layout")
     latents = torch.empty(pages.count * bs, rank, dtype=q.dtype, device=q.device)
     check(kernels().ff_mla_gather(ptr(cache), ptr(pages.blocks), ptr(latents), pages.count, rank, cw, nb, ptr(status_tensor(q.device)), stream_ptr()),
           "ff_mla_gather")
     both = linear(latents, w_kv)
     rc = kernels().ff_attn_prefill_latent(ptr(q), ptr(q_full), ptr(both), ptr(cache), ptr(block_table), ptr(q_start), ptr(q_lens), ptr(ctx_lens),
-                                          ptr(pages.offsets), ptr(out), block_table.shape[0], rows, max_q, heads, dim, width - rank, vdim, q.stride(0),
-                                          width, rank, both.stride(0), both.shape[0], cw, rank, out.stride(0), block_table.shape[1], nb, c_float(scale),
+                                          ptr(pages.offsets), ptr(out), block_table.shape[0], rows, max_q, heads, dim, rot, vdim, q.stride(0),
+                                          q_pitch, width, width - rot, both.stride(0), both.shape[0], cw, rank, out.stride(0), block_table.shape[1], nb, c_float(scale),
                                           window, ptr(head_gate), _head_gate_ld(head_gate, rows, heads), ptr(status_tensor(q.device)), stream_ptr())
     check(rc, "ff_attn_prefill_latent")
     _count(2)

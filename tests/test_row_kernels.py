@@ -40,3 +40,81 @@ def test_rotation_norm_and_cache_write(rows, hq, hkv, dim, rot, norm):
         # largest element of the pair, as the rotation's own test allows
         assert ((a - b).abs() <= 2e-2 + 2e-2 * b.abs()).all()
     assert torch.equal(got[2].cpu(), want[2])                                                   # values are copies
+
+
+def _mla_batch(q_lens, pasts, seed):
+    g = torch.Generator().manual_seed(seed)
+    ql = torch.tensor(q_lens, dtype=torch.int32)
+    ctx = ql + torch.tensor(pasts, dtype=torch.int32)
+    blocks = int(((ctx + 63) // 64).sum()) + 1
+    width = int(((ctx + 63) // 64).max())
+    table, free = torch.zeros(len(q_lens), width, dtype=torch.int32), torch.randperm(blocks, generator=g).tolist()
+    for b, c in enumerate(ctx.tolist()):
+        n = (c + 63) // 64
+        table[b, :n] = torch.tensor([free.pop() for _ in range(n)], dtype=torch.int32)
+    pos = torch.cat([torch.arange(p, p + n) for n, p in zip(q_lens, pasts)]).to(torch.int32)
+    slots = torch.cat([table[b, torch.arange(p, p + n) // 64].long() * 64 + torch.arange(p, p + n) % 64 for b, (n, p) in enumerate(zip(q_lens, pasts))])
+    return g, ql, (torch.cumsum(ql, 0) - ql).to(torch.int32), ctx, table, blocks, pos, slots.to(torch.int32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 3, 200])
+def test_latent_row_step_equals_its_operators(rows):
+    """The fused step gives the bits of rotation and cache write, and the norm's up to its order of additions."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import mla_ops
+    heads, nope = 5, 128
+    g, *_, blocks, pos, slots = _mla_batch([rows], [37], 2)
+    q, kva = torch.randn(rows, heads * (nope + 64), generator=g).to(BF16), torch.randn(rows, 576, generator=g).to(BF16)
+    w = (1 + 0.1 * torch.randn(512, generator=g)).to(BF16)
+    slots[rows // 2] = -1 if rows > 1 else slots[0]
+    q_rope = q.view(rows, heads, -1)[:, :, nope:].reshape(rows, -1).clone()
+    k_rope = kva[:, 512:].clone()
+    ops.rope_inplace(q_rope, pos, heads, 64, 1e4)
+    ops.rope_inplace(k_rope, pos, 1, 64, 1e4)
+    want = torch.zeros(blocks, 1, 64, 576, dtype=BF16)
+    mla_ops.cache_write(ops.rmsnorm(kva[:, :512], w, 1e-6), k_rope, slots, want)
+    for full in (False, True):
+        qd, cache = q.cuda(), torch.zeros_like(want).cuda()
+        q_full = torch.zeros(rows, heads, 576, dtype=BF16, device="cuda") if full else None
+        mla_ops.norm_rope_cache(qd, kva.cuda(), w.cuda(), pos.cuda(), slots.cuda(), cache, heads, nope, 1e4, 1e-6, q_full)
+        torch.cuda.synchronize()
+        ops.check_status()
+        got = q_full[:, :, 512:] if full else qd.view(rows, heads, -1)[:, :, nope:]
+        for a, b in ((got.reshape(rows, -1), q_rope), (cache, want)):
+            assert ((a.cpu().float() - b.float()).abs() <= 2e-2 + 2e-2 * b.float().abs()).all()
+        assert torch.equal(qd.view(rows, heads, -1)[:, :, :nope].cpu(), q.view(rows, heads, -1)[:, :, :nope])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("q_lens,pasts", [([64], [0]), ([1, 130, 63], [70, 0, 129]), ([65, 64], [64, 1])])
+def test_expanded_attention_over_packed_heads(q_lens, pasts):
+    """Keys and values expanded from the latents, queries as the projection leaves them, against attention in 64 bits."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import mla_ops
+    heads, nope, rot, dv, rank = 3, 128, 64, 128, 512
+    g, ql, qs, ctx, table, blocks, *_ = _mla_batch(q_lens, pasts, 5)
+    rows = int(ql.sum())
+    q = torch.randn(rows, heads * (nope + rot), generator=g).to(BF16)
+    cache = torch.randn(blocks, 1, 64, rank + rot, generator=g).to(BF16)
+    w_kv = (0.02 * torch.randn(heads * (nope + dv), rank, generator=g)).to(BF16)
+    scale = (nope + rot) ** -0.5
+    pages = mla_ops.KeyPages.of(ql.tolist(), ctx.tolist(), table, 0, 64, "cuda")
+    out = torch.empty(rows, heads * dv, dtype=BF16, device="cuda")
+    qd = q.cuda()
+    mla_ops.expanded_attention(qd, qd.view(rows, heads, -1), cache.cuda(), w_kv.cuda(), pages, table.cuda(), qs.cuda(), ql.cuda(), ctx.cuda(), max(q_lens),
+                               nope, dv, rank, scale, 0, None, out)
+    torch.cuda.synchronize()
+    ops.check_status()
+    for b in range(len(q_lens)):
+        lat = cache[table[b].long(), 0].reshape(-1, rank + rot)[: int(ctx[b])].double()
+        n, s0 = q_lens[b], int(qs[b])
+        hide = torch.arange(len(lat))[None] > torch.arange(len(lat) - n, len(lat))[:, None]
+        for h in range(heads):
+            k = torch.cat([lat[:, :rank] @ w_kv[h * nope: (h + 1) * nope].double().t(), lat[:, rank:]], 1)
+            v = lat[:, :rank] @ w_kv[heads * nope + h * dv: heads * nope + (h + 1) * dv].double().t()
+            s = (q[s0: s0 + n].view(n, heads, -1)[:, h].double() @ k.t()) * scale
+            want = torch.softmax(s.masked_fill(hide, float("-inf")), -1) @ v
+            got = out[s0: s0 + n].view(n, heads, dv)[:, h].cpu().double()
+            # keys, values, weights and results are rounded to BF16 (2^-9 each): four roundings of values of about 0.5
+            assert ((got - want).abs() <= 1e-2 + 1e-2 * want.abs()).all()
