@@ -2,11 +2,12 @@
 // (activations row-major, weights in the checkpoint's [out, in] layout, FP32 accumulation,
 // one BF16 rounding at the end).
 //
-// gemm_bf16_kernel serves M > 128 (prefill, verification batches): a warp-specialised pipeline
+// Both kernels serve M > 128 (prefill, verification batches) with a warp-specialised pipeline
 // (TMA producer warp -> mbarrier ring -> single-thread tcgen05.mma issuer -> TMEM accumulator ->
-// 4 epilogue warps), persistent over 128 x BN x 64 tiles with double-buffered TMEM accumulators so
-// the epilogue of tile i overlaps the mainloop of tile i+1. Optional fused SwiGLU epilogue
-// (gate|up interleaved per 64 rows of the weight), grouped mode for expert segments, and the
+// 4 epilogue warps), persistent, with double-buffered TMEM accumulators so the epilogue of tile i
+// overlaps the mainloop of tile i+1, and an optional SwiGLU epilogue (gate|up interleaved per 64 rows
+// of the weight). gemm_bf16_pair_kernel: dense problems, 256-row tiles by CTA pairs. gemm_bf16_kernel:
+// 128-row tiles of one CTA, for expert segments (grouped mode), block-diagonal products and the
 // tensor-parallel forms (all-gather -> GEMM, GEMM -> reduce-scatter) with peer stores in the same
 // kernel. Decode shapes (M <= 128) are served by gemm_skinny.cu.
 // This replaces the reference's cuBLAS/cuBLASLt calls (src/backend/cuda/blas.rs:852-1080)
@@ -137,6 +138,144 @@ struct LinTail {
 constexpr int RS_STG_PITCH = 144, RS_STG_BYTES = 32 * RS_STG_PITCH;   // COMM 2 epilogue staging, per warp
 constexpr int COMM_PARTS = 4;       // a 128-row block is pushed (COMM 1) / reduced (COMM 2) in this many pieces
 
+// An epilogue thread's row of a finished tile: tensor memory -> registers -> global. row: row of the result, stored where `live`; tn: column
+// tile, N: columns (of the head), col_off: first column of the head.
+template <int BN>
+__device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict__ Cout, int row, bool live, int ldc, int N, int epi, int tn,
+                                               size_t col_off, const LinTail& tail) {
+  if (epi == 1) {
+    constexpr int HALF = BN / 2;
+    __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + (size_t)tn * HALF;
+    const int ncols_out = N / 2;
+#pragma unroll 1
+    for (int c = 0; c < HALF; c += 16) {
+      uint32_t g[16], u[16];
+      const int gc = (c >> 6) * 128 + (c & 63);      // 64 gate columns, then the matching 64 up columns
+      tmem_ld_x16(taddr + gc, g);
+      tmem_ld_x16(taddr + gc + 64, u);
+      tmem_ld_wait();
+      if (live) {
+        uint32_t o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float g0 = __uint_as_float(g[2 * j]), g1 = __uint_as_float(g[2 * j + 1]);
+          const float u0 = __uint_as_float(u[2 * j]), u1 = __uint_as_float(u[2 * j + 1]);
+          if (tail.gate == 3) { o[j] = pack_bf16x2(gelu_tanh_f(g0) * u0, gelu_tanh_f(g1) * u1); continue; }
+          if (tail.gate == 5) { o[j] = pack_bf16x2(gate_clamped_f(g0, u0, tail.limit), gate_clamped_f(g1, u1, tail.limit)); continue; }
+          // rounding policy "mode 0" of the reference's silu_mul (kernels/act.cu:220-262):
+          // gate and up are BF16 values, silu rounded to BF16, product rounded again.
+          const float a0 = __bfloat162float(__float2bfloat16(silu_f(__bfloat162float(__float2bfloat16(g0)))));
+          const float a1 = __bfloat162float(__float2bfloat16(silu_f(__bfloat162float(__float2bfloat16(g1)))));
+          o[j] = pack_bf16x2(a0 * __bfloat162float(__float2bfloat16(u0)),
+                             a1 * __bfloat162float(__float2bfloat16(u1)));
+        }
+        if (tn * HALF + c + 16 <= ncols_out) {
+          uint4* dst = reinterpret_cast<uint4*>(crow + c);
+          dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+          dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        } else {
+          for (int j = 0; j < 16; ++j)
+            if (tn * HALF + c + j < ncols_out) {
+              const uint32_t w = o[j >> 1];
+              reinterpret_cast<uint16_t*>(crow + c)[j] = (j & 1) ? uint16_t(w >> 16) : uint16_t(w & 0xffff);
+            }
+        }
+      }
+    }
+  } else if (epi == 2) {
+    float* crow = reinterpret_cast<float*>(Cout) + (size_t)row * ldc + (size_t)tn * BN;
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 16) {
+      uint32_t r[16];
+      tmem_ld_x16(taddr + c, r);
+      tmem_ld_wait();
+      if (live) {
+        if (tn * BN + c + 16 <= N) {
+          uint4* dst = reinterpret_cast<uint4*>(crow + c);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dst[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        } else {
+          for (int j = 0; j < 16; ++j) if (tn * BN + c + j < N) crow[c + j] = __uint_as_float(r[j]);
+        }
+      }
+    }
+  } else {
+    __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + col_off + (size_t)tn * BN;
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 32) {
+      uint32_t r[32];
+      tmem_ld_x32(taddr + c, r);
+      tmem_ld_wait();
+      if (tail.bias != nullptr) {
+        const int col = tn * BN + c;
+        if (col + 32 <= N) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint4 bv = __ldg(reinterpret_cast<const uint4*>(tail.bias + col) + j);
+            const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 f = unpack_bf16x2(bw[i]);
+              r[8 * j + 2 * i] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i]) + f.x);
+              r[8 * j + 2 * i + 1] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i + 1]) + f.y);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (col + j < N) r[j] = __float_as_uint(__uint_as_float(r[j]) + __bfloat162float(tail.bias[col + j]));
+        }
+      }
+      if (tail.act == 1) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) { const float v = fmaxf(__uint_as_float(r[j]), 0.f); r[j] = __float_as_uint(v * v); }
+      }
+      if (tail.act == 3) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(gelu_tanh_f(__uint_as_float(r[j])));
+      }
+      if (tail.mul != nullptr && live) {
+        int mr = tail.mul_rows[row];
+        if (mr < 0 || mr >= tail.mul_table) mr = 0;          // reported where the id is first read (embedding)
+        const int col = tn * BN + c;
+        const __nv_bfloat16* f = tail.mul + (size_t)mr * tail.ldm + col;
+        if (col + 32 <= N) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint4 fv = __ldg(reinterpret_cast<const uint4*>(f) + j);
+            const uint32_t fw[4] = {fv.x, fv.y, fv.z, fv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 m = unpack_bf16x2(fw[i]);
+              r[8 * j + 2 * i] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i]) * m.x);
+              r[8 * j + 2 * i + 1] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i + 1]) * m.y);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (col + j < N) r[j] = __float_as_uint(__uint_as_float(r[j]) * __bfloat162float(f[j]));
+        }
+      }
+      if (live) {
+        if (tn * BN + c + 32 <= N) {
+          uint4* dst = reinterpret_cast<uint4*>(crow + c);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            dst[j] = make_uint4(pack_bf16x2(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1])),
+                                pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3])),
+                                pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5])),
+                                pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7])));
+          }
+        } else {
+          for (int j = 0; j < 32; ++j)
+            if (tn * BN + c + j < N) crow[c + j] = __float2bfloat16(__uint_as_float(r[j]));
+        }
+      }
+    }
+  }
+}
+
 template <int BN, int STAGES, int COMM>
 __global__ void __launch_bounds__(COMM == 1 ? 320 : 192, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA1,
@@ -246,66 +385,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tc_fence_after();
       const int row = a_row0 + q * 32 + lane;
       const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * BN;
-      if (epi == 1) {
-        constexpr int HALF = BN / 2;
-        __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + (size_t)tn * HALF;
-        const int ncols_out = N / 2;
-#pragma unroll 1
-        for (int c = 0; c < HALF; c += 16) {
-          uint32_t g[16], u[16];
-          const int gc = (c >> 6) * 128 + (c & 63);      // 64 gate columns, then the matching 64 up columns
-          tmem_ld_x16(taddr + gc, g);
-          tmem_ld_x16(taddr + gc + 64, u);
-          tmem_ld_wait();
-          if (row < row_end) {
-            uint32_t o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float g0 = __uint_as_float(g[2 * j]), g1 = __uint_as_float(g[2 * j + 1]);
-              const float u0 = __uint_as_float(u[2 * j]), u1 = __uint_as_float(u[2 * j + 1]);
-              if (COMM == 0 && tail.gate == 3) { o[j] = pack_bf16x2(gelu_tanh_f(g0) * u0, gelu_tanh_f(g1) * u1); continue; }
-              if (COMM == 0 && tail.gate == 5) { o[j] = pack_bf16x2(gate_clamped_f(g0, u0, tail.limit), gate_clamped_f(g1, u1, tail.limit)); continue; }
-              // rounding policy "mode 0" of the reference's silu_mul (kernels/act.cu:220-262):
-              // gate and up are BF16 values, silu rounded to BF16, product rounded again.
-              const float a0 = __bfloat162float(__float2bfloat16(silu_f(__bfloat162float(__float2bfloat16(g0)))));
-              const float a1 = __bfloat162float(__float2bfloat16(silu_f(__bfloat162float(__float2bfloat16(g1)))));
-              o[j] = pack_bf16x2(a0 * __bfloat162float(__float2bfloat16(u0)),
-                                 a1 * __bfloat162float(__float2bfloat16(u1)));
-            }
-            if (tn * HALF + c + 16 <= ncols_out) {
-              uint4* dst = reinterpret_cast<uint4*>(crow + c);
-              dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-              dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-            } else {
-              for (int j = 0; j < 16; ++j)
-                if (tn * HALF + c + j < ncols_out) {
-                  const uint32_t w = o[j >> 1];
-                  reinterpret_cast<uint16_t*>(crow + c)[j] = (j & 1) ? uint16_t(w >> 16) : uint16_t(w & 0xffff);
-                }
-            }
-          }
-        }
-      } else if (epi == 2) {
-        float* crow = reinterpret_cast<float*>(Cout) + (size_t)row * ldc + (size_t)tn * BN;
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 16) {
-          uint32_t r[16];
-          tmem_ld_x16(taddr + c, r);
-          tmem_ld_wait();
-          if (row < row_end) {
-            if (tn * BN + c + 16 <= N) {
-              uint4* dst = reinterpret_cast<uint4*>(crow + c);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) dst[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-            } else {
-              for (int j = 0; j < 16; ++j) if (tn * BN + c + j < N) crow[c + j] = __uint_as_float(r[j]);
-            }
-          }
-        }
-      } else {
-        __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + (size_t)head * ga.c_cols + (size_t)tn * BN;
-        if (COMM == 2) {
-          // the rows of this tile belong to rank `owner`: they go into its arena slot for source = me,
+      if (COMM == 2) {
+        // the rows of this tile belong to rank `owner`: they go into its arena slot for source = me,
           // 64 columns at a time through a warp-private staging tile
           const int owner = tm / tiles_per_rank;
           __nv_bfloat16* tile_dst = reinterpret_cast<__nv_bfloat16*>(arena_slot(ca.ar, owner, parity, ca.ar.rank)) +
@@ -344,79 +425,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           tma_store_wait<0>();                              // every row of this tile has landed in the owner's slot
           asm volatile("fence.proxy.async;" ::: "memory");
-        } else
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t r[32];
-          tmem_ld_x32(taddr + c, r);
-          tmem_ld_wait();
-          if (COMM == 0 && tail.bias != nullptr) {
-            const int col = tn * BN + c;
-            if (col + 32 <= N) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint4 bv = __ldg(reinterpret_cast<const uint4*>(tail.bias + col) + j);
-                const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const float2 f = unpack_bf16x2(bw[i]);
-                  r[8 * j + 2 * i] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i]) + f.x);
-                  r[8 * j + 2 * i + 1] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i + 1]) + f.y);
-                }
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (col + j < N) r[j] = __float_as_uint(__uint_as_float(r[j]) + __bfloat162float(tail.bias[col + j]));
-            }
-          }
-          if (COMM == 0 && tail.act == 1) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) { const float v = fmaxf(__uint_as_float(r[j]), 0.f); r[j] = __float_as_uint(v * v); }
-          }
-          if (COMM == 0 && tail.act == 3) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(gelu_tanh_f(__uint_as_float(r[j])));
-          }
-          if (COMM == 0 && tail.mul != nullptr && row < row_end) {
-            int mr = tail.mul_rows[row];
-            if (mr < 0 || mr >= tail.mul_table) mr = 0;          // reported where the id is first read (embedding)
-            const int col = tn * BN + c;
-            const __nv_bfloat16* f = tail.mul + (size_t)mr * tail.ldm + col;
-            if (col + 32 <= N) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint4 fv = __ldg(reinterpret_cast<const uint4*>(f) + j);
-                const uint32_t fw[4] = {fv.x, fv.y, fv.z, fv.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const float2 m = unpack_bf16x2(fw[i]);
-                  r[8 * j + 2 * i] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i]) * m.x);
-                  r[8 * j + 2 * i + 1] = __float_as_uint(__uint_as_float(r[8 * j + 2 * i + 1]) * m.y);
-                }
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (col + j < N) r[j] = __float_as_uint(__uint_as_float(r[j]) * __bfloat162float(f[j]));
-            }
-          }
-          if (row < row_end) {
-            if (tn * BN + c + 32 <= N) {
-              uint4* dst = reinterpret_cast<uint4*>(crow + c);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                dst[j] = make_uint4(pack_bf16x2(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1])),
-                                    pack_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3])),
-                                    pack_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5])),
-                                    pack_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7])));
-              }
-            } else {
-              for (int j = 0; j < 32; ++j)
-                if (tn * BN + c + j < N) crow[c + j] = __float2bfloat16(__uint_as_float(r[j]));
-            }
-          }
-        }
+      } else {
+        store_tile_row<BN>(taddr, Cout, row, row < row_end, ldc, N, epi, tn, (size_t)head * ga.c_cols, tail);
       }
       tc_fence_before();
       __syncwarp();
@@ -551,6 +561,122 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 
+// Dense problems: a pair of CTAs per 256 x BN tile (cta_group::2). What bounds the one-CTA form is the way from L2 into shared memory: a
+// 128 x 256 tile takes in 48 KiB per 64-wide K block of 510 tensor cycles, 94 bytes a cycle and SM, and all SMs together got 15 TB/s.
+// Of a pair every CTA loads 128 rows of A and half of B's rows -- 32 KiB for the same work --, the even CTA issues for both, and its
+// commits free the stages of both. Persistent, two accumulators in tensor memory, so the epilogue of a tile runs under the next one's
+// main loop. Prefill of 8121 rows of an 8-layer 8B-sized stack 28.3 -> 26.4 ms, of 8191 rows 33.3 -> 30.7 ms; at these sizes the GPU's power
+// limit holds both forms near 1.4 PFLOP/s inside the products, and the pair form reaches it with less traffic.
+struct alignas(8) PairBars {
+  uint64_t full[8];             // the even CTA's: both CTAs' loads of a stage have landed
+  uint64_t empty[8];            // each CTA's own, freed by the even CTA's commits
+  uint64_t tmem_full[2];
+  uint64_t tmem_empty[2];       // the even CTA's: the eight epilogue warps of the pair have read the accumulator
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+template <int BN, int STAGES>
+__global__ void __launch_bounds__(192, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, void* __restrict__ Cout, int M, int N,
+                      int K, int ldc, int epi, int* status, LinTail tail) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ PairBars bars;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN / 2 * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank();
+  const int tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (N + BN - 1) / BN, tiles = tiles_m * tiles_n;
+  const int kblocks = (K + BK - 1) / BK;
+  const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars.tmem_full[i], 1); mbar_init(&bars.tmem_empty[i], 8); }
+    bars.abort_flag = 0;
+    mbar_fence_init();
+  }
+  pdl_wait();
+  // after the wait: no kernel of this stream that still has tensor memory to allocate can be running. All 512 columns, so that both
+  // CTAs' accumulators have the same addresses.
+  if (warp == 1) { tmem_alloc_pair(&bars.tmem_base, 512); tmem_relinquish_pair(); }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                  // the peer's barriers exist before anything arrives at them
+  tc_fence_after();
+  pdl_trigger();
+  const uint32_t tmem_base = bars.tmem_base;
+  volatile int* abort_flag = &bars.abort_flag;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = first; t < tiles && ok; t += step) {
+        int tm, tn;
+        tile_coords(t, tiles_m, tiles_n, tm, tn);
+        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+          const int s = it % STAGES; const uint32_t ph = (it / STAGES) & 1;
+          if (!mbar_wait(&bars.empty[s], ph ^ 1, abort_flag, status, KID_GEMM_BF16, 5)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(&bars.full[s], 2 * STAGE_BYTES);
+          uint8_t* sa = smem + s * STAGE_BYTES;
+          tma_load_2d_pair(sa, &tmA, &bars.full[s], kb * BK, (2 * tm + rank) * BM);
+          tma_load_2d_pair(sa + A_BYTES, &tmB, &bars.full[s], kb * BK, tn * BN + rank * (BN / 2));
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0 && lane == 0) {
+      constexpr uint32_t idesc = umma_idesc(1, 1, 0, 0, 2 * BM, BN);
+      uint32_t it = 0, tile_it = 0;
+      bool ok = true;
+      for (int t = first; t < tiles && ok; t += step, ++tile_it) {
+        const int acc = tile_it & 1; const uint32_t aph = (tile_it >> 1) & 1;
+        if (!mbar_wait(&bars.tmem_empty[acc], aph ^ 1, abort_flag, status, KID_GEMM_BF16, 6)) { ok = false; break; }
+        tc_fence_after();
+        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&bars.full[s], (it / STAGES) & 1, abort_flag, status, KID_GEMM_BF16, 7)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
+          const uint64_t da = umma_desc_sw128(sa, 16, 1024), db = umma_desc_sw128(sa + A_BYTES, 16, 1024);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_pair(tmem_base + acc * BN, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+          umma_commit_pair(&bars.empty[s]);
+        }
+        if (ok) umma_commit_pair(&bars.tmem_full[acc]);
+      }
+    }
+  } else {
+    const int q = warp & 3;                            // TMEM lane quarter
+    uint32_t tile_it = 0;
+    bool ok = true;
+    for (int t = first; t < tiles && ok; t += step, ++tile_it) {
+      int tm, tn;
+      tile_coords(t, tiles_m, tiles_n, tm, tn);
+      const int acc = tile_it & 1;
+      if (!mbar_wait(&bars.tmem_full[acc], (tile_it >> 1) & 1, abort_flag, status, KID_GEMM_BF16, 8)) ok = false;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const int row = (2 * tm + rank) * BM + q * 32 + lane;
+      store_tile_row<BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * BN, Cout, row, row < M, ldc, N, epi, tn, 0, tail);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_leader(&bars.tmem_empty[acc]);
+    }
+  }
+  __syncthreads();
+  if (bars.abort_flag) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
+  }
+  __syncwarp();
+  cluster_sync_all();                                  // nothing arrives at a CTA's barriers, or reads its stages, after this
+  if (warp == 1) { tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
+}
+
 }  // namespace ff
 
 using namespace ff;
@@ -567,19 +693,25 @@ static int gemm_bf16_launch(const void* X, const void* W, void* Y, int M, int N,
   if (((size_t)ldy * out_bytes) % 16 || ldy < out_cols) return FF_HOST_BAD_ALIGN;
   if (reinterpret_cast<uintptr_t>(Y) & 15) return FF_HOST_BAD_ALIGN;
   CUtensorMap tmA, tmB;
-  constexpr int BN = 256, STAGES = 4;
   int r = make_tmap_2d(&tmA, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, (uint64_t)ldx * 2, BK, BM);
   if (r) return r;
-  r = make_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, BN);
+  // Column tile: 256 wide takes in the fewest bytes per product, 128 wide fills a last wave better (M = 1000, N = 6144: 96 wide tiles on
+  // 74 pairs are two waves, 192 narrow ones three of half the length). A narrow tile is charged 1.15 of half a wide one (24 instead of 16
+  // KiB per 128 columns).
+  const int pairs = sm_count() / 2, tiles_m = (M + 2 * BM - 1) / (2 * BM);
+  auto waves = [&](int bn) { const int t = tiles_m * ((N + bn - 1) / bn); return (t + pairs - 1) / pairs; };
+  const bool narrow = waves(128) * 0.575f < waves(256);
+  const int bn = narrow ? 128 : 256;
+  r = make_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, bn / 2);
   if (r) return r;
-  const int smem = STAGES * (BM * BK * 2 + BN * BK * 2) + 1024;
-  auto kern = gemm_bf16_kernel<BN, STAGES, 0>;
-  r = opt_in_smem(kern, smem); if (r) return r;
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int grid = tiles < sm_count() ? tiles : sm_count();
-  CommArgs none = {};
-  kern<<<grid, 192, smem, stream>>>(tmA, tmA, tmA, tmB, Y, M, N, K, ldy, epi, status, none, GroupArgs{}, tail);
-  return launch_result();
+  const int tiles = tiles_m * ((N + bn - 1) / bn), grid = 2 * (tiles < pairs ? tiles : pairs);
+  auto go = [&](auto kern, int stages) -> int {
+    const int smem = stages * (BM + bn / 2) * BK * 2 + 1024;
+    if (int e = opt_in_smem(kern, smem)) return e;
+    if (int e = launch_pdl(kern, dim3(grid), dim3(192), smem, stream, 2, tmA, tmB, Y, M, N, K, ldy, epi, status, tail)) return e;
+    return launch_result();
+  };
+  return narrow ? go(gemm_bf16_pair_kernel<128, 8>, 8) : go(gemm_bf16_pair_kernel<256, 6>, 6);
 }
 
 FF_EXPORT int ff_gemm_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw, int ldy,

@@ -1,0 +1,54 @@
+"""Products and reductions at the sizes where a tile, a chunk or a split ends."""
+import pytest
+import torch
+
+from flyingfish_b200.ops import ref
+
+BF16 = torch.bfloat16
+
+
+def _rand(shape, seed, dtype=BF16):
+    return torch.randn(shape, generator=torch.Generator().manual_seed(seed)).to(dtype)
+
+
+def _check(got, want, k, dtype=BF16):
+    """One rounding to the result's type, and FP32 sums of k products of unit size (k 2^-24 of their root k norm, with room for the
+    tensor core's alignment of partial products)."""
+    got = got.cpu().double()
+    rounding = 2.0 ** -8 if dtype == BF16 else 0.0
+    assert ((got - want).abs() <= rounding * want.abs() + 2.0 ** -20 * k).all(), (got - want).abs().max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [129, 255, 256, 257, 1000])        # second row tile of a pair empty, ragged, full; several pairs
+@pytest.mark.parametrize("n,k", [(136, 72), (256, 64), (520, 520), (6144, 512)])
+@pytest.mark.parametrize("odt", [BF16, torch.float32])
+def test_pair_gemm(m, n, k, odt):
+    from flyingfish_b200 import ops
+    x, w = _rand((m, k), m), _rand((n, k), n)
+    y = ops.linear(x.cuda(), w.cuda(), out_dtype=odt)
+    torch.cuda.synchronize()
+    ops.check_status()
+    _check(y, x.double() @ w.double().t(), k, odt)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(200, 264, 128), (300, 4096, 200)])
+def test_pair_gemm_tail(m, n, k):
+    from flyingfish_b200 import ops
+    x, w, bias = _rand((m, k), 1), _rand((n, k), 2), _rand((n,), 3)
+    y = ops.linear(x.cuda(), w.cuda(), bias=bias.cuda(), act="relu2")
+    want = (x.double() @ w.double().t() + bias.double()).clamp_min(0) ** 2
+    # the square doubles the sum's relative error: absolute 2 |sum| times it
+    assert ((y.cpu().double() - want).abs() <= 2.0 ** -8 * want + 2.0 ** -19 * k * want.sqrt() + 1e-3).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n", [(129, 256), (700, 5888), (256, 19200)])       # narrow and wide column tiles
+def test_pair_gemm_gate(m, n):
+    from flyingfish_b200 import ops
+    x, w = _rand((m, 128), 4), _rand((n, 128), 5)
+    got = ops.linear_swiglu(x.cuda(), w.cuda()).cpu().float()
+    want = ref.linear_swiglu(x, w).float()
+    # gate and up are rounded to BF16 before the product: sums on either side of a rounding boundary differ by a last bit each
+    assert ((got - want).abs() <= 3 * 2.0 ** -8 * want.abs() + 2e-2).all()
