@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from flyingfish_b200.loaders import quant as qref
 from flyingfish_b200.ops import ref
 
 BF16 = torch.bfloat16
@@ -52,3 +53,11 @@ def test_pair_gemm_gate(m, n):
     want = ref.linear_swiglu(x, w).float()
     # gate and up are rounded to BF16 before the product: sums on either side of a rounding boundary differ by a last bit each
     assert ((got - want).abs() <= 3 * 2.0 ** -8 * want.abs() + 2e-2).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k", [(130, 272), (5, 132), (1, 16), (300, 4)])
+def test_fp8_expansion_is_exact(n, k):
+    from flyingfish_b200.ops import quant_ops
+    codes, scale = qref.quantize_fp8_block_weight(_rand((n, k), 3).float())
+    assert torch.equal(quant_ops.dequant_fp8_block(codes.cuda(), scale.cuda()).cpu(), qref.dequantize_fp8_block(codes, scale))
