@@ -65,11 +65,12 @@ __device__ __forceinline__ void fp8_promote(float (&acc)[NACC], const uint32_t (
 }
 
 // epi: 0 store, 1 SwiGLU over 64/64 interleaved rows (grouped gate/up)
-// TOK: tokens per chunk. 128 for prefill-sized and dense calls (one CTA per SM); 32 for decode-sized grouped calls, where a
+// TOK: tokens per chunk. 128 for prefill-sized and dense calls (one CTA per SM); 32 and 64 for grouped calls with short segments, where a
 // CTA needs few registers and half the shared memory so that two CTAs share an SM and one streams while the other sets up
-// or drains (an expert tile of a decode batch is short: 16 to 56 k-blocks).
+// or drains (an expert tile is short: 16 to 56 k-blocks). 256 experts of 7168 x 2048 with 50 rows each: gate/up and down together
+// 3488 us with chunks of 128, 2036 us with chunks of 64 (codes at the copy rate: 1730 us).
 template <int TOK>
-__global__ void __launch_bounds__(320, TOK <= 32 ? 2 : 1)
+__global__ void __launch_bounds__(320, TOK <= 64 ? 2 : 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                 const float* __restrict__ w_scale, const float* __restrict__ x_scale, __nv_bfloat16* __restrict__ Y,
                 const int* __restrict__ seg_off, const int* __restrict__ counts, int M, int Nw, int K, int ldy,
@@ -235,7 +236,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       }
       if (!ok) break;
       bool final_here = true;
-      if (splits == 1) {
+      if (TOK == 64 || splits == 1) {                        // chunks of 64 are grouped calls, which have no splits
 #pragma unroll
         for (int i = 0; i < TOK / 2; ++i) {
           const int t = blk0 * 16 + i;
@@ -366,9 +367,11 @@ static int gemm_fp8_launch(const void* xq, const float* x_scale, const void* wq,
   if (splits < 1 || (splits > 1 && (!scratch || !tile_counters || experts > 1))) return FF_HOST_BAD_SHAPE;
   if (epi == 1 && (Nw % 128 || ldy < Nw / 2)) return FF_HOST_BAD_SHAPE;
   if (ldy % 8 || (reinterpret_cast<uintptr_t>(y) & 15)) return FF_HOST_BAD_ALIGN;
-  // decode-sized grouped calls (on average at most 24 padded rows per expert): 32-token chunks, two CTAs per SM
-  const bool small = experts > 1 ? (long long)M <= 24ll * experts : M <= 32;
-  const int tok_cap = small ? (experts > 1 ? 32 : (M + 15) / 16 * 16) : (experts > 1 ? F_TOK : (M >= F_TOK ? F_TOK : (M + 15) / 16 * 16));
+  // Grouped calls take the smallest chunk that most segments fit into: 32 tokens up to an average of 8 rows per expert, 64 up to 52 (M
+  // counts 16 rows of padding for each; random segments of that average exceed 64 in one case of twenty, which then streams its weights twice).
+  const int chunk = experts > 1 ? ((long long)M <= 24ll * experts ? 32 : (long long)M <= 68ll * experts ? 64 : F_TOK) : (M <= 32 ? 32 : F_TOK);
+  const bool small = chunk < F_TOK;
+  const int tok_cap = experts > 1 ? chunk : (M >= F_TOK ? F_TOK : (M + 15) / 16 * 16);
   const int per = ((K / 128) + splits - 1) / splits;                     // k-blocks of one split
   if (per * tok_cap * 4 > 64 * 1024) return FF_HOST_TOO_LARGE;           // scale staging
   CUtensorMap tmW, tmX;
@@ -381,17 +384,10 @@ static int gemm_fp8_launch(const void* xq, const float* x_scale, const void* wq,
   int pipe_bytes = budget - staging;
   const int smem = staging + pipe_bytes + 1024;
   dim3 grid((Nw + FBM - 1) / FBM, splits, experts);
-  if (small) {
-    r = opt_in_smem(gemm_fp8_kernel<32>, 111 * 1024); if (r) return r;
-    if (int lr = launch_pdl(gemm_fp8_kernel<32>, grid, dim3(320), smem, s, 0, tmW, tmX, w_scale, x_scale, (__nv_bfloat16*)y,
-                            seg_off, counts, M, Nw, K, ldy, epi, splits, pipe_bytes, staging, tok_cap, scratch, tile_counters,
-                            status, xs_ld)) return lr;
-    return launch_result();
-  }
-  r = opt_in_smem(gemm_fp8_kernel<F_TOK>, 225 * 1024); if (r) return r;
-  if (int lr = launch_pdl(gemm_fp8_kernel<F_TOK>, grid, dim3(320), smem, s, 0, tmW, tmX, w_scale, x_scale, (__nv_bfloat16*)y,
-                          seg_off, counts, M, Nw, K, ldy, epi, splits, pipe_bytes, staging, tok_cap, scratch, tile_counters,
-                          status, xs_ld)) return lr;
+  auto kern = chunk == 32 ? gemm_fp8_kernel<32> : chunk == 64 ? gemm_fp8_kernel<64> : gemm_fp8_kernel<F_TOK>;
+  r = opt_in_smem(kern, budget + 1024); if (r) return r;
+  if (int lr = launch_pdl(kern, grid, dim3(320), smem, s, 0, tmW, tmX, w_scale, x_scale, (__nv_bfloat16*)y, seg_off, counts, M, Nw, K, ldy, epi,
+                          splits, pipe_bytes, staging, tok_cap, scratch, tile_counters, status, xs_ld)) return lr;
   return launch_result();
 }
 

@@ -56,6 +56,31 @@ def test_pair_gemm_gate(m, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("counts", [[64, 1, 65, 0, 50, 33, 63, 47], [16, 17, 0, 32, 33, 1, 31, 30], [100, 128, 129, 16]])   # chunks of 64, 32, 128
+@pytest.mark.parametrize("epi", [0, 1])
+def test_grouped_fp8_chunks(counts, epi):
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import quant_ops
+    e, n, k = len(counts), 256, 384
+    pad = [(c + 15) // 16 * 16 for c in counts]
+    off = [sum(pad[:i]) for i in range(e + 1)]
+    x = _rand((off[-1], k), 7)
+    w = [qref.quantize_fp8_block_weight(_rand((n, k), 10 + i).float()) for i in range(e)]
+    codes, scale = torch.stack([c for c, _ in w]), torch.stack([s for _, s in w])
+    xq, xs = qref.quantize_fp8_act(x)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    y = quant_ops.grouped_gemm_fp8(xq.cuda(), xs.cuda(), codes.cuda(), scale.cuda(), i32(off), i32(counts), off[-1], epi).cpu().float()
+    torch.cuda.synchronize()
+    ops.check_status()
+    for i, c in enumerate(counts):
+        if c:
+            rows = qref.fp8_block_linear(x[off[i]: off[i] + c], codes[i], scale[i])
+            want = ref.silu_mul(quant_ops._deinterleave_cols(rows)).float() if epi else rows.float()
+            got = y[off[i]: off[i] + c]
+            assert ((got - want).abs() <= 3 * 2.0 ** -8 * want.abs() + 2e-2).all()      # roundings as in the gated product above
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n,k", [(130, 272), (5, 132), (1, 16), (300, 4)])
 def test_fp8_expansion_is_exact(n, k):
     from flyingfish_b200.ops import quant_ops
