@@ -4,272 +4,263 @@
 // Wsc : [E_local * Nw, K / 16] bytes, one E4M3 scale per 16 weights
 // global : FP32 per expert (ModelOpt `weight_scale_2`)
 // The decode-sized MoE layer is bound by expert weight bytes, so the weights stay packed in HBM (a quarter of the
-// BF16 bytes) and are expanded on the way into the tensor-core operand:
-//   * four converter warps read the packed codes of a 128-row x 128-wide K block (a warp-wide load covers eight
-//     whole 64-byte row pieces) and its scales straight from global memory, two K blocks ahead in registers,
-//     expand them to BF16 (byte-permute look-ups in registers, four codes at a time, one BF16x2 multiply by the
-//     group's scale; e2m1 * e4m3 is exact in BF16: 2 + 4 significant bits) and write the two 64-wide
-//     128-byte-swizzled sub-tiles that tcgen05.mma reads as its A operand;
-//   * one thread streams the tokens of the segment (the UMMA N side, up to 32 per pass) with TMA;
-//   * one thread issues the MMAs into a TMEM accumulator; the per-expert global scale is applied in FP32 in the
-//     epilogue (more exact than folding it into a BF16 weight), with the optional SwiGLU of gate/up stacks
-//     interleaved per 64 rows. Two CTAs share an SM (97 KiB of shared memory, <= 168 registers), so one CTA's
-//     prologue, pipeline fill and epilogue overlap the other's main loop.
-// Swap-AB like the BF16 grouped kernel of moe.cu (weights = UMMA M, tokens = UMMA N). Segments longer than 32 tokens
-// are processed in passes of 32 that each re-expand the weights, so this kernel is meant for decode-sized segments;
-// prefill-sized calls expand the weights once (quantize.cu) and use the tiled grouped GEMM.
+// BF16 bytes) and are expanded in the registers of the warps that multiply them (mma.sync, weights as the 16-row A fragment, tokens
+// as the 8 columns of B). Why not tcgen05: an instruction of it takes about 190 cycles however few tokens there are, and with 128
+// weight rows x 16 as its operand that caps a GPU at 1.7 TB/s of packed bytes -- measured with the expansion left out, through shared
+// memory and through tensor memory alike (528 us for a gate/up product of 0.9 GB). A 16 x 8 x 16 mma.sync costs what its 8 tokens cost.
+//   * Persistent CTAs, two per SM, walk the (expert, 128 weight rows) tiles of the experts that have tokens. A producer warp keeps a ring
+//     of 256-wide K chunks (codes and scales) in flight with TMA; lanes that read 64-byte pieces of eight rows from global memory
+//     themselves reached 2.9 TB/s with nothing else to do. Eight warps own 16 weight rows each: lane (g, t) takes 16 bytes (32 codes)
+//     of rows g and g + 8 at a time. The codes of a word go to the K slots of two mma in the order in which expanding leaves them;
+//     the tokens are put into shared memory in that order once per slab, as conflict-free 16-byte units.
+//   * Expanding: the three magnitude bits of a code moved to bits 8..6 of a BF16 are the value times 2^-126 (the subnormal 0.5
+//     included); one BF16x2 multiply by the group's scale times 2^118 makes it e2m1 * e4m3 * 2^-8, exactly (2 + 4 significant
+//     bits). The 2^8 goes with the per-expert global scale, which is applied in FP32 in the epilogue, with the optional SwiGLU of
+//     gate/up stacks interleaved per 64 rows.
+//   * Up to 32 tokens per pass (1, 2 or 4 column tiles; the tokens of 512 to 2048 K at a time in 32 KB). Longer segments take
+//     passes that expand again, so this kernel is meant for decode-sized segments; prefill-sized calls use the tiled grouped GEMM
+//     over BF16 weights.
+// 128 experts of 4096 x 1536 with 2 rows each: gate/up and down 658 + 342 us with converters in front of tcgen05, 290 + 154 us now (packed
+// bytes at the copy rate: 138 + 69 us); what is left is integer work, 0.65 of the issue slots busy.
 // Format: kernels/nvfp4_linear.cu and src/fp8.rs:124-147 of the reference.
 #include "ptx.cuh"
 #include "host_util.h"
 #include <cuda_fp8.h>
+#include <type_traits>
 
 namespace ff {
 
-constexpr int F4_BM = 128;           // weight rows per CTA (UMMA M)
-constexpr int F4_KB = 128;           // K per pipeline stage = two 64-wide UMMA sub-tiles
-constexpr int F4_NSUB = F4_KB / 64;
-constexpr int F4_TOK = 32;           // tokens per pass (UMMA N)
-constexpr int F4_STAGES = 2;
-constexpr int F4_SUB = F4_BM * 64 * 2;               // one converted sub-tile: 16 KiB
-constexpr int F4_A_BYTES = F4_NSUB * F4_SUB;         // 32 KiB
-constexpr int F4_X_BYTES = F4_NSUB * F4_TOK * 128;   // 8 KiB
-constexpr int F4_STAGE_BYTES = F4_A_BYTES + F4_X_BYTES;
-constexpr int F4_EPI_TOK = 32;
-constexpr int F4_STAGING = F4_EPI_TOK * F4_BM * 4;   // FP32 transpose tile of the epilogue: 16 KiB
+constexpr int F4_BM = 128;           // weight rows per CTA
+constexpr int F4_KC = 256;           // K of a ring stage: 128 bytes of codes and 16 scales per row
+constexpr int F4_TOK = 32;           // most tokens per pass
+constexpr int F4_WARPS = 8;          // multiplying warps, 16 weight rows each; one more produces
+constexpr int F4_THREADS = 32 * F4_WARPS + 32;
+constexpr int F4_CODES = F4_BM * F4_KC / 2, F4_SCALES = F4_BM * F4_KC / 16, F4_STAGE = F4_CODES + F4_SCALES;      // 18 KiB
+constexpr int F4_STAGES = 3;
+constexpr int F4_X_BYTES = 32 * 1024;                // tokens of a K slab: 8 * NT of them, 2048 / NT wide; then the epilogue's FP32 tile
 
 struct alignas(8) Fp4Bars {
   uint64_t full[F4_STAGES];
   uint64_t empty[F4_STAGES];
-  uint64_t tmem_full;
-  uint64_t tmem_empty;
-  uint32_t tmem_base;
   int abort_flag;
+  int active;
 };
+__device__ __forceinline__ void f4_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }      // the multiplying warps
 
 __device__ __forceinline__ float f4_silu(float x) { return x / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float f4_bfr(float x) { return __bfloat162float(__float2bfloat16(x)); }
-__device__ __forceinline__ float f4_e4m3(uint32_t c) {
-  const __half_raw h = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)c, __NV_E4M3);
-  return __half2float(*reinterpret_cast<const __half*>(&h));
-}
-// E2M1 code -> value: sign | 2-bit exponent | 1-bit mantissa; magnitudes 0, .5, 1, 1.5, 2, 3, 4, 6
-__device__ __forceinline__ float f4_value(uint32_t code) {
-  const uint32_t m = code & 7u;
-  // exponent field 0: 0 or 0.5 (subnormal); otherwise (1 + man / 2) * 2^(exp - 1)
-  const float mag = (m < 2u) ? 0.5f * (float)m : __uint_as_float(((126u + (m >> 1)) << 23) | ((m & 1u) << 22));
-  return (code & 8u) ? -mag : mag;
+
+// Eight codes of a word (low nibble first) times a scale: pairs (0, 4), (1, 5), (2, 6), (3, 7), which share a shift each
+__device__ __forceinline__ void f4_expand8(uint32_t w, __nv_bfloat162 sv, uint32_t (&p)[4]) {
+  constexpr uint32_t MAG = 0x01C001C0u, SGN = 0x80008000u;
+  const uint32_t h = w >> 8;
+  p[0] = ((w << 6) & MAG) | ((w << 12) & SGN);
+  p[1] = ((w << 2) & MAG) | ((w << 8) & SGN);
+  p[2] = ((h << 6) & MAG) | ((h << 12) & SGN);
+  p[3] = ((h << 2) & MAG) | ((h << 8) & SGN);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&p[i]), sv);
+    p[i] = *reinterpret_cast<const uint32_t*>(&r);
+  }
 }
 
-// grid (Nw / 128, E_local), 192 threads: warp 0 token TMA, warp 1 MMA, warps 2..5 converters + epilogue
-__global__ void __launch_bounds__(192, 2)
-moe_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmX, const uint8_t* __restrict__ Wq,
+// two E4M3 scales -> BF16 pairs (each twice) times 2^118
+__device__ __forceinline__ void f4_scale2(uint32_t c, __nv_bfloat162& s0, __nv_bfloat162& s1) {
+  const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)c, __NV_E4M3);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hr));
+  constexpr float UP = 3.3230699894622897e35f;         // 2^118
+  s0 = __float2bfloat162_rn(f.x * UP);
+  s1 = __float2bfloat162_rn(f.y * UP);
+}
+
+__device__ __forceinline__ void f4_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// One pass: `real` (at most 8 NT) tokens from row `grow0` of X against the 128 weight rows that come through the ring. `it`: stages used so far.
+template <int NT>
+__device__ __forceinline__ bool f4_pass(const __nv_bfloat16* __restrict__ X, int grow0, int real, uint8_t* ring, Fp4Bars& bars, uint32_t& it,
+                                        const uint8_t* __restrict__ wsc, int K, uint8_t* xbuf, float gscale, __nv_bfloat16* __restrict__ Y,
+                                        int ldy, int tn, int epi, int* status) {
+  constexpr int SLAB = F4_X_BYTES / (16 * NT);         // K that the tokens in shared memory cover
+  static_assert(SLAB % F4_KC == 0, "a slab holds whole stages");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int chunks = (K + F4_KC - 1) / F4_KC, ra = warp * 16 + g;       // rows ra and ra + 8 have the same swizzle
+  float acc[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+
+  for (int c = 0; c < chunks; ++c, ++it) {
+    const int in_slab = c % (SLAB / F4_KC);
+    if (in_slab == 0) {
+      // tokens of this slab: unit [128-wide K][column tile][i2][token][t] holds x[token][32 t + 8 i2 + {0,4,1,5,2,6,3,7}]
+      f4_sync();
+      const int k0 = c * F4_KC, per = min(SLAB, K - k0) / 8;
+      for (int i = threadIdx.x; i < 8 * NT * per; i += 32 * F4_WARPS) {
+        const int n = i / per, k8 = i - n * per;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (n < real) v = __ldg(reinterpret_cast<const uint4*>(X + (size_t)(grow0 + n) * K + k0) + k8);
+        const int ch = k8 >> 4, tt = (k8 >> 2) & 3, i2 = k8 & 3;
+        *reinterpret_cast<uint4*>(xbuf + ((((ch * NT + (n >> 3)) * 4 + i2) * 8 + (n & 7)) * 4 + tt) * 16) =
+            make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
+      }
+      f4_sync();
+    }
+    const int s = it % F4_STAGES;
+    if (!__all_sync(0xffffffffu, mbar_wait(&bars.full[s], (it / F4_STAGES) & 1, &bars.abort_flag, status, KID_MOE_GEMM, 15))) return false;
+    const uint8_t* st = ring + s * F4_STAGE;
+    uint4 qa[2], qb[2];
+    uint32_t sa[2], sb[2];
+    const int halves = (K - c * F4_KC) >= F4_KC ? 2 : 1;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int piece = ((h * 4 + t) ^ (ra & 7)) << 4;
+      qa[h] = *reinterpret_cast<const uint4*>(st + ra * 128 + piece);
+      qb[h] = *reinterpret_cast<const uint4*>(st + (ra + 8) * 128 + piece);
+      if (wsc == nullptr) {
+        sa[h] = *reinterpret_cast<const unsigned short*>(st + F4_CODES + ra * 16 + h * 8 + t * 2);
+        sb[h] = *reinterpret_cast<const unsigned short*>(st + F4_CODES + (ra + 8) * 16 + h * 8 + t * 2);
+      } else {                                            // rows of scales that are no whole 16 bytes
+        const uint8_t* p = wsc + (size_t)ra * (K / 16) + c * 16 + h * 8 + t * 2;
+        sa[h] = h < halves ? __ldg(reinterpret_cast<const unsigned short*>(p)) : 0;
+        sb[h] = h < halves ? __ldg(reinterpret_cast<const unsigned short*>(p + (size_t)8 * (K / 16))) : 0;
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars.empty[s]);           // in registers
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h < halves) {
+        const uint8_t* xs = xbuf + (size_t)(in_slab * 2 + h) * NT * 2048 + lane * 16;
+        __nv_bfloat162 ga[2], gb[2];
+        f4_scale2(sa[h], ga[0], ga[1]);
+        f4_scale2(sb[h], gb[0], gb[1]);
+        const uint32_t wa[4] = {qa[h].x, qa[h].y, qa[h].z, qa[h].w}, wb[4] = {qb[h].x, qb[h].y, qb[h].z, qb[h].w};
+#pragma unroll
+        for (int i2 = 0; i2 < 4; ++i2) {
+          uint32_t pa[4], pb[4];
+          f4_expand8(wa[i2], ga[i2 >> 1], pa);
+          f4_expand8(wb[i2], gb[i2 >> 1], pb);
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const uint4 x = *reinterpret_cast<const uint4*>(xs + (j * 4 + i2) * 512);
+            f4_mma(acc[j], pa[0], pb[0], pa[1], pb[1], x.x, x.y);
+            f4_mma(acc[j], pa[2], pb[2], pa[3], pb[3], x.z, x.w);
+          }
+        }
+      }
+    }
+  }
+  // ---- epilogue through an FP32 transpose tile [token][128] in the tokens' place
+  float* sT = reinterpret_cast<float*>(xbuf);
+  f4_sync();
+  const int r = ra, t2 = t * 2;
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    sT[(j * 8 + t2) * F4_BM + r] = acc[j][0] * gscale;
+    sT[(j * 8 + t2 + 1) * F4_BM + r] = acc[j][1] * gscale;
+    sT[(j * 8 + t2) * F4_BM + r + 8] = acc[j][2] * gscale;
+    sT[(j * 8 + t2 + 1) * F4_BM + r + 8] = acc[j][3] * gscale;
+  }
+  f4_sync();
+  if (epi == 1) {
+    const int c8 = threadIdx.x & 7;                                     // 32 token rows per sweep, 8 outputs per thread
+    for (int n = threadIdx.x >> 3; n < real; n += 4 * F4_WARPS) {
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int col = c8 * 8 + 2 * j;
+        const float g0 = f4_bfr(sT[n * F4_BM + col]), g1 = f4_bfr(sT[n * F4_BM + col + 1]);
+        const float u0 = f4_bfr(sT[n * F4_BM + 64 + col]), u1 = f4_bfr(sT[n * F4_BM + 64 + col + 1]);
+        o[j] = pack_bf16x2(f4_bfr(f4_silu(g0)) * u0, f4_bfr(f4_silu(g1)) * u1);
+      }
+      *reinterpret_cast<uint4*>(Y + (size_t)(grow0 + n) * ldy + tn * 64 + c8 * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  } else {
+    const int c16 = threadIdx.x & 15;                                   // 16 token rows per sweep
+    for (int n = threadIdx.x >> 4; n < real; n += 2 * F4_WARPS) {
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(sT[n * F4_BM + c16 * 8 + 2 * j], sT[n * F4_BM + c16 * 8 + 2 * j + 1]);
+      *reinterpret_cast<uint4*>(Y + (size_t)(grow0 + n) * ldy + tn * F4_BM + c16 * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+  return true;
+}
+
+// persistent, two CTAs per SM; scale_tma: the scales' rows are multiples of 16 bytes and come with the ring, otherwise the lanes read them
+__global__ void __launch_bounds__(F4_THREADS, 2)
+moe_fp4_grouped_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS, const __nv_bfloat16* __restrict__ X,
                        const uint8_t* __restrict__ Wsc, const float* __restrict__ Wglobal, __nv_bfloat16* __restrict__ Y,
-                       const int* __restrict__ seg_off, const int* __restrict__ counts, int Nw, int K, int ldy, int epi,
-                       int* status, int capacity) {
+                       const int* __restrict__ seg_off, const int* __restrict__ counts, int E, int Nw, int K, int ldy, int epi, int scale_tma,
+                       int capacity, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Fp4Bars bars;
-  const int e = blockIdx.y, tn = blockIdx.x;
-  // a segment reaching past the row buffers (an overflowed dispatch, reported through the status word) is cut there
-  const int cnt = min(counts[e], capacity - seg_off[e]);
-  if (cnt <= 0) return;                                   // uniform for the CTA
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* sT = reinterpret_cast<float*>(smem);             // epilogue staging [32 tokens][128] fp32
-  uint8_t* pipe = smem + F4_STAGING;
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* xbuf = ring + F4_STAGES * F4_STAGE;
+  int3* act = reinterpret_cast<int3*>(xbuf + F4_X_BYTES);                // experts with tokens: id, first row, rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row0 = seg_off[e];
-  const int kblocks = K / F4_KB;
-  const int passes = (cnt + F4_TOK - 1) / F4_TOK;
-
   if (threadIdx.x == 0) {
-    for (int i = 0; i < F4_STAGES; ++i) { mbar_init(&bars.full[i], 5); mbar_init(&bars.empty[i], 1); }
-    mbar_init(&bars.tmem_full, 1); mbar_init(&bars.tmem_empty, 4);
+    tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmS);
+    for (int i = 0; i < F4_STAGES; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.empty[i], F4_WARPS); }
     bars.abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) { tmem_alloc(&bars.tmem_base, 64); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = bars.tmem_base;
-  volatile int* abort_flag = &bars.abort_flag;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmX);
-      uint32_t it = 0; bool ok = true;
-      for (int p = 0; p < passes && ok; ++p) {
-        const int ntok = min(F4_TOK, ((cnt - p * F4_TOK + 15) / 16) * 16);
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % F4_STAGES; const uint32_t ph = (it / F4_STAGES) & 1;
-          if (!mbar_wait(&bars.empty[s], ph ^ 1, abort_flag, status, KID_MOE_GEMM, 11)) { ok = false; break; }
-          mbar_expect_tx(&bars.full[s], F4_NSUB * ntok * 128);
-          uint8_t* sx = pipe + s * F4_STAGE_BYTES + F4_A_BYTES;
-          for (int j = 0; j < F4_NSUB; ++j)
-            for (int r = 0; r < ntok; r += 16)
-              tma_load_2d(sx + j * (F4_TOK * 128) + r * 128, &tmX, &bars.full[s], kb * F4_KB + j * 64,
-                          row0 + p * F4_TOK + r);
-        }
-      }
+  pdl_trigger();
+  pdl_wait();                                             // tokens, offsets and counts are the preceding kernels'
+  if (warp == 1) {
+    int n = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, off = e < E ? seg_off[e] : 0;
+      // a segment reaching past the row buffers (an overflowed dispatch, reported through the status word) is cut there
+      const int cnt = e < E ? min(counts[e], capacity - off) : 0;
+      const uint32_t m = __ballot_sync(0xffffffffu, cnt > 0);
+      if (cnt > 0) act[n + __popc(m & ((1u << lane) - 1))] = make_int3(e, off, cnt);
+      n += __popc(m);
     }
-  } else if (warp == 1) {
+    if (lane == 0) bars.active = n;
+  }
+  __syncthreads();
+  const int tiles_n = Nw / F4_BM, items = bars.active * tiles_n, chunks = (K + F4_KC - 1) / F4_KC;
+  uint32_t it = 0;
+  bool ok = true;
+  if (warp == F4_WARPS) {
     if (lane == 0) {
-      uint32_t it = 0; bool ok = true;
-      for (int p = 0; p < passes && ok; ++p) {
-        const int ntok = min(F4_TOK, ((cnt - p * F4_TOK + 15) / 16) * 16);
-        const uint32_t idesc = umma_idesc(1, 1, 0, 0, F4_BM, ntok);
-        if (!mbar_wait(&bars.tmem_empty, (p & 1) ^ 1, abort_flag, status, KID_MOE_GEMM, 12)) { ok = false; break; }
-        tc_fence_after();
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % F4_STAGES; const uint32_t ph = (it / F4_STAGES) & 1;
-          if (!mbar_wait(&bars.full[s], ph, abort_flag, status, KID_MOE_GEMM, 13)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(pipe + s * F4_STAGE_BYTES);
-#pragma unroll
-          for (int j = 0; j < F4_NSUB; ++j) {
-            const uint64_t da = umma_desc_sw128(sa + j * F4_SUB, 16, 1024);
-            const uint64_t db = umma_desc_sw128(sa + F4_A_BYTES + j * (F4_TOK * 128), 16, 1024);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) umma_f16(tmem_base, da + 2 * k, db + 2 * k, idesc, (kb | j | k) != 0);
+      const uint64_t pol = l2_policy_evict_first();
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const int3 a = act[w / tiles_n];
+        const int wrow = a.x * Nw + (w % tiles_n) * F4_BM;
+        for (int p = 0; p < a.z && ok; p += F4_TOK)
+          for (int c = 0; c < chunks; ++c, ++it) {
+            const int s = it % F4_STAGES;
+            if (!mbar_wait(&bars.empty[s], ((it / F4_STAGES) & 1) ^ 1, &bars.abort_flag, status, KID_MOE_GEMM, 11)) { ok = false; break; }
+            mbar_expect_tx(&bars.full[s], F4_CODES + (scale_tma ? F4_SCALES : 0));
+            tma_load_2d_hint(ring + s * F4_STAGE, &tmW, &bars.full[s], c * (F4_KC / 2), wrow, pol);
+            if (scale_tma) tma_load_2d(ring + s * F4_STAGE + F4_CODES, &tmS, &bars.full[s], c * (F4_KC / 16), wrow);
           }
-          umma_commit(&bars.empty[s]);
-        }
-        if (ok) umma_commit(&bars.tmem_full);
       }
     }
   } else {
-    // ---- converter + epilogue warps. Converter warp cw owns weight rows cw*32 .. cw*32+31 of the tile; load i of
-    // a K block gives lane l the 16 packed bytes (32 weights) of chunk l%4 of row cw*32 + i*8 + l/4, so a warp-wide
-    // load covers eight whole 64-byte row pieces. ------------------------------------------------------------------
-    const int wr = threadIdx.x - 64;                                    // 0..127 (epilogue indexing)
-    const int q = warp & 3;                                             // TMEM lane quarter of this warp
-    const int cw = warp - 2, pc = lane & 3;
-    const size_t grow = (size_t)e * Nw + (size_t)tn * F4_BM + cw * 32 + (lane >> 2);
-    const uint8_t* wq = Wq + grow * (size_t)(K / 2) + pc * 16;
-    const uint8_t* ws = Wsc + grow * (size_t)(K / 16) + pc * 2;
-    const size_t wq_step = (size_t)8 * (K / 2), ws_step = (size_t)8 * (K / 16);      // eight rows further per load
-    const float gscale = Wglobal[e];
-    const int total = passes * kblocks;
-    // register prefetch, two K blocks ahead (two named register sets: no dynamic indexing)
-    uint4 pk0[4], pk1[4];
-    uint32_t sc0[4], sc1[4];
-    auto fetch = [&](uint4 (&pk)[4], uint32_t (&sc)[4], int it) {
-      const int kb = it % kblocks;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        pk[i] = __ldg(reinterpret_cast<const uint4*>(wq + i * wq_step + (size_t)kb * (F4_KB / 2)));
-        sc[i] = __ldg(reinterpret_cast<const unsigned short*>(ws + i * ws_step + (size_t)kb * (F4_KB / 16)));
-      }
-    };
-    // 8 codes of a 32-bit word -> four BF16 pairs times the group's scale (exact in BF16). The magnitude of a code
-    // indexes two 8-entry byte tables (high and low byte of the BF16 value) held in registers: prmt looks up four
-    // codes at once, two more prmt interleave the bytes into BF16 pairs, the sign bits are moved into place.
-    auto expand4 = [&](uint32_t w, __nv_bfloat162 sv) -> uint4 {
-      const uint32_t mag = w & 0x77777777u;
-      const uint32_t hi_a = __byte_perm(0x3f3f3f00u, 0x40404040u, mag);            // codes 0..3: high bytes
-      const uint32_t lo_a = __byte_perm(0xc0800000u, 0xc0804000u, mag);            //             low bytes
-      const uint32_t hi_b = __byte_perm(0x3f3f3f00u, 0x40404040u, mag >> 16);      // codes 4..7
-      const uint32_t lo_b = __byte_perm(0xc0800000u, 0xc0804000u, mag >> 16);
-      uint32_t o[4];
-      o[0] = __byte_perm(lo_a, hi_a, 0x5140) | ((w & 0x00000008u) << 12) | ((w & 0x00000080u) << 24);
-      o[1] = __byte_perm(lo_a, hi_a, 0x7362) | ((w & 0x00000800u) << 4) | ((w & 0x00008000u) << 16);
-      o[2] = __byte_perm(lo_b, hi_b, 0x5140) | ((w & 0x00080000u) >> 4) | ((w & 0x00800000u) << 8);
-      o[3] = __byte_perm(lo_b, hi_b, 0x7362) | ((w & 0x08000000u) >> 12) | (w & 0x80000000u);
-#pragma unroll
-      for (int b2 = 0; b2 < 4; ++b2) {
-        const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&o[b2]), sv);
-        o[b2] = *reinterpret_cast<const uint32_t*>(&r);
-      }
-      return make_uint4(o[0], o[1], o[2], o[3]);
-    };
-    auto convert = [&](const uint4 (&pk)[4], const uint32_t (&sc)[4], uint8_t* stage) {
-      uint8_t* sub = stage + (pc >> 1) * F4_SUB;                        // 64 weights of a row = one sub-tile row
-      const int ch0 = (pc & 1) * 4;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = cw * 32 + i * 8 + (lane >> 2);
-        const __nv_bfloat162 s0 = __float2bfloat162_rn(f4_e4m3(sc[i] & 0xffu));
-        const __nv_bfloat162 s1 = __float2bfloat162_rn(f4_e4m3(sc[i] >> 8));
-        uint8_t* rowp = sub + r * 128;
-        const int x = r & 7;
-        *reinterpret_cast<uint4*>(rowp + (((ch0 + 0) ^ x) << 4)) = expand4(pk[i].x, s0);
-        *reinterpret_cast<uint4*>(rowp + (((ch0 + 1) ^ x) << 4)) = expand4(pk[i].y, s0);
-        *reinterpret_cast<uint4*>(rowp + (((ch0 + 2) ^ x) << 4)) = expand4(pk[i].z, s1);
-        *reinterpret_cast<uint4*>(rowp + (((ch0 + 3) ^ x) << 4)) = expand4(pk[i].w, s1);
-      }
-    };
-    fetch(pk0, sc0, 0);
-    if (total > 1) fetch(pk1, sc1, 1);
-    bool ok = true;
-    int it = 0;
-    for (int p = 0; p < passes && ok; ++p) {
-      const int ntok = min(F4_TOK, ((cnt - p * F4_TOK + 15) / 16) * 16);
-      const int real = min(F4_TOK, cnt - p * F4_TOK);
-      for (int kb = 0; kb < kblocks; ++kb, ++it) {
-        const int s = it % F4_STAGES; const uint32_t ph = (it / F4_STAGES) & 1;
-        if (!mbar_wait(&bars.empty[s], ph ^ 1, abort_flag, status, KID_MOE_GEMM, 14)) { ok = false; break; }
-        uint8_t* sa = pipe + s * F4_STAGE_BYTES;
-        if (it & 1) { convert(pk1, sc1, sa); if (it + 2 < total) fetch(pk1, sc1, it + 2); }
-        else        { convert(pk0, sc0, sa); if (it + 2 < total) fetch(pk0, sc0, it + 2); }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.full[s]);
-      }
-      if (!ok) break;
-      // ---- epilogue of this pass --------------------------------------------------------------------
-      if (!mbar_wait(&bars.tmem_full, p & 1, abort_flag, status, KID_MOE_GEMM, 15)) { ok = false; break; }
-      tc_fence_after();
-      const int nl = q * 32 + lane;                                     // accumulator lane = weight row of the tile
-      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16);
-      const int grow0 = row0 + p * F4_TOK;
-      for (int t0 = 0; t0 < ntok; t0 += F4_EPI_TOK) {                   // the FP32 transpose tile holds 32 tokens
-        const int tcount = min(F4_EPI_TOK, ntok - t0);
-        for (int cc = 0; cc < tcount; cc += 16) {
-          uint32_t r[16];
-          tmem_ld_x16(taddr + t0 + cc, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) sT[(cc + j) * F4_BM + nl] = __uint_as_float(r[j]) * gscale;
-        }
-        if (t0 + F4_EPI_TOK >= ntok) {                                  // accumulator fully read: the next pass may start
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars.tmem_empty);
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (epi == 1) {
-          const int c8 = wr & 7, r0 = wr >> 3;                          // 16 token rows per sweep, 8 outputs per thread
-          for (int t = r0; t < tcount; t += 16) {
-            if (t0 + t >= real) break;
-            uint32_t o[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int col = c8 * 8 + 2 * j;
-              const float g0 = f4_bfr(sT[t * F4_BM + col]), g1 = f4_bfr(sT[t * F4_BM + col + 1]);
-              const float u0 = f4_bfr(sT[t * F4_BM + 64 + col]), u1 = f4_bfr(sT[t * F4_BM + 64 + col + 1]);
-              o[j] = pack_bf16x2(f4_bfr(f4_silu(g0)) * u0, f4_bfr(f4_silu(g1)) * u1);
-            }
-            *reinterpret_cast<uint4*>(Y + (size_t)(grow0 + t0 + t) * ldy + tn * 64 + c8 * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
-        } else {
-          const int c16 = wr & 15, r0 = wr >> 4;                        // 8 token rows per sweep
-          for (int t = r0; t < tcount; t += 8) {
-            if (t0 + t >= real) break;
-            uint32_t o[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(sT[t * F4_BM + c16 * 8 + 2 * j], sT[t * F4_BM + c16 * 8 + 2 * j + 1]);
-            *reinterpret_cast<uint4*>(Y + (size_t)(grow0 + t0 + t) * ldy + tn * F4_BM + c16 * 8) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+      const int3 a = act[w / tiles_n];
+      const int tn = w % tiles_n;
+      const uint8_t* wsc = scale_tma ? nullptr : Wsc + ((size_t)a.x * Nw + (size_t)tn * F4_BM) * (K / 16);
+      const float gscale = Wglobal[a.x] * 256.0f;
+      for (int p = 0; p < a.z && ok; p += F4_TOK) {
+        const int real = min(F4_TOK, a.z - p);
+        auto pass = [&](auto nt) {
+          return f4_pass<decltype(nt)::value>(X, a.y + p, real, ring, bars, it, wsc, K, xbuf, gscale, Y, ldy, tn, epi, status);
+        };
+        ok = real <= 8 ? pass(std::integral_constant<int, 1>{}) : real <= 16 ? pass(std::integral_constant<int, 2>{}) : pass(std::integral_constant<int, 4>{});
       }
     }
   }
-  __syncthreads();
-  if (bars.abort_flag) {
+  if (!ok) {                                              // a wait ran out: copies still in flight land before shared memory is released
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
   }
-  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, 64); }
 }
 
 }  // namespace ff
@@ -281,17 +272,22 @@ FF_EXPORT int ff_moe_grouped_gemm_nvfp4(const void* xs, const void* wq, const vo
                                         const int* seg_off, const int* counts, int E_local, int Nw, int K, int capacity,
                                         int ldy, int epi, int* status, cudaStream_t s) {
   if (E_local <= 0 || Nw <= 0 || K <= 0 || capacity <= 0 || !seg_off || !counts || !wglobal) return FF_HOST_BAD_SHAPE;
-  if (Nw % F4_BM || K % F4_KB || (epi != 0 && epi != 1)) return FF_HOST_BAD_SHAPE;
+  if (Nw % F4_BM || K % 128 || (epi != 0 && epi != 1)) return FF_HOST_BAD_SHAPE;
   if (ldy % 8 || ldy < (epi == 1 ? Nw / 2 : Nw)) return FF_HOST_BAD_ALIGN;
-  if ((reinterpret_cast<uintptr_t>(wq) & 15) || (reinterpret_cast<uintptr_t>(wsc) & 15) ||
+  if ((reinterpret_cast<uintptr_t>(xs) & 15) || (reinterpret_cast<uintptr_t>(wq) & 15) || (reinterpret_cast<uintptr_t>(wsc) & 15) ||
       (reinterpret_cast<uintptr_t>(y) & 15)) return FF_HOST_BAD_ALIGN;
-  CUtensorMap tmX;
-  int r = make_tmap_2d(&tmX, xs, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, capacity, (uint64_t)K * 2, 64, 16);
+  CUtensorMap tmW, tmS;
+  const uint64_t wrows = (uint64_t)E_local * Nw;
+  int r = make_tmap_2d(&tmW, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 2, wrows, K / 2, F4_KC / 2, F4_BM);
   if (r) return r;
-  const int smem = F4_STAGING + F4_STAGES * F4_STAGE_BYTES + 1024;
+  const int scale_tma = K % 256 == 0;                  // a map needs rows of whole 16 bytes
+  tmS = tmW;
+  if (scale_tma) { r = make_tmap_2d(&tmS, wsc, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K / 16, wrows, K / 16, F4_KC / 16, F4_BM, false); if (r) return r; }
+  const int smem = F4_STAGES * F4_STAGE + F4_X_BYTES + E_local * 12 + 1024;
   r = opt_in_smem(moe_fp4_grouped_kernel, smem); if (r) return r;
-  dim3 grid(Nw / F4_BM, E_local);
-  moe_fp4_grouped_kernel<<<grid, 192, smem, s>>>(tmX, (const uint8_t*)wq, (const uint8_t*)wsc, wglobal, (__nv_bfloat16*)y,
-                                                 seg_off, counts, Nw, K, ldy, epi, status, capacity);
+  const long long tiles = (long long)E_local * (Nw / F4_BM);
+  const int grid = tiles < 2 * sm_count() ? (int)tiles : 2 * sm_count();
+  if (int lr_ = launch_pdl(moe_fp4_grouped_kernel, dim3(grid), dim3(F4_THREADS), smem, s, 0, tmW, tmS, (const __nv_bfloat16*)xs, (const uint8_t*)wsc,
+                           wglobal, (__nv_bfloat16*)y, seg_off, counts, E_local, Nw, K, ldy, epi, scale_tma, capacity, status)) return lr_;
   return launch_result();
 }

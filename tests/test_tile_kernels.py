@@ -86,3 +86,33 @@ def test_fp8_expansion_is_exact(n, k):
     from flyingfish_b200.ops import quant_ops
     codes, scale = qref.quantize_fp8_block_weight(_rand((n, k), 3).float())
     assert torch.equal(quant_ops.dequant_fp8_block(codes.cuda(), scale.cuda()).cpu(), qref.dequantize_fp8_block(codes, scale))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("counts", [[1, 8, 0, 9], [16, 17, 32, 33], [70, 0, 0, 2]])      # column tiles of 8, 16 and 32 tokens, further passes
+@pytest.mark.parametrize("k", [128, 384, 768, 2304])         # scale rows of no whole 16 bytes, a ragged stage, token slabs that end inside K
+@pytest.mark.parametrize("epi", [0, 1])
+def test_grouped_nvfp4_passes(counts, k, epi):
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import moe_cuda
+    e, n = len(counts), 256
+    pad = [(c + 15) // 16 * 16 for c in counts]
+    off = [sum(pad[:i]) for i in range(e + 1)]
+    x = _rand((off[-1], k), 7)
+    q = [qref.quantize_nvfp4(_rand((n, k), 20 + i).float()) for i in range(e)]
+    w = moe_cuda.Nvfp4Experts(*(torch.stack([p[j] for p in q]).cuda() for j in range(3)))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    y = moe_cuda.grouped_gemm_nvfp4(x.cuda(), w, i32(off), i32(counts), off[-1], epi).cpu().float()
+    torch.cuda.synchronize()
+    ops.check_status()
+    for i, c in enumerate(counts):
+        if c:
+            full = (qref.e2m1_decode(qref.e2m1_unpack(q[i][0])).view(n, -1, 16) * qref.e4m3_decode(q[i][1])[..., None]).view(n, k).double()
+            rows = x[off[i]: off[i] + c].double() @ full.t() * float(q[i][2])
+            got = y[off[i]: off[i] + c]
+            if epi:
+                g = rows.float().view(c, n // 128, 2, 64)
+                want = ref.silu_mul(torch.cat([g[:, :, 0].reshape(c, -1), g[:, :, 1].reshape(c, -1)], 1).to(BF16)).float()
+                assert ((got - want).abs() <= 3 * 2.0 ** -8 * want.abs() + 2e-2).all()  # roundings as in the gated product above
+            else:
+                _check(got, rows, k)
