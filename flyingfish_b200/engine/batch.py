@@ -110,7 +110,8 @@ class ForwardBatch:
     # -- host fill -----------------------------------------------------------------------------
     def fill(self, *, ids, positions, slots, q_lens, ctx_lens, block_rows, logit_rows, is_decode: bool, nq: int = 1,
              tree_mask=None, kv_start=None, group_rows=None, state_slots=None, singles: int = 0) -> None:
-        """Write one step's metadata into the pinned host buffer (lists of ints)."""
+        """Write one step's metadata into the pinned host buffer (lists of ints; ids, positions and slots also as int32 arrays, which
+        is what a prompt's thousands of rows take)."""
         L = self.layout
         h = self.host
         rows, batch = len(ids), len(q_lens)

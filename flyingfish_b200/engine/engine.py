@@ -15,6 +15,7 @@ from __future__ import annotations
 import time
 from dataclasses import dataclass, field
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -278,16 +279,22 @@ class Engine:
         self._need_blocks([(sp.seq.seq_id, len(sp.tokens)) for sp in spans])
         fb = self.prefill_batch
         ids, positions, slots, q_lens, ctx_lens, block_rows, logit_rows = [], [], [], [], [], [], []
+        # thousands of prompt rows are listed as arrays (8000 rows: 4.4 ms as lists of ints, 0.6 ms); for a few dozen lists are quicker
+        wide = sum(len(sp.tokens) for sp in spans) > 256
         row = 0
         for sp in spans:
             kvs, take = self.kv.seqs[sp.seq.seq_id], len(sp.tokens)
-            sl = self.kv.reserve(sp.seq.seq_id, take)
-            ids += sp.tokens
-            positions += list(range(kvs.length, kvs.length + take))
-            slots += sl
+            if wide:
+                slots.append(self.kv.reserve_span(sp.seq.seq_id, take))
+                ids.append(np.asarray(sp.tokens, dtype=np.int32))
+                positions.append(np.arange(kvs.length, kvs.length + take, dtype=np.int32))
+            else:
+                slots += self.kv.reserve(sp.seq.seq_id, take)
+                ids += sp.tokens
+                positions += range(kvs.length, kvs.length + take)
             q_lens.append(take)
             ctx_lens.append(kvs.length + take)
-            block_rows.append(list(kvs.blocks))
+            block_rows.append(kvs.blocks)
             logit_rows += [row + k for k in sp.want]
             row += take
         mult = getattr(self.model.comm, "size", 1) * 128 if getattr(self.model.comm, "fused", False) else 1
@@ -295,8 +302,13 @@ class Engine:
             # sequence-parallel prefill shards rows over the ranks in 128-row blocks: pad with rows
             # that belong to no sequence (no KV write, no logits)
             pad = (row + mult - 1) // mult * mult - row
-            ids += [0] * pad; positions += [0] * pad; slots += [-1] * pad
+            zeros = np.zeros(pad, np.int32) if wide else [0] * pad
+            ids += [zeros] if wide else zeros
+            positions += [zeros] if wide else zeros
+            slots += [zeros - 1] if wide else [-1] * pad
         state_slots = [sp.seq.state_slot for sp in spans]
+        if wide:
+            ids, positions, slots = (np.concatenate(v) for v in (ids, positions, slots))
         fb.fill(ids=ids, positions=positions, slots=slots, q_lens=q_lens, ctx_lens=ctx_lens, block_rows=block_rows,
                 logit_rows=logit_rows, is_decode=False, state_slots=state_slots if self.state_slots is not None else None,
                 singles=singles)

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass, field
 
+import numpy as np
 import torch
 
 
@@ -113,7 +114,7 @@ class PagedKVCache:
         need = (total + self.block_size - 1) // self.block_size
         return max(0, need - len(s.blocks))
 
-    def reserve(self, seq_id: int, new_tokens: int) -> list[int]:
+    def reserve(self, seq_id: int, new_tokens: int, list_slots: bool = True) -> list[int]:
         """Make room for ``new_tokens`` more tokens and return their slots
         (slot = block * block_size + offset). Does not commit the length."""
         s = self.seqs[seq_id]
@@ -122,8 +123,19 @@ class PagedKVCache:
             raise OutOfBlocks(f"sequence {seq_id} needs {need} blocks, {self.alloc.free_blocks} free")
         for _ in range(need):
             s.blocks.append(self.alloc.alloc())
+        if not list_slots:
+            return []
         bs = self.block_size
         return [s.blocks[p // bs] * bs + p % bs for p in range(s.length, s.length + new_tokens)]
+
+    def reserve_span(self, seq_id: int, new_tokens: int) -> np.ndarray:
+        """:meth:`reserve` for the many rows of a prompt: the slots as an int32 array."""
+        self.reserve(seq_id, new_tokens, list_slots=False)
+        s, bs = self.seqs[seq_id], self.block_size
+        first = s.length // bs
+        pages = np.asarray(s.blocks[first: (s.length + new_tokens + bs - 1) // bs], dtype=np.int32)
+        at = s.length - first * bs
+        return (pages[:, None] * bs + np.arange(bs, dtype=np.int32)).reshape(-1)[at: at + new_tokens]
 
     def commit(self, seq_id: int, new_tokens: int) -> None:
         self.seqs[seq_id].length += new_tokens
