@@ -116,3 +116,19 @@ def test_grouped_nvfp4_passes(counts, k, epi):
                 assert ((got - want).abs() <= 3 * 2.0 ** -8 * want.abs() + 2e-2).all()  # roundings as in the gated product above
             else:
                 _check(got, rows, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ctx", [1, 64, 65, 4000])
+def test_merge_of_many_splits(ctx):
+    """A single sequence is cut into as many splits as it has pages: partials of all, one and most splits without keys."""
+    from flyingfish_b200 import ops
+    hq, hkv, d, blocks = 8, 2, 128, 64
+    q, k, v = _rand((1, hq * d), 1), _rand((blocks, hkv, 64, d), 2), _rand((blocks, hkv, 64, d), 3)
+    table = torch.randperm(blocks, generator=torch.Generator().manual_seed(4)).to(torch.int32)[None]
+    one = torch.ones(1, dtype=torch.int32)
+    want = ref.attention_paged(q, k, v, table, 0 * one, one, ctx * one, hq, hkv, d, d ** -0.5).float()
+    got = ops.attn_decode(q.cuda(), k.cuda(), v.cuda(), table.cuda(), (ctx * one).cuda(), hq, hkv, d, d ** -0.5, max_ctx=blocks * 64)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert ((got.cpu().float() - want).abs() <= 1e-2 + 1e-2 * want.abs()).all()  # BF16 weights and result
