@@ -502,7 +502,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   volatile int* abort_flag = &bars.abort_flag;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&bars.q_full, (k_hi ? TC_Q_BYTES : TC_Q_BYTES / 2) + (LAT ? 16384 : 0));
       const int qx = h * (LAT ? f.q_pitch : dk);
       tma_load_2d(sQ, &tmQ, &bars.q_full, qx, qs + r0);
@@ -553,7 +553,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       if (bad) set_status(status, KID_ATTN_PREFILL, FF_ERR_BOUNDS, b, r0 / TC_BM);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = umma_idesc(1, 1, 0, 0, TC_BM, T2_BN);
       const uint32_t idesc_o = umma_idesc(1, 1, 0, 1, TC_BM, v_hi ? TC_HD : TC_HD / 2);
       const int ksteps = dk >> 4;

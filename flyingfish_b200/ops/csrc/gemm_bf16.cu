@@ -310,7 +310,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* abort_flag = &bars.abort_flag;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
       uint32_t it = 0;
       bool ok = true;
@@ -340,7 +340,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(1, 1, 0, 0, BM, BN);
       uint32_t it = 0, tile_it = 0;
       bool ok = true;
@@ -610,7 +610,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   volatile int* abort_flag = &bars.abort_flag;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int t = first; t < tiles && ok; t += step) {
@@ -627,7 +627,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (rank == 0 && lane == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc(1, 1, 0, 0, 2 * BM, BN);
       uint32_t it = 0, tile_it = 0;
       bool ok = true;

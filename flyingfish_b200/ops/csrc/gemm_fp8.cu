@@ -103,7 +103,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   // The multiplies of up to three k-blocks run ahead of the promotion of the first, which hides the commit -> wait ->
   // load -> arrive latency chain between the MMA thread and the promoting warps.
   const int nbuf = ntok_max <= 64 ? 4 : 2;
-  const int buf_cols = 256 / nbuf;
+  const int buf_cols = 256 / nbuf, buf_shift = nbuf == 4 ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int scale_rows = (Nw + 127) / 128;                                // scale rows per expert
 
@@ -122,9 +122,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 
   pdl_trigger();
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmX);
-      uint32_t it = 0; bool ok = true;
+      RingPos rp; bool ok = true;
       // the weights do not depend on the kernel before this one (which produced the activation codes and scales):
       // the weight tiles of the first stages are requested before the dependency wait, the activation tiles after it
       const int ntok0 = min(TOK, ((cnt + 15) / 16) * 16);
@@ -139,9 +139,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           tma_load_2d(pipe + i * stage_bytes + A_BYTES + r * FBK, &tmX, &bars.full[i], (kb0 + i) * FBK, row0 + r);
       for (int c = 0; c < chunks && ok; ++c) {
         const int ntok = min(TOK, ((cnt - c * TOK + 15) / 16) * 16);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, rp.next(stages)) {
           if (c == 0 && kb - kb0 < pre) continue;                 // requested above
-          const int s = it % stages; const uint32_t ph = (it / stages) & 1;
+          const int s = rp.s; const uint32_t ph = rp.ph;
           if (!mbar_wait(&bars.empty[s], ph ^ 1, abort_flag, status, KID_GEMM_FP8, 1)) { ok = false; break; }
           if (blockIdx.x == 0 && blockIdx.y == 0) FF_TL(status, KID_GEMM_FP8, 10);
           mbar_expect_tx(&bars.full[s], A_BYTES + ntok * FBK);
@@ -153,15 +153,15 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t it = 0, kit = 0; bool ok = true;
+    if (elect_one()) {
+      RingPos rp; uint32_t kit = 0; bool ok = true;
       for (int c = 0; c < chunks && ok; ++c) {
         const int ntok = min(TOK, ((cnt - c * TOK + 15) / 16) * 16);
         const uint32_t idesc = umma_idesc(0, 0, 0, 0, FBM, ntok);        // E4M3 x E4M3 -> FP32
-        for (int kb = kb0; kb < kb1; ++kb, ++it, ++kit) {
-          const int b = kit % nbuf; const uint32_t bph = (kit / nbuf) & 1;
+        for (int kb = kb0; kb < kb1; ++kb, rp.next(stages), ++kit) {
+          const int b = kit & (nbuf - 1); const uint32_t bph = (kit >> buf_shift) & 1;
           if (!mbar_wait(&bars.tmem_empty[b], bph ^ 1, abort_flag, status, KID_GEMM_FP8, 2)) { ok = false; break; }
-          const int s = it % stages; const uint32_t ph = (it / stages) & 1;
+          const int s = rp.s; const uint32_t ph = rp.ph;
           if (blockIdx.x == 0 && blockIdx.y == 0) FF_TL(status, KID_GEMM_FP8, 20);
           if (!mbar_wait(&bars.full[s], ph, abort_flag, status, KID_GEMM_FP8, 3)) { ok = false; break; }
           if (blockIdx.x == 0 && blockIdx.y == 0) FF_TL(status, KID_GEMM_FP8, 21);
@@ -219,8 +219,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       for (int i = 0; i < TOK / 2; ++i) acc[i] = 0.f;
       const int nb = blk1 - blk0;
       for (int kb = 0; kb < nkb && ok; ++kb, ++kit) {
-        const int b0 = kit % nbuf;
-        if (!mbar_wait(&bars.tmem_full[b0], (kit / nbuf) & 1, abort_flag, status, KID_GEMM_FP8, 4)) { ok = false; break; }
+        const int b0 = kit & (nbuf - 1);
+        if (!mbar_wait(&bars.tmem_full[b0], (kit >> buf_shift) & 1, abort_flag, status, KID_GEMM_FP8, 4)) { ok = false; break; }
         if (blockIdx.x == 0 && blockIdx.y == 0 && ee == 0) FF_TL(status, KID_GEMM_FP8, 30);
         tc_fence_after();
         const uint32_t lane_base = tmem_base + (uint32_t(q * 32) << 16) + blk0 * 16;

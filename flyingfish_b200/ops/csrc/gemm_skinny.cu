@@ -292,14 +292,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   // weight tiles (weights are written by no kernel, so this needs no wait on the preceding kernel),
   // while warp 1 allocates TMEM; the other roles meet it at the block barrier.
   const uint32_t pre = (uint32_t)min((long long)stages, u1 - u0);
-  uint64_t pol_w = 0;
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmX);
     for (int i = 0; i < stages; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&bars.tmem_full[i], 1); mbar_init(&bars.tmem_empty[i], 4); }
     bars.abort_flag = 0; bars.flag_a = 0; bars.flag_b = 0;
     mbar_fence_init();
-    pol_w = l2_policy_evict_first();
+    const uint64_t pol_w = l2_policy_evict_first();
     uint32_t it = 0; long long u = u0; Segment sg;
     while (it < pre && next_segment(u, u1, kblocks, sg))
       for (int kb = sg.kb0; kb < sg.kb1 && it < pre; ++kb, ++it) {
@@ -317,15 +316,15 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   if (threadIdx.x == 0) FF_TL(status, KID_GEMM_SKINNY, 1);
 
   if (warp == 0) {
-    if (lane == 0) {
-      const uint64_t pol_x = l2_policy_evict_last();
+    if (elect_one()) {
+      const uint64_t pol_w = l2_policy_evict_first(), pol_x = l2_policy_evict_last();
       pdl_wait();
       FF_TL(status, KID_GEMM_SKINNY, 3);
-      uint32_t it = 0; bool ok = true;
+      uint32_t it = 0; RingPos rp; bool ok = true;
       long long u = u0; Segment sg;
       while (ok && next_segment(u, u1, kblocks, sg)) {
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
-          const int s = it % stages; const uint32_t ph = (it / stages) & 1;
+        for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it, rp.next(stages)) {
+          const int s = rp.s; const uint32_t ph = rp.ph;
           uint8_t* sa = pipe + s * stage_bytes;
           if (it >= pre) {
             if (!mbar_wait(&bars.empty[s], ph ^ 1, abort_flag, status, KID_GEMM_SKINNY, 1)) { ok = false; break; }
@@ -338,17 +337,17 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       FF_TL(status, KID_GEMM_SKINNY, 4);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc(1, 1, 0, 0, STOK, tile_rows);
-      uint32_t it = 0, seg_it = 0; bool ok = true;
+      uint32_t it = 0, seg_it = 0; RingPos rp; bool ok = true;
       long long u = u0; Segment sg;
       while (ok && next_segment(u, u1, kblocks, sg)) {
         const int acc = seg_it & 1; const uint32_t aph = (seg_it >> 1) & 1;
         if (!mbar_wait(&bars.tmem_empty[acc], aph ^ 1, abort_flag, status, KID_GEMM_SKINNY, 2)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * tile_rows;
-        for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it) {
-          const int s = it % stages; const uint32_t ph = (it / stages) & 1;
+        for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++it, rp.next(stages)) {
+          const int s = rp.s; const uint32_t ph = rp.ph;
           if (!mbar_wait(&bars.full[s], ph, abort_flag, status, KID_GEMM_SKINNY, 3)) { ok = false; break; }
           tc_fence_after();
           if (it == 0) FF_TL(status, KID_GEMM_SKINNY, 5);

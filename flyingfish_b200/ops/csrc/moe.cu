@@ -316,13 +316,13 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
   volatile int* abort_flag = &bars.abort_flag;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmX);
-      uint32_t it = 0; bool ok = true;
+      RingPos rp; bool ok = true;
       for (int c = 0; c < chunks && ok; ++c) {
         const int ntok = min(G_TOK, ((cnt - c * G_TOK + 15) / 16) * 16);
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % stages; const uint32_t ph = (it / stages) & 1;
+        for (int kb = 0; kb < kblocks; ++kb, rp.next(stages)) {
+          const int s = rp.s; const uint32_t ph = rp.ph;
           if (!mbar_wait(&bars.empty[s], ph ^ 1, abort_flag, status, KID_MOE_GEMM, 1)) { ok = false; break; }
           mbar_expect_tx(&bars.full[s], A_BYTES + ntok * GBK * 2);
           uint8_t* sa = pipe + s * STAGE_BYTES;
@@ -333,15 +333,15 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t it = 0; bool ok = true;
+    if (elect_one()) {
+      RingPos rp; bool ok = true;
       for (int c = 0; c < chunks && ok; ++c) {
         const int ntok = min(G_TOK, ((cnt - c * G_TOK + 15) / 16) * 16);
         const uint32_t idesc = umma_idesc(1, 1, 0, 0, GBM, ntok);
         if (!mbar_wait(&bars.tmem_empty, (c & 1) ^ 1, abort_flag, status, KID_MOE_GEMM, 2)) { ok = false; break; }
         tc_fence_after();
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % stages; const uint32_t ph = (it / stages) & 1;
+        for (int kb = 0; kb < kblocks; ++kb, rp.next(stages)) {
+          const int s = rp.s; const uint32_t ph = rp.ph;
           if (!mbar_wait(&bars.full[s], ph, abort_flag, status, KID_MOE_GEMM, 3)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(pipe + s * STAGE_BYTES);
