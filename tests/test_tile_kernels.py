@@ -132,3 +132,19 @@ def test_merge_of_many_splits(ctx):
     torch.cuda.synchronize()
     ops.check_status()
     assert ((got.cpu().float() - want).abs() <= 1e-2 + 1e-2 * want.abs()).all()  # BF16 weights and result
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [32, 33, 64, 65])                                 # two CTAs per SM between 33 and 64 rows
+@pytest.mark.parametrize("n,k", [(7168, 2560), (35072, 128), (576, 2560)])      # five splits, none, too few tiles for it
+def test_dense_fp8_pairs(m, n, k):
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import quant_ops
+    x, w = _rand((m, k), m), _rand((n, k), 5)
+    codes, scale = qref.quantize_fp8_block_weight(w.float())
+    y = quant_ops.linear_fp8(x.cuda(), codes.cuda(), scale.cuda()).cpu().float()
+    torch.cuda.synchronize()
+    ops.check_status()
+    want = qref.fp8_block_linear(x, codes, scale).float()
+    # exact block products, FP32 sums of k / 128 of them; device and host quantise activations alike up to a last bit of the scale
+    assert ((y - want).abs() <= 2.0 ** -7 * want.abs() + 2e-3 * k ** 0.5).all()
