@@ -2,11 +2,10 @@
 // stream from HBM, so the job of the kernel is to keep every SM pulling weights at full rate.
 //
 //   * The tokens are the UMMA M dimension (128 TMEM lanes, only ceil16(M) rows are loaded, the rest of
-//     the accumulator is never read) and up to 256 weight rows are the UMMA N dimension. A
-//     tcgen05.mma costs about the same whatever its N, so the weight bytes one instruction consumes
-//     decide how fast an SM can stream: with the weights as the wide B operand (256 rows x 32 bytes per
-//     instruction) the tensor pipe is no longer the limit; with the weights as the 128-row A operand
-//     (swap-AB) it capped an SM near 40 GB/s, below its share of HBM.
+//     the accumulator is never read) and up to 256 weight rows are the UMMA N dimension. One
+//     thread waits for, issues and commits the products of a k-block, and an instruction takes it 40 cycles or more whatever its N, so
+//     the weight bytes an instruction consumes decide how fast an SM can stream: the weights are the wide B operand (up to 256 rows x 32
+//     bytes per instruction), not the 128-row A operand.
 //   * Few weight tiles: cluster split-K. One cluster per tile of `tile_rows` weight rows, CTA s of
 //     the cluster multiplies its share of K and pushes the FP32 partial of token rows t = r (mod S)
 //     into slot s of CTA r's shared memory (distributed-shared-memory stores); after one cluster
@@ -743,28 +742,34 @@ static SkinnyConfig skinny_config(int M, int N, int K, int epi = 0) {
       }
     }
   }
-  // Time model (microseconds). A CTA takes in at most ~60 GB/s (weights plus the activation tile it
-  // re-reads from L2 for every k-block), a pipeline of `st` stages cannot turn a k-block around faster
-  // than the ~1.5 us load latency / st, and all CTAs together cannot beat HBM (~5.9 TB/s on reads).
+  // Time model (microseconds), fitted to the launchable decompositions of eight shapes at 64 tokens and, for the 8B shapes, to whole decode
+  // steps. A CTA takes in about 98 GB/s (weights plus the activation tile it re-reads from L2 for every k-block), a pipeline of `st`
+  // stages cannot turn a k-block around faster than the ~1.5 us load latency / st, and all CTAs together cannot beat HBM (~5.9 TB/s on
+  // reads). On top of the larger of these come 0.08 us per k-block of a CTA (waits and commits), for a cluster 18 ns per row of its tile
+  // (partials of 64 tokens pushed and summed), for stream-K 8 us (partial tiles through global memory). Clusters of two, four
+  // and eight come first: of three or six CTAs they lose in a chain of kernels what they gain alone. Decode steps of the 8-layer 8B-sized stack with 1, 7, 64,
+  // 113 sequences: 1048, 1177, 1677, 1819 us with stream-K for 6144 x 4096 and clusters of six for 4096 x 4096 and 4096 x 14336, 1043, 1184,
+  // 1619, 1615 us with clusters of two and four.
   // The choice must not depend on M: the K split fixes the order of the FP32 additions, and a
   // row's bits may not change with the batch it is computed in. So the model assumes 64 tokens and
   // the receive buffer is sized for those 64 (more tokens get the larger shared-memory budget and the same split).
   const int ntok = 64;
   (void)M;
   auto model = [&](int rows, int kb_per_cta, int st, double ctas) {
-    const double per_kb = (rows + ntok) * 128.0 / 60e3;
+    const double per_kb = (rows + ntok) * 128.0 / 98e3;
     const double lat_kb = 1.5 / st;
     const double t_cta = kb_per_cta * (per_kb > lat_kb ? per_kb : lat_kb);
     const double t_hbm = (double)N * K * 2.0 / 5.9e6;
     (void)ctas;
-    return t_cta > t_hbm ? t_cta : t_hbm;
+    return (t_cta > t_hbm ? t_cta : t_hbm) + 0.08 * kb_per_cta;
   };
   const long long units = (long long)best.tiles * kblocks;
   const int g1 = (int)(units / 2 > 148 ? 148 : (units / 2 < 1 ? 1 : units / 2));
-  // stream-K pays a trip through global scratch for the partial tiles: about 4 us on top
-  double best_cost = model(rows1, (int)((units + g1 - 1) / g1), best.stages, g1) + (g1 > best.tiles ? 4.0 : 0.0);
-  for (int s = 2; s <= 8; ++s) {
-    if (env_s > 0 && s != env_s) continue;
+  double best_cost = model(rows1, (int)((units + g1 - 1) / g1), best.stages, g1) + (g1 > best.tiles || units % g1 ? 8.0 : 0.0);
+  bool pow2 = false;                             // a cluster of two, four or eight beats stream-K: the other sizes are not looked at
+  for (int i = 0; i < 7; ++i) {
+    const int s = (const int[7]){2, 4, 8, 3, 5, 6, 7}[i];
+    if (env_s > 0 ? s != env_s : pow2 && i >= 3) continue;
     if (kblocks / s < 2) continue;
     // one cluster slot is left free: a launch that needs every slot can find one taken when it starts
     // while the preceding kernel drains (programmatic dependent launch), and then runs in two waves
@@ -779,8 +784,8 @@ static SkinnyConfig skinny_config(int M, int N, int K, int epi = 0) {
       const int recv = (s * ((ntok + s - 1) / s) * (rows + SP_PAD) * 4 + 1023) / 1024 * 1024;
       const int st = skinny_stages(rows, recv);
       if (st < 3) continue;
-      const double c = model(rows, (kblocks + s - 1) / s, st, (double)tiles * s);
-      if (c < best_cost - 1e-9 || (env_s > 0 && best.cluster == 1)) { best_cost = c; best = {s, rows, tiles, st, recv}; }
+      const double c = model(rows, (kblocks + s - 1) / s, st, (double)tiles * s) + 0.018 * rows;
+      if (c < best_cost - 1e-9 || (env_s > 0 && best.cluster == 1)) { best_cost = c; best = {s, rows, tiles, st, recv}; pow2 = i < 3; }
     }
   }
   if (best.cluster > 1) {
