@@ -5,9 +5,9 @@
 // global : FP32 per expert (ModelOpt `weight_scale_2`)
 // The decode-sized MoE layer is bound by expert weight bytes, so the weights stay packed in HBM (a quarter of the
 // BF16 bytes) and are expanded in the registers of the warps that multiply them (mma.sync, weights as the 16-row A fragment, tokens
-// as the 8 columns of B). Why not tcgen05: an instruction of it takes about 190 cycles however few tokens there are, and with 128
-// weight rows x 16 as its operand that caps a GPU at 1.7 TB/s of packed bytes -- measured with the expansion left out, through shared
-// memory and through tensor memory alike (528 us for a gate/up product of 0.9 GB). A 16 x 8 x 16 mma.sync costs what its 8 tokens cost.
+// as the 8 columns of B). Why not tcgen05: with converters in front of its 128-row operand the one thread that waits for, issues and
+// commits four products per 64-wide block held a GPU at 1.7 TB/s of packed bytes, with the expansion left out and through shared or
+// tensor memory alike (528 us for a gate/up product of 0.9 GB); here every warp multiplies what it has just expanded.
 //   * Persistent CTAs, two per SM, walk the (expert, 128 weight rows) tiles of the experts that have tokens. A producer warp keeps a ring
 //     of 256-wide K chunks (codes and scales) in flight with TMA; lanes that read 64-byte pieces of eight rows from global memory
 //     themselves reached 2.9 TB/s with nothing else to do. Eight warps own 16 weight rows each: lane (g, t) takes 16 bytes (32 codes)
