@@ -625,6 +625,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           tma_load_2d_pair(sa + A_BYTES, &tmB, &bars.full[s], kb * BK, tn * BN + rank * (BN / 2));
         }
       }
+      // The even CTA's commits arrive at this CTA's barriers: the last one of every stage is waited for, so that none can be on its way
+      // when the CTA leaves (the accumulator's barrier says nothing about the order in which these arrive).
+      for (uint32_t i = it > STAGES ? it - STAGES : 0; i < it && ok; ++i)
+        ok = mbar_wait(&bars.empty[i % STAGES], (i / STAGES) & 1, abort_flag, status, KID_GEMM_BF16, 9);
     }
   } else if (warp == 1) {
     if (rank == 0 && elect_one()) {
@@ -673,7 +677,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
   }
   __syncwarp();
-  cluster_sync_all();                                  // nothing arrives at a CTA's barriers, or reads its stages, after this
+  // Nothing arrives at a CTA's barriers, or reads its stages, after this: its producer has seen the last commit of every stage, its epilogue
+  // warps those of the accumulators, and the peer's epilogue warps have arrived at tmem_empty before they got here.
+  cluster_sync_all();
   if (warp == 1) { tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
 }
 

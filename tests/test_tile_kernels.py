@@ -34,6 +34,20 @@ def test_pair_gemm(m, n, k, odt):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kblocks", [1, 5, 6, 7, 8, 9, 12, 13, 16, 17])          # rings of six and eight stages: not full, full, begun again
+@pytest.mark.parametrize("m,n", [(129, 256), (1536, 4096)])                      # one tile per pair, several
+def test_pair_gemm_ends_with_its_last_stages(m, n, kblocks):
+    """The producers wait for the last commit of every stage they used: a phase that never completes would show in the status word."""
+    from flyingfish_b200 import ops
+    k = 64 * kblocks
+    x, w = _rand((m, k), m), _rand((n, k), n)
+    y = ops.linear(x.cuda(), w.cuda())
+    torch.cuda.synchronize()
+    ops.check_status()
+    _check(y, x.double() @ w.double().t(), k)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [(200, 264, 128), (300, 4096, 200)])
 def test_pair_gemm_tail(m, n, k):
     from flyingfish_b200 import ops
