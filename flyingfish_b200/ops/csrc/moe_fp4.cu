@@ -25,6 +25,7 @@
 // Format: kernels/nvfp4_linear.cu and src/fp8.rs:124-147 of the reference.
 #include "ptx.cuh"
 #include "host_util.h"
+#include "pass_walk.h"
 #include <cuda_fp8.h>
 #include <type_traits>
 
@@ -46,6 +47,12 @@ struct alignas(8) Fp4Bars {
   int active;
 };
 __device__ __forceinline__ void f4_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }      // the multiplying warps
+// the same, and whether any of them passed true
+__device__ __forceinline__ bool f4_sync_any(bool mine) {
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(any) : "r"((uint32_t)mine) : "memory");
+  return any != 0;
+}
 
 __device__ __forceinline__ float f4_silu(float x) { return x / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float f4_bfr(float x) { return __bfloat162float(__float2bfloat16(x)); }
@@ -92,24 +99,25 @@ __device__ __forceinline__ bool f4_pass(const __nv_bfloat16* __restrict__ X, int
 #pragma unroll
   for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
 
-  for (int c = 0; c < chunks; ++c, ++it) {
-    const int in_slab = c % (SLAB / F4_KC);
-    if (in_slab == 0) {
-      // tokens of this slab: unit [128-wide K][column tile][i2][token][t] holds x[token][32 t + 8 i2 + {0,4,1,5,2,6,3,7}]
-      f4_sync();
-      const int k0 = c * F4_KC, per = min(SLAB, K - k0) / 8;
-      for (int i = threadIdx.x; i < 8 * NT * per; i += 32 * F4_WARPS) {
-        const int n = i / per, k8 = i - n * per;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (n < real) v = __ldg(reinterpret_cast<const uint4*>(X + (size_t)(grow0 + n) * K + k0) + k8);
-        const int ch = k8 >> 4, tt = (k8 >> 2) & 3, i2 = k8 & 3;
-        *reinterpret_cast<uint4*>(xbuf + ((((ch * NT + (n >> 3)) * 4 + i2) * 8 + (n & 7)) * 4 + tt) * 16) =
-            make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
-      }
-      f4_sync();
+  constexpr int PER_SLAB = SLAB / F4_KC;
+  auto fill = [&](int c) {
+    // tokens of this slab: unit [128-wide K][column tile][i2][token][t] holds x[token][32 t + 8 i2 + {0,4,1,5,2,6,3,7}]
+    const int k0 = c * F4_KC, per = min(SLAB, K - k0) / 8;
+    for (int i = threadIdx.x; i < 8 * NT * per; i += 32 * F4_WARPS) {
+      const int n = i / per, k8 = i - n * per;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (n < real) v = __ldg(reinterpret_cast<const uint4*>(X + (size_t)(grow0 + n) * K + k0) + k8);
+      const int ch = k8 >> 4, tt = (k8 >> 2) & 3, i2 = k8 & 3;
+      *reinterpret_cast<uint4*>(xbuf + ((((ch * NT + (n >> 3)) * 4 + i2) * 8 + (n & 7)) * 4 + tt) * 16) =
+          make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410), __byte_perm(v.y, v.w, 0x7632));
     }
-    const int s = it % F4_STAGES;
-    if (!__all_sync(0xffffffffu, mbar_wait(&bars.full[s], (it / F4_STAGES) & 1, &bars.abort_flag, status, KID_MOE_GEMM, 15))) return false;
+  };
+  auto wait = [&](int) {
+    return __all_sync(0xffffffffu, mbar_wait(&bars.full[it % F4_STAGES], (it / F4_STAGES) & 1, &bars.abort_flag, status, KID_MOE_GEMM, 15)) != 0;
+  };
+  auto multiply = [&](int c) {
+    const int in_slab = c % PER_SLAB, s = it % F4_STAGES;
+    ++it;
     const uint8_t* st = ring + s * F4_STAGE;
     uint4 qa[2], qb[2];
     uint32_t sa[2], sb[2];
@@ -152,10 +160,10 @@ __device__ __forceinline__ bool f4_pass(const __nv_bfloat16* __restrict__ X, int
         }
       }
     }
-  }
+  };
+  if (!walk_pass(chunks, PER_SLAB, f4_sync, fill, wait, multiply, f4_sync_any)) return false;
   // ---- epilogue through an FP32 transpose tile [token][128] in the tokens' place
   float* sT = reinterpret_cast<float*>(xbuf);
-  f4_sync();
   const int r = ra, t2 = t * 2;
 #pragma unroll
   for (int j = 0; j < NT; ++j) {

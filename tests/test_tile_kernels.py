@@ -1,4 +1,6 @@
 """Products and reductions at the sizes where a tile, a chunk or a split ends."""
+import subprocess
+
 import pytest
 import torch
 
@@ -130,6 +132,49 @@ def test_grouped_nvfp4_passes(counts, k, epi):
                 assert ((got - want).abs() <= 3 * 2.0 ** -8 * want.abs() + 2e-2).all()  # roundings as in the gated product above
             else:
                 _check(got, rows, k)
+
+
+_WALK = r"""
+#include <atomic>
+#include <barrier>
+#include <cstdio>
+#include <thread>
+#include <vector>
+#include "pass_walk.h"
+constexpr int WARPS = 8;
+int main() {
+  int bad = 0;
+  for (int chunks : {1, 2, 5, 9})
+    for (int per_slab : {1, 2, 8})
+      for (int warp = -1; warp < WARPS; ++warp)            // -1: nobody gives up
+        for (int at = 0; at < (warp < 0 ? 1 : chunks); ++at) {
+          std::barrier sync(WARPS);
+          std::atomic<int> failed{0}, held{0}, done{0};
+          std::vector<std::thread> ts;
+          for (int w = 0; w < WARPS; ++w)
+            ts.emplace_back([&, w] {
+              auto meet = [&] { sync.arrive_and_wait(); };
+              auto any = [&](bool f) { failed += f; meet(); return failed.load() > 0; };
+              held += ff::walk_pass(chunks, per_slab, meet, [](int) {}, [&](int c) { return w != warp || c != at; }, [&](int) { ++done; }, any);
+            });
+          for (auto& t : ts) t.join();
+          const int want = warp < 0 ? WARPS * chunks : (WARPS - 1) * chunks + at;      // a warp that gave up multiplies nothing more
+          bad += held != (warp < 0 ? WARPS : 0) || done != want;
+        }
+  std::printf("%d", bad);
+  return bad != 0;
+}
+"""
+
+
+def test_warps_of_a_packed_pass_leave_together(tmp_path):
+    """The kernel's own walk on eight host threads: whichever warp's wait gives up at whichever stage, all eight come out of the pass (a
+    barrier that one of them no longer meets would hold the rest for good) and all say that it does not hold."""
+    from flyingfish_b200.ops import build
+    src, exe = tmp_path / "walk.cpp", tmp_path / "walk"
+    src.write_text(_WALK)
+    subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-I", str(build.CSRC), str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)], timeout=60, capture_output=True, text=True, check=True).stdout == "0"
 
 
 @pytest.mark.gpu
