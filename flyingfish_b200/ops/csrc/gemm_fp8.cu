@@ -339,19 +339,24 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 }  // namespace ff
 using namespace ff;
 
-// Dense calls of 33 to 64 tokens run two CTAs per SM (chunks of 64) where that fills nine tenths of the 296 places: one CTA's set-up and
-// reduction run under the other's stream (36864 x 7168 72 -> 55 us, 7168 x 18432 50 -> 41, 7168 x 16384 46 -> 41). Fewer CTAs would leave SMs
-// with one CTA and half a pipeline (24576 x 1536: 35 us with one CTA per SM, 46 with up to two).
-static bool fp8_paired(int M, int tiles, int splits) { return M > 32 && M <= 64 && tiles * splits >= 266; }
+// Dense calls of 33 to 64 tokens run two CTAs per SM (chunks of 64) where a result has tiles for nine tenths of the 296 places: one CTA's
+// set-up and drain run under the other's stream (36864 x 7168: 72 us with one CTA per SM, 54 with two). Fewer tiles would leave SMs with one CTA
+// and half a pipeline (24576 x 1536: 35 us with one CTA per SM, 46 with up to two).
+static bool fp8_paired(int M, int tiles) { return M > 32 && M <= 64 && tiles >= 266; }
 
+// The K split must not depend on M up to 128: it fixes the order of the FP32 additions, and a row's bits may not change with the batch it is
+// computed in. More splits for two CTAs per SM at 33 to 64 tokens alone broke that; at all sizes they lose where a split gets few k-blocks
+// (4096 x 7168, nine splits for four: 30 us for 21 at 64 tokens, 39 for 25 at 128).
 FF_EXPORT int ff_gemm_fp8_plan(int M, int N, int K, long long* scratch_bytes, long long* counter_bytes) {
   const int tiles = (N + FBM - 1) / FBM;
   const int kblocks = (K + FBK - 1) / FBK;
-  const int chunks = (M + F_TOK - 1) / F_TOK;      // further than 64 tokens dense calls use 128-token chunks
-  const int maxs = kblocks / 4 > 0 ? kblocks / 4 : 1;
-  auto split_for = [&](int ctas) { const int s = tiles * chunks < ctas ? ctas / (tiles * chunks) : 1; return s > maxs ? maxs : s; };
-  int splits = split_for(148);
-  if (fp8_paired(M, tiles, split_for(296))) splits = split_for(296);
+  const int chunks = (M + F_TOK - 1) / F_TOK;
+  int splits = 1;
+  if (tiles * chunks < 148) {
+    splits = 148 / (tiles * chunks);
+    const int maxs = kblocks / 4 > 0 ? kblocks / 4 : 1;
+    if (splits > maxs) splits = maxs;
+  }
   if (scratch_bytes) *scratch_bytes = splits > 1 ? (long long)splits * M * N * 4 : 0;
   if (counter_bytes) *counter_bytes = (long long)tiles * chunks * 4;
   return splits;
@@ -371,7 +376,7 @@ static int gemm_fp8_launch(const void* xq, const float* x_scale, const void* wq,
   if (ldy % 8 || (reinterpret_cast<uintptr_t>(y) & 15)) return FF_HOST_BAD_ALIGN;
   // Grouped calls take the smallest chunk that most segments fit into: 32 tokens up to an average of 8 rows per expert, 64 up to 52 (M
   // counts 16 rows of padding for each; random segments of that average exceed 64 in one case of twenty, which then streams its weights twice).
-  const int chunk = experts > 1 ? ((long long)M <= 24ll * experts ? 32 : (long long)M <= 68ll * experts ? 64 : F_TOK) : (M <= 32 ? 32 : fp8_paired(M, (Nw + FBM - 1) / FBM, splits) ? 64 : F_TOK);
+  const int chunk = experts > 1 ? ((long long)M <= 24ll * experts ? 32 : (long long)M <= 68ll * experts ? 64 : F_TOK) : (M <= 32 ? 32 : fp8_paired(M, (Nw + FBM - 1) / FBM) ? 64 : F_TOK);
   const bool small = chunk < F_TOK;
   const int tok_cap = experts > 1 ? chunk : (M >= F_TOK ? F_TOK : (M + 15) / 16 * 16);
   const int per = ((K / 128) + splits - 1) / splits;                     // k-blocks of one split

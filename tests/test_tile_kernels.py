@@ -193,9 +193,29 @@ def test_merge_of_many_splits(ctx):
     assert ((got.cpu().float() - want).abs() <= 1e-2 + 1e-2 * want.abs()).all()  # BF16 weights and result
 
 
+@pytest.mark.parametrize("n,k", [(7168, 18432), (7168, 2560), (4096, 7168), (6144, 4096), (34048, 512), (33920, 512), (576, 2560), (128, 128)])
+def test_fp8_split_does_not_depend_on_the_rows(n, k):
+    import ctypes
+    from flyingfish_b200.ops.lib import kernels
+    assert len({kernels().ff_gemm_fp8_plan(m, n, k, *(ctypes.byref(ctypes.c_longlong()) for _ in range(2))) for m in range(1, 129)}) == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k", [(7168, 2560), (4096, 7168), (34048, 512), (33920, 512)])      # splits, none with one and two CTAs per SM
+def test_fp8_rows_keep_their_bits_in_any_decode_batch(n, k):
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import quant_ops
+    x = _rand((128, k), 1).cuda()
+    codes, scale = (t.cuda() for t in qref.quantize_fp8_block_weight(_rand((n, k), 2).float()))
+    y = quant_ops.linear_fp8(x, codes, scale)
+    for m in (1, 5, 32, 33, 64, 65):
+        assert torch.equal(quant_ops.linear_fp8(x[:m].contiguous(), codes, scale), y[:m]), m
+    ops.check_status()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m", [32, 33, 64, 65])                                 # two CTAs per SM between 33 and 64 rows
-@pytest.mark.parametrize("n,k", [(7168, 2560), (35072, 128), (576, 2560)])      # five splits, none, too few tiles for it
+@pytest.mark.parametrize("n,k", [(7168, 2560), (35072, 128), (576, 2560)])      # two splits, none, too few tiles for it
 def test_dense_fp8_pairs(m, n, k):
     from flyingfish_b200 import ops
     from flyingfish_b200.ops import quant_ops
