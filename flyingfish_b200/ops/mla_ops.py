@@ -184,8 +184,9 @@ EXPAND_MAX_KEYS = 1 << 16        # most key rows expanded at a time
 def expands(q: torch.Tensor, width: int, dim: int, rot: int, vdim: int, longest: int) -> bool:
     """Whether :func:`expanded_attention` serves a batch whose longest portion has ``longest`` rows: on the tensor cores a head of
     dim + rot elements costs a fraction of one as wide as the latent, which pays for the expansion from a few dozen rows on. Narrow
-    latents have the tcgen05 kernel in the latent space."""
-    return q.is_cuda and q.dtype == torch.bfloat16 and width > 128 and dim <= 128 and rot <= 64 and vdim <= 128 and longest >= EXPAND_MIN_ROWS
+    latents have the tcgen05 kernel in the latent space. The kernel's head parts are whole 16-element steps of a product."""
+    steps = dim % 16 == 0 and rot % 16 == 0 and vdim % 16 == 0
+    return q.is_cuda and q.dtype == torch.bfloat16 and width > 128 and dim <= 128 and rot <= 64 and vdim <= 128 and steps and longest >= EXPAND_MIN_ROWS
 
 
 @dataclass

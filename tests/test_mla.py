@@ -80,3 +80,26 @@ def test_tiered_experts_on_gpu():
     out = [first] + [m.engine.decode([seq])[0] for _ in range(9)]
     assert sum(x == y for x, y in zip(out, plain)) >= 8, (out, plain)
     assert prov.stats["cpu_rows"] > 0 and prov.stats["gpu_rows"] > 0 and prov.stats["h2d_expert_bytes"] > 0
+
+
+def test_only_widths_of_whole_steps_are_expanded():
+    """Heads whose parts are no multiples of 16 elements stay in the latent space, which serves them."""
+    from types import SimpleNamespace
+    from flyingfish_b200.ops import mla_ops
+    q = SimpleNamespace(is_cuda=True, dtype=torch.bfloat16)
+    assert mla_ops.expands(q, 576, 128, 64, 128, 64) and mla_ops.expands(q, 576, 16, 16, 16, 64)
+    assert not any(mla_ops.expands(q, 576, *w, 64) for w in ((24, 64, 128), (128, 40, 128), (128, 64, 72)))
+
+
+@pytest.mark.gpu
+def test_prompt_of_a_model_with_24_wide_keys():
+    """70 rows, more than a portion needs to be expanded: the unrotated key part of 24 elements goes through the latent space."""
+    from _oracle import assert_rows_mostly_close
+    from flyingfish_b200 import ops
+    from flyingfish_b200.config import named_shape
+    spec = named_shape("deepseek-v3-mini")
+    spec.mla.qk_nope_dim = 24
+    cpu, gpu = (Model.load(spec, Settings(capacity=256, max_batch=4, graph=False), device=d, seed=0) for d in ("cpu", "cuda"))
+    g = torch.Generator().manual_seed(6)
+    assert_rows_mostly_close(cpu, gpu, [torch.randint(0, 2048, (n,), generator=g).tolist() for n in (70, 9)], rel=0.08, frac=0.6)
+    ops.check_status()
