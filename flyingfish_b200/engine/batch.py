@@ -63,6 +63,7 @@ class ForwardBatch:
         self.n_logit_rows = 0
         self.use_tree_mask = False
         self._bt_sig: list = []           # block list last written to each block-table row of the host buffer
+        self.key_pages: tuple | None = None   # what a model's layers derive once from this step's block lists; fill() drops it
 
     # -- device views (fixed addresses) ------------------------------------------------------
     def _v(self, off: int, n: int) -> torch.Tensor:
@@ -118,6 +119,7 @@ class ForwardBatch:
         assert rows <= L.max_rows and batch <= L.max_batch, "batch exceeds the layout capacity"
         assert len(logit_rows) <= L.n_logit
         self.rows, self.batch, self.nq, self.is_decode, self.singles = rows, batch, nq, is_decode, singles
+        self.key_pages = None
         h[L.ids: L.ids + rows] = torch.as_tensor(ids, dtype=torch.int32)
         h[L.positions: L.positions + rows] = torch.as_tensor(positions, dtype=torch.int32)
         h[L.slots: L.slots + rows] = torch.as_tensor(slots, dtype=torch.int32)

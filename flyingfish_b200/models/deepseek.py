@@ -149,20 +149,17 @@ class DeepseekModel(DecoderModel):
                                 self.scale, a.kv_lora_rank)
         return ops.head_linear(lat.view(rows, -1), m.w_uv(heads))
 
-    def hidden_states(self, b, kv, inputs_embeds=None):
-        self._pages = None                      # pages the portions of this step can see, listed by its first layer
-        return super().hidden_states(b, kv, inputs_embeds)
-
     def _key_pages(self, b, kv):
-        """The pages of a step's portions, or None where keys and values of all heads would take over ``EXPAND_MAX_BYTES``."""
-        if self._pages is None:
+        """The pages of a step's portions, or None where keys and values of all heads would take over ``EXPAND_MAX_BYTES``. Listed by the
+        step's first layer and kept with the step: one model serves several engines, also from several threads."""
+        if b.key_pages is None:
             L, h, n = b.layout, b.host, b.batch
             table = h[L.block_table: L.block_table + L.max_batch * L.max_blocks].view(L.max_batch, L.max_blocks)[:n]
             ctx = h[L.ctx_lens: L.ctx_lens + n].tolist()
             keys = sum((c + kv.block_size - 1) // kv.block_size for c in ctx) * kv.block_size
             fits = 2 * keys * self.spec.heads * (self.mla.qk_nope_dim + self.mla.v_head_dim) <= EXPAND_MAX_BYTES
-            self._pages = (mla_ops.KeyPages.of(h[L.q_lens: L.q_lens + n].tolist(), ctx, table, 0, kv.block_size, b.device) if fits else None,)
-        return self._pages[0]
+            b.key_pages = (mla_ops.KeyPages.of(h[L.q_lens: L.q_lens + n].tolist(), ctx, table, 0, kv.block_size, b.device) if fits else None,)
+        return b.key_pages[0]
 
     def _attend_oracle(self, i: int, q: torch.Tensor, kva: torch.Tensor, m: MlaWeights, b, kv) -> torch.Tensor:
         """[rows, heads * v] through the latent space, operator by operator (CPU)."""

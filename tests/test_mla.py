@@ -103,3 +103,30 @@ def test_prompt_of_a_model_with_24_wide_keys():
     g = torch.Generator().manual_seed(6)
     assert_rows_mostly_close(cpu, gpu, [torch.randint(0, 2048, (n,), generator=g).tolist() for n in (70, 9)], rel=0.08, frac=0.6)
     ops.check_status()
+
+
+def _portions(q_lens, pasts):
+    """A filled batch of prompt portions (host side), its sequences' pages one after the other from block 1 on."""
+    from flyingfish_b200.engine.batch import BatchLayout, ForwardBatch
+    ctx = [n + p for n, p in zip(q_lens, pasts)]
+    pages = [(c + 63) // 64 for c in ctx]
+    at = [1 + sum(pages[:i]) for i in range(len(pages))]
+    fb = ForwardBatch(BatchLayout(len(q_lens), sum(q_lens), max(pages)), torch.device("cpu"))
+
+    def fill():
+        fb.fill(ids=[0] * sum(q_lens), positions=[0] * sum(q_lens), slots=[0] * sum(q_lens), q_lens=q_lens, ctx_lens=ctx,
+                block_rows=[list(range(a, a + n)) for a, n in zip(at, pages)], logit_rows=[], is_decode=False)
+    fill()
+    return fb, fill
+
+
+def test_pages_belong_to_the_step():
+    """Steps of two engines that share a model, layer by layer in turn, and the next step of one of them."""
+    m = Model.load("deepseek-v3-mini", Settings(capacity=256, max_batch=4, graph=False), device="cpu", seed=0).engine
+    net, (a, _), (b, fill) = m.model, _portions([70], [0]), _portions([100, 64], [60, 64])
+    for _ in range(2):
+        assert net._key_pages(a, m.kv).blocks.tolist() == [1, 2] and net._key_pages(b, m.kv).blocks.tolist() == [1, 2, 3, 4, 5]
+    first = net._key_pages(b, m.kv)
+    assert net._key_pages(b, m.kv) is first
+    fill()
+    assert net._key_pages(b, m.kv) is not first
