@@ -22,6 +22,10 @@ from .weights import LayerWeights, ModelWeights, TPInfo, build_decoder_weights
 
 
 EXPAND_MAX_BYTES = 2 << 30       # most memory that a layer's expanded keys and values take
+# A step's portions are expanded from this many query rows per visible key on (a portion's rows, weighted by its context). The expansion costs
+# by the key, the latent space by the row and key. One layer at the published widths, latent space against expanded: 64 rows in front of 16,000
+# tokens 1748 / 855 us, 23 rows per key 553 / 622, 10 rows 634 / 1314, a portion of 64 rows beside fifteen of 8 rows behind 2000 tokens 612 / 1612.
+EXPAND_MIN_ROWS_PER_KEY = 32
 
 
 @dataclass
@@ -129,8 +133,9 @@ class DeepseekModel(DecoderModel):
         return self.comm.row_linear(o, m.wo)
 
     def _attend(self, i: int, q: torch.Tensor, kva: torch.Tensor, m: MlaWeights, b, kv) -> torch.Tensor:
-        """[rows, heads * v] on the GPU. Portions of prompts expand the visible latents to keys and values; decoded tokens, short
-        portions and contexts beyond the expansion's memory go through the latent space."""
+        """[rows, heads * v] on the GPU. Portions of prompts expand the visible latents to keys and values; decoded tokens, portions that
+        are short against what they see, and contexts beyond the expansion's memory go through the latent space. The step decides for all
+        its portions, and the forms round at different places: a portion's bits may depend on the portions beside it."""
         s, a, heads, rows = self.spec, self.mla, self.spec.heads, q.shape[0]
         cache, nope, dv = kv.k[i], a.qk_nope_dim, a.v_head_dim
         form = (kva, m.kv_a_ln, b.positions, b.slots, cache, heads, nope, s.rope_theta, s.rms_eps)
@@ -150,15 +155,17 @@ class DeepseekModel(DecoderModel):
         return ops.head_linear(lat.view(rows, -1), m.w_uv(heads))
 
     def _key_pages(self, b, kv):
-        """The pages of a step's portions, or None where keys and values of all heads would take over ``EXPAND_MAX_BYTES``. Listed by the
+        """The pages of a step's portions, or None where expanding them does not pay or would take over ``EXPAND_MAX_BYTES``. Listed by the
         step's first layer and kept with the step: one model serves several engines, also from several threads."""
         if b.key_pages is None:
             L, h, n = b.layout, b.host, b.batch
             table = h[L.block_table: L.block_table + L.max_batch * L.max_blocks].view(L.max_batch, L.max_blocks)[:n]
             ctx = h[L.ctx_lens: L.ctx_lens + n].tolist()
+            lens = h[L.q_lens: L.q_lens + n].tolist()
             keys = sum((c + kv.block_size - 1) // kv.block_size for c in ctx) * kv.block_size
             fits = 2 * keys * self.spec.heads * (self.mla.qk_nope_dim + self.mla.v_head_dim) <= EXPAND_MAX_BYTES
-            b.key_pages = (mla_ops.KeyPages.of(h[L.q_lens: L.q_lens + n].tolist(), ctx, table, 0, kv.block_size, b.device) if fits else None,)
+            pays = sum(q * c for q, c in zip(lens, ctx)) >= EXPAND_MIN_ROWS_PER_KEY * sum(ctx)
+            b.key_pages = (mla_ops.KeyPages.of(lens, ctx, table, 0, kv.block_size, b.device) if fits and pays else None,)
         return b.key_pages[0]
 
     def _attend_oracle(self, i: int, q: torch.Tensor, kva: torch.Tensor, m: MlaWeights, b, kv) -> torch.Tensor:

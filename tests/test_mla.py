@@ -130,3 +130,48 @@ def test_pages_belong_to_the_step():
     assert net._key_pages(b, m.kv) is first
     fill()
     assert net._key_pages(b, m.kv) is not first
+
+
+@pytest.mark.parametrize("q_lens,pasts,pays", [([64], [0], True), ([64], [900], True), ([64, 64], [500, 0], True), ([64] + [1] * 5, [0] + [200] * 5, False),
+                                               ([200, 20, 20], [0, 500, 500], True), ([64, 20, 20], [0, 300, 300], False)])
+def test_portions_are_expanded_where_rows_pay_for_keys(q_lens, pasts, pays):
+    m = Model.load("deepseek-v3-mini", Settings(capacity=256, max_batch=4, graph=False), device="cpu", seed=0).engine
+    assert (m.model._key_pages(_portions(q_lens, pasts)[0], m.kv) is not None) == pays
+
+
+@pytest.mark.gpu
+def test_expanded_and_latent_prompts_agree(monkeypatch):
+    """Portions of 70 + 9 rows and, behind them, 80 + 40: expanded, over the memory limit, over the key limit and too few rows per key."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.engine.engine import Span
+    from flyingfish_b200.models import deepseek
+    from flyingfish_b200.ops import mla_ops
+    g = torch.Generator().manual_seed(8)
+    ids = [torch.randint(0, 2048, (n,), generator=g).tolist() for n in (150, 49)]
+    m = Model.load("deepseek-v3-mini", Settings(capacity=256, max_batch=4, graph=False), device="cuda", seed=0)
+    asked, real = [], mla_ops.expanded_attention
+    monkeypatch.setattr(mla_ops, "expanded_attention", lambda *x, **k: (asked.append(1), real(*x, **k))[1])
+
+    def logits():
+        asked.clear()
+        seqs, out = [m.engine.add_sequence(p) for p in ids], []
+        for lo, hi in (((0, 0), (70, 9)), ((70, 9), (150, 49))):
+            fb = m.engine._fill_spans([Span(s, p[a: b], list(range(b - a))) for s, p, a, b in zip(seqs, ids, lo, hi)])
+            out.append(m.engine.model.forward(fb, m.engine.kv, return_logits=True).float().cpu())
+            for s, a, b in zip(seqs, lo, hi):
+                m.engine.kv.commit(s.seq_id, b - a)
+        for s in seqs:
+            m.engine.free_sequence(s.seq_id)
+        return torch.cat(out)
+    want = logits()
+    assert len(asked) == 2 * m.spec.layers
+    for where, name, value in ((deepseek, "EXPAND_MAX_BYTES", 0), (mla_ops, "EXPAND_MAX_KEYS", 64), (deepseek, "EXPAND_MIN_ROWS_PER_KEY", 1000)):
+        with monkeypatch.context() as mp:
+            mp.setattr(where, name, value)
+            got = logits()
+        assert not asked
+        # The forms round to BF16 at different places (2^-9 of a value each, a few per layer). A rounding may turn an expert choice, which
+        # changes a row and those that see it: most rows agree.
+        err = (got - want).norm(dim=-1) / want.norm(dim=-1)
+        assert torch.isfinite(got).all() and (err <= 2e-2).float().mean() >= 0.6, (name, err.sort().values)
+    ops.check_status()
