@@ -7,8 +7,8 @@
 // 4 epilogue warps), persistent, with double-buffered TMEM accumulators so the epilogue of tile i
 // overlaps the mainloop of tile i+1, and an optional SwiGLU epilogue (gate|up interleaved per 64 rows
 // of the weight). gemm_bf16_pair_kernel: dense problems, 256-row tiles by CTA pairs. gemm_bf16_kernel:
-// 128-row tiles of one CTA, for expert segments (grouped mode), block-diagonal products and the
-// tensor-parallel forms (all-gather -> GEMM, GEMM -> reduce-scatter) with peer stores in the same
+// 128-row tiles of one CTA, for dense problems whose rows or K do not suit a pair, expert segments (grouped mode),
+// block-diagonal products and the tensor-parallel forms (all-gather -> GEMM, GEMM -> reduce-scatter) with peer stores in the same
 // kernel. Decode shapes (M <= 128) are served by gemm_skinny.cu.
 // This replaces the reference's cuBLAS/cuBLASLt calls (src/backend/cuda/blas.rs:852-1080)
 // and its mma.sync skinny kernel (kernels/gemm_skinny.cu).
@@ -707,6 +707,22 @@ static int gemm_bf16_launch(const void* X, const void* W, void* Y, int M, int N,
   const int pairs = sm_count() / 2, tiles_m = (M + 2 * BM - 1) / (2 * BM);
   auto waves = [&](int bn) { const int t = tiles_m * ((N + bn - 1) / bn); return (t + pairs - 1) / pairs; };
   const bool narrow = waves(128) * 0.575f < waves(256);
+  // Tiles of one CTA where they finish in clearly fewer waves: 256-row tiles of pairs pad rows more, and at short K a pair's set-up and its
+  // epilogue take what its main loop saves. A wave of one-CTA tiles is charged 1 / 0.79 of a pair's (1 / 0.97 behind a SwiGLU epilogue at K up
+  // to 2048, 1 / 1.05 at K up to 512 and for a single wave at K up to 1024). Of 1507 sizes (42 shapes of 512 x 512 to 65536 x 2048 and 57344 x
+  // 8192, 130 to 8192 rows) that is the quicker form within 2 % at all but 18, within 5 % at those. One-CTA / pair tiles: 1100 x 4096 x 14336
+  // 98 / 128 us, 320 x 24576 x 1536 29 / 32, 4096 x 32768 x 512 157 / 179. K is walked in the same order: the bits are the same.
+  const int ctas = sm_count(), waves1 = (((M + BM - 1) / BM) * ((N + 255) / 256) + ctas - 1) / ctas;
+  const float share = K <= 512 || (K <= 1024 && waves1 == 1) ? 1.05f : epi == 1 && K <= 2048 ? 0.97f : 0.79f;
+  if (waves1 < share * (narrow ? 0.575f * waves(128) : (float)waves(256))) {
+    constexpr int BN = 256, STAGES = 4;
+    if (int e = make_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, BN)) return e;
+    const int smem = STAGES * (BM + BN) * BK * 2 + 1024, tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    auto kern = gemm_bf16_kernel<BN, STAGES, 0>;
+    if (int e = opt_in_smem(kern, smem)) return e;
+    kern<<<tiles < ctas ? tiles : ctas, 192, smem, stream>>>(tmA, tmA, tmA, tmB, Y, M, N, K, ldy, epi, status, CommArgs{}, GroupArgs{}, tail);
+    return launch_result();
+  }
   const int bn = narrow ? 128 : 256;
   r = make_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, bn / 2);
   if (r) return r;

@@ -61,6 +61,43 @@ def test_pair_gemm_tail(m, n, k):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("form", ["plain", "fp32", "pitches", "bias relu2", "bias gelu factors", "swiglu", "gated 3", "gated 5"])
+@pytest.mark.parametrize("k", [64, 520, 584, 2048])
+def test_pairs_and_single_ctas_give_the_same_bits(form, k):
+    """Sixteen column tiles: 1000 rows are one wave of pairs and 1100 rows two, where 128-row tiles of one CTA need one (of K up to 512
+    both sizes take those). The rows that both calls have must agree, whatever the epilogue and the pitches."""
+    from flyingfish_b200 import ops
+    x = _rand((1100, k + 8), 1).cuda()[:, : k]                                  # rows 16 bytes apart from being contiguous
+    n = 4096 if form.startswith(("swiglu", "gated")) else 4072                   # a ragged last tile where the form takes one
+    w = (_rand((n, k + 16), 2) * 0.1).cuda()[:, 8: k + 8]
+    bias, table, ids = _rand((n,), 3).cuda(), _rand((7, n), 4).cuda(), torch.randint(0, 7, (1100,), generator=torch.Generator().manual_seed(5)).to(torch.int32).cuda()
+
+    def run(m):
+        if form == "fp32":
+            return ops.linear(x[:m], w, out_dtype=torch.float32)
+        if form == "pitches":
+            out = torch.full((m, n + 24), 7.0, dtype=BF16, device="cuda")
+            ops.linear(x[:m], w, out=out[:, 8: n + 8])
+            assert (out[:, :8] == 7).all() and (out[:, n + 8:] == 7).all()
+            return out
+        if form == "bias relu2":
+            return ops.linear(x[:m], w, bias=bias, act="relu2")
+        if form == "bias gelu factors":
+            return ops.linear(x[:m], w, bias=bias, act="gelu_tanh", mul=(table, ids[:m].contiguous()))
+        if form == "swiglu" or form.startswith("gated"):
+            mode = 0 if form == "swiglu" else int(form[-1])
+            return ops.linear_swiglu(x[:m], w, mode=mode, limit=1.5)
+        return ops.linear(x[:m], w)
+    many, few = run(1100), run(1000)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(many[:1000], few)
+    if form in ("plain", "fp32"):
+        want = x.cpu().double() @ w.cpu().double().t()
+        _check(many, want, k, torch.float32 if form == "fp32" else BF16)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n", [(129, 256), (700, 5888), (256, 19200)])       # narrow and wide column tiles
 def test_pair_gemm_gate(m, n):
     from flyingfish_b200 import ops
