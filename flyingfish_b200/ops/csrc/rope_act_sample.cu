@@ -470,12 +470,18 @@ sample_rows_kernel(const float* __restrict__ logits, int* __restrict__ out_ids, 
 using namespace ff;
 
 // Rows per CTA: four where that still leaves several CTAs per SM (fewer angles made twice, three vectors of a thread in flight), one
-// for decode batches.
+// for decode batches. Few or narrow heads leave threads idle in a CTA per row and take two or four rows as soon as every SM has a CTA: 4 + 1
+// heads of 64 (24 vector pairs a row) at 2367 rows 12.3 -> 4.8 us, 8.6 with a thread per vector pair. More rows than four gain only for a head
+// or two of the smallest (8192 rows of 1 + 1 heads of 16: 9.8 -> 4.6 us, 6.1 with a thread per pair) and cost others (4.7 -> 5.6).
 static int rope_launch(void* qkv, const int* positions, const int* slots, void* kcache, void* vcache, const float* inv_freq, int rows, int hq,
                        int hkv, int dim, int rot_dim, int block_size, int num_blocks, float theta, int ldqkv, int* status, const float* cos_sin,
                        const void* q_weight, const void* k_weight, float eps, cudaStream_t s) {
   if (rows <= 0 || dim % 16 || rot_dim > dim || rot_dim % 2 || ldqkv % 8) return FF_HOST_BAD_SHAPE;
-  const int R = rows >= 4 * 4 * 148 && rot_dim <= 1024 ? 4 : 1;
+  int R = rows >= 4 * 4 * 148 ? 4 : 1;
+  const int pairs = (hq + 2 * hkv) * (dim / 16);
+  while (R < 4 && R * pairs < ROPE_THREADS && rows >= 2 * R * 148) R *= 2;
+  while (R >= 4 && 2 * R * pairs <= 64 && rows >= 2 * R * 296) R *= 2;
+  if (rot_dim > 1024) R = 1;
   const size_t smem = (size_t)R * (rot_dim / 2) * sizeof(float2);
   auto kern = q_weight ? rope_kv_paged_kernel<true> : rope_kv_paged_kernel<false>;
   if (smem > 48 * 1024)

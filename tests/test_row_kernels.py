@@ -13,8 +13,8 @@ def _packed(rows, heads, dim, seed):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows", [1, 7, 2368, 2371])          # one row per CTA, the first size with four, a ragged last CTA
-@pytest.mark.parametrize("hq,hkv,dim,rot", [(4, 1, 128, 128), (64, 4, 128, 128), (3, 2, 128, 64), (5, 1, 64, 64), (2, 2, 48, 32)])
+@pytest.mark.parametrize("rows", [1, 7, 299, 600, 2368, 2371, 4741])  # one row per CTA, two and four for few heads, four, ragged ones, more for one head
+@pytest.mark.parametrize("hq,hkv,dim,rot", [(4, 1, 128, 128), (64, 4, 128, 128), (3, 2, 128, 64), (5, 1, 64, 64), (2, 2, 48, 32), (1, 1, 16, 16)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_rotation_norm_and_cache_write(rows, hq, hkv, dim, rot, norm):
     """Rotation and cache write are the oracle's bits; with head norms the sums of squares meet in another order, which moves a normed
