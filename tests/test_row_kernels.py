@@ -12,34 +12,67 @@ def _packed(rows, heads, dim, seed):
     return torch.randn(rows, heads * dim, generator=g).to(BF16)
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("rows", [1, 7, 299, 600, 2368, 2371, 4741])  # one row per CTA, two and four for few heads, four, ragged ones, more for one head
-@pytest.mark.parametrize("hq,hkv,dim,rot", [(4, 1, 128, 128), (64, 4, 128, 128), (3, 2, 128, 64), (5, 1, 64, 64), (2, 2, 48, 32), (1, 1, 16, 16)])
-@pytest.mark.parametrize("norm", [False, True])
-def test_rotation_norm_and_cache_write(rows, hq, hkv, dim, rot, norm):
-    """Rotation and cache write are the oracle's bits; with head norms the sums of squares meet in another order, which moves a normed
-    value by at most its last bit (2^-8 relative) before it is turned."""
-    from flyingfish_b200 import ops
-    qkv = _packed(rows, hq + 2 * hkv, dim, rows + dim)
-    g = torch.Generator().manual_seed(1)
+def _batch(rows, hq, hkv, dim):
+    g = torch.Generator().manual_seed(rows + dim)
     nb = (rows + 63) // 64 + 1
     slots = torch.randperm(nb * 64, generator=g)[:rows].to(torch.int32)
     slots[rows // 2] = -1 if rows > 1 else slots[0]
     pos = torch.randint(0, 9000, (rows,), generator=g).to(torch.int32)
-    w = [(1 + 0.1 * torch.randn(dim, generator=g)).to(BF16) for _ in range(2)]
-    kw = dict(q_norm=w[0], k_norm=w[1], eps=1e-6) if norm else {}
-    want = [qkv.clone(), torch.zeros(nb, hkv, 64, dim, dtype=BF16), torch.zeros(nb, hkv, 64, dim, dtype=BF16)]
-    ops.rope_kv_paged(want[0], pos, slots, want[1], want[2], hq, hkv, dim, 1e6, rot, **kw)       # CPU oracle
-    got = [qkv.cuda(), torch.zeros_like(want[1]).cuda(), torch.zeros_like(want[2]).cuda()]
-    ops.rope_kv_paged(got[0], pos.cuda(), slots.cuda(), got[1], got[2], hq, hkv, dim, 1e6, rot, **{k: v.cuda() if k != "eps" else v for k, v in kw.items()})
+    return _packed(rows, hq + 2 * hkv, dim, rows + dim), pos, slots, [torch.zeros(nb, hkv, 64, dim, dtype=BF16) for _ in range(2)]
+
+
+ROWS = [1, 7, 299, 600, 2368, 2371, 4741]   # one row per CTA, two and four for few heads, the first size with four for all, ragged ones, more for one head
+HEADS = [(4, 1, 128, 128), (64, 4, 128, 128), (3, 2, 128, 64), (5, 1, 64, 64), (2, 2, 48, 32), (1, 1, 16, 16)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", ROWS)
+@pytest.mark.parametrize("hq,hkv,dim,rot", HEADS)
+def test_rotation_and_cache_write(rows, hq, hkv, dim, rot):
+    """With the angles given, rotation and cache write are the oracle's bits; the kernel that makes the angles itself turns by those of the
+    table kernel, which differ from the host's by a last bit of BF16 (and by what FP32 gives an angle of up to 9000)."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import vision_ops
+    qkv, pos, slots, caches = _batch(rows, hq, hkv, dim)
+    table = ops.rope_table(pos, rot, 1e6)
+    want, got = [[qkv.to(d), *(c.to(d) for c in caches)] for d in ("cpu", "cuda")]
+    vision_ops.rope_table_apply_(want[0], table, hq, dim, rot, slots, want[1], want[2], hkv)
+    vision_ops.rope_table_apply_(got[0], table.cuda(), hq, dim, rot, slots.cuda(), got[1], got[2], hkv)
+    assert all(torch.equal(a.cpu(), b) for a, b in zip(got, want))
+    own, by_table = [[qkv.cuda(), *(c.cuda() for c in caches)] for _ in range(2)]
+    angles = ops.rope_table(pos.cuda(), rot, 1e6)
+    ops.rope_kv_paged(own[0], pos.cuda(), slots.cuda(), own[1], own[2], hq, hkv, dim, 1e6, rot)
+    vision_ops.rope_table_apply_(by_table[0], angles, hq, dim, rot, slots.cuda(), by_table[1], by_table[2], hkv)
+    assert all(torch.equal(a, b) for a, b in zip(own, by_table))
+    assert (angles.cpu() - table).abs().max() <= 2.0 ** -8 + 9000 * 2.0 ** -22
     torch.cuda.synchronize()
     ops.check_status()
-    for a, b in zip(got, want):
-        a, b = a.cpu().float(), b.float()
-        # sine and cosine may differ by a last bit of BF16 between the host's and the device's functions: an absolute 2^-7 of the
-        # largest element of the pair, as the rotation's own test allows
-        assert ((a - b).abs() <= 2e-2 + 2e-2 * b.abs()).all()
-    assert torch.equal(got[2].cpu(), want[2])                                                   # values are copies
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", ROWS)
+@pytest.mark.parametrize("hq,hkv,dim,rot", HEADS)
+def test_head_norms_before_the_rotation(rows, hq, hkv, dim, rot):
+    """At position 0 what is left is the norm: the oracle's up to its last bit (2^-7 of a value at most), since the sums of squares meet in
+    another order. Elsewhere the pass gives the bits of that norm followed by the plain rotation."""
+    from flyingfish_b200 import ops
+    qkv, pos, slots, caches = _batch(rows, hq, hkv, dim)
+    g = torch.Generator().manual_seed(1)
+    w = [(1 + 0.1 * torch.randn(dim, generator=g)).to(BF16) for _ in range(2)]
+    kw = dict(q_norm=w[0].cuda(), k_norm=w[1].cuda(), eps=1e-6)
+
+    def turned(x, positions, **norms):
+        out = [x.cuda(), *(c.cuda() for c in caches)]
+        ops.rope_kv_paged(out[0], positions.cuda(), slots.cuda(), out[1], out[2], hq, hkv, dim, 1e6, rot, **norms)
+        return out
+    normed = turned(qkv, torch.zeros_like(pos), **kw)[0].cpu()
+    heads = qkv.view(rows, -1, dim)
+    want = torch.cat([ref.rmsnorm(heads[:, :hq], w[0], 1e-6), ref.rmsnorm(heads[:, hq: hq + hkv], w[1], 1e-6)], 1).view(rows, -1).float()
+    assert ((normed[:, : want.shape[1]].float() - want).abs() <= 2.0 ** -7 * want.abs()).all()
+    assert torch.equal(normed[:, want.shape[1]:], qkv[:, want.shape[1]:])                        # values are copies
+    assert all(torch.equal(a, b) for a, b in zip(turned(qkv, pos, **kw), turned(normed, pos)))
+    torch.cuda.synchronize()
+    ops.check_status()
 
 
 def _mla_batch(q_lens, pasts, seed):
@@ -60,7 +93,7 @@ def _mla_batch(q_lens, pasts, seed):
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows", [1, 3, 200])
 def test_latent_row_step_equals_its_operators(rows):
-    """The fused step gives the bits of rotation and cache write, and the norm's up to its order of additions."""
+    """The fused step gives the bits of the rotation kernel and the cache write, and the norm's up to its order of additions."""
     from flyingfish_b200 import ops
     from flyingfish_b200.ops import mla_ops
     heads, nope = 5, 128
@@ -68,12 +101,12 @@ def test_latent_row_step_equals_its_operators(rows):
     q, kva = torch.randn(rows, heads * (nope + 64), generator=g).to(BF16), torch.randn(rows, 576, generator=g).to(BF16)
     w = (1 + 0.1 * torch.randn(512, generator=g)).to(BF16)
     slots[rows // 2] = -1 if rows > 1 else slots[0]
-    q_rope = q.view(rows, heads, -1)[:, :, nope:].reshape(rows, -1).clone()
-    k_rope = kva[:, 512:].clone()
-    ops.rope_inplace(q_rope, pos, heads, 64, 1e4)
-    ops.rope_inplace(k_rope, pos, 1, 64, 1e4)
+    q_rope = q.view(rows, heads, -1)[:, :, nope:].reshape(rows, -1).cuda()
+    k_rope = kva[:, 512:].cuda()
+    ops.rope_inplace(q_rope, pos.cuda(), heads, 64, 1e4)
+    ops.rope_inplace(k_rope, pos.cuda(), 1, 64, 1e4)
     want = torch.zeros(blocks, 1, 64, 576, dtype=BF16)
-    mla_ops.cache_write(ops.rmsnorm(kva[:, :512], w, 1e-6), k_rope, slots, want)
+    mla_ops.cache_write(ops.rmsnorm(kva[:, :512], w, 1e-6), k_rope.cpu(), slots, want)
     for full in (False, True):
         qd, cache = q.cuda(), torch.zeros_like(want).cuda()
         q_full = torch.zeros(rows, heads, 576, dtype=BF16, device="cuda") if full else None
@@ -81,8 +114,11 @@ def test_latent_row_step_equals_its_operators(rows):
         torch.cuda.synchronize()
         ops.check_status()
         got = q_full[:, :, 512:] if full else qd.view(rows, heads, -1)[:, :, nope:]
-        for a, b in ((got.reshape(rows, -1), q_rope), (cache, want)):
-            assert ((a.cpu().float() - b.float()).abs() <= 2e-2 + 2e-2 * b.float().abs()).all()
+        assert torch.equal(got.reshape(rows, -1), q_rope)
+        cache = cache.cpu()
+        assert torch.equal(cache[..., 512:], want[..., 512:])
+        a, b = cache[..., :512].float(), want[..., :512].float()
+        assert ((a - b).abs() <= 2.0 ** -7 * b.abs()).all()                                     # one last bit
         assert torch.equal(qd.view(rows, heads, -1)[:, :, :nope].cpu(), q.view(rows, heads, -1)[:, :, :nope])
 
 
