@@ -21,7 +21,7 @@ from .decoder import DecoderModel
 from .weights import LayerWeights, ModelWeights, TPInfo, build_decoder_weights
 
 
-EXPAND_MAX_BYTES = 2 << 30       # most memory that a layer's expanded keys and values take
+EXPAND_MAX_BYTES = 2 << 30       # most memory that a layer's expanded keys and values take (out of the planner's reserve)
 # A step's portions are expanded from this many query rows per visible key on (a portion's rows, weighted by its context). The expansion costs
 # by the key, the latent space by the row and key. One layer at the published widths, latent space against expanded: 64 rows in front of 16,000
 # tokens 1748 / 855 us, 23 rows per key 553 / 622, 10 rows 634 / 1314, a portion of 64 rows beside fifteen of 8 rows behind 2000 tokens 612 / 1612.

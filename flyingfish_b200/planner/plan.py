@@ -107,7 +107,7 @@ def plan_memory(spec: ModelSpec, settings: Settings, info: DeviceInfo, weights_b
     budget = total
     if settings.device_budget_gib is not None:
         budget = min(total, int(settings.device_budget_gib * (1 << 30)))
-    reserve = total // 16
+    reserve = total // 16              # among it what a step takes beyond its rows: expanded keys and values of latent attention
     free_after_weights = min(info.free_bytes, budget - weights_bytes) - reserve
     if free_after_weights <= 0:
         raise PlanError(f"model weights ({weights_bytes >> 20} MiB) leave no room inside the budget "

@@ -89,3 +89,26 @@ def test_plan_memory_refuses_when_too_small():
     p_full = plan_memory(spec8, Settings(capacity=4096, max_batch=256), big, 16 << 30)
     p_small = plan_memory(spec8, Settings(capacity=4096, max_batch=256, device_budget_gib=40), big, 16 << 30)
     assert p_small.kv_blocks < p_full.kv_blocks
+
+
+@pytest.mark.parametrize("past,new", [(0, 1), (0, 64), (0, 300), (63, 1), (63, 2), (64, 128), (70, 257)])
+def test_slots_as_an_array_are_those_of_the_list(past, new):
+    slots = []
+    for span in (False, True):
+        kv = PagedKVCache(1, 1, 16, 40, 64, torch.float32, torch.device("cpu"))
+        for other in (0, 1):                                     # pages of two sequences between one another
+            kv.add_sequence(other)
+        for _ in range(past):
+            for other in (0, 1):
+                kv.reserve(other, 1); kv.commit(other, 1)
+        slots.append(list(kv.reserve_span(1, new)) if span else kv.reserve(1, new))
+    assert slots[0] == slots[1]
+
+
+def test_the_reserve_holds_what_latent_attention_expands():
+    from flyingfish_b200.models.deepseek import EXPAND_MAX_BYTES
+    from flyingfish_b200.ops.mla_ops import EXPAND_MAX_KEYS
+    latents = EXPAND_MAX_KEYS * 512 * 2                          # gathered rows in front of the expansion
+    spec, gib = named_shape("deepseek-v3-shape"), 1 << 30
+    p = plan_memory(spec, Settings(capacity=1024, max_batch=8), DeviceInfo(total_bytes=180 * gib, free_bytes=179 * gib), 100 * gib)
+    assert p.reserve_bytes >= 2 * (EXPAND_MAX_BYTES + latents)
