@@ -158,8 +158,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
     ``csrc/gemm_f32.cu`` (true 32-bit products).
 
     CUDA path: tcgen05 kernels -- the weight-streaming decode kernel of ``csrc/gemm_skinny.cu`` (tokens on
-    the UMMA M side, cluster split-K or stream-K) for M <= 128, the persistent 128x256x64 kernel of
-    ``csrc/gemm_bf16.cu`` otherwise. ``w`` may be an FP8-resident weight (``quant_ops.Fp8Weight``): the block-scaled
+    the UMMA M side, cluster split-K or stream-K) for M <= 128, the persistent kernels of ``csrc/gemm_bf16.cu`` otherwise
+    (256-row tiles by CTA pairs, or 128-row tiles of one CTA where those fill fewer waves). ``w`` may be an FP8-resident weight (``quant_ops.Fp8Weight``): the block-scaled
     W8A8 GEMM of ``csrc/gemm_fp8.cu`` (CPU: its oracle) runs instead."""
     if not isinstance(w, torch.Tensor):
         _require(bias is None and act is None and mul is None, "linear: FP8-resident weights take no bias or activation")

@@ -226,8 +226,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         const uint32_t lane_base = tmem_base + (uint32_t(q * 32) << 16) + blk0 * 16;
         const uint32_t taddr[2] = {lane_base + b0 * buf_cols, 0};
         const float* const sp[2] = {sXs + kb * ntok + blk0 * 16, nullptr};
-        // (promoting two k-blocks per round was measured: the extra registers spill under the 168-register cap of a
-        // ten-warp CTA and the kernel gets slower)
+        // (promoting two k-blocks per round was measured with chunks of 128: the extra registers spill under the 168-register cap
+        // of its ten warps and the kernel gets slower; chunks of 32 and 64 share an SM and have about 100)
         fp8_promote<TOK / 32, 1, 0, TOK / 2>(acc, taddr, sp, nb);
         tc_fence_before();
         __syncwarp();

@@ -747,9 +747,11 @@ static SkinnyConfig skinny_config(int M, int N, int K, int epi = 0) {
   // stages cannot turn a k-block around faster than the ~1.5 us load latency / st, and all CTAs together cannot beat HBM (~5.9 TB/s on
   // reads). On top of the larger of these come 0.08 us per k-block of a CTA (waits and commits), for a cluster 18 ns per row of its tile
   // (partials of 64 tokens pushed and summed), for stream-K 8 us (partial tiles through global memory). Clusters of two, four
-  // and eight come first: of three or six CTAs they lose in a chain of kernels what they gain alone. Decode steps of the 8-layer 8B-sized stack with 1, 7, 64,
-  // 113 sequences: 1048, 1177, 1677, 1819 us with stream-K for 6144 x 4096 and clusters of six for 4096 x 4096 and 4096 x 14336, 1043, 1184,
-  // 1619, 1615 us with clusters of two and four.
+  // and eight come first: of three or six CTAs they lose in a chain of kernels what they gain alone. The captured decode step of the 8-layer
+  // 8B-sized stack, replayed back to back with 1, 7, 64, 113 sequences (a call adds its host work, 105 to 344 us): 1048, 1177, 1677, 1819 us with
+  // stream-K for 6144 x 4096 and clusters of six for 4096 x 4096 and 4096 x 14336, 1043, 1184, 1619, 1615 us with clusters of two and four.
+  // Alone, back to back, some products are slower so (8192 x 8192, one token: 23 -> 26 us); captured steps of no stack tried were, against the
+  // former choice, issue loop and merge together: 70B-sized layers 0.88 to 0.91 of the time from 1 to 128 sequences, five others 0.81 to 0.98.
   // The choice must not depend on M: the K split fixes the order of the FP32 additions, and a
   // row's bits may not change with the batch it is computed in. So the model assumes 64 tokens and
   // the receive buffer is sized for those 64 (more tokens get the larger shared-memory budget and the same split).

@@ -1,7 +1,7 @@
-"""Multi-head latent attention operators: latent cache write, absorbed attention over the paged
-latent cache, per-head batched projections. CUDA: ``csrc/mla.cu`` (+ the grouped tcgen05 GEMM for the
-per-head W_UK / W_UV products); CPU: FP32 oracles. :func:`latent_norm_kv` and :func:`latent_attention` are the forms for any
-widths, windows and 32-bit, with ``ops.head_linear`` for the per-head products."""
+"""Multi-head latent attention operators: the step between projections and attention (norm, rotations, latent cache write), absorbed
+attention over the paged latent cache, attention of prompts over expanded keys and values. CUDA: ``csrc/mla.cu``, ``csrc/attention_tc.cu``,
+``ops.head_linear`` for the per-head products (:func:`per_head_linear`, over the grouped GEMM, for head-major operands); CPU: FP32 oracles.
+:func:`latent_norm_kv` and :func:`latent_attention` are the forms for any widths, windows and 32-bit."""
 from __future__ import annotations
 
 import ctypes

@@ -225,7 +225,7 @@ def _rudorax_table(spec: ModelSpec, rows: int, ctx: int, iters: int, device) -> 
     for name, n, k in (("qkv projection", nq, W), ("output projection", W, H * d)):
         w, r = rn(n, k), x if k == W else rn(rows, k)
         pair(name, lambda: ops.linear(r, w), pair.gemm(n, k), name, lambda: ops.linear(r, w), pair.gemm(n, k))
-    # head norm + rotation + cache write against the two norms, the rotation and the cache write of the like layer
+    # head norm + rotation + cache write against those of the like layer
     batch = rows if decode else rows // ctx
     pg = _Paged(batch, ctx, G, d, dev)
     slots, pos = i32(torch.randperm(pg.k.shape[0] * 64, device=dev)[:rows]), i32(torch.arange(rows, device=dev)) % ctx
@@ -235,10 +235,7 @@ def _rudorax_table(spec: ModelSpec, rows: int, ctx: int, iters: int, device) -> 
     table = ops.rope_angles(pos, fr, amp)
 
     def like_norm_rope():
-        q, k = qkv[:, : H * d].reshape(rows * H, d), qkv[:, H * d: (H + G) * d].reshape(rows * G, d)
-        qkv[:, : H * d] = ops.rmsnorm(q.contiguous(), qn, 1e-5).view(rows, -1)
-        qkv[:, H * d: (H + G) * d] = ops.rmsnorm(k.contiguous(), kn, 1e-5).view(rows, -1)
-        ops.rope_kv_paged(qkv, pos, slots, pg.k, pg.v, H, G, d, 1e4)
+        ops.rope_kv_paged(qkv, pos, slots, pg.k, pg.v, H, G, d, 1e4, q_norm=qn, k_norm=kn, eps=1e-5)
     byts = 2 * rows * d * (2 * H + 2 * G + 2 * G)
     qnf, knf = qn.float(), kn.float()
     pair("head norm + rotation + cache write", lambda: ops.head_norm_kv(qkv, slots, pg.k, pg.v, H, G, d, d, 1e-5, q_weight=qnf, k_weight=knf, cos_sin=table),
@@ -387,10 +384,7 @@ def _kabavik_table(spec: ModelSpec, rows: int, ctx: int, iters: int, device) -> 
     table = ops.rope_angles(pos, ops.rope_frequencies(freqs, dev), amp)
 
     def like_norm_rope():
-        q, k = qkv[:, : H * d].reshape(rows * H, d), qkv[:, H * d: (H + G) * d].reshape(rows * G, d)
-        qkv[:, : H * d] = ops.rmsnorm(q.contiguous(), qn, 1e-5).view(rows, -1)
-        qkv[:, H * d: (H + G) * d] = ops.rmsnorm(k.contiguous(), kn, 1e-5).view(rows, -1)
-        ops.rope_kv_paged(qkv, pos, slots, pg.k, pg.v, H, G, d, 1e4)
+        ops.rope_kv_paged(qkv, pos, slots, pg.k, pg.v, H, G, d, 1e4, q_norm=qn, k_norm=kn, eps=1e-5)
     byts = (2 * rows * d * (2 * H + 4 * G), 0)
     pair("row norms, rotation + cache write", lambda: ops.head_norm_kv(qkv, slots, pg.k, pg.v, H, G, d, d, 1e-5, q_weight=wq, k_weight=wk, cos_sin=table,
          whole=True, halves=True), byts, "head norms, rotation + cache write", like_norm_rope, byts)
@@ -427,41 +421,35 @@ def _kabavik_table(spec: ModelSpec, rows: int, ctx: int, iters: int, device) -> 
     rot, at0 = H * d, H * (d + T)
     byts = (2 * rows * (2 * H * T + 2 * (R + T)), 0)
 
-    def like_latent():
-        c = ops.rmsnorm(p[:, at0: at0 + R].contiguous(), w16[:R].contiguous(), 1e-5)
-        kr, qr = p[:, at0 + R: at0 + R + T].contiguous(), p[:, rot: at0].contiguous()
-        ops.rope_inplace(qr, pos, H, T, 1e4)
-        ops.rope_inplace(kr, pos, 1, T, 1e4)
-        mla_ops.cache_write(c, kr, slots, lg.k)
+    packed, kva = rn(rows, H * (d + T)), rn(rows, R + T)            # the like layer's query heads and latent rows
+    like_latent = lambda: mla_ops.norm_rope_cache(packed, kva, w16[:R], pos, slots, lg.k, H, d, 1e4, 1e-5, q if decode else None)
     pair("latent norm, rotations + cache write", lambda: mla_ops.latent_norm_kv(p, slots, lg.k, q, rot, at0, R, R, wn, ltab, 1e-5), byts,
          "norm, rotations, cache write", like_latent, byts)
     uk, uv, out = rn(H, R, d), rn(H, d, R), rn(rows, H * R)
     per_head = lambda a, b: (2 * (rows * H * (a + b) + H * a * b), 2 * rows * H * a * b)
     xq = p[:, :rot]
     pair("queries into the latent space", lambda: ops.head_linear(xq, uk, out=q.view(rows, -1), out_cols=R + T), per_head(d, R), "per-head projection",
-         lambda: mla_ops.per_head_linear(xq.reshape(rows, H, d), uk), per_head(d, R))
+         lambda: ops.head_linear(packed, uk, out=q.view(rows, -1), x_cols=d + T, out_cols=R + T), per_head(d, R))
     pair("results out of the latent space", lambda: ops.head_linear(out, uv), per_head(R, d), "per-head projection",
-         lambda: mla_ops.per_head_linear(out.view(rows, H, R), uv), per_head(R, d))
+         lambda: ops.head_linear(out, uv), per_head(R, d))
     q.normal_()
     gate = p[:, at0 + R + T: at0 + R + T + H]
     unbound = dataclasses.replace(lat, window=0)
     lc = lambda l: cost(l, R + T, seen(l), 2 * R + T, 2 * R + T)
-    like = lambda: mla_ops.attention(q, lg.k, lg.table, qs, ql, lg.ctx, rows // batch, ctx, lat.scale, R)
     if decode:
         pair("latent attention, window, gated", lambda: mla_ops.latent_attention(q, lg.k, lg.table, qs, ql, lg.ctx, 1, ctx, lat.scale, R, lat.window, gate, out,
-             decode=True), lc(lat), "latent attention, full", like, lc(unbound))
-    else:       # prompts: expansion and attention here, the latent space there; the cost is that of the expanded form for both
-        def like_latent_attention():
-            mla_ops.per_head_linear(xq.reshape(rows, H, d), uk)
-            mla_ops.per_head_linear(like(), uv)
-        pages = mla_ops.KeyPages.of([ctx] * batch, [ctx] * batch, lg.table.cpu(), lat.window, 64, dev)
+             decode=True), lc(lat), "latent attention, full",
+             lambda: mla_ops.attention(q, lg.k, lg.table, qs, ql, lg.ctx, rows // batch, ctx, lat.scale, R), lc(unbound))
+    else:       # prompts: both layers expand the latents that their rows see
+        seen_pages = lambda window: mla_ops.KeyPages.of([ctx] * batch, [ctx] * batch, lg.table.cpu(), window, 64, dev)
+        pages, every = seen_pages(lat.window), seen_pages(0)
         w_kv, res = rn(H * 2 * d, R), rn(rows, H * d)
         expansion, ec = pair.gemm(H * 2 * d, R), lambda l: cost(l, R + T, seen(l), 2 * d + T, 2 * d + T)
         add = lambda a, b: (a[0] + b[0], a[1] + b[1])
         pair("latents expanded, attention, window, gated", lambda: mla_ops.expanded_attention(xq, q, lg.k, w_kv, pages, lg.table, qs, ql, lg.ctx, ctx, d, d, R,
-             lat.scale, lat.window, gate, res), add(expansion, ec(lat)), "queries to latents, attention, results out of latents",
-             like_latent_attention,
-             add(expansion, ec(unbound)))
+             lat.scale, lat.window, gate, res), add(expansion, ec(lat)), "latents expanded, attention, full",
+             lambda: mla_ops.expanded_attention(packed, packed.view(rows, H, -1), lg.k, w_kv, every, lg.table, qs, ql, lg.ctx, ctx, d, d, R, lat.scale, 0,
+             None, res), add(expansion, ec(unbound)))
     if decode:
         wv = rn(spec.vocab, W)
         pair("logits, 32-bit", lambda: ops.linear(x, wv, out_dtype=f32), pair.gemm(spec.vocab, W, out_bytes=4), "logits", lambda: ops.linear(x, wv),
