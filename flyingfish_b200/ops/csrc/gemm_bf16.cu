@@ -138,17 +138,18 @@ struct LinTail {
 constexpr int RS_STG_PITCH = 144, RS_STG_BYTES = 32 * RS_STG_PITCH;   // COMM 2 epilogue staging, per warp
 constexpr int COMM_PARTS = 4;       // a 128-row block is pushed (COMM 1) / reduced (COMM 2) in this many pieces
 
-// An epilogue thread's row of a finished tile: tensor memory -> registers -> global. row: row of the result, stored where `live`; tn: column
-// tile, N: columns (of the head), col_off: first column of the head.
-template <int BN>
-__device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict__ Cout, int row, bool live, int ldc, int N, int epi, int tn,
-                                               size_t col_off, const LinTail& tail) {
+// An epilogue thread's row of a finished tile: tensor memory -> registers -> global. row: row of the result, stored where `live`; col0: first
+// of the tile's `width` columns (a multiple of 32, of 128 with epi 1), N: columns (of the head), col_off: first column of the head. The PARTS
+// warps that share the row take turns with its groups of columns.
+template <int PARTS>
+__device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict__ Cout, int row, bool live, int ldc, int N, int epi, int col0,
+                                               int width, size_t col_off, const LinTail& tail, int part) {
   if (epi == 1) {
-    constexpr int HALF = BN / 2;
-    __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + (size_t)tn * HALF;
+    const int half = width / 2, out0 = col0 / 2;
+    __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + out0;
     const int ncols_out = N / 2;
 #pragma unroll 1
-    for (int c = 0; c < HALF; c += 16) {
+    for (int c = 16 * part; c < half; c += 16 * PARTS) {
       uint32_t g[16], u[16];
       const int gc = (c >> 6) * 128 + (c & 63);      // 64 gate columns, then the matching 64 up columns
       tmem_ld_x16(taddr + gc, g);
@@ -169,13 +170,13 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
           o[j] = pack_bf16x2(a0 * __bfloat162float(__float2bfloat16(u0)),
                              a1 * __bfloat162float(__float2bfloat16(u1)));
         }
-        if (tn * HALF + c + 16 <= ncols_out) {
+        if (out0 + c + 16 <= ncols_out) {
           uint4* dst = reinterpret_cast<uint4*>(crow + c);
           dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
           dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
         } else {
           for (int j = 0; j < 16; ++j)
-            if (tn * HALF + c + j < ncols_out) {
+            if (out0 + c + j < ncols_out) {
               const uint32_t w = o[j >> 1];
               reinterpret_cast<uint16_t*>(crow + c)[j] = (j & 1) ? uint16_t(w >> 16) : uint16_t(w & 0xffff);
             }
@@ -183,31 +184,31 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
       }
     }
   } else if (epi == 2) {
-    float* crow = reinterpret_cast<float*>(Cout) + (size_t)row * ldc + (size_t)tn * BN;
+    float* crow = reinterpret_cast<float*>(Cout) + (size_t)row * ldc + col0;
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 16) {
+    for (int c = 16 * part; c < width; c += 16 * PARTS) {
       uint32_t r[16];
       tmem_ld_x16(taddr + c, r);
       tmem_ld_wait();
       if (live) {
-        if (tn * BN + c + 16 <= N) {
+        if (col0 + c + 16 <= N) {
           uint4* dst = reinterpret_cast<uint4*>(crow + c);
 #pragma unroll
           for (int j = 0; j < 4; ++j) dst[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         } else {
-          for (int j = 0; j < 16; ++j) if (tn * BN + c + j < N) crow[c + j] = __uint_as_float(r[j]);
+          for (int j = 0; j < 16; ++j) if (col0 + c + j < N) crow[c + j] = __uint_as_float(r[j]);
         }
       }
     }
   } else {
-    __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + col_off + (size_t)tn * BN;
+    __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + col_off + col0;
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 32) {
+    for (int c = 32 * part; c < width; c += 32 * PARTS) {
       uint32_t r[32];
       tmem_ld_x32(taddr + c, r);
       tmem_ld_wait();
       if (tail.bias != nullptr) {
-        const int col = tn * BN + c;
+        const int col = col0 + c;
         if (col + 32 <= N) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -237,7 +238,7 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
       if (tail.mul != nullptr && live) {
         int mr = tail.mul_rows[row];
         if (mr < 0 || mr >= tail.mul_table) mr = 0;          // reported where the id is first read (embedding)
-        const int col = tn * BN + c;
+        const int col = col0 + c;
         const __nv_bfloat16* f = tail.mul + (size_t)mr * tail.ldm + col;
         if (col + 32 <= N) {
 #pragma unroll
@@ -258,7 +259,7 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
         }
       }
       if (live) {
-        if (tn * BN + c + 32 <= N) {
+        if (col0 + c + 32 <= N) {
           uint4* dst = reinterpret_cast<uint4*>(crow + c);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -269,7 +270,7 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
           }
         } else {
           for (int j = 0; j < 32; ++j)
-            if (tn * BN + c + j < N) crow[c + j] = __float2bfloat16(__uint_as_float(r[j]));
+            if (col0 + c + j < N) crow[c + j] = __float2bfloat16(__uint_as_float(r[j]));
         }
       }
     }
@@ -277,7 +278,7 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
 }
 
 template <int BN, int STAGES, int COMM>
-__global__ void __launch_bounds__(COMM == 1 ? 320 : 192, 1)
+__global__ void __launch_bounds__(COMM == 2 ? 192 : 320, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA1,
                  const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmB, void* __restrict__ Cout, int M, int N, int K, int ldc, int epi,
                  int* status, CommArgs ca, GroupArgs ga, LinTail tail) {
@@ -298,7 +299,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars.tmem_full[i], 1); mbar_init(&bars.tmem_empty[i], 4); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars.tmem_full[i], 1); mbar_init(&bars.tmem_empty[i], COMM ? 4 : 8); }
     bars.abort_flag = 0; bars.is_last = 0;
     mbar_fence_init();
   }
@@ -369,8 +370,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (ok) umma_commit(&bars.tmem_full[acc]);
       }
     }
-  } else if (warp < 6) {
-    // epilogue warps 2..5 ; TMEM lane quarter = warp % 4
+  } else if (warp < (COMM ? 6 : 10)) {
+    // epilogue warps 2..5, without communication 2..9 in two per quarter; TMEM lane quarter = warp % 4
     const int q = warp & 3;
     const int e = (warp - 2) * 32 + lane;
     uint32_t tile_it = 0;
@@ -426,7 +427,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tma_store_wait<0>();                              // every row of this tile has landed in the owner's slot
           asm volatile("fence.proxy.async;" ::: "memory");
       } else {
-        store_tile_row<BN>(taddr, Cout, row, row < row_end, ldc, N, epi, tn, (size_t)head * ga.c_cols, tail);
+        store_tile_row<COMM ? 1 : 2>(taddr, Cout, row, row < row_end, ldc, N, epi, tn * BN, BN, (size_t)head * ga.c_cols, tail, COMM ? 0 : (warp - 2) >> 2);
       }
       tc_fence_before();
       __syncwarp();
@@ -567,33 +568,48 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // commits free the stages of both. Persistent, two accumulators in tensor memory, so the epilogue of a tile runs under the next one's
 // main loop. Prefill of 8121 rows of an 8-layer 8B-sized stack 28.3 -> 26.4 ms, of 8191 rows 33.3 -> 30.7 ms; at these sizes the GPU's power
 // limit holds both forms near 1.4 PFLOP/s inside the products, and the pair form reaches it with less traffic.
+constexpr int PAIR_STAGES = 11;                      // most stages of a ring
+constexpr int PAIR_RING = 224 * 1024;                // its bytes
 struct alignas(8) PairBars {
-  uint64_t full[8];             // the even CTA's: both CTAs' loads of a stage have landed
-  uint64_t empty[8];            // each CTA's own, freed by the even CTA's commits
+  uint64_t full[PAIR_STAGES];   // the even CTA's: both CTAs' loads of a stage have landed
+  uint64_t empty[PAIR_STAGES];  // each CTA's own, freed by the even CTA's commits
   uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];       // the even CTA's: the eight epilogue warps of the pair have read the accumulator
+  uint64_t tmem_empty[2];       // the even CTA's: the sixteen epilogue warps of the pair have read the accumulator
   uint32_t tmem_base;
   int abort_flag;
 };
 
-template <int BN, int STAGES>
-__global__ void __launch_bounds__(192, 1)
-gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, void* __restrict__ Cout, int M, int N,
-                      int K, int ldc, int epi, int* status, LinTail tail) {
+// A ring as deep as shared memory takes (7 stages 256 wide, 11 stages 64 wide: 200 rows times 4096 x 14336 50.6 -> 40.0 us) and two epilogue warps
+// per 32 rows, since the last tile's epilogue is not hidden: 130 x 4096 x 4096 17.5 -> 16.1 us.
+// Tiles of a launch: `wide` columns of tiles w1 wide, then tiles w2 wide up to N; every width a multiple of 32 (of 128 with epi 1), at most 256.
+struct PairTiles { int w1, wide, w2; };
+
+// tile t: row tile, first column and width. The wide tiles come first, the narrow ones fill the last wave.
+__device__ __forceinline__ void pair_tile(const PairTiles& pt, int t, int tiles_m, int tiles_n2, int& tm, int& col0, int& width) {
+  const int n1 = pt.wide * tiles_m;
+  int tn;
+  if (t < n1) { tile_coords(t, tiles_m, pt.wide, tm, tn); col0 = tn * pt.w1; width = pt.w1; }
+  else { tile_coords(t - n1, tiles_m, tiles_n2, tm, tn); col0 = pt.wide * pt.w1 + tn * pt.w2; width = pt.w2; }
+}
+
+__global__ void __launch_bounds__(320, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2,
+                      void* __restrict__ Cout, int M, int N, int K, int ldc, int epi, const PairTiles pt, int stages, int* status, LinTail tail) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ PairBars bars;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN / 2 * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+  constexpr int A_BYTES = BM * BK * 2;
+  const int stage_bytes = A_BYTES + (pt.wide ? pt.w1 : pt.w2) * BK;                          // half of B's rows per CTA
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
-  const int tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (N + BN - 1) / BN, tiles = tiles_m * tiles_n;
+  const int tiles_m = (M + 2 * BM - 1) / (2 * BM), rest = N - pt.wide * pt.w1, tiles_n2 = rest > 0 ? (rest + pt.w2 - 1) / pt.w2 : 0, tiles = tiles_m * (pt.wide + tiles_n2);
   const int kblocks = (K + BK - 1) / BK;
   const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB);
-    for (int i = 0; i < STAGES; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars.tmem_full[i], 1); mbar_init(&bars.tmem_empty[i], 8); }
+    tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB1); tma_prefetch_desc(&tmB2);
+    for (int i = 0; i < stages; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars.tmem_full[i], 1); mbar_init(&bars.tmem_empty[i], 16); }
     bars.abort_flag = 0;
     mbar_fence_init();
   }
@@ -612,41 +628,46 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   if (warp == 0) {
     if (elect_one()) {
       uint32_t it = 0;
+      RingPos rp;
       bool ok = true;
       for (int t = first; t < tiles && ok; t += step) {
-        int tm, tn;
-        tile_coords(t, tiles_m, tiles_n, tm, tn);
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % STAGES; const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&bars.empty[s], ph ^ 1, abort_flag, status, KID_GEMM_BF16, 5)) { ok = false; break; }
-          if (rank == 0) mbar_expect_tx(&bars.full[s], 2 * STAGE_BYTES);
-          uint8_t* sa = smem + s * STAGE_BYTES;
+        int tm, col0, width;
+        pair_tile(pt, t, tiles_m, tiles_n2, tm, col0, width);
+        const CUtensorMap* tmB = t < pt.wide * tiles_m ? &tmB1 : &tmB2;
+        const uint32_t bytes = 2 * A_BYTES + width * BK * 2;
+        for (int kb = 0; kb < kblocks; ++kb, ++it, rp.next(stages)) {
+          const int s = rp.s;
+          if (!mbar_wait(&bars.empty[s], rp.ph ^ 1, abort_flag, status, KID_GEMM_BF16, 5)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(&bars.full[s], bytes);
+          uint8_t* sa = smem + s * stage_bytes;
           tma_load_2d_pair(sa, &tmA, &bars.full[s], kb * BK, (2 * tm + rank) * BM);
-          tma_load_2d_pair(sa + A_BYTES, &tmB, &bars.full[s], kb * BK, tn * BN + rank * (BN / 2));
+          tma_load_2d_pair(sa + A_BYTES, tmB, &bars.full[s], kb * BK, col0 + rank * (width >> 1));
         }
       }
       // The even CTA's commits arrive at this CTA's barriers: the last one of every stage is waited for, so that none can be on its way
       // when the CTA leaves (the accumulator's barrier says nothing about the order in which these arrive).
-      for (uint32_t i = it > STAGES ? it - STAGES : 0; i < it && ok; ++i)
-        ok = mbar_wait(&bars.empty[i % STAGES], (i / STAGES) & 1, abort_flag, status, KID_GEMM_BF16, 9);
+      for (uint32_t i = it > (uint32_t)stages ? it - stages : 0; i < it && ok; ++i)
+        ok = mbar_wait(&bars.empty[i % stages], (i / stages) & 1, abort_flag, status, KID_GEMM_BF16, 9);
     }
   } else if (warp == 1) {
     if (rank == 0 && elect_one()) {
-      constexpr uint32_t idesc = umma_idesc(1, 1, 0, 0, 2 * BM, BN);
-      uint32_t it = 0, tile_it = 0;
+      const uint32_t idesc1 = umma_idesc(1, 1, 0, 0, 2 * BM, pt.w1), idesc2 = umma_idesc(1, 1, 0, 0, 2 * BM, pt.w2);
+      uint32_t tile_it = 0;
+      RingPos rp;
       bool ok = true;
       for (int t = first; t < tiles && ok; t += step, ++tile_it) {
         const int acc = tile_it & 1; const uint32_t aph = (tile_it >> 1) & 1;
         if (!mbar_wait(&bars.tmem_empty[acc], aph ^ 1, abort_flag, status, KID_GEMM_BF16, 6)) { ok = false; break; }
         tc_fence_after();
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
-          const int s = it % STAGES;
-          if (!mbar_wait(&bars.full[s], (it / STAGES) & 1, abort_flag, status, KID_GEMM_BF16, 7)) { ok = false; break; }
+        const uint32_t idesc = t < pt.wide * tiles_m ? idesc1 : idesc2;
+        for (int kb = 0; kb < kblocks; ++kb, rp.next(stages)) {
+          const int s = rp.s;
+          if (!mbar_wait(&bars.full[s], rp.ph, abort_flag, status, KID_GEMM_BF16, 7)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
+          const uint32_t sa = smem_u32(smem + s * stage_bytes);
           const uint64_t da = umma_desc_sw128(sa, 16, 1024), db = umma_desc_sw128(sa + A_BYTES, 16, 1024);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_pair(tmem_base + acc * BN, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+          for (int k = 0; k < BK / UMMA_K; ++k) umma_f16_pair(tmem_base + acc * 256, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
           umma_commit_pair(&bars.empty[s]);
         }
         if (ok) umma_commit_pair(&bars.tmem_full[acc]);
@@ -657,15 +678,15 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     uint32_t tile_it = 0;
     bool ok = true;
     for (int t = first; t < tiles && ok; t += step, ++tile_it) {
-      int tm, tn;
-      tile_coords(t, tiles_m, tiles_n, tm, tn);
+      int tm, col0, width;
+      pair_tile(pt, t, tiles_m, tiles_n2, tm, col0, width);
       const int acc = tile_it & 1;
       if (!mbar_wait(&bars.tmem_full[acc], (tile_it >> 1) & 1, abort_flag, status, KID_GEMM_BF16, 8)) ok = false;
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       const int row = (2 * tm + rank) * BM + q * 32 + lane;
-      store_tile_row<BN>(tmem_base + (uint32_t(q * 32) << 16) + acc * BN, Cout, row, row < M, ldc, N, epi, tn, 0, tail);
+      store_tile_row<2>(tmem_base + (uint32_t(q * 32) << 16) + acc * 256, Cout, row, row < M, ldc, N, epi, col0, width, 0, tail, (warp - 2) >> 2);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(&bars.tmem_empty[acc]);
@@ -687,6 +708,60 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
 using namespace ff;
 
+// What a pair takes for a tile w columns wide, in cycles per 64-wide K block where a 256-wide one takes 552: the time of a wave beyond the second at
+// K = 4096 and 2048 rows, 24.3, 21.8, 20.0, 17.7, 16.1, 15.3 and 14.4 us for 256 down to 64 columns in steps of 32. Narrow tiles are bound
+// by the 128 rows of A that each CTA loads for them.
+static float pair_cost(int w) { return w >= 128 ? 178.0f + 1.46f * w : 291.0f + 0.58f * w; }
+
+// The tiles of M x N for `pairs` pairs that take tile t, t + pairs, ...: as many wide columns as fill whole waves, the rest in tiles so narrow that
+// the last wave is full too. Returns what the busiest pair takes, in units of pair_cost. Against one width for all tiles (256 or 128): 1000 rows
+// times 6144 x 4096 (18 columns of 224, the rest of 128 wide) 42.9 -> 40.3 us, 700 x 4096 x 14336 (192 wide) 77.9 -> 66.5, 2039 x 7168 x 18432 529 ->
+// 413, 2500 x 4096 x 14336 256 -> 219. K is walked in the same order in tiles of all widths: the bits are the same.
+static float pair_plan(int M, int N, int epi, int pairs, PairTiles& best) {
+  const int step = epi == 1 ? 128 : 32, tiles_m = (M + 2 * BM - 1) / (2 * BM);
+  float least = 0.f;
+  for (int w1 = 256; w1 >= 64; w1 -= step) {
+    const int cols = (N + w1 - 1) / w1, full = cols * tiles_m / pairs;
+    for (int w2 = w1; w2 >= 64; w2 -= step)
+      for (int k = 0; k < 2; ++k) {
+        // all columns w1 wide, or those of the last whole wave (k = 0) or the one before it (k = 1)
+        int wide = w2 == w1 ? cols : (full - k) * pairs / tiles_m;
+        if (wide < 0 || (w2 == w1 && k) || (w2 < w1 && wide >= cols)) continue;
+        const int rest = N - wide * w1, n1 = wide * tiles_m, n2 = rest > 0 ? tiles_m * ((rest + w2 - 1) / w2) : 0;
+        const int q1 = n1 / pairs, r1 = n1 % pairs;
+        // pairs that got q1 wide tiles take the first narrow ones; the others what is left then
+        const int low = (n2 + pairs - 1) / pairs, over = n2 - (pairs - r1), high = over > 0 ? (over + pairs - 1) / pairs : 0;
+        float t = q1 * pair_cost(w1) + low * pair_cost(w2);
+        if (r1) { const float h = (q1 + 1) * pair_cost(w1) + high * pair_cost(w2); t = t > h ? t : h; }
+        if (least == 0.f || t < least * 0.995f) { least = t; best = PairTiles{w1, wide, w2}; }
+      }
+  }
+  return least;
+}
+
+// the plan as {w1, wide, w2} (host only)
+FF_EXPORT int ff_gemm_bf16_pair_tiles(int M, int N, int epi, int pairs, int* tiles) {
+  if (M <= 0 || N <= 0 || pairs <= 0 || epi < 0 || epi > 2) return FF_HOST_BAD_SHAPE;
+  PairTiles pt;
+  pair_plan(M, N, epi, pairs, pt);
+  tiles[0] = pt.w1; tiles[1] = pt.wide; tiles[2] = pt.w2;
+  return FF_HOST_OK;
+}
+
+static int pair_launch(const CUtensorMap& tmA, const void* W, void* Y, int M, int N, int K, int ldw, int ldy, int epi, const PairTiles& pt,
+                       const LinTail& tail, int* status, cudaStream_t stream) {
+  const int pairs = sm_count() / 2, tiles_m = (M + 2 * BM - 1) / (2 * BM), rest = N - pt.wide * pt.w1;
+  const int tiles = tiles_m * (pt.wide + (rest > 0 ? (rest + pt.w2 - 1) / pt.w2 : 0)), grid = 2 * (tiles < pairs ? tiles : pairs);
+  CUtensorMap tmB1, tmB2;
+  if (int e = make_tmap_2d(&tmB1, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, pt.w1 / 2)) return e;
+  if (int e = make_tmap_2d(&tmB2, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, pt.w2 / 2)) return e;
+  const int fit = PAIR_RING / (BM * BK * 2 + (pt.wide ? pt.w1 : pt.w2) * BK), stages = fit < PAIR_STAGES ? fit : PAIR_STAGES;
+  constexpr int SMEM = PAIR_RING + 1024;
+  if (int e = opt_in_smem(gemm_bf16_pair_kernel, SMEM)) return e;
+  if (int e = launch_pdl(gemm_bf16_pair_kernel, dim3(grid), dim3(320), SMEM, stream, 2, tmA, tmB1, tmB2, Y, M, N, K, ldy, epi, pt, stages, status, tail)) return e;
+  return launch_result();
+}
+
 // Y[M,N] = X[M,K] · W[N,K]ᵀ. epi: 0 bf16 out, 1 fused SwiGLU (out has N/2 columns), 2 fp32 out.
 // ldx / ldw / ldy in elements. Returns 0 or an error code (see host_util.h).
 static int gemm_bf16_launch(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw, int ldy,
@@ -698,15 +773,11 @@ static int gemm_bf16_launch(const void* X, const void* W, void* Y, int M, int N,
   const int out_bytes = (epi == 2) ? 4 : 2;
   if (((size_t)ldy * out_bytes) % 16 || ldy < out_cols) return FF_HOST_BAD_ALIGN;
   if (reinterpret_cast<uintptr_t>(Y) & 15) return FF_HOST_BAD_ALIGN;
-  CUtensorMap tmA, tmB;
-  int r = make_tmap_2d(&tmA, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, (uint64_t)ldx * 2, BK, BM);
-  if (r) return r;
-  // Column tile: 256 wide takes in the fewest bytes per product, 128 wide fills a last wave better (M = 1000, N = 6144: 96 wide tiles on
-  // 74 pairs are two waves, 192 narrow ones three of half the length). A narrow tile is charged 1.15 of half a wide one (24 instead of 16
-  // KiB per 128 columns).
-  const int pairs = sm_count() / 2, tiles_m = (M + 2 * BM - 1) / (2 * BM);
-  auto waves = [&](int bn) { const int t = tiles_m * ((N + bn - 1) / bn); return (t + pairs - 1) / pairs; };
-  const bool narrow = waves(128) * 0.575f < waves(256);
+  CUtensorMap tmA;
+  if (int e = make_tmap_2d(&tmA, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, (uint64_t)ldx * 2, BK, BM)) return e;
+  const int pairs = sm_count() / 2;
+  PairTiles pt;
+  const float pair_waves = pair_plan(M, N, epi, pairs, pt) / pair_cost(256);
   // Tiles of one CTA where they finish in clearly fewer waves: 256-row tiles of pairs pad rows more, and at short K a pair's set-up and its
   // epilogue take what its main loop saves. A wave of one-CTA tiles is charged 1 / 0.79 of a pair's (1 / 0.97 behind a SwiGLU epilogue at K up
   // to 2048, 1 / 1.05 at K up to 512 and for a single wave at K up to 1024). Of 1507 sizes (42 shapes of 512 x 512 to 65536 x 2048 and 57344 x
@@ -714,26 +785,17 @@ static int gemm_bf16_launch(const void* X, const void* W, void* Y, int M, int N,
   // 98 / 128 us, 320 x 24576 x 1536 29 / 32, 4096 x 32768 x 512 157 / 179. K is walked in the same order: the bits are the same.
   const int ctas = sm_count(), waves1 = (((M + BM - 1) / BM) * ((N + 255) / 256) + ctas - 1) / ctas;
   const float share = K <= 512 || (K <= 1024 && waves1 == 1) ? 1.05f : epi == 1 && K <= 2048 ? 0.97f : 0.79f;
-  if (waves1 < share * (narrow ? 0.575f * waves(128) : (float)waves(256))) {
+  if (waves1 < share * pair_waves) {
     constexpr int BN = 256, STAGES = 4;
+    CUtensorMap tmB;
     if (int e = make_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, BN)) return e;
     const int smem = STAGES * (BM + BN) * BK * 2 + 1024, tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     auto kern = gemm_bf16_kernel<BN, STAGES, 0>;
     if (int e = opt_in_smem(kern, smem)) return e;
-    kern<<<tiles < ctas ? tiles : ctas, 192, smem, stream>>>(tmA, tmA, tmA, tmB, Y, M, N, K, ldy, epi, status, CommArgs{}, GroupArgs{}, tail);
+    kern<<<tiles < ctas ? tiles : ctas, 320, smem, stream>>>(tmA, tmA, tmA, tmB, Y, M, N, K, ldy, epi, status, CommArgs{}, GroupArgs{}, tail);
     return launch_result();
   }
-  const int bn = narrow ? 128 : 256;
-  r = make_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, bn / 2);
-  if (r) return r;
-  const int tiles = tiles_m * ((N + bn - 1) / bn), grid = 2 * (tiles < pairs ? tiles : pairs);
-  auto go = [&](auto kern, int stages) -> int {
-    const int smem = stages * (BM + bn / 2) * BK * 2 + 1024;
-    if (int e = opt_in_smem(kern, smem)) return e;
-    if (int e = launch_pdl(kern, dim3(grid), dim3(192), smem, stream, 2, tmA, tmB, Y, M, N, K, ldy, epi, status, tail)) return e;
-    return launch_result();
-  };
-  return narrow ? go(gemm_bf16_pair_kernel<128, 8>, 8) : go(gemm_bf16_pair_kernel<256, 6>, 6);
+  return pair_launch(tmA, W, Y, M, N, K, ldw, ldy, epi, pt, tail, status, stream);
 }
 
 FF_EXPORT int ff_gemm_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw, int ldy,
@@ -788,7 +850,7 @@ FF_EXPORT int ff_gemm_bf16_heads(const void* X, const void* W, void* Y, int M, i
   CommArgs none = {};
   GroupArgs ga = {};
   ga.heads = heads; ga.a_cols = a_cols; ga.c_cols = c_cols;
-  kern<<<grid, 192, smem, stream>>>(tmA, tmA, tmA, tmB, Y, M, N, K, ldy, 0, status, none, ga, LinTail{});
+  kern<<<grid, 320, smem, stream>>>(tmA, tmA, tmA, tmB, Y, M, N, K, ldy, 0, status, none, ga, LinTail{});
   return launch_result();
 }
 
@@ -816,7 +878,7 @@ FF_EXPORT int ff_moe_grouped_gemm_tiled(const void* Xs, const void* W, void* Y, 
   GroupArgs ga = {seg_off, counts, E_local};
   LinTail tail = {};
   if (limit > 0.f) { tail.gate = 5; tail.limit = limit; }
-  kern<<<sm_count(), 192, smem, stream>>>(tmA, tmA, tmA, tmB, Y, capacity, Nw, K, ldy, epi, status, none, ga, tail);
+  kern<<<sm_count(), 320, smem, stream>>>(tmA, tmA, tmA, tmB, Y, capacity, Nw, K, ldy, epi, status, none, ga, tail);
   return launch_result();
 }
 

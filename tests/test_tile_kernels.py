@@ -108,6 +108,57 @@ def test_pair_gemm_gate(m, n):
     assert ((got - want).abs() <= 3 * 2.0 ** -8 * want.abs() + 2e-2).all()
 
 
+def _pair_tiles(m, n, epi, pairs=74):
+    import ctypes
+    from flyingfish_b200.ops.lib import kernels
+    out = (ctypes.c_int * 3)()
+    assert kernels().ff_gemm_bf16_pair_tiles(m, n, epi, pairs, out) == 0
+    return tuple(out)
+
+
+@pytest.mark.parametrize("epi", [0, 1])
+def test_pair_tiles_cover_the_columns(epi):
+    """Widths the tensor cores and the epilogue take, wide columns that leave something to the narrow ones or nothing, no empty column."""
+    mixed = 0
+    for m in (129, 256, 257, 700, 1000, 2500, 8191, 70000):
+        for n in (256, 512, 768, 4096, 6144, 28672) + (() if epi else (1, 31, 32, 63, 65, 136, 257, 576, 129280)):
+            for pairs in (1, 16, 74):
+                w1, wide, w2 = _pair_tiles(m, n, epi, pairs)
+                step = 128 if epi else 32
+                assert w1 % step == w2 % step == 0 and 64 <= w2 <= w1 <= 256
+                rest = n - wide * w1
+                assert rest > -w1 and wide * w1 + max(0, -(-rest // w2)) * w2 >= n
+                mixed += 0 < wide and rest > 0 and w1 != w2
+    assert mixed > 10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,mixed", [(1000, 6144, 128, True), (2500, 4096, 704, True), (300, 6144, 832, False), (600, 4104, 64, False)])
+def test_pair_gemm_of_two_widths(m, n, k, mixed):
+    """Wide and narrow tiles in one launch and tiles of one odd width, rings of 7 to 11 stages begun again, a last tile past the columns."""
+    from flyingfish_b200 import ops
+    w1, wide, w2 = _pair_tiles(m, n, 0)
+    assert (0 < wide * w1 < n and w1 != w2) if mixed else wide == 0 and w2 < 256
+    x, w = _rand((m, k), m), _rand((n, k), n)
+    y = ops.linear(x.cuda(), w.cuda())
+    torch.cuda.synchronize()
+    ops.check_status()
+    _check(y, x.double() @ w.double().t(), k)
+
+
+@pytest.mark.gpu
+def test_pair_gemm_gate_of_two_widths():
+    from flyingfish_b200 import ops
+    m, n = 300, 28672
+    w1, wide, w2 = _pair_tiles(m, n, 1)
+    assert 0 < wide * w1 < n and (w1, w2) == (256, 128)
+    x, w = _rand((m, 64), 4), _rand((n, 64), 5)
+    got, want = ops.linear_swiglu(x.cuda(), w.cuda()), ops.silu_mul_interleaved(ops.linear(x.cuda(), w.cuda()))
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(got, want)                                # the activation kernel rounds at the same places
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("counts", [[64, 1, 65, 0, 50, 33, 63, 47], [16, 17, 0, 32, 33, 1, 31, 30], [100, 128, 129, 16]])   # chunks of 64, 32, 128
 @pytest.mark.parametrize("epi", [0, 1])
