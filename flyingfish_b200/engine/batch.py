@@ -13,6 +13,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 
@@ -50,7 +51,10 @@ class ForwardBatch:
         self.layout = layout
         self.device = torch.device(device)
         pin = self.device.type == "cuda" if pinned is None else pinned
-        self.host = torch.zeros(layout.total, dtype=torch.int32, pin_memory=pin)
+        pinned = torch.zeros(layout.total + 4 + layout.max_batch, dtype=torch.int32, pin_memory=pin)
+        self.host = pinned[: layout.total]
+        self.results = pinned[layout.total:]     # where a step's device status (four words) and ids are copied to
+        self._words = self.host.numpy()   # the same memory: a field is written in about a microsecond, through a tensor in four
         self.dev = torch.zeros(layout.total, dtype=torch.int32, device=self.device)
         # host-side scalars of the current step
         self.batch = 0
@@ -114,63 +118,61 @@ class ForwardBatch:
         """Write one step's metadata into the pinned host buffer (lists of ints; ids, positions and slots also as int32 arrays, which
         is what a prompt's thousands of rows take)."""
         L = self.layout
-        h = self.host
+        h = self._words
         rows, batch = len(ids), len(q_lens)
         assert rows <= L.max_rows and batch <= L.max_batch, "batch exceeds the layout capacity"
         assert len(logit_rows) <= L.n_logit
         self.rows, self.batch, self.nq, self.is_decode, self.singles = rows, batch, nq, is_decode, singles
         self.key_pages = None
-        h[L.ids: L.ids + rows] = torch.as_tensor(ids, dtype=torch.int32)
-        h[L.positions: L.positions + rows] = torch.as_tensor(positions, dtype=torch.int32)
-        h[L.slots: L.slots + rows] = torch.as_tensor(slots, dtype=torch.int32)
-        ql = torch.as_tensor(q_lens, dtype=torch.int32)
+        h[L.ids: L.ids + rows] = ids
+        h[L.positions: L.positions + rows] = positions
+        h[L.slots: L.slots + rows] = slots
+        ql = np.asarray(q_lens, dtype=np.int32)
+        ends = np.cumsum(ql, dtype=np.int32)
         h[L.q_lens: L.q_lens + batch] = ql
-        qs = torch.zeros(batch, dtype=torch.int32)
-        if batch > 1:
-            qs[1:] = torch.cumsum(ql, 0)[:-1].to(torch.int32)
-        h[L.q_start: L.q_start + batch] = qs
-        h[L.row_start: L.row_start + batch] = qs
-        h[L.row_start + batch] = int(ql.sum()) if batch else 0
+        h[L.q_start: L.q_start + batch] = h[L.row_start: L.row_start + batch] = ends - ql
+        h[L.row_start + batch] = ends[-1] if batch else 0
         if state_slots is not None:
-            h[L.state_slots: L.state_slots + batch] = torch.as_tensor(state_slots, dtype=torch.int32)
+            h[L.state_slots: L.state_slots + batch] = state_slots
             self.state_slots = list(state_slots)
-        h[L.ctx_lens: L.ctx_lens + batch] = torch.as_tensor(ctx_lens, dtype=torch.int32)
+        h[L.ctx_lens: L.ctx_lens + batch] = ctx_lens
         self.n_logit_rows = len(logit_rows)
-        h[L.logit_rows: L.logit_rows + len(logit_rows)] = torch.as_tensor(logit_rows, dtype=torch.int32)
-        bt = h[L.block_table: L.block_table + L.max_batch * L.max_blocks].view(L.max_batch, L.max_blocks)
+        h[L.logit_rows: L.logit_rows + len(logit_rows)] = logit_rows
+        bt = h[L.block_table: L.block_table + L.max_batch * L.max_blocks].reshape(L.max_batch, L.max_blocks)
         # a decode batch keeps the same sequences in the same rows for many steps and a block list changes only when
         # a sequence crosses a block boundary: rows whose list is unchanged are not rewritten (the pinned buffer
         # still holds them), which takes most of the host time out of a decode step
         sig = self._bt_sig
         for i, row in enumerate(block_rows):
-            t = tuple(row)
-            if i < len(sig) and sig[i] == t:
+            if type(row) is not list:
+                row = list(row)
+            if i < len(sig) and sig[i] == row:
                 continue
-            n = len(t)
+            row = row.copy()                      # the caller's list goes on growing
+            n = len(row)
             assert n <= L.max_blocks
             if n:
-                bt[i, :n] = torch.as_tensor(t, dtype=torch.int32)
+                bt[i, :n] = row
             if i < len(sig):
-                sig[i] = t
+                sig[i] = row
             else:
-                sig.extend([None] * (i - len(sig)) + [t])
+                sig.extend([None] * (i - len(sig)) + [row])
         if L.max_groups:
-            ks = torch.zeros(batch, dtype=torch.int32)
+            ks = h[L.kv_start: L.kv_start + batch]
+            ks[:] = 0
             if kv_start is not None:
-                ks[: len(kv_start)] = torch.as_tensor(kv_start, dtype=torch.int32)
-            h[L.kv_start: L.kv_start + batch] = ks
-            gt = h[L.groups: L.groups + L.max_batch * L.max_groups].view(L.max_batch, L.max_groups)
+                ks[: len(kv_start)] = kv_start
+            gt = h[L.groups: L.groups + L.max_batch * L.max_groups].reshape(L.max_batch, L.max_groups)
             for i, row in enumerate(group_rows or []):
                 if row:
                     assert len(row) <= L.max_groups
-                    gt[i, : len(row)] = torch.as_tensor(row, dtype=torch.int32)
+                    gt[i, : len(row)] = row
         self.max_q_len = int(max(q_lens)) if batch else 0
         self.max_ctx = int(max(ctx_lens)) if batch else 0
         self.use_tree_mask = tree_mask is not None
         if tree_mask is not None:
-            # bit 63 may be set: store the two's complement value
-            tm = torch.as_tensor([m - (1 << 64) if m >= (1 << 63) else m for m in tree_mask], dtype=torch.int64)
-            h[L.tree_mask: L.tree_mask + 2 * rows].view(torch.int64)[:] = tm
+            # 64 bits per row, bit 63 may be set
+            h[L.tree_mask: L.tree_mask + 2 * rows] = np.array([m & (1 << 64) - 1 for m in tree_mask], dtype=np.uint64).view(np.int32)
 
     def h2d_bytes(self) -> int:
         return self.layout.total * 4

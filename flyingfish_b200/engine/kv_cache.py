@@ -137,6 +137,20 @@ class PagedKVCache:
         at = s.length - first * bs
         return (pages[:, None] * bs + np.arange(bs, dtype=np.int32)).reshape(-1)[at: at + new_tokens]
 
+    def reserve_step(self, seq_ids: list[int]) -> tuple[list[SequenceKV], np.ndarray, np.ndarray]:
+        """One more token of every sequence of a decode step, reserved for all of them or for none: the sequences, their lengths and
+        the tokens' slots (int32)."""
+        held, bs = [self.seqs[i] for i in seq_ids], self.block_size
+        short = [s for s in held if s.length >= len(s.blocks) * bs]
+        need = sum(self.blocks_needed(s.seq_id, 1) for s in short)
+        if need > self.alloc.free_blocks:
+            raise OutOfBlocks(f"step needs {need} KV blocks, {self.alloc.free_blocks} free")
+        for s in short:
+            self.reserve(s.seq_id, 1, list_slots=False)
+        at = np.array([s.length for s in held], dtype=np.int32)
+        pages = np.array([s.blocks[s.length // bs] for s in held], dtype=np.int32)
+        return held, at, pages * bs + at % bs
+
     def commit(self, seq_id: int, new_tokens: int) -> None:
         self.seqs[seq_id].length += new_tokens
 

@@ -60,6 +60,14 @@ def _rows2d(t: torch.Tensor) -> tuple[int, int]:
     return t.shape[0], t.stride(0)
 
 
+def copy_async(dst: torch.Tensor, src: torch.Tensor) -> None:
+    """Copy of equal contiguous tensors, host (pinned) or device, on the current stream, also as part of a captured graph. The caller keeps
+    both alive and the host side untouched until the copy has run."""
+    _require(dst.dtype == src.dtype and dst.shape == src.shape and dst.is_contiguous() and src.is_contiguous(), "copy_async: equal contiguous tensors")
+    _require(all(t.is_cuda or t.is_pinned() for t in (dst, src)), "copy_async: device or pinned memory")
+    check(kernels().ff_copy_async(ptr(dst), ptr(src), c_longlong(dst.numel() * dst.element_size()), stream_ptr()), "ff_copy_async")
+
+
 # ------------------------------------------------------------------------------------------
 # workspace (split-K partials, attention split partials): one per device, grown outside of
 # graph capture only

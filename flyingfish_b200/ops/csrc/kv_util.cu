@@ -49,3 +49,11 @@ FF_EXPORT int ff_kv_move_rows(const unsigned long long* caches, int tensors, con
   return launch_pdl(kv_move_rows_kernel<false>, grid, dim3(threads), 0, s, 0, caches, dst_slots,
                     static_cast<uint4*>(staging), heads, block_size, dim, num_blocks, status);
 }
+
+// a copy between device and pinned host memory in stream order
+FF_EXPORT int ff_copy_async(void* dst, const void* src, long long bytes, cudaStream_t s) {
+  if (bytes <= 0 || dst == nullptr || src == nullptr) return FF_HOST_BAD_SHAPE;
+  const cudaError_t e = cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDefault, s);
+  if (e != cudaSuccess) { cudaGetLastError(); return static_cast<int>(e); }
+  return FF_HOST_OK;
+}
