@@ -281,6 +281,42 @@ def test_merge_of_many_splits(ctx):
     assert ((got.cpu().float() - want).abs() <= 1e-2 + 1e-2 * want.abs()).all()  # BF16 weights and result
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens,hq,hkv", [
+    ([0, 1, 64, 65, 320, 321, 384, 640], 8, 2),              # padding, whole pages, one page more; one split and several in a launch
+    ([2000, 63, 700], 16, 1),                                # more than eight splits beside one
+    ([300] * 100 + [900, 0], 32, 8),                         # so many rows that short sequences are not split
+])
+@pytest.mark.parametrize("nq", [1, 3])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_splits_by_length(lens, hq, hkv, nq, sinks):
+    """A sequence is cut by its own length: results against the oracle, and the bits of a row beside sequences of other lengths."""
+    from flyingfish_b200 import ops
+    d, blocks, batch = 128, 64, len(lens)
+    lens = [max(n, nq) if n else 0 for n in lens]
+    pool = 40
+    q, k, v = _rand((batch * nq, hq * d), 1), _rand((pool, hkv, 64, d), 2), _rand((pool, hkv, 64, d), 3)
+    table = torch.stack([torch.randint(0, pool, (blocks,), generator=torch.Generator().manual_seed(b)) for b in range(batch)]).to(torch.int32)
+    ctx = torch.tensor(lens, dtype=torch.int32)
+    sk = torch.randn(hq, generator=torch.Generator().manual_seed(9)) if sinks else None
+    run = lambda c: ops.attn_decode(q.cuda(), k.cuda(), v.cuda(), table.cuda(), c.cuda(), hq, hkv, d, d ** -0.5, nq=nq, max_ctx=blocks * 64, sinks=sk.cuda() if sinks else None)
+    got = run(ctx)
+    torch.cuda.synchronize()
+    ops.check_status()
+    live = [b for b in range(batch) if lens[b]]
+    for b in live[:12] + live[-2:]:
+        one = torch.ones(1, dtype=torch.int32)
+        want = ref.attention_paged(q[b * nq: (b + 1) * nq], k, v, table[b: b + 1], 0 * one, nq * one, ctx[b: b + 1], hq, hkv, d, d ** -0.5, None, 0, sk).float()
+        assert ((got[b * nq: (b + 1) * nq].cpu().float() - want).abs() <= 1e-2 + 1e-2 * want.abs()).all()      # BF16 weights and result
+    other = torch.where(ctx > 0, (ctx * 3) // 4 + nq, ctx)
+    for first in (True, False):                              # the first sequence beside others, the others beside another first one
+        mixed = torch.cat([ctx[:1], other[1:]]) if first else torch.cat([other[:1], ctx[1:]])
+        again = run(mixed)
+        for b in range(batch):
+            if int(mixed[b]) == lens[b]:
+                assert torch.equal(again[b * nq: (b + 1) * nq], got[b * nq: (b + 1) * nq])
+
+
 @pytest.mark.parametrize("n,k", [(7168, 18432), (7168, 2560), (4096, 7168), (6144, 4096), (34048, 512), (33920, 512), (576, 2560), (128, 128)])
 def test_fp8_split_does_not_depend_on_the_rows(n, k):
     import ctypes
