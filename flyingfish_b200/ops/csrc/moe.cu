@@ -201,24 +201,27 @@ moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ pos, uint
 // ---------------------------------------------------------------------------------------
 // count / scan / permute
 // ---------------------------------------------------------------------------------------
-__global__ void moe_count_kernel(const int* __restrict__ ids, int n_assign, int E, int e_lo, int e_hi,
-                                 int* __restrict__ counts, int* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_assign) return;
-  const int e = ids[i];
-  if (e == -1) return;                       // assignment served elsewhere (another tier / rank)
-  if (e < 0 || e >= E) { set_status(status, KID_MOE_DISPATCH, FF_ERR_BOUNDS, i, e); return; }
-  if (e >= e_lo && e < e_hi) atomicAdd(&counts[e - e_lo], 1);
-}
-
-// One block: seg_off[e] = sum of pad16(count) over earlier experts; cursors zeroed; total rows
-// (padded) written to seg_off[E_local]. capacity = rows the sorted buffer can hold.
+// One block: assignments of every expert, seg_off[e] = sum of pad16(count) over earlier experts; cursors zeroed; total rows
+// (padded) written to seg_off[E_local]. capacity = rows the sorted buffer can hold. A memset, a count over many blocks and a scan were three
+// launches in a row, 5.7 us of 256 assignments and 8.8 of 16312; one is 3.0 us of 256.
+// It does not let the next kernel start early, and the permutations are launched plainly: the grouped FP8 product reads counts and offsets in
+// front of its wait on the kernel before it, so they have to be complete before the permutation starts.
 __global__ void __launch_bounds__(1024)
-moe_scan_kernel(const int* __restrict__ counts, int* __restrict__ seg_off, int* __restrict__ cursors, int E_local,
-                int capacity, int* status) {
-  __shared__ int s[1024];
-  const int t = threadIdx.x;
-  const int c = t < E_local ? ((counts[t] + 15) / 16) * 16 : 0;
+moe_count_scan_kernel(const int* __restrict__ ids, int n_assign, int E, int e_lo, int e_hi, int* __restrict__ counts, int* __restrict__ seg_off,
+                      int* __restrict__ cursors, int capacity, int* status) {
+  __shared__ int n[1024], s[1024];
+  const int t = threadIdx.x, E_local = e_hi - e_lo;
+  n[t] = 0;
+  __syncthreads();
+  pdl_wait();
+  for (int i = t; i < n_assign; i += 1024) {
+    const int e = ids[i];
+    if (e == -1) continue;                     // assignment served elsewhere (another tier / rank)
+    if (e < 0 || e >= E) { set_status(status, KID_MOE_DISPATCH, FF_ERR_BOUNDS, i, e); continue; }
+    if (e >= e_lo && e < e_hi) atomicAdd(&n[e - e_lo], 1);
+  }
+  __syncthreads();
+  const int c = t < E_local ? ((n[t] + 15) / 16) * 16 : 0;
   s[t] = c;
   __syncthreads();
   for (int o = 1; o < 1024; o <<= 1) {
@@ -227,7 +230,7 @@ moe_scan_kernel(const int* __restrict__ counts, int* __restrict__ seg_off, int* 
     s[t] += v;
     __syncthreads();
   }
-  if (t < E_local) { seg_off[t] = s[t] - c; cursors[t] = 0; }
+  if (t < E_local) { counts[t] = n[t]; seg_off[t] = s[t] - c; cursors[t] = 0; }
   if (t == E_local - 1) {
     seg_off[E_local] = s[t];
     if (s[t] > capacity) set_status(status, KID_MOE_DISPATCH, FF_ERR_CAPACITY, s[t], capacity);
@@ -252,6 +255,26 @@ moe_permute_kernel(const uint4* __restrict__ x, const int* __restrict__ ids, con
   const uint4* src = x + (size_t)row * ldx_vecs;
   uint4* dst = sorted + (size_t)slot * vecs;
   for (int v = threadIdx.x; v < vecs; v += blockDim.x) dst[v] = src[v];
+}
+
+// The same for rows that are quantised already: E4M3 codes (vecs 16-byte vectors a row) and their `groups` FP32 scales. A row is quantised once and
+// not once per expert, and the padding between the segments not at all: 64 rows for 256 experts 77 us behind the permutation, 2.5 in front of it.
+__global__ void __launch_bounds__(128)
+moe_permute_fp8_kernel(const uint4* __restrict__ codes, const float* __restrict__ scales, const int* __restrict__ ids, const int* __restrict__ seg_off,
+                       int* __restrict__ cursors, uint4* __restrict__ sorted, float* __restrict__ sorted_scales, int* __restrict__ pos, int vecs,
+                       int groups, int top_k, int e_lo, int e_hi, int capacity) {
+  const int a = blockIdx.x;
+  const int e = ids[a];
+  __shared__ int slot_s;
+  if (e < e_lo || e >= e_hi) { if (threadIdx.x == 0) pos[a] = -1; return; }
+  if (threadIdx.x == 0) slot_s = seg_off[e - e_lo] + atomicAdd(&cursors[e - e_lo], 1);
+  __syncthreads();
+  const int slot = slot_s;
+  if (threadIdx.x == 0) pos[a] = slot < capacity ? slot : -1;
+  if (slot >= capacity) return;
+  const int row = a / top_k;
+  for (int v = threadIdx.x; v < vecs; v += 128) sorted[(size_t)slot * vecs + v] = codes[(size_t)row * vecs + v];
+  for (int g = threadIdx.x; g < groups; g += 128) sorted_scales[(size_t)slot * groups + g] = scales[(size_t)row * groups + g];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -523,13 +546,24 @@ FF_EXPORT int ff_moe_dispatch_local(const void* x, const int* ids, int rows, int
   if (rows <= 0 || top_k < 1 || hidden % 8 || el < 1 || el > 1024 || ldx % 8) return FF_HOST_BAD_SHAPE;
   if (elem_bytes != 2 && elem_bytes != 4) return FF_HOST_UNSUPPORTED;
   const int per_vec = 16 / elem_bytes;
-  cudaError_t e = cudaMemsetAsync(counts, 0, (size_t)el * 4, s);
-  if (e != cudaSuccess) return (int)e;
   const int n = rows * top_k;
-  moe_count_kernel<<<(n + 255) / 256, 256, 0, s>>>(ids, n, E, e_lo, e_hi, counts, status);
-  moe_scan_kernel<<<1, 1024, 0, s>>>(counts, seg_off, cursors, el, capacity, status);
+  if (int r = launch_pdl(moe_count_scan_kernel, dim3(1), dim3(1024), 0, s, 0, ids, n, E, e_lo, e_hi, counts, seg_off, cursors, capacity, status)) return r;
   moe_permute_kernel<<<n, 128, 0, s>>>((const uint4*)x, ids, seg_off, cursors, (uint4*)sorted, pos, hidden / per_vec, top_k, e_lo, e_hi,
                                        capacity, ldx / per_vec);
+  return launch_result();
+}
+
+// codes [rows, hidden] E4M3 with scales [rows, hidden / 128]; sorted [capacity, hidden] and sorted_scales [capacity, hidden / 128]
+FF_EXPORT int ff_moe_dispatch_fp8(const void* codes, const float* scales, const int* ids, int rows, int top_k, int hidden, int E, int e_lo, int e_hi,
+                                  int* counts, int* seg_off, int* cursors, void* sorted, float* sorted_scales, int* pos, int capacity,
+                                  int* status, cudaStream_t s) {
+  const int el = e_hi - e_lo;
+  if (rows <= 0 || top_k < 1 || hidden <= 0 || hidden % 128 || el < 1 || el > 1024) return FF_HOST_BAD_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(sorted)) & 15) return FF_HOST_BAD_ALIGN;
+  const int n = rows * top_k;
+  if (int r = launch_pdl(moe_count_scan_kernel, dim3(1), dim3(1024), 0, s, 0, ids, n, E, e_lo, e_hi, counts, seg_off, cursors, capacity, status)) return r;
+  moe_permute_fp8_kernel<<<n, 128, 0, s>>>((const uint4*)codes, scales, ids, seg_off, cursors, (uint4*)sorted, sorted_scales, pos, hidden / 16, hidden / 128,
+                                           top_k, e_lo, e_hi, capacity);
   return launch_result();
 }
 

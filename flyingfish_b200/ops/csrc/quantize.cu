@@ -36,18 +36,10 @@ __device__ __forceinline__ uint32_t e2m1_code(float v) {
   return idx | (v < 0.f ? 8u : 0u);
 }
 
-// one warp per (row, 128-group): lane holds 4 consecutive elements
-__global__ void quant_fp8_1x128_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
-                                       float* __restrict__ scale, int rows, int K, int ldx, int ue8m0, long long ldq,
-                                       long long lds) {
-  pdl_trigger();
-  pdl_wait();
-  const int groups = K >> 7;
-  const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// a warp quantises 128 elements, four per lane
+__device__ __forceinline__ void quant_group(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, int ue8m0) {
   const int lane = threadIdx.x & 31;
-  if (wid >= (long long)rows * groups) return;
-  const int row = (int)(wid / groups), g = (int)(wid % groups);
-  const uint2 raw = *reinterpret_cast<const uint2*>(x + (size_t)row * ldx + g * 128 + lane * 4);
+  const uint2 raw = *reinterpret_cast<const uint2*>(x + lane * 4);
   const float2 a = unpack_bf16x2(raw.x), b = unpack_bf16x2(raw.y);
   float amax = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y)));
   amax = warp_max(amax);
@@ -57,8 +49,37 @@ __global__ void quant_fp8_1x128_kernel(const __nv_bfloat16* __restrict__ x, uint
   // true division (not a reciprocal multiply) so the codes match the host codec bit for bit
   const uint32_t packed = (uint32_t)to_e4m3(__fdiv_rn(a.x, s)) | ((uint32_t)to_e4m3(__fdiv_rn(a.y, s)) << 8) |
                           ((uint32_t)to_e4m3(__fdiv_rn(b.x, s)) << 16) | ((uint32_t)to_e4m3(__fdiv_rn(b.y, s)) << 24);
-  *reinterpret_cast<uint32_t*>(q + (size_t)row * ldq + g * 128 + lane * 4) = packed;
-  if (lane == 0) scale[(size_t)row * lds + g] = s;
+  *reinterpret_cast<uint32_t*>(q + lane * 4) = packed;
+  if (lane == 0) *scale = s;
+}
+
+// one warp per (row, 128-group)
+__global__ void quant_fp8_1x128_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
+                                       float* __restrict__ scale, int rows, int K, int ldx, int ue8m0, long long ldq,
+                                       long long lds) {
+  pdl_trigger();
+  pdl_wait();
+  const int groups = K >> 7;
+  const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (wid >= (long long)rows * groups) return;
+  const int row = (int)(wid / groups), g = (int)(wid % groups);
+  quant_group(x + (size_t)row * ldx + g * 128, q + (size_t)row * ldq + g * 128, scale + (size_t)row * lds + g, ue8m0);
+}
+
+// The rows of expert segments (row seg_off[e] + i for i < counts[e]) and not the padding between them; grid (experts, warps' turns), 8 warps.
+// 512 rows of 2048 in 256 segments padded to 16 rows: 15.6 us for all 4608 rows, 8.0 us for the segments'.
+__global__ void __launch_bounds__(256)
+quant_fp8_segments_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, const int* __restrict__ seg_off,
+                          const int* __restrict__ counts, int capacity, int K) {
+  pdl_trigger();
+  pdl_wait();
+  const int e = blockIdx.x, row0 = seg_off[e], groups = K >> 7;
+  const int n = min(counts[e], capacity - row0) * groups;          // a segment cut at the end of the buffer, as the products cut it
+  for (int i = blockIdx.y * 8 + (threadIdx.x >> 5); i < n; i += 8 * gridDim.y) {
+    const int r = i / groups, g = i - r * groups;
+    const size_t at = (size_t)(row0 + r) * groups + g;
+    quant_group(x + at * 128, q + at * 128, scale + at, 0);
+  }
 }
 
 // VEC codes of a row per thread (16 where rows are whole vectors; a vector lies in one scale block). Bound by DRAM, 3 bytes a weight:
@@ -165,6 +186,16 @@ FF_EXPORT int ff_quant_fp8_1x128_strided(const void* x, void* q, float* scale, i
   if (int lr = launch_pdl(quant_fp8_1x128_kernel, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, s, 0,
                           (const __nv_bfloat16*)x, (uint8_t*)q, scale, rows, K, ldx, 0, ldq, lds)) return lr;
   return launch_result();
+}
+
+// the rows of expert segments: x, q [capacity, K], scale [capacity, K / 128]
+FF_EXPORT int ff_quant_fp8_segments(const void* x, void* q, float* scale, const int* seg_off, const int* counts, int experts, int capacity, int K,
+                                    int rows_per_expert, cudaStream_t s) {
+  if (experts <= 0 || capacity <= 0 || K <= 0 || K % 128 || rows_per_expert < 1) return FF_HOST_BAD_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(x) & 7) || (reinterpret_cast<uintptr_t>(q) & 3)) return FF_HOST_BAD_ALIGN;
+  const int turns = (rows_per_expert * (K / 128) + 15) / 16;       // about two groups a warp in a segment of average length
+  return launch_pdl(quant_fp8_segments_kernel, dim3(experts, turns < 1 ? 1 : turns > 64 ? 64 : turns), dim3(256), 0, s, 0, (const __nv_bfloat16*)x, (uint8_t*)q, scale,
+                    seg_off, counts, capacity, K);
 }
 
 FF_EXPORT int ff_dequant_fp8_block(const void* q, const float* scale, void* out, int N, int K, cudaStream_t s) {

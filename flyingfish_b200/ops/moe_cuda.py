@@ -58,17 +58,19 @@ def _gu_interleaved(w_gate_up: torch.Tensor) -> torch.Tensor:
     return t
 
 
+def _dispatch_plan(rows: int, top_k: int, el: int, dev):
+    capacity = ((rows * top_k + 16 * el + 15) // 16) * 16
+    meta = torch.empty(3 * el + 1, dtype=torch.int32, device=dev)
+    pos = torch.empty(rows * top_k, dtype=torch.int32, device=dev)
+    return meta[:el], meta[el: 2 * el + 1], meta[2 * el + 1:], pos, capacity
+
+
 def dispatch_local(x, ids, n_experts_total: int, e_lo: int, e_hi: int):
     """Device-side count / scan / permute for the experts [e_lo, e_hi) owned locally.
     Returns (sorted rows, pos, seg_off, counts, capacity)."""
     rows, hidden = x.shape
-    top_k = ids.shape[1]
-    el = e_hi - e_lo
-    capacity = ((rows * top_k + 16 * el + 15) // 16) * 16
-    dev = x.device
-    meta = torch.empty(3 * el + 1, dtype=torch.int32, device=dev)
-    counts, seg_off, cursors = meta[:el], meta[el: 2 * el + 1], meta[2 * el + 1:]
-    pos = torch.empty(rows * top_k, dtype=torch.int32, device=dev)
+    top_k, dev = ids.shape[1], x.device
+    counts, seg_off, cursors, pos, capacity = _dispatch_plan(rows, top_k, e_hi - e_lo, dev)
     # rows between the segments are never written; a GEMM computes them and stores nothing of them. The buffer comes from the
     # allocator per call: a captured step has its own
     sorted_x = torch.empty(capacity, hidden, dtype=x.dtype, device=dev)
@@ -76,8 +78,23 @@ def dispatch_local(x, ids, n_experts_total: int, e_lo: int, e_hi: int):
                                          ptr(counts), ptr(seg_off), ptr(cursors), ptr(sorted_x), ptr(pos), capacity,
                                          x.element_size(), ptr(status_tensor(dev)), stream_ptr())
     check(rc, "ff_moe_dispatch_local")
-    _count(3)
+    _count(2)
     return sorted_x, pos, seg_off, counts, capacity
+
+
+def dispatch_fp8(codes, scales, ids, n_experts_total: int, e_lo: int, e_hi: int):
+    """:func:`dispatch_local` of quantised rows (E4M3 codes [rows, hidden], FP32 scales [rows, hidden / 128]): (sorted codes, their scales,
+    pos, seg_off, counts, capacity)."""
+    rows, hidden = codes.shape
+    top_k, dev = ids.shape[1], codes.device
+    counts, seg_off, cursors, pos, capacity = _dispatch_plan(rows, top_k, e_hi - e_lo, dev)
+    xq = torch.empty(capacity, hidden, dtype=torch.uint8, device=dev)
+    xs = torch.empty(capacity, hidden // 128, dtype=torch.float32, device=dev)
+    rc = kernels().ff_moe_dispatch_fp8(ptr(codes), ptr(scales), ptr(ids), rows, top_k, hidden, n_experts_total, e_lo, e_hi, ptr(counts), ptr(seg_off),
+                                       ptr(cursors), ptr(xq), ptr(xs), ptr(pos), capacity, ptr(status_tensor(dev)), stream_ptr())
+    check(rc, "ff_moe_dispatch_fp8")
+    _count(2)
+    return xq, xs, pos, seg_off, counts, capacity
 
 
 TILED_MIN_ROWS = int(os.environ.get("FF_MOE_TILED_MIN", "96"))

@@ -32,6 +32,19 @@ def quant_fp8_act(x: torch.Tensor, ue8m0: bool = False) -> tuple[torch.Tensor, t
     return q, s
 
 
+def quant_fp8_segments(x: torch.Tensor, seg_off: torch.Tensor, counts: torch.Tensor, rows_per_expert: int) -> tuple[torch.Tensor, torch.Tensor]:
+    """:func:`quant_fp8_act` of the rows of expert segments; what lies between them stays unwritten. ``rows_per_expert``: about how many
+    rows a segment has."""
+    m, k = x.shape
+    _require(x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and k % 128 == 0, "quant_fp8_segments: bf16 rows, K % 128 == 0")
+    q = torch.empty(m, k, dtype=torch.uint8, device=x.device)
+    s = torch.empty(m, k // 128, dtype=torch.float32, device=x.device)
+    check(kernels().ff_quant_fp8_segments(ptr(x), ptr(q), ptr(s), ptr(seg_off), ptr(counts), counts.numel(), m, k, max(1, rows_per_expert), stream_ptr()),
+          "ff_quant_fp8_segments")
+    _count()
+    return q, s
+
+
 def linear_fp8(x: torch.Tensor, w_codes: torch.Tensor, w_scale: torch.Tensor) -> torch.Tensor:
     """W8A8 block-scaled linear: ``x`` BF16 [M, K]; weight E4M3 codes [N, K] + FP32 128x128 scales."""
     if not x.is_cuda:
@@ -164,10 +177,9 @@ def experts_forward_fp8(x: torch.Tensor, weights: torch.Tensor, ids: torch.Tenso
         return out.to(x.dtype)
     from . import moe_cuda
     _require(gate_up.interleaved, "experts_forward_fp8: the gate/up experts must be interleaved per 64 rows")
-    xs, pos, seg_off, counts, cap = moe_cuda.dispatch_local(x.contiguous(), ids.contiguous(), total, e_lo, e_lo + el)
-    xq, xsc = quant_fp8_act(xs)
+    xq, xsc, pos, seg_off, counts, cap = moe_cuda.dispatch_fp8(*quant_fp8_act(x.contiguous()), ids.contiguous(), total, e_lo, e_lo + el)
     h = grouped_gemm_fp8(xq, xsc, gate_up.codes, gate_up.scale, seg_off, counts, cap, epi=1)
-    hq, hsc = quant_fp8_act(h)
+    hq, hsc = quant_fp8_segments(h, seg_off, counts, rows * ids.shape[1] // total)
     y = grouped_gemm_fp8(hq, hsc, down.codes, down.scale, seg_off, counts, cap, epi=0)
     return moe_cuda.combine(y, pos, ids, weights.contiguous(), rows, hidden)
 

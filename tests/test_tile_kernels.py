@@ -185,6 +185,33 @@ def test_grouped_fp8_chunks(counts, epi):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows,hidden,experts,top_k", [(1, 128, 4, 1), (64, 1152, 32, 8), (200, 512, 7, 3), (3000, 256, 1000, 4)])
+def test_quantised_rows_dispatched(rows, hidden, experts, top_k):
+    """Rows quantised in front of the dispatch, and rows of segments, have the codes and scales of rows quantised behind it."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import moe_cuda, quant_ops
+    x = _rand((rows, hidden), rows).cuda()
+    g = torch.Generator().manual_seed(rows)
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(rows)]).to(torch.int32).cuda()
+    xq, xs, pos, seg_off, counts, cap = moe_cuda.dispatch_fp8(*quant_ops.quant_fp8_act(x), ids, experts, 0, experts)
+    want_q, want_s = quant_ops.quant_fp8_act(x)
+    row = torch.arange(rows, device="cuda").repeat_interleave(top_k)
+    at = pos.long()
+    assert at.unique().numel() == rows * top_k
+    assert torch.equal(xq[at], want_q[row]) and torch.equal(xs[at], want_s[row])
+    assert torch.equal(counts.long(), torch.bincount(ids.view(-1).long(), minlength=experts))
+    assert torch.equal(seg_off[1:].long() - seg_off[:-1].long(), (counts.long() + 15) // 16 * 16)
+    lo, n = seg_off[:-1].long()[ids.view(-1).long()], counts.long()[ids.view(-1).long()]
+    assert bool(((at >= lo) & (at < lo + n)).all())
+    h = _rand((cap, hidden), 5).cuda()
+    hq, hs = quant_ops.quant_fp8_segments(h, seg_off, counts, max(1, rows * top_k // experts))
+    want_q, want_s = quant_ops.quant_fp8_act(h)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(hq[at], want_q[at]) and torch.equal(hs[at], want_s[at])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n,k", [(130, 272), (5, 132), (1, 16), (300, 4)])
 def test_fp8_expansion_is_exact(n, k):
     from flyingfish_b200.ops import quant_ops
