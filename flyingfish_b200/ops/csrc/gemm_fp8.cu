@@ -38,7 +38,7 @@ __device__ __forceinline__ float bfr8(float x) { return __bfloat162float(__float
 // issued before the single wait, so the fixed latency of the wait -> load -> arrive chain is paid once per call.
 // acc[16 u + j] += partial[u][j] * scale[u][j], k-blocks in order (the summation order of the contract).
 template <int U, int P, int OFF, int NACC>
-__device__ __forceinline__ void fp8_promote(float (&acc)[NACC], const uint32_t (&taddr)[2], const float* const (&sp)[2],
+__device__ __forceinline__ void fp8_promote(float (&acc)[NACC], const uint32_t (&taddr)[2], const float* (&sp)[2],
                                             int nb) {
   uint32_t r[P][U][16];
 #pragma unroll
@@ -69,8 +69,14 @@ __device__ __forceinline__ void fp8_promote(float (&acc)[NACC], const uint32_t (
 // CTA needs few registers and half the shared memory so that two CTAs share an SM and one streams while the other sets up
 // or drains (an expert tile is short: 16 to 56 k-blocks). 256 experts of 7168 x 2048 with 50 rows each: gate/up and down together
 // 3488 us with chunks of 128, 2036 us with chunks of 64 (codes at the copy rate: 1730 us).
-template <int TOK>
-__global__ void __launch_bounds__(320, TOK <= 64 ? 2 : 1)
+// CTAS: CTAs per SM. P: K blocks promoted per round; a warp waits for a block, reads it, multiplies and hands it back, about 0.25 us one after the
+// other at 64 tokens, and two blocks in a round share the waits. A dense call of 33 to 64 tokens that does not fill two CTAs per SM has the
+// registers for it. Together with scale rows that lie 4 floats apart from a multiple of 32 in shared memory (staging them put 32 lanes on one
+// bank): 64 rows times 7168 x 16384 and 7168 x 18432 49 -> 41.5 us, 24576 x 1536 21.1 -> 18.9 (before: 53.5 us alone, 37.4 without
+// promotion, 39.7 without staging, 29.3 without both).
+constexpr int SX_PAD = 4;
+template <int TOK, int CTAS, int P>
+__global__ void __launch_bounds__(320, CTAS)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                 const float* __restrict__ w_scale, const float* __restrict__ x_scale, __nv_bfloat16* __restrict__ Y,
                 const int* __restrict__ seg_off, const int* __restrict__ counts, int M, int Nw, int K, int ldy,
@@ -88,7 +94,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   // staging is sized by the host for the tokens of this launch (tok_cap) and the k-blocks of one split: what it
   // does not take is pipeline depth, and the bytes in flight per SM are what bounds the weight stream
   __nv_bfloat16* sT = reinterpret_cast<__nv_bfloat16*>(smem);            // [tok_cap][128] bf16
-  float* sXs = reinterpret_cast<float*>(smem + tok_cap * FBM * 2);       // scale products [ntok][nkb]
+  float* sXs = reinterpret_cast<float*>(smem + tok_cap * FBM * 2);       // scale products [nkb][ntok + SX_PAD]
   uint8_t* pipe = smem + stage_off;
   constexpr int A_BYTES = FBM * FBK;                                     // 16 KiB of E4M3
   const int kblocks_total = (K + FBK - 1) / FBK;
@@ -210,7 +216,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int i = i0 + u * 256;
-          if (i < ntok * nkb) { const int t = i / nkb, kb = i - t * nkb; sXs[kb * ntok + t] = v[u]; }
+          if (i < ntok * nkb) { const int t = i / nkb, kb = i - t * nkb; sXs[kb * (ntok + SX_PAD) + t] = v[u]; }
         }
       }
       asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -218,21 +224,31 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 #pragma unroll
       for (int i = 0; i < TOK / 2; ++i) acc[i] = 0.f;
       const int nb = blk1 - blk0;
-      for (int kb = 0; kb < nkb && ok; ++kb, ++kit) {
-        const int b0 = kit & (nbuf - 1);
-        if (!mbar_wait(&bars.tmem_full[b0], (kit >> buf_shift) & 1, abort_flag, status, KID_GEMM_FP8, 4)) { ok = false; break; }
+      for (int kb = 0; kb < nkb && ok;) {
+        const int n = P == 2 && kb + 1 < nkb ? 2 : 1;
+        uint32_t taddr[2];
+        const float* sp[2];
+        const uint32_t lane_base = tmem_base + (uint32_t(q * 32) << 16) + blk0 * 16;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          const int b = (kit + p) & (nbuf - 1);
+          if (ok && p < n && !mbar_wait(&bars.tmem_full[b], ((kit + p) >> buf_shift) & 1, abort_flag, status, KID_GEMM_FP8, 4)) ok = false;
+          taddr[p] = lane_base + b * buf_cols;
+          sp[p] = sXs + (kb + p) * (ntok + SX_PAD) + blk0 * 16;
+        }
+        if (!ok) break;
         if (blockIdx.x == 0 && blockIdx.y == 0 && ee == 0) FF_TL(status, KID_GEMM_FP8, 30);
         tc_fence_after();
-        const uint32_t lane_base = tmem_base + (uint32_t(q * 32) << 16) + blk0 * 16;
-        const uint32_t taddr[2] = {lane_base + b0 * buf_cols, 0};
-        const float* const sp[2] = {sXs + kb * ntok + blk0 * 16, nullptr};
-        // (promoting two k-blocks per round was measured with chunks of 128: the extra registers spill under the 168-register cap
-        // of its ten warps and the kernel gets slower; chunks of 32 and 64 share an SM and have about 100)
-        fp8_promote<TOK / 32, 1, 0, TOK / 2>(acc, taddr, sp, nb);
+        // (two K blocks per round with chunks of 128: the extra registers spill under the 168-register cap of its ten warps and the kernel gets
+        // slower; chunks of 32 and 64 with two CTAs on an SM have about 100)
+        if (P == 2 && n == 2) fp8_promote<TOK / 32, P, 0, TOK / 2>(acc, taddr, sp, nb);
+        else fp8_promote<TOK / 32, 1, 0, TOK / 2>(acc, taddr, sp, nb);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.tmem_empty[b0]);
+        if (lane == 0)
+          for (int p = 0; p < n; ++p) mbar_arrive(&bars.tmem_empty[(kit + p) & (nbuf - 1)]);
         if (blockIdx.x == 0 && blockIdx.y == 0 && ee == 0) FF_TL(status, KID_GEMM_FP8, 31);
+        kb += n; kit += n;
       }
       if (!ok) break;
       bool final_here = true;
@@ -260,34 +276,50 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         final_here = bars.is_last != 0;
         if (final_here) {
           __threadfence();
-          // partials are added in split order (fixed summation order). Thread -> four adjacent columns and every
-          // eighth token: eight 16-byte loads of one split in flight per thread, the sums go straight into the staging tile
+          // partials are added in split order (fixed summation order). Thread -> four adjacent columns and every eighth token, four
+          // tokens at a time; SB splits' loads are in flight together and the sums go straight into the staging tile. One CTA adds the
+          // partials of a tile while the GPU waits for it: with one split of eight tokens in flight, fourteen splits of 576 x 7168
+          // at 64 tokens took the whole product 38 us, now 30.
+          constexpr int SB = TOK == 128 ? 4 : 2;
           const int c4 = (ee & 31) * 4, tg = ee >> 5;          // tg 0 .. 7
           const int ncol = tn * FBM + c4;
           const bool vec = (Nw & 3) == 0 && ncol + 3 < Nw;
-          for (int tb = 0; tb < ntok; tb += 64) {              // bands of 64 tokens: eight tokens per thread and band
-            float4 sum[8];
+          for (int tb = 0; tb < ntok; tb += 32) {              // bands of 32 tokens: four tokens per thread and band
+            float4 sum[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s = 0; s < splits; ++s) {
-              const float* ps = scratch + ((size_t)s * M + grow0) * Nw + ncol;
-              float4 v[8];
+            for (int j = 0; j < 4; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int s0 = 0; s0 < splits; s0 += SB) {
+              float4 v[SB][4];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const int t = tb + tg + 8 * j;
-                v[j] = (t < real && vec) ? __ldcg(reinterpret_cast<const float4*>(ps + (size_t)t * Nw))
-                                         : make_float4(0.f, 0.f, 0.f, 0.f);
-                if (t < real && !vec) {                        // ragged right edge, or rows that are not 16-byte aligned
-                  float e4[4] = {0.f, 0.f, 0.f, 0.f};
-                  for (int q2 = 0; q2 < 4 && ncol + q2 < Nw; ++q2) e4[q2] = __ldcg(ps + (size_t)t * Nw + q2);
-                  v[j] = make_float4(e4[0], e4[1], e4[2], e4[3]);
+              for (int u = 0; u < SB; ++u) {
+                const float* ps = scratch + ((size_t)(s0 + u) * M + grow0) * Nw + ncol;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const int t = tb + tg + 8 * j;
+                  v[u][j] = s0 + u < splits && t < real && vec ? __ldcg(reinterpret_cast<const float4*>(ps + (size_t)t * Nw)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
               }
 #pragma unroll
-              for (int j = 0; j < 8; ++j) { sum[j].x += v[j].x; sum[j].y += v[j].y; sum[j].z += v[j].z; sum[j].w += v[j].w; }
-            }
+              for (int u = 0; u < SB; ++u)
+                if (s0 + u < splits) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+                  for (int j = 0; j < 4; ++j) { sum[j].x += v[u][j].x; sum[j].y += v[u][j].y; sum[j].z += v[u][j].z; sum[j].w += v[u][j].w; }
+                }
+            }
+            if (!vec)                                          // ragged right edge, or rows that are not 16-byte aligned
+              for (int s1 = 0; s1 < splits; ++s1)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const int t = tb + tg + 8 * j;
+                  const float* ps = scratch + ((size_t)s1 * M + grow0 + t) * Nw + ncol;
+                  if (t >= real) continue;
+                  if (ncol < Nw) sum[j].x += __ldcg(ps);
+                  if (ncol + 1 < Nw) sum[j].y += __ldcg(ps + 1);
+                  if (ncol + 2 < Nw) sum[j].z += __ldcg(ps + 2);
+                  if (ncol + 3 < Nw) sum[j].w += __ldcg(ps + 3);
+                }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
               const int t = tb + tg + 8 * j;
               if (t < ntok) {
                 __nv_bfloat162* d = reinterpret_cast<__nv_bfloat162*>(sT + t * FBM + c4);
@@ -376,8 +408,9 @@ static int gemm_fp8_launch(const void* xq, const float* x_scale, const void* wq,
   if (ldy % 8 || (reinterpret_cast<uintptr_t>(y) & 15)) return FF_HOST_BAD_ALIGN;
   // Grouped calls take the smallest chunk that most segments fit into: 32 tokens up to an average of 8 rows per expert, 64 up to 52 (M
   // counts 16 rows of padding for each; random segments of that average exceed 64 in one case of twenty, which then streams its weights twice).
-  const int chunk = experts > 1 ? ((long long)M <= 24ll * experts ? 32 : (long long)M <= 68ll * experts ? 64 : F_TOK) : (M <= 32 ? 32 : fp8_paired(M, (Nw + FBM - 1) / FBM) ? 64 : F_TOK);
-  const bool small = chunk < F_TOK;
+  const int chunk = experts > 1 ? ((long long)M <= 24ll * experts ? 32 : (long long)M <= 68ll * experts ? 64 : F_TOK) : (M <= 32 ? 32 : M <= 64 ? 64 : F_TOK);
+  const bool single = experts == 1 && chunk == 64 && !fp8_paired(M, (Nw + FBM - 1) / FBM);      // dense, 33 to 64 tokens, one CTA per SM
+  const bool small = chunk < F_TOK && !single;
   const int tok_cap = experts > 1 ? chunk : (M >= F_TOK ? F_TOK : (M + 15) / 16 * 16);
   const int per = ((K / 128) + splits - 1) / splits;                     // k-blocks of one split
   if (per * tok_cap * 4 > 64 * 1024) return FF_HOST_TOO_LARGE;           // scale staging
@@ -386,12 +419,12 @@ static int gemm_fp8_launch(const void* xq, const float* x_scale, const void* wq,
   if (r) return r;
   r = make_tmap_2d(&tmX, xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, M, (uint64_t)ldxq, FBK, 16);
   if (r) return r;
-  const int staging = (tok_cap * FBM * 2 + per * tok_cap * 4 + 1023) / 1024 * 1024;
+  const int staging = (tok_cap * FBM * 2 + per * (tok_cap + SX_PAD) * 4 + 1023) / 1024 * 1024;
   const int budget = small ? 110 * 1024 : 224 * 1024;
   int pipe_bytes = budget - staging;
   const int smem = staging + pipe_bytes + 1024;
   dim3 grid((Nw + FBM - 1) / FBM, splits, experts);
-  auto kern = chunk == 32 ? gemm_fp8_kernel<32> : chunk == 64 ? gemm_fp8_kernel<64> : gemm_fp8_kernel<F_TOK>;
+  auto kern = chunk == 32 ? gemm_fp8_kernel<32, 2, 1> : single ? gemm_fp8_kernel<64, 1, 2> : chunk == 64 ? gemm_fp8_kernel<64, 2, 1> : gemm_fp8_kernel<F_TOK, 1, 1>;
   r = opt_in_smem(kern, budget + 1024); if (r) return r;
   if (int lr = launch_pdl(kern, grid, dim3(320), smem, s, 0, tmW, tmX, w_scale, x_scale, (__nv_bfloat16*)y, seg_off, counts, M, Nw, K, ldy, epi,
                           splits, pipe_bytes, staging, tok_cap, scratch, tile_counters, status, xs_ld)) return lr;

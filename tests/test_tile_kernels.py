@@ -212,6 +212,24 @@ def test_quantised_rows_dispatched(rows, hidden, experts, top_k):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 16, 33, 64, 100])
+@pytest.mark.parametrize("n,k", [(576, 7168), (136, 2048), (1536, 1152)])       # fourteen, four and two splits, a ragged edge
+def test_fp8_partials_of_many_splits(m, n, k):
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import quant_ops
+    x = _rand((m, k), m)
+    codes, scale = qref.quantize_fp8_block_weight(_rand((n, k), n).float())
+    y = quant_ops.linear_fp8(x.cuda(), codes.cuda(), scale.cuda())
+    torch.cuda.synchronize()
+    ops.check_status()
+    xq, xs = qref.quantize_fp8_act(x)
+    wide = lambda c: c.view(torch.float8_e4m3fn).double()
+    want = (wide(xq) * xs.double().repeat_interleave(128, 1)[:, :k]) @ (wide(codes) * scale.double().repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)[:, :k]).t()
+    # one rounding of the result; the products of a K block are aligned to its largest partial sum (13 bits, a few times root 128)
+    assert ((y.cpu().double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -11 * k ** 0.5).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n,k", [(130, 272), (5, 132), (1, 16), (300, 4)])
 def test_fp8_expansion_is_exact(n, k):
     from flyingfish_b200.ops import quant_ops
