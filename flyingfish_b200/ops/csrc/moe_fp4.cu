@@ -57,14 +57,18 @@ __device__ __forceinline__ bool f4_sync_any(bool mine) {
 __device__ __forceinline__ float f4_silu(float x) { return x / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float f4_bfr(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
-// Eight codes of a word (low nibble first) times a scale: pairs (0, 4), (1, 5), (2, 6), (3, 7), which share a shift each
+// Eight codes of a word (low nibble first) times a scale: pairs (0, 4), (1, 5), (2, 6), (3, 7), one code per half. A code n alone in its half, times
+// 2^6 + 2^12, has its magnitude at bits 8..6 and its sign at bit 15, and nothing of it reaches the other half: one multiplication, which the FMA pipe
+// does, takes the place of two shifts and a merge on the ALU, whose half rate is what expanding is bound by (17 ALU operations a word
+// with shifts, 9 so). The products of 32
+// sequences over 128 experts of 4096 x 1536: 198 -> 187 us on average.
 __device__ __forceinline__ void f4_expand8(uint32_t w, __nv_bfloat162 sv, uint32_t (&p)[4]) {
-  constexpr uint32_t MAG = 0x01C001C0u, SGN = 0x80008000u;
+  constexpr uint32_t KEEP = 0x81C081C0u;
   const uint32_t h = w >> 8;
-  p[0] = ((w << 6) & MAG) | ((w << 12) & SGN);
-  p[1] = ((w << 2) & MAG) | ((w << 8) & SGN);
-  p[2] = ((h << 6) & MAG) | ((h << 12) & SGN);
-  p[3] = ((h << 2) & MAG) | ((h << 8) & SGN);
+  p[0] = ((w & 0x000F000Fu) * 0x1040u) & KEEP;
+  p[1] = ((w & 0x00F000F0u) * 0x0104u) & KEEP;
+  p[2] = ((h & 0x000F000Fu) * 0x1040u) & KEEP;
+  p[3] = ((h & 0x00F000F0u) * 0x0104u) & KEEP;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&p[i]), sv);
