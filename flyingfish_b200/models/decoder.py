@@ -106,7 +106,8 @@ class DecoderModel:
             return self._hidden_states_sp(b, kv)
         if self._chain_ok(b):
             return self._hidden_states_chain(b, kv, inputs_embeds)
-        if b.positions.is_cuda and b.positions.shape[0] <= ops.SKINNY_MAX_M and self.d == 128 and not s.qk_norm:
+        if b.positions.is_cuda and self.d == 128 and not s.qk_norm and \
+                (b.positions.shape[0] <= ops.SKINNY_MAX_M or type(self)._attention is DecoderModel._attention):
             # one cos/sin table per step for the fused QKV + rotary + KV-write kernels of all layers
             self._rope_cs = ops.rope_table(b.positions, self.d, s.rope_theta)
         if inputs_embeds is None:

@@ -475,12 +475,12 @@ def linear_rope_kv(x: torch.Tensor, wqkv: torch.Tensor, positions: torch.Tensor,
                    rot_dim: int | None = None, inv_freq: torch.Tensor | None = None,
                    cos_sin: torch.Tensor | None = None) -> torch.Tensor:
     """Fused QKV projection + rotary embedding + paged KV write: ``qkv = x @ wqkv.T`` with Q and K
-    rotated and K/V stored at ``slots``. Decode shapes with 128-dim heads run as one kernel (the
+    rotated and K/V stored at ``slots``. 128-dim heads run as one kernel (the
     rotation and the cache write are the GEMM's epilogue; ``cos_sin`` from :func:`rope_table` is
     reused across layers); everything else as GEMM + rope kernel."""
     m = x.shape[0]
     n = wqkv.shape[0]
-    fused = (FUSE_ROPE and _is_cuda(x) and m <= SKINNY_MAX_M and dim == 128 and n == (hq + 2 * hkv) * 128 and x.dtype == BF16
+    fused = (FUSE_ROPE and _is_cuda(x) and dim == 128 and n == (hq + 2 * hkv) * 128 and x.dtype == BF16
              and kcache.dim() == 4 and kcache.is_contiguous() and vcache.is_contiguous())
     if not fused:
         qkv = linear(x, wqkv)
@@ -494,15 +494,21 @@ def linear_rope_kv(x: torch.Tensor, wqkv: torch.Tensor, positions: torch.Tensor,
     k = x.shape[1]
     out = torch.empty(m, n, dtype=BF16, device=x.device)
     lib = kernels()
+    if cos_sin is None:
+        cos_sin = rope_table(positions, rot_dim or dim, theta, inv_freq)
+    _require(cos_sin.shape == (m, (rot_dim or dim) // 2, 2) and cos_sin.is_contiguous(), "linear_rope_kv: cos/sin table shape")
+    if m > SKINNY_MAX_M:
+        rc = lib.ff_gemm_bf16_rope_kv(ptr(x), ptr(wqkv), ptr(out), m, n, k, ldx, ldw, n, ptr(cos_sin), ptr(slots), ptr(kcache), ptr(vcache), hq, hkv,
+                                      rot_dim or dim, bs, nb, ptr(status_tensor(x.device)), stream_ptr())
+        check(rc, "ff_gemm_bf16_rope_kv")
+        _count()
+        return out
     scratch_b, counter_b = c_longlong(0), c_longlong(0)
     grid = lib.ff_gemm_skinny_plan_epi(m, n, k, 2, ctypes.byref(scratch_b), ctypes.byref(counter_b))
     check(min(grid, 0), "ff_gemm_skinny_plan_epi")
     ws = workspace(x.device)
     scratch = ws.ensure("gemm_scratch", scratch_b.value // 4) if scratch_b.value > 0 else None
     _require(counter_b.value // 4 <= ws.gemm_counters.numel(), "linear_rope_kv: too many column tiles for counters")
-    if cos_sin is None:
-        cos_sin = rope_table(positions, rot_dim or dim, theta, inv_freq)
-    _require(cos_sin.shape == (m, (rot_dim or dim) // 2, 2) and cos_sin.is_contiguous(), "linear_rope_kv: cos/sin table shape")
     rc = lib.ff_gemm_skinny_rope_kv(ptr(x), ptr(wqkv), ptr(out), m, n, k, ldx, ldw, n, grid, ptr(scratch),
                                     ptr(ws.gemm_counters), ptr(cos_sin), ptr(slots), ptr(kcache), ptr(vcache),
                                     hq, hkv, rot_dim or dim, bs, nb, ptr(status_tensor(x.device)), stream_ptr())

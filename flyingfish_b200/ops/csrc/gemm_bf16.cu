@@ -93,7 +93,7 @@ __device__ __forceinline__ bool next_tile(const GroupArgs& g, TileWalk& w, int t
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 
-// epi: 0 = store bf16; 1 = SwiGLU (every 128 columns of a tile are 64 gate then the matching 64 up columns; output
+// epi: 3 = rotary embedding and cache write (LinTail); 0 = store bf16; 1 = SwiGLU (every 128 columns of a tile are 64 gate then the matching 64 up columns; output
 // has N/2 columns); 2 = store fp32.
 // COMM (tensor-parallel prefill, rows split evenly over the ranks in 128-row blocks):
 //   1 = all-gather -> GEMM : A is row-sharded. Four extra warps per CTA (all CTAs together) push this
@@ -133,17 +133,22 @@ struct LinTail {
   const __nv_bfloat16* bias; int act;
   const __nv_bfloat16* mul; const int* mul_rows; int ldm, mul_table;
   int gate; float limit;
+  // epi 3: rotation of q and k heads and the paged cache write behind a QKV product with heads of 128
+  const float2* cos_sin;               // [rows, rhalf], rounded to BF16 (ff_rope_table)
+  const int* slots;
+  __nv_bfloat16 *kcache, *vcache;
+  int hq, hkv, rhalf, block_size, num_blocks;
 };
 
 constexpr int RS_STG_PITCH = 144, RS_STG_BYTES = 32 * RS_STG_PITCH;   // COMM 2 epilogue staging, per warp
 constexpr int COMM_PARTS = 4;       // a 128-row block is pushed (COMM 1) / reduced (COMM 2) in this many pieces
 
 // An epilogue thread's row of a finished tile: tensor memory -> registers -> global. row: row of the result, stored where `live`; col0: first
-// of the tile's `width` columns (a multiple of 32, of 128 with epi 1), N: columns (of the head), col_off: first column of the head. The PARTS
+// of the tile's `width` columns (a multiple of 32, of 128 with epi 1 and 3), N: columns (of the head), col_off: first column of the head. The PARTS
 // warps that share the row take turns with its groups of columns.
 template <int PARTS>
 __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict__ Cout, int row, bool live, int ldc, int N, int epi, int col0,
-                                               int width, size_t col_off, const LinTail& tail, int part) {
+                                               int width, size_t col_off, const LinTail& tail, int part, int* status) {
   if (epi == 1) {
     const int half = width / 2, out0 = col0 / 2;
     __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + out0;
@@ -180,6 +185,62 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
               const uint32_t w = o[j >> 1];
               reinterpret_cast<uint16_t*>(crow + c)[j] = (j & 1) ? uint16_t(w >> 16) : uint16_t(w & 0xffff);
             }
+        }
+      }
+    }
+  } else if (epi == 3) {
+    // The values are rounded to BF16 and turned in BF16 arithmetic, as the rotation kernel turns the stored rows: the bits are the same. A pass
+    // over the rows of its own took 72 us of a layer at 8121 rows (32 + 16 heads) and 11 at 1000; here it runs under the next tile's main loop.
+#pragma unroll 1
+    for (int h0 = 0; h0 < width; h0 += 128) {
+      const int head = (col0 + h0) >> 7;
+      if (head >= tail.hq + 2 * tail.hkv) break;
+      const bool is_v = head >= tail.hq + tail.hkv;
+      __nv_bfloat16* cached = nullptr;
+      if (live && head >= tail.hq) {
+        const int slot = tail.slots[row], blk = slot / tail.block_size, kvh = is_v ? head - tail.hq - tail.hkv : head - tail.hq;
+        if (slot >= 0 && blk >= tail.num_blocks) { if (part == 0) set_status(status, KID_ROPE_KV, FF_ERR_BOUNDS, row, slot); }
+        else if (slot >= 0) {                             // a negative slot: a padding row, nothing cached
+          if (part == 0) dbg_write_once(status, KID_ROPE_KV, is_v ? DBG_KV_V : DBG_KV_K, (long long)slot * tail.hkv + kvh);
+          cached = (is_v ? tail.vcache : tail.kcache) + (((size_t)blk * tail.hkv + kvh) * tail.block_size + (slot - blk * tail.block_size)) * 128;
+        }
+      }
+      __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + col0 + h0;
+#pragma unroll 1
+      for (int c = 16 * part; c < 64; c += 16 * PARTS) {
+        uint32_t a[16], b[16];
+        tmem_ld_x16(taddr + h0 + c, a);
+        tmem_ld_x16(taddr + h0 + c + 64, b);
+        tmem_ld_wait();
+        if (live) {
+          auto r = [](float x) { return __bfloat162float(__float2bfloat16(x)); };
+          uint32_t lo[8], hi[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float x[2], y[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              x[e] = r(__uint_as_float(a[2 * j + e]));
+              y[e] = r(__uint_as_float(b[2 * j + e]));
+              if (!is_v && c + 2 * j + e < tail.rhalf) {
+                const float2 t = __ldg(tail.cos_sin + (size_t)row * tail.rhalf + c + 2 * j + e);
+                const float u = x[e], v = y[e];
+                x[e] = r(u * t.x) - r(v * t.y);
+                y[e] = r(v * t.x) + r(u * t.y);
+              }
+            }
+            lo[j] = pack_bf16x2(x[0], x[1]);
+            hi[j] = pack_bf16x2(y[0], y[1]);
+          }
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            __nv_bfloat16* dst = k ? cached : crow;
+            if (dst == nullptr) continue;
+            reinterpret_cast<uint4*>(dst + c)[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            reinterpret_cast<uint4*>(dst + c)[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+            reinterpret_cast<uint4*>(dst + 64 + c)[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            reinterpret_cast<uint4*>(dst + 64 + c)[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+          }
         }
       }
     }
@@ -427,7 +488,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tma_store_wait<0>();                              // every row of this tile has landed in the owner's slot
           asm volatile("fence.proxy.async;" ::: "memory");
       } else {
-        store_tile_row<COMM ? 1 : 2>(taddr, Cout, row, row < row_end, ldc, N, epi, tn * BN, BN, (size_t)head * ga.c_cols, tail, COMM ? 0 : (warp - 2) >> 2);
+        store_tile_row<COMM ? 1 : 2>(taddr, Cout, row, row < row_end, ldc, N, epi, tn * BN, BN, (size_t)head * ga.c_cols, tail, COMM ? 0 : (warp - 2) >> 2, status);
       }
       tc_fence_before();
       __syncwarp();
@@ -581,7 +642,7 @@ struct alignas(8) PairBars {
 
 // A ring as deep as shared memory takes (7 stages 256 wide, 11 stages 64 wide: 200 rows times 4096 x 14336 50.6 -> 40.0 us) and two epilogue warps
 // per 32 rows, since the last tile's epilogue is not hidden: 130 x 4096 x 4096 17.5 -> 16.1 us.
-// Tiles of a launch: `wide` columns of tiles w1 wide, then tiles w2 wide up to N; every width a multiple of 32 (of 128 with epi 1), at most 256.
+// Tiles of a launch: `wide` columns of tiles w1 wide, then tiles w2 wide up to N; every width a multiple of 32 (of 128 with epi 1 and 3), at most 256.
 struct PairTiles { int w1, wide, w2; };
 
 // tile t: row tile, first column and width. The wide tiles come first, the narrow ones fill the last wave.
@@ -686,7 +747,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (!ok) break;
       tc_fence_after();
       const int row = (2 * tm + rank) * BM + q * 32 + lane;
-      store_tile_row<2>(tmem_base + (uint32_t(q * 32) << 16) + acc * 256, Cout, row, row < M, ldc, N, epi, col0, width, 0, tail, (warp - 2) >> 2);
+      store_tile_row<2>(tmem_base + (uint32_t(q * 32) << 16) + acc * 256, Cout, row, row < M, ldc, N, epi, col0, width, 0, tail, (warp - 2) >> 2, status);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(&bars.tmem_empty[acc]);
@@ -718,7 +779,7 @@ static float pair_cost(int w) { return w >= 128 ? 178.0f + 1.46f * w : 291.0f + 
 // times 6144 x 4096 (18 columns of 224, the rest of 128 wide) 42.9 -> 40.3 us, 700 x 4096 x 14336 (192 wide) 77.9 -> 66.5, 2039 x 7168 x 18432 529 ->
 // 413, 2500 x 4096 x 14336 256 -> 219. K is walked in the same order in tiles of all widths: the bits are the same.
 static float pair_plan(int M, int N, int epi, int pairs, PairTiles& best) {
-  const int step = epi == 1 ? 128 : 32, tiles_m = (M + 2 * BM - 1) / (2 * BM);
+  const int step = epi == 1 || epi == 3 ? 128 : 32, tiles_m = (M + 2 * BM - 1) / (2 * BM);
   float least = 0.f;
   for (int w1 = 256; w1 >= 64; w1 -= step) {
     const int cols = (N + w1 - 1) / w1, full = cols * tiles_m / pairs;
@@ -741,7 +802,7 @@ static float pair_plan(int M, int N, int epi, int pairs, PairTiles& best) {
 
 // the plan as {w1, wide, w2} (host only)
 FF_EXPORT int ff_gemm_bf16_pair_tiles(int M, int N, int epi, int pairs, int* tiles) {
-  if (M <= 0 || N <= 0 || pairs <= 0 || epi < 0 || epi > 2) return FF_HOST_BAD_SHAPE;
+  if (M <= 0 || N <= 0 || pairs <= 0 || epi < 0 || epi > 3) return FF_HOST_BAD_SHAPE;
   PairTiles pt;
   pair_plan(M, N, epi, pairs, pt);
   tiles[0] = pt.w1; tiles[1] = pt.wide; tiles[2] = pt.w2;
@@ -815,6 +876,20 @@ FF_EXPORT int ff_gemm_bf16_act(const void* X, const void* W, void* Y, int M, int
   return gemm_bf16_launch(X, W, Y, M, N, K, ldx, ldw, ldy, 0,
                           LinTail{static_cast<const __nv_bfloat16*>(bias), act, static_cast<const __nv_bfloat16*>(mul), mul_rows, ldm, mul_table, 0},
                           status, stream);
+}
+
+// QKV product with rotary embedding and paged cache write in the epilogue (heads of 128, N = (hq + 2 hkv) * 128): the bits of ff_gemm_bf16 and
+// ff_rope_kv_paged. cos_sin: [M, rot_dim / 2] pairs from ff_rope_table; caches [blocks, hkv, block_size, 128]; negative slots are skipped.
+FF_EXPORT int ff_gemm_bf16_rope_kv(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw, int ldy, const float* cos_sin,
+                                   const int* slots, void* kcache, void* vcache, int hq, int hkv, int rot_dim, int block_size, int num_blocks,
+                                   int* status, cudaStream_t stream) {
+  if (hq <= 0 || hkv <= 0 || N != (hq + 2 * hkv) * 128 || rot_dim <= 0 || rot_dim > 128 || rot_dim % 2 || block_size <= 0 || num_blocks <= 0) return FF_HOST_BAD_SHAPE;
+  if (cos_sin == nullptr || slots == nullptr || ((reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15)) return FF_HOST_BAD_ALIGN;
+  LinTail tail = {};
+  tail.cos_sin = reinterpret_cast<const float2*>(cos_sin); tail.slots = slots;
+  tail.kcache = static_cast<__nv_bfloat16*>(kcache); tail.vcache = static_cast<__nv_bfloat16*>(vcache);
+  tail.hq = hq; tail.hkv = hkv; tail.rhalf = rot_dim / 2; tail.block_size = block_size; tail.num_blocks = num_blocks;
+  return gemm_bf16_launch(X, W, Y, M, N, K, ldx, ldw, ldy, 3, tail, status, stream);
 }
 
 // Gate/up projection (rows interleaved per 64) with the activation in the epilogue, rounded once. gate 3: tanh-GELU(gate) * up, 5: the

@@ -327,6 +327,29 @@ def test_merge_of_many_splits(ctx):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m", [129, 300, 1000])
+@pytest.mark.parametrize("hq,hkv,k,rot", [(8, 2, 1024, 128), (32, 8, 256, 128), (5, 1, 520, 64)])      # tiles of pairs and of single CTAs, a part turned
+def test_rotation_in_the_product_of_prompts(m, hq, hkv, k, rot):
+    """The bits of the product followed by the rotation kernel, in the rows and in the cache; padding rows are not cached."""
+    from flyingfish_b200 import ops
+    n, blocks = (hq + 2 * hkv) * 128, 20
+    x, w = _rand((m, k), 1).cuda(), (_rand((n, k), 2) * 0.1).cuda()
+    g = torch.Generator().manual_seed(m)
+    pos = torch.randint(0, 9000, (m,), generator=g).to(torch.int32).cuda()
+    slots = torch.randperm(blocks * 64, generator=g)[:m].to(torch.int32)
+    slots[::7] = -1
+    slots = slots.cuda()
+    cache = lambda: [torch.full((blocks, hkv, 64, 128), 3.0, dtype=BF16, device="cuda") for _ in range(2)]
+    (k0, v0), (k1, v1) = cache(), cache()
+    want = ops.linear(x, w)
+    ops.rope_kv_paged(want, pos, slots, k0, v0, hq, hkv, 128, 5e5, rot)
+    got = ops.linear_rope_kv(x, w, pos, slots, k1, v1, hq, hkv, 128, 5e5, rot)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(got, want) and torch.equal(k0, k1) and torch.equal(v0, v1)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("lens,hq,hkv", [
     ([0, 1, 64, 65, 320, 321, 384, 640], 8, 2),              # padding, whole pages, one page more; one split and several in a launch
     ([2000, 63, 700], 16, 1),                                # more than eight splits beside one
