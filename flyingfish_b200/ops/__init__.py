@@ -482,6 +482,9 @@ def linear_rope_kv(x: torch.Tensor, wqkv: torch.Tensor, positions: torch.Tensor,
     n = wqkv.shape[0]
     fused = (FUSE_ROPE and _is_cuda(x) and dim == 128 and n == (hq + 2 * hkv) * 128 and x.dtype == BF16
              and kcache.dim() == 4 and kcache.is_contiguous() and vcache.is_contiguous())
+    if m > SKINNY_MAX_M and fused:                       # what the two kernels take and the one does not
+        fused = (type(wqkv) is torch.Tensor and wqkv.dtype == kcache.dtype == vcache.dtype == BF16 and wqkv.shape[1] == x.shape[1] and
+                 (kcache.data_ptr() | vcache.data_ptr()) % 16 == 0)
     if not fused:
         qkv = linear(x, wqkv)
         rope_kv_paged(qkv, positions, slots, kcache, vcache, hq, hkv, dim, theta, rot_dim, inv_freq)
@@ -889,6 +892,67 @@ def attn_prefill(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, bl
     check(rc, "ff_attn_prefill")
     _count()
     return out
+
+
+# ------------------------------------------------------------------------------------------
+# the layers of a dense decoder over prompt rows in one call
+# ------------------------------------------------------------------------------------------
+class _DenseLayer(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("wqkv", "wo", "post_ln", "wgu", "wdown", "next_ln", "kcache", "vcache")]
+
+
+class _DenseStack(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("x", "n", "qkv", "att", "mid", "o", "cos_sin", "slots", "block_table", "q_start", "q_lens",
+                                        "ctx_lens", "scratch", "counters", "status")] + \
+               [(n, c_longlong) for n in ("scratch_bytes", "counter_bytes")] + \
+               [(n, c_int) for n in ("layers", "rows", "hidden", "ffn", "hq", "hkv", "batch", "max_q_len", "max_blocks", "num_blocks", "window")] + \
+               [(n, c_float) for n in ("scale", "eps")]
+
+
+def dense_stack(x: torch.Tensor, n: torch.Tensor, layers: list[tuple[torch.Tensor, ...]], positions: torch.Tensor, slots: torch.Tensor,
+                block_table: torch.Tensor, q_start: torch.Tensor, q_lens: torch.Tensor, ctx_lens: torch.Tensor, max_q_len: int, hq: int, hkv: int,
+                ffn: int, scale: float, eps: float, theta: float, window: int = 0, cos_sin: torch.Tensor | None = None) -> torch.Tensor | None:
+    """Layers of :func:`linear_rope_kv`, :func:`attn_prefill`, :func:`linear`, :func:`add_rmsnorm`, :func:`linear_swiglu`, :func:`linear` and
+    :func:`add_rmsnorm` over prompt rows, launched by one native call: the same kernels, the same bits. ``x`` [rows, hidden]: the residual, updated in
+    place; ``n``: its normed rows, overwritten and returned. A layer: (wqkv, wo, post_ln, wgu interleaved, wdown, next_ln, K cache, V cache),
+    contiguous BF16, heads and cache rows of 128 elements, pages of 64; None, and nothing launched, where a layer is anything else. ``cos_sin``:
+    :func:`rope_table` of the positions, if it is there already."""
+    rows, hidden = x.shape
+    qkv_dim, att_dim = (hq + 2 * hkv) * 128, hq * 128
+    _require(x.is_cuda and x.shape == n.shape and x.dtype == n.dtype == BF16 and x.is_contiguous() and n.is_contiguous(), "dense_stack: contiguous BF16 rows")
+    cache = layers[0][6].shape
+    shapes = ((qkv_dim, hidden), (hidden, att_dim), (hidden,), (2 * ffn, hidden), (hidden, ffn), (hidden,), cache, cache)
+    if hidden % 8 or ffn % 128 or len(cache) != 4 or cache[1:] != (hkv, 64, 128):
+        return None
+    table = (_DenseLayer * len(layers))()
+    for entry, tensors in zip(table, layers):
+        at = []
+        for t, shape in zip(tensors, shapes):
+            if type(t) is not torch.Tensor or t.dtype is not BF16 or t.shape != shape or not t.is_contiguous() or not t.is_cuda:
+                return None
+            at.append(t.data_ptr())
+            if at[-1] % 16:
+                return None
+        entry.wqkv, entry.wo, entry.post_ln, entry.wgu, entry.wdown, entry.next_ln, entry.kcache, entry.vcache = at
+    meta = (positions, slots, block_table, q_start, q_lens, ctx_lens)
+    _require(all(t.is_cuda and t.dtype == torch.int32 and t.is_contiguous() for t in meta) and positions.numel() == slots.numel() == rows and
+             block_table.shape[0] == q_start.numel() == q_lens.numel() == ctx_lens.numel(), "dense_stack: int32 metadata")
+    lib, ws = kernels(), workspace(x.device)
+    sb, cb = c_longlong(0), c_longlong(0)
+    check(lib.ff_dense_stack_workspace(rows, hidden, ffn, hq, hkv, ctypes.byref(sb), ctypes.byref(cb)), "ff_dense_stack_workspace")
+    scratch = ws.ensure("gemm_scratch", sb.value // 4)
+    if cos_sin is None:
+        cos_sin = rope_table(positions, 128, theta)
+    _require(cos_sin.shape == (rows, 64, 2) and cos_sin.is_contiguous() and cos_sin.dtype == torch.float32, "dense_stack: rotation table")
+    new = lambda width: torch.empty(rows, width, dtype=BF16, device=x.device)
+    qkv, att, mid, o = new(qkv_dim), new(att_dim), new(ffn), new(hidden)
+    at = lambda t: None if t is None else t.data_ptr()
+    form = _DenseStack(*(at(t) for t in (x, n, qkv, att, mid, o, cos_sin, *meta[1:], scratch, ws.gemm_counters, status_tensor(x.device))),
+                       scratch.numel() * 4, ws.gemm_counters.numel() * 4, len(layers), rows, hidden, ffn, hq, hkv, block_table.shape[0], max_q_len,
+                       block_table.shape[1], cache[0], window, scale, eps)
+    check(lib.ff_dense_stack(table, ctypes.byref(form), stream_ptr()), "ff_dense_stack")
+    _count(7 * len(layers))
+    return n
 
 
 # ------------------------------------------------------------------------------------------

@@ -1,0 +1,107 @@
+// The layers of a dense decoder over a batch of prompt rows, launched by one call: per layer QKV product with rotation and cache write, attention, O
+// product, residual and norm, gate/up product with SwiGLU, down product, residual and norm -- the launchers that the operators of the
+// Python side call one by one, in the same order and with the same arguments. Nothing is computed here. What it is for: a launch through the
+// operators takes 20 us of host time, so that prompts of up to a hundred rows were bound by the host (37 rows, 8 layers of an 8B-sized stack: 64
+// launches, 1519 -> 1283 us a call).
+#include "host_util.h"
+#include <stddef.h>
+
+#pragma GCC visibility push(default)      // as where they are defined
+extern "C" {
+int ff_gemm_skinny_plan(int, int, int, long long*, long long*);
+int ff_gemm_skinny_plan_epi(int, int, int, int, long long*, long long*);
+int ff_gemm_skinny(const void*, const void*, void*, int, int, int, int, int, int, int, float*, int*, int*, cudaStream_t);
+int ff_gemm_skinny_swiglu(const void*, const void*, void*, int, int, int, int, int, int, int, float*, int*, int, float, int*, cudaStream_t);
+int ff_gemm_skinny_rope_kv(const void*, const void*, void*, int, int, int, int, int, int, int, float*, int*, const float*, const int*, void*, void*, int, int,
+                           int, int, int, int*, cudaStream_t);
+int ff_gemm_bf16(const void*, const void*, void*, int, int, int, int, int, int, int, int*, cudaStream_t);
+int ff_gemm_bf16_rope_kv(const void*, const void*, void*, int, int, int, int, int, int, const float*, const int*, void*, void*, int, int, int, int, int, int*,
+                         cudaStream_t);
+int ff_attn_prefill_tc(const void*, const void*, const void*, const int*, const int*, const int*, const int*, void*, int, int, int, int, int, int, int, int, int,
+                       int, int, float, int, int, const float*, const void*, int, int, int, float, const void*, int, int*, cudaStream_t);
+int ff_add_rmsnorm(const void*, void*, const void*, void*, void*, int, int, int, int, float, int, int*, cudaStream_t);
+}
+#pragma GCC visibility pop
+
+using namespace ff;
+
+struct FfDenseLayer { const void *wqkv, *wo, *post_ln, *wgu, *wdown, *next_ln; void *kcache, *vcache; };
+
+// x: residual rows [rows, hidden], n: normed rows, in and out; qkv, att, mid, o: rows of (hq + 2 hkv) * 128, hq * 128, ffn and hidden elements.
+// cos_sin: rotation table of the rows (ff_rope_table).
+struct FfDenseStack {
+  void *x, *n, *qkv, *att, *mid, *o;
+  const float* cos_sin;
+  const int *slots, *block_table, *q_start, *q_lens, *ctx_lens;
+  float* scratch;
+  int* counters;
+  int* status;
+  long long scratch_bytes, counter_bytes;
+  int layers, rows, hidden, ffn, hq, hkv, batch, max_q_len, max_blocks, num_blocks, window;
+  float scale, eps;
+};
+
+static const int DENSE_SKINNY = 128;       // rows up to which the decode product serves
+
+// scratch of the decode products of a stack's shapes, in bytes
+FF_EXPORT int ff_dense_stack_workspace(int rows, int hidden, int ffn, int hq, int hkv, long long* scratch_bytes, long long* counter_bytes) {
+  *scratch_bytes = *counter_bytes = 0;
+  if (rows <= 0 || rows > DENSE_SKINNY) return rows <= 0 ? FF_HOST_BAD_SHAPE : FF_HOST_OK;
+  auto take = [&](int grid, long long sb, long long cb) {
+    if (sb > *scratch_bytes) *scratch_bytes = sb;
+    if (cb > *counter_bytes) *counter_bytes = cb;
+    return grid < 0 ? grid : FF_HOST_OK;
+  };
+  long long sb = 0, cb = 0;
+  int g = ff_gemm_skinny_plan_epi(rows, (hq + 2 * hkv) * 128, hidden, 2, &sb, &cb);
+  if (int r = take(g, sb, cb)) return r;
+  g = ff_gemm_skinny_plan(rows, hidden, hq * 128, &sb, &cb);
+  if (int r = take(g, sb, cb)) return r;
+  g = ff_gemm_skinny_plan_epi(rows, 2 * ffn, hidden, 1, &sb, &cb);
+  if (int r = take(g, sb, cb)) return r;
+  g = ff_gemm_skinny_plan(rows, hidden, ffn, &sb, &cb);
+  return take(g, sb, cb);
+}
+
+FF_EXPORT int ff_dense_stack(const FfDenseLayer* layers, const FfDenseStack* a, cudaStream_t s) {
+  if (layers == nullptr || a == nullptr || a->layers <= 0 || a->rows <= 0 || a->hidden % 8 || a->ffn % 128 || a->hq <= 0 || a->hkv <= 0 || a->cos_sin == nullptr) return FF_HOST_BAD_SHAPE;
+  const int rows = a->rows, hidden = a->hidden, ffn = a->ffn, qkv_dim = (a->hq + 2 * a->hkv) * 128, att_dim = a->hq * 128;
+  const bool few = rows <= DENSE_SKINNY;
+  if (few) {
+    long long sb = 0, cb = 0;
+    if (int r = ff_dense_stack_workspace(rows, hidden, ffn, a->hq, a->hkv, &sb, &cb)) return r;
+    if (sb > a->scratch_bytes || cb > a->counter_bytes) return FF_HOST_TOO_LARGE;
+  }
+  auto product = [&](const void* x, const void* w, void* y, int n, int k) -> int {
+    if (!few) return ff_gemm_bf16(x, w, y, rows, n, k, k, k, n, 0, a->status, s);
+    const int grid = ff_gemm_skinny_plan(rows, n, k, nullptr, nullptr);
+    return grid < 0 ? grid : ff_gemm_skinny(x, w, y, rows, n, k, k, k, n, grid, a->scratch, a->counters, a->status, s);
+  };
+  for (int i = 0; i < a->layers; ++i) {
+    const FfDenseLayer& l = layers[i];
+    if (few) {
+      const int grid = ff_gemm_skinny_plan_epi(rows, qkv_dim, hidden, 2, nullptr, nullptr);
+      if (grid < 0) return grid;
+      if (int r = ff_gemm_skinny_rope_kv(a->n, l.wqkv, a->qkv, rows, qkv_dim, hidden, hidden, hidden, qkv_dim, grid, a->scratch, a->counters, a->cos_sin, a->slots,
+                                         l.kcache, l.vcache, a->hq, a->hkv, 128, 64, a->num_blocks, a->status, s)) return r;
+    } else if (int r = ff_gemm_bf16_rope_kv(a->n, l.wqkv, a->qkv, rows, qkv_dim, hidden, hidden, hidden, qkv_dim, a->cos_sin, a->slots, l.kcache, l.vcache, a->hq,
+                                            a->hkv, 128, 64, a->num_blocks, a->status, s)) {
+      return r;
+    }
+    if (int r = ff_attn_prefill_tc(a->qkv, l.kcache, l.vcache, a->block_table, a->q_start, a->q_lens, a->ctx_lens, a->att, a->batch, rows, a->max_q_len, a->hq,
+                                   a->hkv, 128, 128, qkv_dim, att_dim, a->max_blocks, a->num_blocks, a->scale, a->window, 0, nullptr, nullptr, 0, 128, 0, 0.f,
+                                   nullptr, 0, a->status, s)) return r;
+    if (int r = product(a->att, l.wo, a->o, hidden, att_dim)) return r;
+    if (int r = ff_add_rmsnorm(a->o, a->x, l.post_ln, a->n, nullptr, 0, rows, hidden, hidden, a->eps, 0, a->status, s)) return r;
+    if (few) {
+      const int grid = ff_gemm_skinny_plan_epi(rows, 2 * ffn, hidden, 1, nullptr, nullptr);
+      if (grid < 0) return grid;
+      if (int r = ff_gemm_skinny_swiglu(a->n, l.wgu, a->mid, rows, 2 * ffn, hidden, hidden, hidden, ffn, grid, a->scratch, a->counters, 0, 0.f, a->status, s)) return r;
+    } else if (int r = ff_gemm_bf16(a->n, l.wgu, a->mid, rows, 2 * ffn, hidden, hidden, hidden, ffn, 1, a->status, s)) {
+      return r;
+    }
+    if (int r = product(a->mid, l.wdown, a->o, hidden, ffn)) return r;
+    if (int r = ff_add_rmsnorm(a->o, a->x, l.next_ln, a->n, nullptr, 0, rows, hidden, hidden, a->eps, 0, a->status, s)) return r;
+  }
+  return FF_HOST_OK;
+}
