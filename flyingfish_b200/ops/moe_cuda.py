@@ -241,14 +241,21 @@ class Nvfp4Experts:
     def supported(self) -> bool:
         return self.n % 128 == 0 and self.k % 128 == 0
 
+    def prompts(self) -> bool:
+        """Whether ``csrc/moe_fp4_tc.cu`` takes this stack."""
+        return self.supported() and self.k % 256 == 0 and self.experts <= 768
+
 
 def grouped_gemm_nvfp4(xs, w: Nvfp4Experts, seg_off, counts, capacity: int, epi: int,
-                       out: torch.Tensor | None = None) -> torch.Tensor:
+                       out: torch.Tensor | None = None, rows_per_expert: float = 0.0) -> torch.Tensor:
+    """``rows_per_expert``: the caller's estimate of the mean segment length; from ``FP4_TC_MIN_ROWS`` on the tcgen05 kernel of
+    ``csrc/moe_fp4_tc.cu`` expands a weight tile once for up to 256 rows, below it ``csrc/moe_fp4.cu`` in the registers of the warps that
+    multiply, once for up to 32."""
     n_out = w.n // 2 if epi == 1 else w.n
     y = out if out is not None else torch.empty(capacity, n_out, dtype=torch.bfloat16, device=xs.device)
-    rc = kernels().ff_moe_grouped_gemm_nvfp4(ptr(xs), ptr(w.codes), ptr(w.scales), ptr(w.global_scale), ptr(y), ptr(seg_off),
-                                             ptr(counts), w.experts, w.n, w.k, capacity, n_out, epi,
-                                             ptr(status_tensor(xs.device)), stream_ptr())
+    fn = kernels().ff_moe_grouped_gemm_nvfp4_tc if rows_per_expert >= FP4_TC_MIN_ROWS and w.prompts() else kernels().ff_moe_grouped_gemm_nvfp4
+    rc = fn(ptr(xs), ptr(w.codes), ptr(w.scales), ptr(w.global_scale), ptr(y), ptr(seg_off), ptr(counts), w.experts, w.n, w.k, capacity, n_out, epi,
+            ptr(status_tensor(xs.device)), stream_ptr())
     check(rc, "ff_moe_grouped_gemm_nvfp4")
     _count()
     return y
@@ -261,12 +268,14 @@ def experts_forward_nvfp4(x, weights, ids, gate_up: Nvfp4Experts, down: Nvfp4Exp
     rows, hidden = x.shape
     total = n_experts_total if n_experts_total is not None else gate_up.experts
     xs, pos, seg_off, counts, cap = dispatch_local(x.contiguous(), ids.contiguous(), total, e_lo, e_lo + gate_up.experts)
-    h = grouped_gemm_nvfp4(xs, gate_up, seg_off, counts, cap, epi=1)
-    y = grouped_gemm_nvfp4(h, down, seg_off, counts, cap, epi=0)
+    rpe = rows * ids.shape[1] / max(total, 1)
+    h = grouped_gemm_nvfp4(xs, gate_up, seg_off, counts, cap, epi=1, rows_per_expert=rpe)
+    y = grouped_gemm_nvfp4(h, down, seg_off, counts, cap, epi=0, rows_per_expert=rpe)
     return combine(y, pos, ids, weights.contiguous(), rows, hidden)
 
 
 FP4_DECODE_MAX_ROWS = int(os.environ.get("FF_FP4_MAX_ROWS_PER_EXPERT", "32"))
+FP4_TC_MIN_ROWS = 16.0           # expert layer at 12.5 rows an expert 652 us packed / 740 on tcgen05, at 16 757 / 742
 
 
 def pack_experts_nvfp4(weights) -> int:

@@ -267,6 +267,48 @@ def test_grouped_nvfp4_passes(counts, k, epi):
                 _check(got, rows, k)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("counts,n,k", [
+    ([1, 16, 0, 17, 63], 256, 256),                          # one K chunk, boxes of 64 rows that reach past a segment and past the buffer
+    ([64, 65, 255], 384, 768),                               # whole boxes and one row more, an odd number of chunks
+    ([256, 257, 0, 600], 256, 1280),                         # whole passes and further ones
+    ([33] * 50, 512, 512),                                   # more tiles than CTAs: accumulators and rings begun again
+])
+@pytest.mark.parametrize("epi", [0, 1])
+def test_grouped_nvfp4_for_prompts(counts, n, k, epi):
+    """The tcgen05 kernel against 64 bits, and rows that belong to no segment untouched."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import moe_cuda
+    e = len(counts)
+    pad = [(c + 15) // 16 * 16 for c in counts]
+    off = [sum(pad[:i]) for i in range(e + 1)]
+    x = _rand((off[-1], k), 7)
+    kinds = [qref.quantize_nvfp4(_rand((n, k), 20 + i).float()) for i in range(min(e, 5))]
+    q = [kinds[i % len(kinds)] for i in range(e)]
+    w = moe_cuda.Nvfp4Experts(*(torch.stack([p[j] for p in q]).cuda() for j in range(3)))
+    assert w.prompts()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    out = torch.full((off[-1], n // (2 if epi else 1)), 5.0, dtype=BF16, device="cuda")
+    y = moe_cuda.grouped_gemm_nvfp4(x.cuda(), w, i32(off), i32(counts), off[-1], epi, out=out, rows_per_expert=1e6).cpu().float()
+    torch.cuda.synchronize()
+    ops.check_status()
+    for i, c in enumerate(counts):
+        assert (y[off[i] + c: off[i + 1]] == 5).all()
+        if c:
+            full = (qref.e2m1_decode(qref.e2m1_unpack(q[i][0])).view(n, -1, 16) * qref.e4m3_decode(q[i][1])[..., None]).view(n, k).double()
+            rows = x[off[i]: off[i] + c].double() @ full.t() * float(q[i][2])
+            got = y[off[i]: off[i] + c]
+            if epi:
+                g = rows.float().view(c, n // 128, 2, 64)
+                g, u = g[:, :, 0].reshape(c, -1).double(), g[:, :, 1].reshape(c, -1).double()
+                # gate (slope of silu at most 1.1), up, silu and the product are each rounded to BF16, 2^-9 of themselves; twice that, and FP32 sums
+                act = torch.nn.functional.silu(g)
+                bound = 2.0 ** -8 * (1.1 * g.abs() + 3 * act.abs()) * u.abs() + 2.0 ** -20 * k * (1 + g.abs() + u.abs())
+                assert ((got - act * u).abs() <= bound).all()
+            else:
+                _check(got, rows, k)
+
+
 _WALK = r"""
 #include <atomic>
 #include <barrier>
