@@ -75,6 +75,35 @@ def test_head_norms_before_the_rotation(rows, hq, hkv, dim, rot):
     ops.check_status()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,hidden,top_k", [(1, 8, 1), (3, 1032, 3), (70, 4104, 9), (5, 2048, 16)])      # parts of a CTA, of its loads, the most choices
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_expert_rows_dispatched_and_combined(rows, hidden, top_k, accumulate):
+    """Rows reach every choice's place; the weighted sum skips choices served elsewhere."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import moe_cuda
+    experts, g = 24, torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, hidden, generator=g).to(BF16)
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(rows)]).to(torch.int32)
+    w = torch.rand(rows, top_k, generator=g)
+    lo, hi = 3, experts - 2                                   # the others' choices belong to another rank
+    xs, pos, _, _, cap = moe_cuda.dispatch_local(x.cuda(), ids.cuda(), experts, lo, hi)
+    served = ((ids >= lo) & (ids < hi)).view(-1)
+    assert torch.equal(pos.cpu() >= 0, served)
+    assert torch.equal(xs[pos.long()[served.cuda()]].cpu(), x.repeat_interleave(top_k, 0)[served])
+    y, out = torch.randn(cap, hidden, generator=g).to(BF16).cuda(), torch.randn(rows, hidden, generator=g).to(BF16).cuda()
+    before = out.double().cpu()
+    got = moe_cuda.combine(y, pos, ids.cuda(), w.cuda(), rows, hidden, **(dict(out=out, accumulate=True) if accumulate else {}))
+    torch.cuda.synchronize()
+    ops.check_status()
+    terms = y.cpu().double()[pos.long().cpu().clamp_min(0)].view(rows, top_k, hidden) * (w.double() * served.view(rows, top_k))[..., None]
+    want, size = terms.sum(1), terms.abs().sum(1)
+    if accumulate:
+        want, size = want + before, size + before.abs()
+    # one rounding of the result, a rounding of FP32 per addition
+    assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + (top_k + 1) * 2.0 ** -23 * size).all()
+
+
 def _mla_batch(q_lens, pasts, seed):
     g = torch.Generator().manual_seed(seed)
     ql = torch.tensor(q_lens, dtype=torch.int32)
