@@ -121,10 +121,10 @@ class DecoderModel:
         if self.trace is not None:
             self.trace.record("embed", x)
         stack = self._stack_layers(b, kv)
-        done = stack is not None and ops.dense_stack(
+        done = 0 if stack is None else ops.dense_stack(
             x, n, stack, b.positions, b.slots, b.block_table, b.q_start, b.q_lens, b.ctx_lens, b.max_q_len, self.hq, self.hkv, w.layers[0].wdown.shape[1],
-            self.scale, s.rms_eps, s.rope_theta, -1 if self.bidirectional else 0, self._rope_cs) is not None
-        for i in range(0 if done else s.layers):
+            self.scale, s.rms_eps, s.rope_theta, -1 if self.bidirectional else 0, self._rope_cs)
+        for i in range(done, s.layers):
             lw = w.layers[i]
             o = self._attention(i, n, b, kv)
             n = ops.add_rmsnorm(o, x, lw.post_ln, s.rms_eps)
@@ -141,12 +141,13 @@ class DecoderModel:
             self.normed_sink.append(n)
         return n
 
-    # -- prompts of few rows: all layers launched by one native call --------------------------------
+    # -- prompts of few rows: layers launched by native calls --------------------------------
     def _stack_layers(self, b: ForwardBatch, kv: PagedKVCache) -> list[tuple[torch.Tensor, ...]] | None:
         """The layers' tensors for :func:`ops.dense_stack`, or None where the operators are called one by one: steps that it does not cover, and
-        prompts of so many rows that the device is busier than the host (a layer of an 8B-sized stack takes the host about 0.15 ms; the one
-        call has its host work in front of the first layer). Prefill of 8 layers, operators / native call: 16 rows 1520 / 1235 us, 37 1509 / 1283,
-        100 1523 / 1466, 128 1531 / 1514; from 140 rows on, where the rows leave the decode product, 1651 / 1686 and more."""
+        prompts of so many rows that the device is busier than the host (a layer of an 8B-sized stack takes the host about 0.15 ms; the
+        native calls have their host work in front of the second layer). Prefill of 8 layers, operators / native
+        calls: 16 rows 1511 / 1195 us, 37 1495 / 1249, 100 1526 / 1439, 128 1535 / 1484; from 140 rows on, where the rows leave the decode product, no
+        difference or slower (200 1662 / 1688)."""
         from ..ops import lib
         w, s, me = self.w, self.spec, type(self)
         if b.is_decode or b.rows > STACK_MAX_ROWS or not b.positions.is_cuda or self.trace is not None or self.capture_taps or lib.DEBUG_CHECKS:

@@ -2,7 +2,7 @@
 // product, residual and norm, gate/up product with SwiGLU, down product, residual and norm -- the launchers that the operators of the
 // Python side call one by one, in the same order and with the same arguments. Nothing is computed here. What it is for: a launch through the
 // operators takes 20 us of host time, so that prompts of up to a hundred rows were bound by the host (37 rows, 8 layers of an 8B-sized stack: 64
-// launches, 1519 -> 1283 us a call).
+// launches, 1495 -> 1249 us a call).
 #include "host_util.h"
 #include <stddef.h>
 
