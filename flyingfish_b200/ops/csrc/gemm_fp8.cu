@@ -64,6 +64,56 @@ __device__ __forceinline__ void fp8_promote(float (&acc)[NACC], const uint32_t (
     }
 }
 
+// Partials are added in split order (fixed summation order). Thread -> four adjacent columns and every eighth token, J tokens at a time; SB splits' loads
+// are in flight together and the sums go straight into the staging tile. One CTA adds the partials of a tile while the GPU waits for it: with
+// one split of eight tokens in flight, fourteen splits of 576 x 7168 at 64 tokens took the whole product 38 us, with two splits of four 30, with
+// eight of two 24. Few splits have no eight loads for two tokens. (It spills less than the loop in the kernel's own body did, which the promotion
+// loop paid for: 64 rows times 7168 x 16384 46 -> 42 us, 100 rows 73 -> 60.)
+template <int SB, int J>
+__device__ __forceinline__ void fp8_add_partials(const float* part, __nv_bfloat16* sT, int ee, int col0, int Nw, size_t stride, int ntok, int real,
+                                                 int splits) {
+  const int c4 = (ee & 31) * 4, tg = ee >> 5, ncol = col0 + c4;          // tg 0 .. 7
+  const bool vec = (Nw & 3) == 0 && ncol + 3 < Nw;
+  for (int tb = tg; tb < ntok; tb += 8 * J) {
+    float4 sum[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* ps = part + (size_t)tb * Nw + ncol;
+    for (int s0 = 0; s0 < splits; s0 += SB) {
+      float4 v[SB][J];
+#pragma unroll
+      for (int u = 0; u < SB; ++u, ps += stride)
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+          v[u][j] = vec && s0 + u < splits && tb + 8 * j < real ? __ldcg(reinterpret_cast<const float4*>(ps + (size_t)(8 * j) * Nw)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < SB; ++u)
+        if (s0 + u < splits) {
+#pragma unroll
+          for (int j = 0; j < J; ++j) { sum[j].x += v[u][j].x; sum[j].y += v[u][j].y; sum[j].z += v[u][j].z; sum[j].w += v[u][j].w; }
+        }
+    }
+    if (!vec)                                          // ragged right edge, or rows that are not 16-byte aligned
+      for (int s1 = 0; s1 < splits; ++s1)
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const float* at = part + s1 * stride + (size_t)(tb + 8 * j) * Nw + ncol;
+          if (tb + 8 * j >= real) continue;
+          if (ncol < Nw) sum[j].x += __ldcg(at);
+          if (ncol + 1 < Nw) sum[j].y += __ldcg(at + 1);
+          if (ncol + 2 < Nw) sum[j].z += __ldcg(at + 2);
+          if (ncol + 3 < Nw) sum[j].w += __ldcg(at + 3);
+        }
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+      if (tb + 8 * j < ntok) {
+        __nv_bfloat162* d = reinterpret_cast<__nv_bfloat162*>(sT + (tb + 8 * j) * FBM + c4);
+        d[0] = __floats2bfloat162_rn(sum[j].x, sum[j].y);
+        d[1] = __floats2bfloat162_rn(sum[j].z, sum[j].w);
+      }
+  }
+}
+
 // epi: 0 store, 1 SwiGLU over 64/64 interleaved rows (grouped gate/up)
 // TOK: tokens per chunk. 128 for prefill-sized and dense calls (one CTA per SM); 32 and 64 for grouped calls with short segments, where a
 // CTA needs few registers and half the shared memory so that two CTAs share an SM and one streams while the other sets up
@@ -276,58 +326,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         final_here = bars.is_last != 0;
         if (final_here) {
           __threadfence();
-          // partials are added in split order (fixed summation order). Thread -> four adjacent columns and every eighth token, four
-          // tokens at a time; SB splits' loads are in flight together and the sums go straight into the staging tile. One CTA adds the
-          // partials of a tile while the GPU waits for it: with one split of eight tokens in flight, fourteen splits of 576 x 7168
-          // at 64 tokens took the whole product 38 us, now 30.
-          constexpr int SB = TOK == 128 ? 4 : 2;
-          const int c4 = (ee & 31) * 4, tg = ee >> 5;          // tg 0 .. 7
-          const int ncol = tn * FBM + c4;
-          const bool vec = (Nw & 3) == 0 && ncol + 3 < Nw;
-          for (int tb = 0; tb < ntok; tb += 32) {              // bands of 32 tokens: four tokens per thread and band
-            float4 sum[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s0 = 0; s0 < splits; s0 += SB) {
-              float4 v[SB][4];
-#pragma unroll
-              for (int u = 0; u < SB; ++u) {
-                const float* ps = scratch + ((size_t)(s0 + u) * M + grow0) * Nw + ncol;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const int t = tb + tg + 8 * j;
-                  v[u][j] = s0 + u < splits && t < real && vec ? __ldcg(reinterpret_cast<const float4*>(ps + (size_t)t * Nw)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-              }
-#pragma unroll
-              for (int u = 0; u < SB; ++u)
-                if (s0 + u < splits) {
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) { sum[j].x += v[u][j].x; sum[j].y += v[u][j].y; sum[j].z += v[u][j].z; sum[j].w += v[u][j].w; }
-                }
-            }
-            if (!vec)                                          // ragged right edge, or rows that are not 16-byte aligned
-              for (int s1 = 0; s1 < splits; ++s1)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const int t = tb + tg + 8 * j;
-                  const float* ps = scratch + ((size_t)s1 * M + grow0 + t) * Nw + ncol;
-                  if (t >= real) continue;
-                  if (ncol < Nw) sum[j].x += __ldcg(ps);
-                  if (ncol + 1 < Nw) sum[j].y += __ldcg(ps + 1);
-                  if (ncol + 2 < Nw) sum[j].z += __ldcg(ps + 2);
-                  if (ncol + 3 < Nw) sum[j].w += __ldcg(ps + 3);
-                }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int t = tb + tg + 8 * j;
-              if (t < ntok) {
-                __nv_bfloat162* d = reinterpret_cast<__nv_bfloat162*>(sT + t * FBM + c4);
-                d[0] = __floats2bfloat162_rn(sum[j].x, sum[j].y);
-                d[1] = __floats2bfloat162_rn(sum[j].z, sum[j].w);
-              }
-            }
-          }
+          const float* ps = scratch + (size_t)grow0 * Nw;
+          if (TOK == 64 && CTAS == 1 && splits > 4) fp8_add_partials<8, 2>(ps, sT, ee, tn * FBM, Nw, (size_t)M * Nw, ntok, real, splits);
+          else fp8_add_partials<TOK == 128 ? 4 : 2, 4>(ps, sT, ee, tn * FBM, Nw, (size_t)M * Nw, ntok, real, splits);
         }
       }
       if (final_here) {
