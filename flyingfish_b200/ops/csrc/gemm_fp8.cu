@@ -122,8 +122,8 @@ __device__ __forceinline__ void fp8_add_partials(const float* part, __nv_bfloat1
 // CTAS: CTAs per SM. P: K blocks promoted per round; a warp waits for a block, reads it, multiplies and hands it back, about 0.25 us one after the
 // other at 64 tokens, and two blocks in a round share the waits. A dense call of 33 to 64 tokens that does not fill two CTAs per SM has the
 // registers for it. Together with scale rows that lie 4 floats apart from a multiple of 32 in shared memory (staging them put 32 lanes on one
-// bank): 64 rows times 7168 x 16384 and 7168 x 18432 49 -> 41.5 us, 24576 x 1536 21.1 -> 18.9 (before: 53.5 us alone, 37.4 without
-// promotion, 39.7 without staging, 29.3 without both).
+// bank): 64 rows times 7168 x 16384 and 7168 x 18432 49 -> 41.5 us, 24576 x 1536 21.1 -> 18.9 (with what
+// is noted at the partial sums and the staging 32 to 35 and 17 now).
 constexpr int SX_PAD = 4;
 template <int TOK, int CTAS, int P>
 __global__ void __launch_bounds__(320, CTAS)
@@ -251,24 +251,26 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       const int blk1 = half == 0 ? (nblk + 1) / 2 : nblk;
       // scale products of this chunk and K range -> shared memory [kb][ntok] (the product of the two scales is what
       // every partial sum is multiplied by: staged once, so that no global load sits between a k-block's arrival and
-      // its promotion); eight independent loads per thread in flight
-      for (int i0 = ee; i0 < ntok * nkb; i0 += 256 * 8) {
-        float v[8];
+      // its promotion). A warp takes every eighth token, its lanes the K blocks, sixteen independent loads per
+      // thread in flight. With a division per scale and eight loads, staging took a third of the product: 7168 x 16384 with 64 rows 42 -> 32 us, with
+      // 100 60 -> 43; 36864 x 7168 with 64 rows 55 -> 48, with 100 91 -> 64; 256 experts of 7168 x 2048 with 50 rows each 2256 -> 2032.
+      for (int t0 = ee >> 5; t0 < ntok; t0 += 64)
+        for (int k0 = lane; k0 < nkb; k0 += 64) {
+          float wv[2], v[2][8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int i = i0 + u * 256;
-          v[u] = 0.f;
-          if (i < ntok * nkb) {
-            const int t = i / nkb, kb = i - t * nkb;
-            if (t < real) v[u] = ws_row[kb0 + kb] * x_scale[(size_t)(grow0 + t) * xs_ld + kb0 + kb];
+          for (int h = 0; h < 2; ++h) {
+            const bool in = k0 + 32 * h < nkb;
+            const float* xp = x_scale + (size_t)(grow0 + t0) * xs_ld + kb0 + k0 + 32 * h;
+            wv[h] = in ? ws_row[kb0 + k0 + 32 * h] : 0.f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[h][u] = in && t0 + 8 * u < real ? xp[(size_t)(8 * u) * xs_ld] : 0.f;
           }
-        }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int i = i0 + u * 256;
-          if (i < ntok * nkb) { const int t = i / nkb, kb = i - t * nkb; sXs[kb * (ntok + SX_PAD) + t] = v[u]; }
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (k0 + 32 * h < nkb && t0 + 8 * u < ntok) sXs[(k0 + 32 * h) * (ntok + SX_PAD) + t0 + 8 * u] = wv[h] * v[h][u];
         }
-      }
       asm volatile("bar.sync 1, 256;" ::: "memory");
       float acc[TOK / 2];                                 // columns (blk0 + i / 16) * 16 + i % 16
 #pragma unroll
