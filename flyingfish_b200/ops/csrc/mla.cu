@@ -53,7 +53,9 @@ __device__ __forceinline__ uint32_t toff(int r, int c, int chp) { return (uint32
 // out     : [total rows][heads][512] bf16
 // part_o  : fp32 [B][nsplit][max_rows][512], part_ml fp32 [B][nsplit][max_rows][2]  (max_rows = max_q * heads)
 // grid (pairs of 16-row tiles, nsplit, B), 256 threads. FULL: the DeepSeek geometry, otherwise the widths of `f` (576 and 512 above
-// stand for them).
+// stand for them). 128 heads over 1024 keys, one query each: 64 sequences 130 us with the queries read again from shared memory at every page,
+// 115 so; 200 keys 45 / 41; 32 of 3000 193 / 172; eight of 1024 no difference.
+constexpr int QREGS = 28;
 template <bool FULL>
 __global__ void __launch_bounds__(256)
 mla_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
@@ -129,6 +131,14 @@ mla_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __rest
   };
   if (p0 < p1) issue(p0, 0);
   const uint32_t sQa = smem_u32(sQ), sPa = smem_u32(sP);
+  // queries of the first QREGS steps of 16 stay in registers: shared memory, which a warp read for its queries as much as for its keys at every page,
+  // is what the scores wait for (one CTA per SM leaves a thread 255 registers; with 24 steps 119 us, with all 36 127, for 64 sequences)
+  __syncthreads();
+  uint32_t qa[QREGS][4];
+  if (FULL)
+#pragma unroll
+    for (int kk = 0; kk < QREGS; ++kk)
+      ldsm4(sQa + toff((lane & 7) + (((lane >> 3) & 1) << 3), 2 * kk + (lane >> 4), chp), qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3]);
   for (int p = p0; p < p1; ++p) {
     const int buf = (p - p0) & 1;
     if (p + 1 < p1) { issue(p + 1, buf ^ 1); cp_wait<1>(); } else { cp_wait<0>(); }
@@ -136,8 +146,17 @@ mla_attn_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __rest
     const uint32_t sKa = smem_u32(sK[buf]);
     // S[16 rows][16 keys of this warp]
     float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    if (FULL) {
+#pragma unroll
+      for (int kk = 0; kk < QREGS; ++kk) {
+        uint32_t b0, b1, b2, b3;
+        ldsm4(sKa + toff(warp * 16 + ((lane >> 4) << 3) + (lane & 7), 2 * kk + ((lane >> 3) & 1), chp), b0, b1, b2, b3);
+        mma(s[0], qa[kk], b0, b1);
+        mma(s[1], qa[kk], b2, b3);
+      }
+    }
 #pragma unroll 4
-    for (int kk = 0; kk < ld / 16; ++kk) {
+    for (int kk = FULL ? QREGS : 0; kk < ld / 16; ++kk) {
       uint32_t a[4], b0, b1, b2, b3;
       ldsm4(sQa + toff((lane & 7) + (((lane >> 3) & 1) << 3), 2 * kk + (lane >> 4), chp), a[0], a[1], a[2], a[3]);
       ldsm4(sKa + toff(warp * 16 + ((lane >> 4) << 3) + (lane & 7), 2 * kk + ((lane >> 3) & 1), chp), b0, b1, b2, b3);
