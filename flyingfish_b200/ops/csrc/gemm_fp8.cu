@@ -67,8 +67,9 @@ __device__ __forceinline__ void fp8_promote(float (&acc)[NACC], const uint32_t (
 // Partials are added in split order (fixed summation order). Thread -> four adjacent columns and every eighth token, J tokens at a time; SB splits' loads
 // are in flight together and the sums go straight into the staging tile. One CTA adds the partials of a tile while the GPU waits for it: with
 // one split of eight tokens in flight, fourteen splits of 576 x 7168 at 64 tokens took the whole product 38 us, with two splits of four 30, with
-// eight of two 24. Few splits have no eight loads for two tokens. (It spills less than the loop in the kernel's own body did, which the promotion
-// loop paid for: 64 rows times 7168 x 16384 46 -> 42 us, 100 rows 73 -> 60.)
+// eight of two 24. Few splits have no eight loads for two tokens. Two CTAs of 64 tokens on an SM rarely have splits: two tokens there leave the
+// promotion loop its registers (256 experts with 28 rows each 1181 -> 1156 us, 36864 x 7168 with 64 rows 58.8 -> 57.2). As a function it spills less than
+// the loop in the kernel's own body did, which the promotion loop paid for: 64 rows times 7168 x 16384 46 -> 42 us, 100 rows 73 -> 60.
 template <int SB, int J>
 __device__ __forceinline__ void fp8_add_partials(const float* part, __nv_bfloat16* sT, int ee, int col0, int Nw, size_t stride, int ntok, int real,
                                                  int splits) {
@@ -330,7 +331,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           __threadfence();
           const float* ps = scratch + (size_t)grow0 * Nw;
           if (TOK == 64 && CTAS == 1 && splits > 4) fp8_add_partials<8, 2>(ps, sT, ee, tn * FBM, Nw, (size_t)M * Nw, ntok, real, splits);
-          else fp8_add_partials<TOK == 128 ? 4 : 2, 4>(ps, sT, ee, tn * FBM, Nw, (size_t)M * Nw, ntok, real, splits);
+          else fp8_add_partials<TOK == 128 ? 4 : 2, TOK == 64 && CTAS == 2 ? 2 : 4>(ps, sT, ee, tn * FBM, Nw, (size_t)M * Nw, ntok, real, splits);
         }
       }
       if (final_here) {
