@@ -202,17 +202,6 @@ struct DecodeForm {
 __device__ __forceinline__ int first_visible(int pos, int window, int chunk) {
   return window > 0 ? max(0, pos - window + 1) : (chunk > 0 ? max(0, pos) / chunk * chunk : 0);
 }
-// Pages that a split of a sequence takes. The launch has `nsplit` splits for sequences of the cache's whole capacity; a sequence that is
-// shorter is cut into fewer: as many CTAs as fit the GPU at once (three per SM, `items` of them work beside each other per split) are enough, and a CTA
-// of one or two pages spends its time on its start and end. Up to five pages, about four waves of which fill up evenly. The rule looks at the
-// sequence's own length and the size of the launch only: a row's bits do not depend on the lengths beside it. 32 / 8 heads, capacity
-// 4096, us before / after: one sequence of 1024 9.0 / 6.7, seven of 150 to 2850 21.8 / 14.0 (merge 6.6 / 3.9), 113 of 120 to 480 39.1 / 36.9; 64 / 4 heads,
-// 32 of 1000 41.6 / 25.5.
-constexpr int DEC_SLOTS = 444, DEC_PAGES = 5;
-__device__ __forceinline__ int pages_per_split(int pages, int nsplit, int items) {
-  const int even = (pages + nsplit - 1) / nsplit, filled = (int)(((long long)items * pages + DEC_SLOTS - 1) / DEC_SLOTS);
-  return max(max(even, 1), min(filled, DEC_PAGES));
-}
 __device__ __forceinline__ float gate_factor(const __nv_bfloat16* gate, int ldg, size_t row, int head, int dv, int d, int head_gate) {
   return gate == nullptr ? 1.0f : 1.0f / (1.0f + expf(-__bfloat162float(gate[row * ldg + (head_gate ? head : head * dv + d)])));
 }
@@ -268,12 +257,17 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   const int skip = pfirst - nkeep;                     // pages between the kept ones and the window's first
   auto page_of = [&](int p) { return EXTRA && p >= nkeep ? p + skip : p; };
   const int first = EXTRA ? 0 : pfirst, last = EXTRA ? pages - skip : pages;
-  // by_length: the split goes by the sequence's length and the merge knows it (ctx_lens); otherwise all splits share the pages evenly
-  const bool by_length = !EXTRA && window == 0 && kv_start == nullptr && pstride == 0 && split_counters == nullptr;
-  const int per = by_length ? pages_per_split(pages, nsplit, gridDim.y * gridDim.z) : (last - first + nsplit - 1) / nsplit;
+  // The splits of a launch share a sequence's pages evenly. Where a sequence is cut fixes its result's bits (another running maximum rounds
+  // every probability anew), so the cut depends on the sequence's own pages and the number of splits alone. counted: the merge is told the
+  // lengths (attn_decode_launch) and reads the splits that have pages; the others leave, and a sequence of one split is written without a merge.
+  // Attention and merge of a layer, capacity 4096, us with all splits written and read / so: 32 / 8 heads, one sequence of 1024 13.6 / 10.8, seven of
+  // 150 to 2850 28.2 / 24.8, 16 of 20 to 180 23.6 / 12.8; 64 / 4 heads, 32 of 700 to 1300 49.2 / 42.0. (A cut by a sequence's length and the
+  // batch, up to five pages a split, took 10.8, 19.5, 12.5 and 31.0, but moved the logits of a model with experts by 0.05 of their size.)
+  const int per = (last - first + nsplit - 1) / nsplit;
   const int p0 = first + split * per, p1 = min(last, p0 + per);
-  if (by_length && split > 0 && p0 >= p1) return;      // the merge does not read this split
-  const bool whole = pstride == 0 && (nsplit == 1 || (by_length && per >= pages));
+  const bool counted = !EXTRA && window == 0 && kv_start == nullptr && pstride == 0 && split_counters == nullptr;
+  if (counted && split > 0 && p0 >= p1) return;
+  const bool whole = pstride == 0 && (nsplit == 1 || (counted && per >= pages));
   const int rows_total = nq * G;
   const int rows_used = min(16, rows_total - rt * 16);
 
@@ -444,7 +438,7 @@ template <bool MANY>
 __global__ void __launch_bounds__(128)
 attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, __nv_bfloat16* __restrict__ out,
                   int rows_per_seq, int nsplit, const float* __restrict__ sinks, int hq, int dv, const __nv_bfloat16* __restrict__ gate,
-                  int ldg, int head_gate, const int* __restrict__ ctx_lens, int items) {
+                  int ldg, int head_gate, const int* __restrict__ ctx_lens) {
   __shared__ float4 s_acc[MANY ? 4 : 1][HD / 4];
   pdl_trigger();
   pdl_wait();
@@ -453,12 +447,12 @@ attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ pa
   const float2* ml = reinterpret_cast<const float2*>(part_ml);
   const int d = threadIdx.x;
   float M = NEG_BIG;
-  if (ctx_lens != nullptr) {                       // splits by length: this sequence's own number; one of them has written the result itself
-    const int pages = (ctx_lens[b] + PAGE - 1) / PAGE, per = pages_per_split(pages, nsplit, items);
+  if (ctx_lens != nullptr) {                       // splits of this sequence that have pages; a single one has written the result itself
+    const int pages = (ctx_lens[b] + PAGE - 1) / PAGE, per = (pages + nsplit - 1) / nsplit;
     if (per >= pages) return;
     nsplit = (pages + per - 1) / per;
   }
-  if (!MANY || nsplit <= 8) {
+  if (!MANY) {
     if (d >= dv) return;
     float2 v[8];
     float o[8];
@@ -672,9 +666,9 @@ static int attn_decode_launch(const void* q, const void* kcache, const void* vca
   if (int r = launch_result()) return r;
   if (pstride != 0) return 0;                      // partials only: the caller merges after the other kernel has added its own
   if (nsplit > 1 && split_counters == nullptr) {
-    // splits by length in the instances without EXTRA, as the kernel decides
+    // the lengths go to the merge where the kernel counts a sequence's own splits
     if (int lr_ = launch_pdl(nsplit > 8 ? attn_merge_kernel<true> : attn_merge_kernel<false>, dim3(batch * nq * hq), dim3(128), 0, s, 0, part_o, part_ml, (__nv_bfloat16*)out, nq * hq, nsplit, sinks, hq, f.dv, f.gate, f.ldg, f.head_gate,
-                           extra || f.window > 0 || kv_start != nullptr || !wide ? (const int*)nullptr : ctx_lens, hkv * row_tiles * batch)) return lr_;
+                           extra || f.window > 0 || kv_start != nullptr || !wide ? (const int*)nullptr : ctx_lens)) return lr_;
     return launch_result();
   }
   return 0;
@@ -708,7 +702,7 @@ FF_EXPORT int ff_attn_merge(const float* part_o, const float* part_ml, void* out
   if (batch <= 0 || rows_per_seq <= 0 || nsplit < 1) return FF_HOST_BAD_SHAPE;
   if (int lr_ = launch_pdl(nsplit > 8 ? attn_merge_kernel<true> : attn_merge_kernel<false>, dim3(batch * rows_per_seq), dim3(128), 0, s, 0, part_o, part_ml,
                            (__nv_bfloat16*)out, rows_per_seq, nsplit, (const float*)nullptr, rows_per_seq, HD,
-                           (const __nv_bfloat16*)nullptr, 0, 0, (const int*)nullptr, 0)) return lr_;
+                           (const __nv_bfloat16*)nullptr, 0, 0, (const int*)nullptr)) return lr_;
   return launch_result();
 }
 

@@ -427,6 +427,29 @@ def test_splits_by_length(lens, hq, hkv, nq, sinks):
                 assert torch.equal(again[b * nq: (b + 1) * nq], got[b * nq: (b + 1) * nq])
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens,hq,hkv", [
+    ([0, 1, 64, 65, 320, 1000, 4096], 8, 2),                 # more splits than most of them have pages: some leave, some are alone
+    ([1500, 150, 2850], 32, 8),
+    ([300, 64, 700] * 40, 32, 8),                            # two splits, one of them without pages
+])
+@pytest.mark.parametrize("nq", [1, 2])
+def test_splits_share_the_pages_evenly(lens, hq, hkv, nq):
+    """A window that reaches past every context hides nothing, and its launch writes and merges all splits: the same bits. They fix how a
+    sequence is cut, which fixes how its probabilities are rounded."""
+    from flyingfish_b200 import ops
+    d, blocks, pool = 128, 64, 40
+    lens = [max(n, nq) if n else 0 for n in lens]
+    q, k, v = _rand((len(lens) * nq, hq * d), 1), _rand((pool, hkv, 64, d), 2), _rand((pool, hkv, 64, d), 3)
+    table = torch.stack([torch.randint(0, pool, (blocks,), generator=torch.Generator().manual_seed(b)) for b in range(len(lens))]).to(torch.int32).cuda()
+    run = lambda window: ops.attn_decode(q.cuda(), k.cuda(), v.cuda(), table, torch.tensor(lens, dtype=torch.int32, device="cuda"), hq, hkv, d, d ** -0.5,
+                                         nq=nq, max_ctx=blocks * 64, window=window)
+    full, wide = run(0), run(1 << 20)
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(full, wide)
+
+
 @pytest.mark.parametrize("n,k", [(7168, 18432), (7168, 2560), (4096, 7168), (6144, 4096), (34048, 512), (33920, 512), (576, 2560), (128, 128)])
 def test_fp8_split_does_not_depend_on_the_rows(n, k):
     import ctypes
