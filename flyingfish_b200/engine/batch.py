@@ -53,7 +53,7 @@ class ForwardBatch:
         pin = self.device.type == "cuda" if pinned is None else pinned
         pinned = torch.zeros(layout.total + 4 + layout.max_batch, dtype=torch.int32, pin_memory=pin)
         self.host = pinned[: layout.total]
-        self.results = pinned[layout.total:]     # where a step's device status (four words) and ids are copied to
+        self.results = pinned[layout.total:]     # where the engine reads a step's device status (four words) and ids
         self._words = self.host.numpy()   # the same memory: a field is written in about a microsecond, through a tensor in four
         self.dev = torch.zeros(layout.total, dtype=torch.int32, device=self.device)
         # host-side scalars of the current step

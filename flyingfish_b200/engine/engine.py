@@ -62,8 +62,6 @@ class _Graph:
         self.batch: ForwardBatch | None = None
         self.out: torch.Tensor | None = None
         self.logits: torch.Tensor | None = None
-        self.ids: np.ndarray | None = None         # pinned copy of ``out``, written by the replayed step
-        self.status: np.ndarray | None = None      # pinned copy of the device status, likewise
 
 
 @dataclass
@@ -404,7 +402,7 @@ class Engine:
             if all(len(sp.tokens) == 1 for sp in spans):
                 for sp in spans:
                     sp.seq.pending = sp.tokens[0]
-                _, logits, _, _ = self._launch_decode([sp.seq for sp in spans])
+                _, logits, _ = self._launch_decode([sp.seq for sp in spans])
                 for sp in spans:
                     self.kv.commit(sp.seq.seq_id, 1)
                 rows = [i for i, sp in enumerate(spans) for _ in sp.want]
@@ -510,7 +508,8 @@ class Engine:
 
     def capture(self, bucket: int) -> _Graph:
         """Capture the decode step for a batch bucket: one eager warm-up on padding rows (which
-        write no KV), then stream capture of the same step."""
+        write no KV), then stream capture of the same step. A replay reads the step's metadata from the batch's device
+        buffer (``batch.dev``), which the caller has written, and leaves ids and logits in ``out`` and ``logits``."""
         key = (bucket, 1)
         g = self.graphs.get(key)
         if g is not None:
@@ -531,14 +530,8 @@ class Engine:
         torch.cuda.current_stream(self.device).wait_stream(side)
         torch.cuda.synchronize(self.device)
         graph = torch.cuda.CUDAGraph()
-        # the copies of the step's metadata and of its results are part of the graph: one launch and one wait per step
-        status = ops.status_tensor(self.device)[:4]
         with torch.cuda.graph(graph):
-            ops.copy_async(fb.dev, fb.host)
             out = self.model.forward(fb, self.kv)
-            ops.copy_async(fb.results[4:], out)
-            ops.copy_async(fb.results[:4], status)
-        g.ids, g.status = fb.results[4:].numpy(), fb.results[:4].numpy()
         g.graph, g.batch, g.out, g.logits = graph, fb, out, getattr(self.model, "last_logits", None)
         self.graphs[key] = g
         self.stats["captures"] += 1
@@ -551,23 +544,24 @@ class Engine:
             if held[s.seq_id].length >= cap:
                 raise OutOfBlocks(f"sequence {s.seq_id} reached the KV capacity {cap}")
 
-    def _launch_decode(self, seqs: list[Sequence]) -> tuple[torch.Tensor, torch.Tensor | None, ForwardBatch, _Graph | None]:
+    def _launch_decode(self, seqs: list[Sequence]) -> tuple[torch.Tensor, torch.Tensor | None, ForwardBatch]:
         """Upload and launch the decode step of every sequence's pending token (a graph replay where graphs are on);
-        returns (greedy ids, logits, batch), all of the padded bucket, and the graph. Commits nothing; the caller waits for the
+        returns (greedy ids, logits, batch), all of the padded bucket. Commits nothing; the caller waits for the
         device before it launches the next step, which writes the batch's pinned buffer."""
         bucket = bucket_for(len(seqs))
         if self.use_graph and getattr(self.model, "expert_provider", None) is None:
             g = self.capture(bucket)
             fb = g.batch
             self._fill_decode(fb, seqs, bucket)
+            fb.upload()
             g.graph.replay()
             self.stats["graph_replays"] += 1
-            return g.out, g.logits, fb, g
+            return g.out, g.logits, fb
         fb = self._decode_batch(bucket)
         self._fill_decode(fb, seqs, bucket)
         fb.upload()
         out = self.model.forward(fb, self.kv)
-        return out, getattr(self.model, "last_logits", None), fb, None
+        return out, getattr(self.model, "last_logits", None), fb
 
     def decode(self, seqs: list[Sequence]) -> list[int]:
         """One decode step for the given sequences (each must have a pending token)."""
@@ -582,17 +576,13 @@ class Engine:
             if provider is not None:
                 provider.begin_token()
             self._check_capacity(seqs)
-            out, _, fb, g = self._launch_decode(seqs)
-            if g is not None:
-                torch.cuda.current_stream(self.device).synchronize()
-                toks = g.ids[:n].tolist()
-                if g.status[0]:
-                    self._after_sync()
-            else:
-                toks = [int(t) for t in out[:n].cpu().tolist()] if provider is not None else self._read_ids(out[:n])
+            out, _, fb = self._launch_decode(seqs)
             if provider is not None:
+                toks = [int(t) for t in out[:n].cpu().tolist()]
                 provider.finish_token()
                 self._after_sync()
+            else:
+                toks = self._read_ids(out[:n])
             self.stats["h2d_bytes"] += fb.h2d_bytes()
             self.stats["d2h_bytes"] += 4 * fb.batch
             for s, t in zip(seqs, toks):
@@ -817,8 +807,8 @@ class Engine:
         if n:
             ops.copy_async(read[4: n + 4], ids)
         ops.copy_async(read[:4], ops.status_tensor(self.device)[:4])
-        torch.cuda.current_stream(self.device).synchronize()
         got = read.numpy()
+        torch.cuda.current_stream(self.device).synchronize()
         if got[0]:
             self._after_sync()
         return got[4: n + 4].tolist()

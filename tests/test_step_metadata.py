@@ -77,3 +77,43 @@ def test_a_replayed_step_reports_the_device_status():
     seqs = [eng.add_sequence([1, 2, 3, 4 + i]) for i in range(3)]
     eng.prefill(seqs)
     assert eng.decode(seqs) == first
+
+
+@pytest.mark.gpu
+def test_a_captured_step_reads_the_device_buffer():
+    """Steps staged in device memory and replayed, the ids fed back there, are those of ``Engine.decode``: ids, logits and cache."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.api import Model
+    from flyingfish_b200.config import Settings
+    from flyingfish_b200.engine.engine import bucket_for
+    m = Model.load("tiny-llama", Settings(capacity=256, max_batch=4), device="cuda:0", seed=0)
+    eng, steps, bucket = m.engine, 5, bucket_for(3)
+
+    def start():
+        eng.reset()
+        for t in eng.kv.k + eng.kv.v:
+            t.zero_()
+        seqs = [eng.add_sequence([1, 2, 3, 4 + i][: 2 + i]) for i in range(3)]
+        eng.prefill(seqs)
+        return seqs
+    seqs = start()
+    g = eng.capture(bucket)
+    want = [(eng.decode(seqs), g.logits[:3].clone()) for _ in range(steps)]
+    cached = lambda: [t[eng.kv.seqs[s.seq_id].blocks] for t in eng.kv.k + eng.kv.v for s in seqs]
+    cache = cached()
+    seqs = start()
+    fb, staged = g.batch, []
+    for _ in range(steps):
+        eng._fill_decode(fb, seqs, bucket)
+        staged.append(fb.host.to("cuda"))
+        for s in seqs:
+            eng.kv.commit(s.seq_id, 1)
+    ids, prev = fb.dev[fb.layout.ids: fb.layout.ids + bucket], torch.tensor([s.pending for s in seqs] + [0] * (bucket - 3), dtype=torch.int32, device="cuda")
+    for meta, (toks, logits) in zip(staged, want):
+        fb.dev.copy_(meta)
+        ids.copy_(prev)
+        g.graph.replay()
+        prev = g.out
+        assert g.out[:3].tolist() == toks and torch.equal(g.logits[:3], logits)
+    ops.check_status()
+    assert all(torch.equal(a, b) for a, b in zip(cache, cached()))
