@@ -204,8 +204,6 @@ moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ pos, uint
 // One block: assignments of every expert, seg_off[e] = sum of pad16(count) over earlier experts; cursors zeroed; total rows
 // (padded) written to seg_off[E_local]. capacity = rows the sorted buffer can hold. A memset, a count over many blocks and a scan were three
 // launches in a row, 5.7 us of 256 assignments and 8.8 of 16312; one is 3.0 us of 256.
-// It does not let the next kernel start early, and the permutations are launched plainly: the grouped FP8 product reads counts and offsets in
-// front of its wait on the kernel before it, so they have to be complete before the permutation starts.
 __global__ void __launch_bounds__(1024)
 moe_count_scan_kernel(const int* __restrict__ ids, int n_assign, int E, int e_lo, int e_hi, int* __restrict__ counts, int* __restrict__ seg_off,
                       int* __restrict__ cursors, int capacity, int* status) {

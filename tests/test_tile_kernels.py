@@ -212,6 +212,35 @@ def test_quantised_rows_dispatched(rows, hidden, experts, top_k):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows,experts,top_k", [(64, 256, 8), (5, 8, 2)])
+def test_grouped_fp8_waits_for_its_offsets(rows, experts, top_k):
+    """Counts and offsets by a kernel that lets the next ones start before it has written them. The buffers hold zeros until then: a product
+    that read too early would store nothing."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import moe_cuda, quant_ops
+    from flyingfish_b200.ops.lib import check, kernels, ptr, status_tensor, stream_ptr
+    n, k, cap = 256, 512, (rows * top_k + 16 * experts + 15) // 16 * 16
+    logits, x = torch.randn(rows, experts, generator=torch.Generator().manual_seed(1)).cuda(), _rand((rows, 8), 2).cuda()
+    xq, xs = quant_ops.quant_fp8_act(_rand((1, k), 3).cuda().expand(cap, k).contiguous())      # all rows alike: their order in a segment is free
+    codes = torch.randint(0, 120, (experts, n, k), generator=torch.Generator().manual_seed(4), dtype=torch.uint8).cuda()
+    scale = torch.rand(experts, n // 128, k // 128, generator=torch.Generator().manual_seed(5)).cuda()
+    i32 = lambda m: torch.zeros(m, dtype=torch.int32, device="cuda")
+    ids, pos, weights, sorted_x = i32(rows * top_k), i32(rows * top_k), torch.empty(rows * top_k, device="cuda"), torch.empty(cap, 8, dtype=BF16, device="cuda")
+    full = lambda: torch.full((cap, n), 5.0, dtype=BF16, device="cuda")
+    for _ in range(5):
+        counts, seg_off, y = i32(experts), i32(experts + 1), full()
+        torch.cuda._sleep(1_000_000)                          # so that the launches below are all queued before the first runs
+        check(kernels().ff_moe_plan(ptr(logits), None, ptr(weights), ptr(ids), ptr(counts), ptr(seg_off), ptr(pos), rows, experts, experts, top_k,
+                                    moe_cuda.SCORE_MODES["softmax"], experts, 1, ptr(x), ptr(sorted_x), 8, 8, 2, cap, ptr(status_tensor("cuda")), stream_ptr()), "plan")
+        quant_ops.grouped_gemm_fp8(xq, xs, codes, scale, seg_off, counts, cap, 0, out=y)
+        torch.cuda.synchronize()
+        ops.check_status()
+        assert int(counts.sum()) == rows * top_k
+        assert torch.equal(y, quant_ops.grouped_gemm_fp8(xq, xs, codes, scale, seg_off, counts, cap, 0, out=full()))
+        assert int((y != 5).any(1).sum()) == rows * top_k
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m", [1, 16, 33, 64, 100])
 @pytest.mark.parametrize("n,k", [(576, 7168), (136, 2048), (1536, 1152)])       # fourteen, four and two splits, a ragged edge
 def test_fp8_partials_of_many_splits(m, n, k):
