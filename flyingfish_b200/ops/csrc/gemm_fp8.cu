@@ -421,7 +421,7 @@ static int gemm_fp8_launch(const void* xq, const float* x_scale, const void* wq,
   const bool small = chunk < F_TOK && !single;
   const int tok_cap = experts > 1 ? chunk : (M >= F_TOK ? F_TOK : (M + 15) / 16 * 16);
   const int per = ((K / 128) + splits - 1) / splits;                     // k-blocks of one split
-  if (per * tok_cap * 4 > 64 * 1024) return FF_HOST_TOO_LARGE;           // scale staging
+  if (per * tok_cap * 4 > 64 * 1024) return FF_HOST_TOO_LARGE;           // scales of a split, without the padding of their rows
   CUtensorMap tmW, tmX;
   int r = make_tmap_2d(&tmW, wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, (uint64_t)experts * Nw, (uint64_t)K, FBK, FBM);
   if (r) return r;
@@ -429,7 +429,9 @@ static int gemm_fp8_launch(const void* xq, const float* x_scale, const void* wq,
   if (r) return r;
   const int staging = (tok_cap * FBM * 2 + per * (tok_cap + SX_PAD) * 4 + 1023) / 1024 * 1024;
   const int budget = small ? 110 * 1024 : 224 * 1024;
-  int pipe_bytes = budget - staging;
+  const int pipe_bytes = budget - staging;
+  // with scales at their limit one stage is left (26 KiB of two CTAs' 110); a ring without any would never move
+  if (pipe_bytes < FBM * FBK + (tok_cap < chunk ? tok_cap : chunk) * FBK) return FF_HOST_TOO_LARGE;
   const int smem = staging + pipe_bytes + 1024;
   dim3 grid((Nw + FBM - 1) / FBM, splits, experts);
   auto kern = chunk == 32 ? gemm_fp8_kernel<32, 2, 1> : single ? gemm_fp8_kernel<64, 1, 2> : chunk == 64 ? gemm_fp8_kernel<64, 2, 1> : gemm_fp8_kernel<F_TOK, 1, 1>;

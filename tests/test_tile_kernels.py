@@ -513,3 +513,19 @@ def test_dense_fp8_pairs(m, n, k):
     want = qref.fp8_block_linear(x, codes, scale).float()
     # exact block products, FP32 sums of k / 128 of them; device and host quantise activations alike up to a last bit of the scale
     assert ((y - want).abs() <= 2.0 ** -7 * want.abs() + 2e-3 * k ** 0.5).all()
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 48, 64, 65, 128])
+def test_fp8_scales_leave_a_stage(m):
+    """The longest K whose scales are taken still leaves the ring a stage; beyond it a product is refused. (Refusals come in front of the tensor
+    maps, which need a driver: where there is none, anything but "too large" was accepted.)"""
+    from flyingfish_b200.ops.lib import kernels, ptr
+    too_large, cap = -5, (m + 15) // 16 * 16
+    buf, ints = torch.zeros(64, dtype=torch.uint8), torch.zeros(4, dtype=torch.int32)
+
+    def call(k):
+        return kernels().ff_gemm_fp8(ptr(buf), ptr(buf), ptr(buf), ptr(buf), ptr(buf), None, None, 1, m, 128, k, 128, 0, 1, None, None, ptr(ints), None)
+    longest = 64 * 1024 // (4 * cap) * 128
+    assert call(longest + 128) == too_large
+    if not torch.cuda.is_available():
+        assert call(longest) != too_large
