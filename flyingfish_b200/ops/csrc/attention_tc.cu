@@ -29,6 +29,7 @@
 // (third_party/flash-attention/adapter.cu:147-162, device/src/lib.rs:422-940).
 #include "ptx.cuh"
 #include "host_util.h"
+#include "launchers.h"
 
 namespace ff {
 

@@ -3,25 +3,8 @@
 // Python side call one by one, in the same order and with the same arguments. Nothing is computed here. What it is for: a launch through the
 // operators takes 20 us of host time, so that prompts of up to a hundred rows were bound by the host (37 rows, 8 layers of an 8B-sized stack: 64
 // launches, 1495 -> 1249 us a call).
-#include "host_util.h"
+#include "launchers.h"
 #include <stddef.h>
-
-#pragma GCC visibility push(default)      // as where they are defined
-extern "C" {
-int ff_gemm_skinny_plan(int, int, int, long long*, long long*);
-int ff_gemm_skinny_plan_epi(int, int, int, int, long long*, long long*);
-int ff_gemm_skinny(const void*, const void*, void*, int, int, int, int, int, int, int, float*, int*, int*, cudaStream_t);
-int ff_gemm_skinny_swiglu(const void*, const void*, void*, int, int, int, int, int, int, int, float*, int*, int, float, int*, cudaStream_t);
-int ff_gemm_skinny_rope_kv(const void*, const void*, void*, int, int, int, int, int, int, int, float*, int*, const float*, const int*, void*, void*, int, int,
-                           int, int, int, int*, cudaStream_t);
-int ff_gemm_bf16(const void*, const void*, void*, int, int, int, int, int, int, int, int*, cudaStream_t);
-int ff_gemm_bf16_rope_kv(const void*, const void*, void*, int, int, int, int, int, int, const float*, const int*, void*, void*, int, int, int, int, int, int*,
-                         cudaStream_t);
-int ff_attn_prefill_tc(const void*, const void*, const void*, const int*, const int*, const int*, const int*, void*, int, int, int, int, int, int, int, int, int,
-                       int, int, float, int, int, const float*, const void*, int, int, int, float, const void*, int, int*, cudaStream_t);
-int ff_add_rmsnorm(const void*, void*, const void*, void*, void*, int, int, int, int, float, int, int*, cudaStream_t);
-}
-#pragma GCC visibility pop
 
 using namespace ff;
 

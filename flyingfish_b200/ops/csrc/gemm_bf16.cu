@@ -15,6 +15,7 @@
 #include "ptx.cuh"
 #include "comm.cuh"
 #include "host_util.h"
+#include "launchers.h"
 
 namespace ff {
 

@@ -27,6 +27,7 @@
 #include "ptx.cuh"
 #include "comm.cuh"
 #include "host_util.h"
+#include "launchers.h"
 #include <mutex>
 #include <vector>
 #include "skinny_common.cuh"

@@ -10,6 +10,7 @@
 // kernels/add_rmsnorm_capture.cu).
 #include "ptx.cuh"
 #include "host_util.h"
+#include "launchers.h"
 
 namespace ff {
 

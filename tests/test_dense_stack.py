@@ -1,6 +1,27 @@
 """The layers of a dense decoder launched by one native call against the operators called one by one."""
+import re
+from pathlib import Path
+
 import pytest
 import torch
+
+CSRC = Path(__file__).resolve().parent.parent / "flyingfish_b200" / "ops" / "csrc"
+
+
+def test_launchers_have_one_declaration():
+    """C linkage: a prototype copied by hand would go on linking against a definition whose parameters have changed. The header that declares
+    them is included where they are defined and where they are called."""
+    declared = set(re.findall(r"FF_EXPORT int (ff_\w+)\(", (CSRC / "launchers.h").read_text()))
+    assert declared
+    for src in CSRC.glob("*.cu"):
+        text = src.read_text()
+        assert not re.findall(r"\bint ff_\w+\([^;{}]*\)\s*;", text), src.name
+        defined = set(re.findall(r"FF_EXPORT int (ff_\w+)\(", text))
+        called = set(re.findall(r"\b(ff_\w+)\(", text)) - defined
+        if defined & declared or src.stem == "dense_stack":
+            assert '#include "launchers.h"' in text, src.name
+        if src.stem == "dense_stack":
+            assert called <= declared
 
 
 @pytest.mark.gpu
