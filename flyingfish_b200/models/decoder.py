@@ -26,7 +26,7 @@ from .weights import ModelWeights
 from . import moe as moe_mod
 
 
-STACK_MAX_ROWS = 128            # most prompt rows whose layers are launched by one native call
+STACK_MAX_ROWS = ops.SKINNY_MAX_M            # most prompt rows whose layers are launched by native calls: those of the decode product
 
 
 class NoComm:

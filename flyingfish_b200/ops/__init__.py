@@ -916,13 +916,13 @@ def dense_stack(x: torch.Tensor, n: torch.Tensor, layers: list[tuple[torch.Tenso
     :func:`add_rmsnorm` over prompt rows, launched by native calls: the same kernels, the same bits. ``x`` [rows, hidden]: the residual, updated in
     place; ``n``: its normed rows, overwritten. A layer: (wqkv, wo, post_ln, wgu interleaved, wdown, next_ln, K cache, V cache),
     contiguous BF16, heads and cache rows of 128 elements, pages of 64; returns how many layers were launched, those in front of the first that is
-    anything else. ``cos_sin``: :func:`rope_table` of the positions, if it is there already.
+    anything else, none for more than ``SKINNY_MAX_M`` rows. ``cos_sin``: :func:`rope_table` of the positions, if it is there already.
 
     The first layer is launched by itself: the device works on it while the other layers' tensors are looked at (37 rows, 8 layers: the first product
     started 174 us behind the embedding; 1294 us a call with all layers at once, 1260 so)."""
     rows, hidden = x.shape
     qkv_dim, att_dim = (hq + 2 * hkv) * 128, hq * 128
-    if not (x.is_cuda and x.shape == n.shape and x.dtype == n.dtype == BF16 and x.is_contiguous() and n.is_contiguous()):
+    if rows > SKINNY_MAX_M or not (x.is_cuda and x.shape == n.shape and x.dtype == n.dtype == BF16 and x.is_contiguous() and n.is_contiguous()):
         return 0
     cache = layers[0][6].shape
     shapes = ((qkv_dim, hidden), (hidden, att_dim), (hidden,), (2 * ffn, hidden), (hidden, ffn), (hidden,), cache, cache)

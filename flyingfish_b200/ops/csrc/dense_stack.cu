@@ -24,12 +24,12 @@ struct FfDenseStack {
   float scale, eps;
 };
 
-static const int DENSE_SKINNY = 128;       // rows up to which the decode product serves
-
-// scratch of the decode products of a stack's shapes, in bytes
+// scratch of the decode products of a stack's shapes, in bytes. Rows beyond what the decode product takes (FF_SKINNY_MAX_ROWS) are refused: there the
+// operators called one by one are as quick.
 FF_EXPORT int ff_dense_stack_workspace(int rows, int hidden, int ffn, int hq, int hkv, long long* scratch_bytes, long long* counter_bytes) {
   *scratch_bytes = *counter_bytes = 0;
-  if (rows <= 0 || rows > DENSE_SKINNY) return rows <= 0 ? FF_HOST_BAD_SHAPE : FF_HOST_OK;
+  if (rows <= 0) return FF_HOST_BAD_SHAPE;
+  if (rows > FF_SKINNY_MAX_ROWS) return FF_HOST_TOO_LARGE;
   auto take = [&](int grid, long long sb, long long cb) {
     if (sb > *scratch_bytes) *scratch_bytes = sb;
     if (cb > *counter_bytes) *counter_bytes = cb;
@@ -49,40 +49,25 @@ FF_EXPORT int ff_dense_stack_workspace(int rows, int hidden, int ffn, int hq, in
 FF_EXPORT int ff_dense_stack(const FfDenseLayer* layers, const FfDenseStack* a, cudaStream_t s) {
   if (layers == nullptr || a == nullptr || a->layers <= 0 || a->rows <= 0 || a->hidden % 8 || a->ffn % 128 || a->hq <= 0 || a->hkv <= 0 || a->cos_sin == nullptr) return FF_HOST_BAD_SHAPE;
   const int rows = a->rows, hidden = a->hidden, ffn = a->ffn, qkv_dim = (a->hq + 2 * a->hkv) * 128, att_dim = a->hq * 128;
-  const bool few = rows <= DENSE_SKINNY;
-  if (few) {
-    long long sb = 0, cb = 0;
-    if (int r = ff_dense_stack_workspace(rows, hidden, ffn, a->hq, a->hkv, &sb, &cb)) return r;
-    if (sb > a->scratch_bytes || cb > a->counter_bytes) return FF_HOST_TOO_LARGE;
-  }
+  long long sb = 0, cb = 0;
+  if (int r = ff_dense_stack_workspace(rows, hidden, ffn, a->hq, a->hkv, &sb, &cb)) return r;
+  if (sb > a->scratch_bytes || cb > a->counter_bytes) return FF_HOST_TOO_LARGE;
   auto product = [&](const void* x, const void* w, void* y, int n, int k) -> int {
-    if (!few) return ff_gemm_bf16(x, w, y, rows, n, k, k, k, n, 0, a->status, s);
     const int grid = ff_gemm_skinny_plan(rows, n, k, nullptr, nullptr);
     return grid < 0 ? grid : ff_gemm_skinny(x, w, y, rows, n, k, k, k, n, grid, a->scratch, a->counters, a->status, s);
   };
   for (int i = 0; i < a->layers; ++i) {
     const FfDenseLayer& l = layers[i];
-    if (few) {
-      const int grid = ff_gemm_skinny_plan_epi(rows, qkv_dim, hidden, 2, nullptr, nullptr);
-      if (grid < 0) return grid;
-      if (int r = ff_gemm_skinny_rope_kv(a->n, l.wqkv, a->qkv, rows, qkv_dim, hidden, hidden, hidden, qkv_dim, grid, a->scratch, a->counters, a->cos_sin, a->slots,
-                                         l.kcache, l.vcache, a->hq, a->hkv, 128, 64, a->num_blocks, a->status, s)) return r;
-    } else if (int r = ff_gemm_bf16_rope_kv(a->n, l.wqkv, a->qkv, rows, qkv_dim, hidden, hidden, hidden, qkv_dim, a->cos_sin, a->slots, l.kcache, l.vcache, a->hq,
-                                            a->hkv, 128, 64, a->num_blocks, a->status, s)) {
-      return r;
-    }
+    const int gq = ff_gemm_skinny_plan_epi(rows, qkv_dim, hidden, 2, nullptr, nullptr), gu = ff_gemm_skinny_plan_epi(rows, 2 * ffn, hidden, 1, nullptr, nullptr);
+    if (gq < 0 || gu < 0) return gq < 0 ? gq : gu;
+    if (int r = ff_gemm_skinny_rope_kv(a->n, l.wqkv, a->qkv, rows, qkv_dim, hidden, hidden, hidden, qkv_dim, gq, a->scratch, a->counters, a->cos_sin, a->slots,
+                                       l.kcache, l.vcache, a->hq, a->hkv, 128, 64, a->num_blocks, a->status, s)) return r;
     if (int r = ff_attn_prefill_tc(a->qkv, l.kcache, l.vcache, a->block_table, a->q_start, a->q_lens, a->ctx_lens, a->att, a->batch, rows, a->max_q_len, a->hq,
                                    a->hkv, 128, 128, qkv_dim, att_dim, a->max_blocks, a->num_blocks, a->scale, a->window, 0, nullptr, nullptr, 0, 128, 0, 0.f,
                                    nullptr, 0, a->status, s)) return r;
     if (int r = product(a->att, l.wo, a->o, hidden, att_dim)) return r;
     if (int r = ff_add_rmsnorm(a->o, a->x, l.post_ln, a->n, nullptr, 0, rows, hidden, hidden, a->eps, 0, a->status, s)) return r;
-    if (few) {
-      const int grid = ff_gemm_skinny_plan_epi(rows, 2 * ffn, hidden, 1, nullptr, nullptr);
-      if (grid < 0) return grid;
-      if (int r = ff_gemm_skinny_swiglu(a->n, l.wgu, a->mid, rows, 2 * ffn, hidden, hidden, hidden, ffn, grid, a->scratch, a->counters, 0, 0.f, a->status, s)) return r;
-    } else if (int r = ff_gemm_bf16(a->n, l.wgu, a->mid, rows, 2 * ffn, hidden, hidden, hidden, ffn, 1, a->status, s)) {
-      return r;
-    }
+    if (int r = ff_gemm_skinny_swiglu(a->n, l.wgu, a->mid, rows, 2 * ffn, hidden, hidden, hidden, ffn, gu, a->scratch, a->counters, 0, 0.f, a->status, s)) return r;
     if (int r = product(a->mid, l.wdown, a->o, hidden, ffn)) return r;
     if (int r = ff_add_rmsnorm(a->o, a->x, l.next_ln, a->n, nullptr, 0, rows, hidden, hidden, a->eps, 0, a->status, s)) return r;
   }

@@ -15,7 +15,6 @@
 #include "ptx.cuh"
 #include "comm.cuh"
 #include "host_util.h"
-#include "launchers.h"
 
 namespace ff {
 

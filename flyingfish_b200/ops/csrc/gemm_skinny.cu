@@ -32,6 +32,8 @@
 #include <vector>
 #include "skinny_common.cuh"
 
+static_assert(FF_SKINNY_MAX_ROWS == ff::STOK, "rows of a decode product");
+
 namespace ff {
 
 constexpr int SK_MAX_STAGES = 8;

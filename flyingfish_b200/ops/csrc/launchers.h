@@ -2,6 +2,8 @@
 #pragma once
 #include "host_util.h"
 
+constexpr int FF_SKINNY_MAX_ROWS = 128;        // most rows of the products of gemm_skinny.cu
+
 // gemm_skinny.cu
 FF_EXPORT int ff_gemm_skinny_plan(int M, int N, int K, long long* scratch_bytes, long long* counter_bytes);
 FF_EXPORT int ff_gemm_skinny_plan_epi(int M, int N, int K, int epi, long long* scratch_bytes, long long* counter_bytes);
@@ -12,11 +14,6 @@ FF_EXPORT int ff_gemm_skinny_swiglu(const void* X, const void* W, void* Y, int M
 FF_EXPORT int ff_gemm_skinny_rope_kv(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw, int ldy, int grid, float* scratch, int* counters,
                                      const float* cos_sin, const int* slots, void* kcache, void* vcache, int hq, int hkv, int rot_dim, int block_size,
                                      int num_blocks, int* status, cudaStream_t stream);
-
-// gemm_bf16.cu
-FF_EXPORT int ff_gemm_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw, int ldy, int epi, int* status, cudaStream_t stream);
-FF_EXPORT int ff_gemm_bf16_rope_kv(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw, int ldy, const float* cos_sin, const int* slots,
-                                   void* kcache, void* vcache, int hq, int hkv, int rot_dim, int block_size, int num_blocks, int* status, cudaStream_t stream);
 
 // attention_tc.cu
 FF_EXPORT int ff_attn_prefill_tc(const void* q, const void* kcache, const void* vcache, const int* block_table, const int* q_start, const int* q_lens,

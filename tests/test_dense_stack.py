@@ -27,7 +27,7 @@ def test_launchers_have_one_declaration():
 @pytest.mark.gpu
 @pytest.mark.parametrize("lens,pasts", [([1], [0]), ([37], [0]), ([5, 64, 59], [0, 70, 3]), ([129], [0]), ([300, 1, 211], [10, 0, 64])])
 def test_native_layers_give_the_bits_of_the_operators(lens, pasts, monkeypatch):
-    """Rows of the decode product and of the pair product, several sequences, portions behind a context."""
+    """One and several sequences, portions behind a context; more rows than the decode product takes are left to the operators."""
     import copy
     from flyingfish_b200 import ops
     from flyingfish_b200.config import Settings, named_shape
@@ -52,10 +52,10 @@ def test_native_layers_give_the_bits_of_the_operators(lens, pasts, monkeypatch):
             monkeypatch.setattr(decoder, "STACK_MAX_ROWS", 1024)
         calls = []
         real = ops.dense_stack
-        monkeypatch.setattr(ops, "dense_stack", lambda *a, **k: calls.append(1) or real(*a, **k))
+        monkeypatch.setattr(ops, "dense_stack", lambda *a, **k: calls.append(real(*a, **k)) or calls[-1])
         eng.prefill(seqs)
         monkeypatch.setattr(ops, "dense_stack", real)
-        assert bool(calls) == native
+        assert bool(calls) == native and all(n == (spec.layers if sum(lens) <= ops.SKINNY_MAX_M else 0) for n in calls)
         ops.check_status()
         return net.last_logits.clone(), net.last_residual.clone(), [t.clone() for t in eng.kv.k + eng.kv.v]
     a, b = run(False), run(True)
