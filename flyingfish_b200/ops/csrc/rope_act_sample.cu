@@ -252,7 +252,9 @@ template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-template <typename T>
+// U: 16-byte vectors of BF16 logits in flight per thread. A row of 128 K logits is 256 KB read by one CTA, in latency-bound rounds of loads. Four need
+// more registers than two CTAs on an SM have, two do not; which is the better follows from how many rows an SM gets (ff_argmax_rows).
+template <typename T, int U>
 __global__ void __launch_bounds__(1024)
 argmax_rows_kernel(const T* __restrict__ logits, int* __restrict__ out_ids, float* __restrict__ out_vals, int vocab,
                    int ld, int id_offset, const int* __restrict__ valid_rows, int* status) {
@@ -269,19 +271,18 @@ argmax_rows_kernel(const T* __restrict__ logits, int* __restrict__ out_ids, floa
   const T* p = logits + (size_t)row * ld;
   int i0 = 0;
   if (sizeof(T) == 2 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-    // 16-byte vectors, four in flight per thread: a row of 128 K logits is 256 KB read by one CTA, in latency-bound rounds of loads. 64 rows
-    // with two in flight / four: 16.4 / 10.1 us, one row 8.9 / 9.4 (eight: 11.5 and 10.7).
-    constexpr int U = 4;
     const int nvec = vocab >> 3;
     const uint4* pv = reinterpret_cast<const uint4*>(p);
     for (int i = threadIdx.x; i < nvec; i += U * blockDim.x) {
       uint4 u[U];
 #pragma unroll
-      for (int h = 0; h < U; ++h)
-        if (i + h * (int)blockDim.x < nvec) u[h] = pv[i + h * blockDim.x];
+      for (int h = 0; h < U; ++h) {
+        if (h == 0 || i + h * (int)blockDim.x < nvec) u[h] = pv[i + h * blockDim.x];
+        else if (U == 2) u[h] = make_uint4(0, 0, 0, 0);      // the load as a select: 256 rows of 128 K logits 20.0 -> 18.9 us; with four 8.5 -> 8.8 for one row
+      }
 #pragma unroll
       for (int h = 0; h < U; ++h) {
-        if (i + h * (int)blockDim.x >= nvec) break;
+        if (h > 0 && i + h * (int)blockDim.x >= nvec) break;
         const uint32_t* w = reinterpret_cast<const uint32_t*>(&u[h]);
         const int base = (i + h * blockDim.x) * 8;
 #pragma unroll
@@ -573,10 +574,12 @@ FF_EXPORT int ff_argmax_rows(const void* logits, int* out_ids, float* out_vals, 
   if (rows <= 0 || vocab <= 0) return FF_HOST_BAD_SHAPE;
   int lr;
   if (dtype == 0) {
-    lr = launch_pdl(argmax_rows_kernel<__nv_bfloat16>, dim3(rows), dim3(1024), 0, s, 0, (const __nv_bfloat16*)logits, out_ids,
-                    out_vals, vocab, ld, id_offset, valid_rows, status);
+    // While every row has an SM of its own, four vectors in flight are as quick or quicker (128 rows of 128 K logits 15.9 -> 12.8 us with a cold cache, 14.6 -> 8.8
+    // with a warm one; one row 10.8 and 10.8); beyond, two rows on an SM are: 149 rows 20.5 with four, 17.9 with two, 256 rows 22.5 and 18.9, 1024 rows 69 and 56.
+    lr = launch_pdl(rows <= sm_count() ? argmax_rows_kernel<__nv_bfloat16, 4> : argmax_rows_kernel<__nv_bfloat16, 2>, dim3(rows), dim3(1024), 0, s, 0,
+                    (const __nv_bfloat16*)logits, out_ids, out_vals, vocab, ld, id_offset, valid_rows, status);
   } else {
-    lr = launch_pdl(argmax_rows_kernel<float>, dim3(rows), dim3(1024), 0, s, 0, (const float*)logits, out_ids, out_vals, vocab,
+    lr = launch_pdl(argmax_rows_kernel<float, 1>, dim3(rows), dim3(1024), 0, s, 0, (const float*)logits, out_ids, out_vals, vocab,
                     ld, id_offset, valid_rows, status);
   }
   if (lr) return lr;

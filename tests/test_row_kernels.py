@@ -183,3 +183,17 @@ def test_expanded_attention_over_packed_heads(q_lens, pasts):
             got = out[s0: s0 + n].view(n, heads, dv)[:, h].cpu().double()
             # keys, values, weights and results are rounded to BF16 (2^-9 each): four roundings of values of about 0.5
             assert ((got - want).abs() <= 1e-2 + 1e-2 * want.abs()).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [8, 1000, 16384, 40008, 49160])          # parts of a round of two and of four vectors, a tail of single logits
+def test_argmax_by_rows_of_an_sm(vocab):
+    """Both instances: a row per SM at most, and more. Equal logits give the lower id."""
+    from flyingfish_b200 import ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for rows in (1, sms, sms + 1, 2 * sms + 3):
+        lg = (torch.randn(rows, vocab, generator=torch.Generator().manual_seed(rows)) * 4).round().to(BF16)       # many ties
+        got = ops.argmax_rows(lg.cuda()).cpu().long()
+        top = lg == lg.amax(1, keepdim=True)
+        assert torch.equal(got, top.int().argmax(1))
+    ops.check_status()
