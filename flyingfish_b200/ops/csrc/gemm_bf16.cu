@@ -93,8 +93,8 @@ __device__ __forceinline__ bool next_tile(const GroupArgs& g, TileWalk& w, int t
 
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 
-// epi: 3 = rotary embedding and cache write (LinTail); 0 = store bf16; 1 = SwiGLU (every 128 columns of a tile are 64 gate then the matching 64 up columns; output
-// has N/2 columns); 2 = store fp32.
+// epi: 0 = store bf16; 1 = SwiGLU (every 128 columns of a tile are 64 gate then the matching 64 up columns; output has N/2 columns); 2 = store fp32;
+// 3 = rotary embedding and cache write (LinTail).
 // COMM (tensor-parallel prefill, rows split evenly over the ranks in 128-row blocks):
 //   1 = all-gather -> GEMM : A is row-sharded. Four extra warps per CTA (all CTAs together) push this
 //       rank's shard into every peer's arena with plain peer stores, a quarter of a 128-row block at a
@@ -840,12 +840,13 @@ static int gemm_bf16_launch(const void* X, const void* W, void* Y, int M, int N,
   PairTiles pt;
   const float pair_waves = pair_plan(M, N, epi, pairs, pt) / pair_cost(256);
   // Tiles of one CTA where they finish in clearly fewer waves: 256-row tiles of pairs pad rows more, and at short K a pair's set-up and its
-  // epilogue take what its main loop saves. A wave of one-CTA tiles is charged 1 / 0.79 of a pair's (1 / 0.97 behind a SwiGLU epilogue at K up
-  // to 2048, 1 / 1.05 at K up to 512 and for a single wave at K up to 1024). Of 1507 sizes (42 shapes of 512 x 512 to 65536 x 2048 and 57344 x
-  // 8192, 130 to 8192 rows) that is the quicker form within 2 % at all but 18, within 5 % at those. One-CTA / pair tiles: 1100 x 4096 x 14336
-  // 98 / 128 us, 320 x 24576 x 1536 29 / 32, 4096 x 32768 x 512 157 / 179. K is walked in the same order: the bits are the same.
+  // epilogue take what its main loop saves. A wave of one-CTA tiles is charged 1 / 0.86 of a pair's; with a SwiGLU epilogue 1 / 0.79, at K up to 2048
+  // 1 / 0.97; 1 / 1.05 at K up to 512, and at K up to 1024 for a single wave or a SwiGLU epilogue. Both forms in turn at 736 sizes (24 shapes of 512 x 512 to
+  // 65536 x 2048, 129 to 8191 rows): that is the quicker form within 2 % at all but 6, within 3.3 % at those. One-CTA / pair tiles: 1100 x 4096 x 14336
+  // 95 / 104 us, 1100 x 8192 x 1024 21 / 23, 4096 x 32768 x 512 152 / 180, 600 x 36864 x 7168 251 / 263.
+  // K is walked in the same order: the bits are the same.
   const int ctas = sm_count(), waves1 = (((M + BM - 1) / BM) * ((N + 255) / 256) + ctas - 1) / ctas;
-  const float share = K <= 512 || (K <= 1024 && waves1 == 1) ? 1.05f : epi == 1 && K <= 2048 ? 0.97f : 0.79f;
+  const float share = K <= 512 || (K <= 1024 && (waves1 == 1 || epi == 1)) ? 1.05f : epi != 1 ? 0.86f : K <= 2048 ? 0.97f : 0.79f;
   if (waves1 < share * pair_waves) {
     constexpr int BN = 256, STAGES = 4;
     CUtensorMap tmB;
