@@ -166,8 +166,6 @@ moe_fp4_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             q[j] = *reinterpret_cast<const uint2*>(st + row * 128 + (((2 * j + (part >> 1)) ^ sw) << 4) + (part & 1) * 8);
             sc[j] = st[FT_CODES + row * 16 + j * 4 + part];
           }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars.p_empty[pp.s]);  // in registers
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             __nv_bfloat162 s2, unused;
@@ -190,6 +188,9 @@ moe_fp4_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             if (lane == 0) mbar_arrive(&bars.a_full[ap.s]);
             ap.next(FT_STAGES);
           }
+          // The chunk is given back behind the stores that its codes went into. An arrival right behind the loads does not wait for them: where the tensor
+          // cores held the expanding warps up (segments from about 150 rows) the refill overtook the loads of the chunk's last K blocks.
+          if (ok && lane == 0) mbar_arrive(&bars.p_empty[pp.s]);
         }
     }
   } else {                                                  // finished tiles: lane = weight row, columns = rows of the segment

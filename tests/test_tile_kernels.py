@@ -338,6 +338,32 @@ def test_grouped_nvfp4_for_prompts(counts, n, k, epi):
                 _check(got, rows, k)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,prompts", [(256, True), (300, True), (40, True), (32, False), (5, False)])
+def test_packed_experts_repeat_their_bits(rows, prompts):
+    """Rings refilled many times while the tensor cores hold the warps up that read them: every launch the bits of the first, and those near 64 bits."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import moe_cuda
+    e, n, k = 24, 2048, 4096
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    codes = torch.randint(0, 256, (e, n, k // 2), dtype=torch.uint8, device="cuda", generator=g)
+    scales = torch.randint(40, 60, (e, n, k // 16), dtype=torch.uint8, device="cuda", generator=g)
+    w = moe_cuda.Nvfp4Experts(codes, scales, torch.ones(e, device="cuda"))
+    pad = (rows + 15) // 16 * 16
+    x = torch.randn(e * pad, k, device="cuda", generator=g).to(BF16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    off, counts = i32([pad * i for i in range(e + 1)]), i32([rows] * e)
+    run = lambda: moe_cuda.grouped_gemm_nvfp4(x, w, off, counts, e * pad, 0, rows_per_expert=1e6 if prompts else 0.0).view(e, pad, n)[:, :rows]
+    first = run().clone()
+    assert all(torch.equal(run(), first) for _ in range(20))
+    ops.check_status()
+    for i in (0, e - 1):
+        full = (qref.e2m1_decode(qref.e2m1_unpack(codes[i].cpu())).view(n, -1, 16) * qref.e4m3_decode(scales[i].cpu())[..., None]).view(n, k).double()
+        want = x[i * pad: i * pad + rows].cpu().double() @ full.t()
+        # one rounding of the result; FP32 sums of k products of the size of the weights
+        assert ((first[i].cpu().double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * k * full.abs().max()).all()
+
+
 _WALK = r"""
 #include <atomic>
 #include <barrier>
