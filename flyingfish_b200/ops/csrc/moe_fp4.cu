@@ -112,8 +112,6 @@ __device__ __forceinline__ bool f4_pass(const __nv_bfloat16* __restrict__ X, int
         sb[h] = h < halves ? __ldg(reinterpret_cast<const unsigned short*>(p + (size_t)8 * (K / 16))) : 0;
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&bars.empty[s]);           // in registers
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (h < halves) {
@@ -136,6 +134,10 @@ __device__ __forceinline__ bool f4_pass(const __nv_bfloat16* __restrict__ X, int
         }
       }
     }
+    // The stage is given back behind its last multiplication, and the arrival's address goes through that sum (epi is 0 or 1): an arrival does not wait
+    // for loads in front of it, and right behind them a refill could overtake those that have not returned.
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars.empty[s + (__float_as_uint(acc[0][0]) & ((uint32_t)epi >> 1))]);
   };
   if (!walk_pass(chunks, PER_SLAB, f4_sync, fill, wait, multiply, f4_sync_any)) return false;
   // ---- epilogue through an FP32 transpose tile [token][128] in the tokens' place
