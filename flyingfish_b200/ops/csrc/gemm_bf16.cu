@@ -635,13 +635,14 @@ struct alignas(8) PairBars {
   uint64_t full[PAIR_STAGES];   // the even CTA's: both CTAs' loads of a stage have landed
   uint64_t empty[PAIR_STAGES];  // each CTA's own, freed by the even CTA's commits
   uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];       // the even CTA's: the sixteen epilogue warps of the pair have read the accumulator
+  uint64_t tmem_empty[2];       // the even CTA's: the epilogue warps of the pair have read the accumulator
   uint32_t tmem_base;
   int abort_flag;
 };
 
-// A ring as deep as shared memory takes (7 stages 256 wide, 11 stages 64 wide: 200 rows times 4096 x 14336 50.6 -> 40.0 us) and two epilogue warps
-// per 32 rows, since the last tile's epilogue is not hidden: 130 x 4096 x 4096 17.5 -> 16.1 us.
+// A ring as deep as shared memory takes (7 stages 256 wide, 11 stages 64 wide: 200 rows times 4096 x 14336 50.6 -> 40.0 us). PARTS: epilogue warps that
+// share 32 rows. Two where the epilogue computes (SwiGLU, 4096 x 8192 x 1024: 110 us with one, 70 with two; GELU 3 %, rotation and cache write 2 %), one
+// where it only stores: the second costs 0.2 us at a launch's ends (one / two: 1000 x 2048 x 2048 11.5 / 11.8 us, 1500 x 1024 x 1024 7.7 / 8.2).
 // Tiles of a launch: `wide` columns of tiles w1 wide, then tiles w2 wide up to N; every width a multiple of 32 (of 128 with epi 1 and 3), at most 256.
 struct PairTiles { int w1, wide, w2; };
 
@@ -653,7 +654,8 @@ __device__ __forceinline__ void pair_tile(const PairTiles& pt, int t, int tiles_
   else { tile_coords(t - n1, tiles_m, tiles_n2, tm, tn); col0 = pt.wide * pt.w1 + tn * pt.w2; width = pt.w2; }
 }
 
-__global__ void __launch_bounds__(320, 1)
+template <int PARTS>
+__global__ void __launch_bounds__(64 + 128 * PARTS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ CUtensorMap tmB2,
                       void* __restrict__ Cout, int M, int N, int K, int ldc, int epi, const PairTiles pt, int stages, int* status, LinTail tail) {
   extern __shared__ uint8_t smem_raw[];
@@ -670,7 +672,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB1); tma_prefetch_desc(&tmB2);
     for (int i = 0; i < stages; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars.tmem_full[i], 1); mbar_init(&bars.tmem_empty[i], 16); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars.tmem_full[i], 1); mbar_init(&bars.tmem_empty[i], 8 * PARTS); }
     bars.abort_flag = 0;
     mbar_fence_init();
   }
@@ -747,7 +749,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (!ok) break;
       tc_fence_after();
       const int row = (2 * tm + rank) * BM + q * 32 + lane;
-      store_tile_row<2>(tmem_base + (uint32_t(q * 32) << 16) + acc * 256, Cout, row, row < M, ldc, N, epi, col0, width, 0, tail, (warp - 2) >> 2, status);
+      store_tile_row<PARTS>(tmem_base + (uint32_t(q * 32) << 16) + acc * 256, Cout, row, row < M, ldc, N, epi, col0, width, 0, tail, (warp - 2) >> 2, status);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(&bars.tmem_empty[acc]);
@@ -816,10 +818,15 @@ static int pair_launch(const CUtensorMap& tmA, const void* W, void* Y, int M, in
   CUtensorMap tmB1, tmB2;
   if (int e = make_tmap_2d(&tmB1, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, pt.w1 / 2)) return e;
   if (int e = make_tmap_2d(&tmB2, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, pt.w2 / 2)) return e;
-  const int fit = PAIR_RING / (BM * BK * 2 + (pt.wide ? pt.w1 : pt.w2) * BK), stages = fit < PAIR_STAGES ? fit : PAIR_STAGES;
+  // Large results at short K are limited by power, and a seventh stage of 256 columns only loads earlier than needed: 4096 x 24576 x 1536 221 us with
+  // seven, 218 with six, 8191 x 8192 x 1024 111.1 / 110.3; from K = 2048 on no difference.
+  const int stage_bytes = BM * BK * 2 + (pt.wide ? pt.w1 : pt.w2) * BK, fit = PAIR_RING / stage_bytes;
+  const int stages = fit == 7 && K <= 1536 ? 6 : fit < PAIR_STAGES ? fit : PAIR_STAGES;
   constexpr int SMEM = PAIR_RING + 1024;
-  if (int e = opt_in_smem(gemm_bf16_pair_kernel, SMEM)) return e;
-  if (int e = launch_pdl(gemm_bf16_pair_kernel, dim3(grid), dim3(320), SMEM, stream, 2, tmA, tmB1, tmB2, Y, M, N, K, ldy, epi, pt, stages, status, tail)) return e;
+  const bool stores = (epi == 0 || epi == 2) && tail.bias == nullptr && tail.act == 0 && tail.mul == nullptr;
+  auto kern = stores ? gemm_bf16_pair_kernel<1> : gemm_bf16_pair_kernel<2>;
+  if (int e = opt_in_smem(kern, SMEM)) return e;
+  if (int e = launch_pdl(kern, dim3(grid), dim3(stores ? 192 : 320), SMEM, stream, 2, tmA, tmB1, tmB2, Y, M, N, K, ldy, epi, pt, stages, status, tail)) return e;
   return launch_result();
 }
 
@@ -841,12 +848,13 @@ static int gemm_bf16_launch(const void* X, const void* W, void* Y, int M, int N,
   const float pair_waves = pair_plan(M, N, epi, pairs, pt) / pair_cost(256);
   // Tiles of one CTA where they finish in clearly fewer waves: 256-row tiles of pairs pad rows more, and at short K a pair's set-up and its
   // epilogue take what its main loop saves. A wave of one-CTA tiles is charged 1 / 0.86 of a pair's; with a SwiGLU epilogue 1 / 0.79, at K up to 2048
-  // 1 / 0.97; 1 / 1.05 at K up to 512, and at K up to 1024 for a single wave or a SwiGLU epilogue. Both forms in turn at 736 sizes (24 shapes of 512 x 512 to
+  // 1 / 0.97; 1 / 1.05 at K up to 512, and at K up to 1024 for a single wave or a SwiGLU epilogue (tanh-GELU, which computes more: 4096 x 8192 x
+  // 1024 53 / 47 us). Both forms in turn at 736 sizes (24 shapes of 512 x 512 to
   // 65536 x 2048, 129 to 8191 rows): that is the quicker form within 2 % at all but 6, within 3.3 % at those. One-CTA / pair tiles: 1100 x 4096 x 14336
   // 95 / 104 us, 1100 x 8192 x 1024 21 / 23, 4096 x 32768 x 512 152 / 180, 600 x 36864 x 7168 251 / 263.
   // K is walked in the same order: the bits are the same.
   const int ctas = sm_count(), waves1 = (((M + BM - 1) / BM) * ((N + 255) / 256) + ctas - 1) / ctas;
-  const float share = K <= 512 || (K <= 1024 && (waves1 == 1 || epi == 1)) ? 1.05f : epi != 1 ? 0.86f : K <= 2048 ? 0.97f : 0.79f;
+  const float share = K <= 512 || (K <= 1024 && (waves1 == 1 || (epi == 1 && tail.gate == 0))) ? 1.05f : epi != 1 ? 0.86f : K <= 2048 ? 0.97f : 0.79f;
   if (waves1 < share * pair_waves) {
     constexpr int BN = 256, STAGES = 4;
     CUtensorMap tmB;
