@@ -1,5 +1,6 @@
-// Grouped expert GEMM over NVFP4 weights for prompts, on tcgen05 (formats, rounding and epilogues as in moe_fp4.cu, which serves segments of a
-// few rows):  Y[seg rows, Nw] = Xs[seg rows, K] · (e2m1(Wq[e]) * e4m3(Wsc[e]) * global[e])[Nw, K]ᵀ
+// Grouped expert GEMM over NVFP4 weights for batches of 16 and more rows an expert on average, on tcgen05 (formats, rounding and epilogues as in
+// moe_fp4.cu, which serves segments of a few rows; prompts of more than 32 rows an expert take the BF16 copies that the layer keeps):
+//   Y[seg rows, Nw] = Xs[seg rows, K] · (e2m1(Wq[e]) * e4m3(Wsc[e]) * global[e])[Nw, K]ᵀ
 // moe_fp4.cu expands a weight tile once for every 32 rows of a segment, which is what its time goes by; here it is expanded once for up to 256.
 // Whole expert layer (128 experts of 4096 x 1536), us with moe_fp4.cu / here: 8 rows an expert 540 / 738, 12.5 652 / 740, 16 757 / 742, 32
 // 1241 / 759; on BF16 copies of the experts 752, 846, 845 and 878. The packed bytes take 207.

@@ -275,7 +275,10 @@ def experts_forward_nvfp4(x, weights, ids, gate_up: Nvfp4Experts, down: Nvfp4Exp
 
 
 FP4_DECODE_MAX_ROWS = int(os.environ.get("FF_FP4_MAX_ROWS_PER_EXPERT", "32"))
-FP4_TC_MIN_ROWS = 16.0           # expert layer at 12.5 rows an expert 652 us packed / 740 on tcgen05, at 16 757 / 742
+# Rows an expert from which the tcgen05 kernel is the quicker one. A product, us with csrc/moe_fp4.cu / on tcgen05 at 12 and 16 rows an expert: 128 experts of
+# 3072 x 4096 427 / 469 and 515 / 464, 128 of 4096 x 1536 219 / 244 and 256 / 242, 64 of 2048 x 2048 88 / 88 and 97 / 84, 256 of 4096 x 7168 1799 / 2130
+# and 2187 / 2132, 16 of 16384 x 5120 325 / 392 and 430 / 394, 8 of 28672 x 4096 235 / 291 and 290 / 287
+FP4_TC_MIN_ROWS = 16.0
 
 
 def pack_experts_nvfp4(weights) -> int:
