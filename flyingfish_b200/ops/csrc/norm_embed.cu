@@ -32,8 +32,11 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // unit_offset: 1 -> weight is (1 + w) (Gemma convention), 0 -> w
 // NVEC: vectors per thread. One instance for all widths held 64 values in registers and left four CTAs on an SM, and the weight was asked for
 // behind the row's sum. 8121 rows of 4096 76 -> 57 us, one row 4.2 -> 3.0 (the sums are taken in the same order).
-template <int MODE, int NVEC>
-__global__ void __launch_bounds__(NORM_THREADS, NVEC == 1 ? 8 : NVEC == 2 ? (MODE == 2 ? 6 : 8) : NVEC == 4 ? 3 : 2)
+// Rows wider than 8192 (NVEC 8): four CTAs on an SM, five of the embedding, three of the sum, whose second operand needs the registers: as many as do without
+// spilling. FIVE: the instance of the plain norm that has five, by loading a vector when its turn comes, which is what one wave of that
+// size is worth (norm_of): rows of 16384, two CTAs on an SM / four / five, us: 1 row 3.8 / 4.1 / 5.1, 600 9.5 / 8.5 / 7.2, 1000 12.5 / 10.0 / 11.8.
+template <int MODE, int NVEC, bool FIVE = false>
+__global__ void __launch_bounds__(NORM_THREADS, NVEC == 1 ? 8 : NVEC == 2 ? (MODE == 2 ? 6 : 8) : NVEC == 4 ? 3 : MODE == 2 ? 3 : MODE == 1 || FIVE ? 5 : 4)
 norm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ res, const int* __restrict__ ids,
             const __nv_bfloat16* __restrict__ table, const __nv_bfloat16* __restrict__ w,
             __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ capture, int capture_stride, int hidden,
@@ -59,7 +62,7 @@ norm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ res
   for (int i = 0; i < NVEC; ++i) {
     const int idx = threadIdx.x + i * NORM_THREADS;
     if (idx < nvec) {
-      v[i] = reinterpret_cast<const uint4*>(src)[idx];
+      if (!FIVE) v[i] = reinterpret_cast<const uint4*>(src)[idx];
       if (MODE == 2) rv[i] = reinterpret_cast<const uint4*>(res + (size_t)row * hidden)[idx];
       if (NVEC <= 4) wv[i] = __ldg(reinterpret_cast<const uint4*>(w) + idx);
     }
@@ -68,7 +71,7 @@ norm_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ res
   for (int i = 0; i < NVEC; ++i) {
     const int idx = threadIdx.x + i * NORM_THREADS;
     if (idx < nvec) {
-      uint4 a = v[i];
+      uint4 a = FIVE ? reinterpret_cast<const uint4*>(src)[idx] : v[i];
       if (MODE == 2) {
         uint32_t* ap = reinterpret_cast<uint32_t*>(&a);
         const uint32_t* rp = reinterpret_cast<const uint32_t*>(&rv[i]);
@@ -152,8 +155,9 @@ static int check_hidden(int hidden) {
 
 // the instance with as many vectors per thread as the row takes
 template <int MODE>
-static auto norm_of(int hidden) {
+static auto norm_of(int hidden, int rows) {
   const int n = (hidden / 8 + NORM_THREADS - 1) / NORM_THREADS;
+  if (MODE == 0 && n > 4 && rows > 4 * sm_count() && rows <= 5 * sm_count()) return norm_kernel<MODE, 8, MODE == 0>;
   return n <= 1 ? norm_kernel<MODE, 1> : n <= 2 ? norm_kernel<MODE, 2> : n <= 4 ? norm_kernel<MODE, 4> : norm_kernel<MODE, 8>;
 }
 
@@ -162,7 +166,7 @@ FF_EXPORT int ff_rmsnorm(const void* x, const void* w, void* out, int rows, int 
   if (int r = check_hidden(hidden)) return r;
   if (rows <= 0) return FF_HOST_BAD_SHAPE;
   if (ldx % 8) return FF_HOST_BAD_ALIGN;
-  if (int lr_ = launch_pdl(norm_of<0>(hidden), dim3(rows), dim3(NORM_THREADS), 0, s, 0, (const __nv_bfloat16*)x, nullptr, nullptr, nullptr,
+  if (int lr_ = launch_pdl(norm_of<0>(hidden, rows), dim3(rows), dim3(NORM_THREADS), 0, s, 0, (const __nv_bfloat16*)x, nullptr, nullptr, nullptr,
       (const __nv_bfloat16*)w, (__nv_bfloat16*)out, nullptr, 0, hidden, 0, eps, unit_offset, ldx, status)) return lr_;
   return launch_result();
 }
@@ -171,7 +175,7 @@ FF_EXPORT int ff_embed_rmsnorm(const int* ids, const void* table, const void* w,
                                int hidden, int vocab, float eps, int unit_offset, int* status, cudaStream_t s) {
   if (int r = check_hidden(hidden)) return r;
   if (rows <= 0) return FF_HOST_BAD_SHAPE;
-  if (int lr_ = launch_pdl(norm_of<1>(hidden), dim3(rows), dim3(NORM_THREADS), 0, s, 0, nullptr, (__nv_bfloat16*)res, ids, (const __nv_bfloat16*)table,
+  if (int lr_ = launch_pdl(norm_of<1>(hidden, rows), dim3(rows), dim3(NORM_THREADS), 0, s, 0, nullptr, (__nv_bfloat16*)res, ids, (const __nv_bfloat16*)table,
       (const __nv_bfloat16*)w, (__nv_bfloat16*)out, nullptr, 0, hidden, vocab, eps, unit_offset, hidden, status)) return lr_;
   return launch_result();
 }
@@ -183,7 +187,7 @@ FF_EXPORT int ff_add_rmsnorm(const void* x, void* res, const void* w, void* out,
   if (int r = check_hidden(hidden)) return r;
   if (rows <= 0) return FF_HOST_BAD_SHAPE;
   if (ldx % 8 || capture_stride % 8) return FF_HOST_BAD_ALIGN;
-  if (int lr_ = launch_pdl(norm_of<2>(hidden), dim3(rows), dim3(NORM_THREADS), 0, s, 0, (const __nv_bfloat16*)x, (__nv_bfloat16*)res, nullptr, nullptr,
+  if (int lr_ = launch_pdl(norm_of<2>(hidden, rows), dim3(rows), dim3(NORM_THREADS), 0, s, 0, (const __nv_bfloat16*)x, (__nv_bfloat16*)res, nullptr, nullptr,
       (const __nv_bfloat16*)w, (__nv_bfloat16*)out, (__nv_bfloat16*)capture, capture_stride, hidden, 0, eps,
       unit_offset, ldx, status)) return lr_;
   return launch_result();

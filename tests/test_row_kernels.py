@@ -197,3 +197,23 @@ def test_argmax_by_rows_of_an_sm(vocab):
         top = lg == lg.amax(1, keepdim=True)
         assert torch.equal(got, top.int().argmax(1))
     ops.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hidden", [8200, 16384])                # parts of a thread's vectors, all of them
+@pytest.mark.parametrize("waves", [1, 4, 5, 6])
+def test_norm_of_wide_rows(hidden, waves):
+    """Rows around the waves at which another instance runs: the bits of the same rows normed a few at a time, and those near 64 bits."""
+    from flyingfish_b200 import ops
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    w = (1 + 0.1 * torch.randn(hidden, generator=torch.Generator().manual_seed(1))).to(BF16)
+    for rows in (waves * sms, waves * sms + 1):
+        x = torch.randn(rows, hidden, generator=torch.Generator().manual_seed(rows)).to(BF16).cuda()
+        got = ops.rmsnorm(x, w.cuda(), 1e-6)
+        few = torch.cat([ops.rmsnorm(part.contiguous(), w.cuda(), 1e-6) for part in x.split(100)])
+        assert torch.equal(got, few)
+        some = x[:: max(1, rows // 20)].cpu().double()
+        want = some * torch.rsqrt(some.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+        # one rounding of the result; the sum and its root in FP32
+        assert ((got[:: max(1, rows // 20)].cpu().double() - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs()).all()
+    ops.check_status()
