@@ -462,14 +462,15 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
 // (+ optional residual-style accumulate into `out` when accumulate != 0). pos < 0 skips
 // (assignment owned by another rank).
 // ---------------------------------------------------------------------------------------
-// Bound by DRAM for prompts, by latency for decode steps: a CTA takes 128 vectors of a row, whose choices' loads are in flight
-// together, instead of a row, one choice after the other. Cold, eight choices: 32 x 4096 16.4 -> 10.2 us, 64 x 7168 26.6 -> 10.2, 2039 x 4096 45 -> 41.
-constexpr int COMBINE_THREADS = 128, COMBINE_LOADS = 8;
-__global__ void __launch_bounds__(COMBINE_THREADS)
+// Bound by DRAM for prompts, by latency for decode steps: LOADS choices of VECS vectors have their loads in flight together, in place of one choice after
+// the other. Us before / so: with a cold cache 64 x 7168 with eight choices 26.7 / 10.2, 2039 x 4096 45 / 39; warm 2039 x 4096 35 / 28, 8191 x 7168 196 / 163, with
+// two choices 65 / 62, with one 44 / 40.
+template <int LOADS, int VECS>
+__global__ void __launch_bounds__(256)
 moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos, const int* __restrict__ ids,
                    const float* __restrict__ w, __nv_bfloat16* __restrict__ out, int hidden, int top_k, int ldy,
                    int accumulate) {
-  const int row = blockIdx.x, v = blockIdx.y * COMBINE_THREADS + threadIdx.x;
+  const int row = blockIdx.x, nvec = hidden / 8, step = gridDim.y * blockDim.x;
   __shared__ int s_pos[16], s_id[16]; __shared__ float s_w[16];
   pdl_wait();
   // the choices in the order of their expert ids (equal ids in the order of the choices): each finds its own place
@@ -483,34 +484,44 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ 
     s_pos[place] = at; s_w[place] = wt;
   }
   __syncthreads();
-  if (v < hidden / 8) {
-    float acc[8];
+  for (int v0 = blockIdx.y * blockDim.x + threadIdx.x; v0 < nvec; v0 += VECS * step) {
+    float acc[VECS][8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    for (int j0 = 0; j0 < top_k; j0 += COMBINE_LOADS) {
-      uint4 d[COMBINE_LOADS];
+    for (int q = 0; q < VECS; ++q)
 #pragma unroll
-      for (int u = 0; u < COMBINE_LOADS; ++u)
-        if (j0 + u < top_k && s_pos[j0 + u] >= 0) d[u] = reinterpret_cast<const uint4*>(y + (size_t)s_pos[j0 + u] * ldy)[v];
+      for (int i = 0; i < 8; ++i) acc[q][i] = 0.f;
+    for (int j0 = 0; j0 < top_k; j0 += LOADS) {
+      uint4 d[LOADS][VECS];
 #pragma unroll
-      for (int u = 0; u < COMBINE_LOADS; ++u) {
+      for (int u = 0; u < LOADS; ++u)
+        if (j0 + u < top_k && s_pos[j0 + u] >= 0)
+#pragma unroll
+          for (int q = 0; q < VECS; ++q)
+            if (q == 0 || v0 + q * step < nvec) d[u][q] = reinterpret_cast<const uint4*>(y + (size_t)s_pos[j0 + u] * ldy)[v0 + q * step];
+#pragma unroll
+      for (int u = 0; u < LOADS; ++u) {
         if (j0 + u >= top_k || s_pos[j0 + u] < 0) continue;
-        const uint32_t* dp = reinterpret_cast<const uint32_t*>(&d[u]);
         const float ww = s_w[j0 + u];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { const float2 f = unpack_bf16x2(dp[i]); acc[2 * i] += ww * f.x; acc[2 * i + 1] += ww * f.y; }
+        for (int q = 0; q < VECS; ++q) {
+          const uint32_t* dp = reinterpret_cast<const uint32_t*>(&d[u][q]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { const float2 f = unpack_bf16x2(dp[i]); acc[q][2 * i] += ww * f.x; acc[q][2 * i + 1] += ww * f.y; }
+        }
       }
     }
-    uint4 o;
-    if (accumulate) {
-      const uint4 prev = reinterpret_cast<const uint4*>(out + (size_t)row * hidden)[v];
-      const uint32_t* pp = reinterpret_cast<const uint32_t*>(&prev);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) { const float2 f = unpack_bf16x2(pp[i]); acc[2 * i] += f.x; acc[2 * i + 1] += f.y; }
+    for (int q = 0; q < VECS; ++q) {
+      if (q > 0 && v0 + q * step >= nvec) break;
+      uint4* dst = reinterpret_cast<uint4*>(out + (size_t)row * hidden) + v0 + q * step;
+      if (accumulate) {
+        const uint4 prev = *dst;
+        const uint32_t* pp = reinterpret_cast<const uint32_t*>(&prev);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { const float2 f = unpack_bf16x2(pp[i]); acc[q][2 * i] += f.x; acc[q][2 * i + 1] += f.y; }
+      }
+      *dst = make_uint4(pack_bf16x2(acc[q][0], acc[q][1]), pack_bf16x2(acc[q][2], acc[q][3]), pack_bf16x2(acc[q][4], acc[q][5]), pack_bf16x2(acc[q][6], acc[q][7]));
     }
-    o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]);
-    o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
-    reinterpret_cast<uint4*>(out + (size_t)row * hidden)[v] = o;
   }
 }
 
@@ -610,6 +621,10 @@ FF_EXPORT int ff_moe_grouped_gemm(const void* xs, const void* w, void* y, const 
 FF_EXPORT int ff_moe_combine(const void* y, const int* pos, const int* ids, const float* w, void* out, int rows,
                              int hidden, int top_k, int ldy, int accumulate, cudaStream_t s) {
   if (rows <= 0 || hidden % 8 || top_k < 1 || top_k > 16 || ldy % 8) return FF_HOST_BAD_SHAPE;
-  return launch_pdl(moe_combine_kernel, dim3(rows, (hidden / 8 + COMBINE_THREADS - 1) / COMBINE_THREADS), dim3(COMBINE_THREADS), 0, s, 0, (const __nv_bfloat16*)y,
-                    pos, ids, w, (__nv_bfloat16*)out, hidden, top_k, ldy, accumulate);
+  // From some hundred rows on a CTA per row fills the GPU, and a row's set-up (its choices, two barriers) is paid once; fewer rows are spread over CTAs: a
+  // CTA per row / spread, us: 300 rows of 4096 with eight choices 6.1 / 5.1, 600 rows 7.2 / 7.4; with two choices 300 rows 3.1 / 2.8, 511 rows 3.6 / 4.1.
+  const bool whole = rows >= (top_k <= 4 ? 320 : 512);
+  const int threads = whole ? 128 : 256, spread = whole ? 1 : (hidden / 8 + threads - 1) / threads;
+  auto kern = top_k == 1 ? moe_combine_kernel<1, 2> : top_k == 2 ? moe_combine_kernel<2, 2> : top_k <= 4 ? moe_combine_kernel<4, 2> : moe_combine_kernel<8, 1>;
+  return launch_pdl(kern, dim3(rows, spread), dim3(threads), 0, s, 0, (const __nv_bfloat16*)y, pos, ids, w, (__nv_bfloat16*)out, hidden, top_k, ldy, accumulate);
 }

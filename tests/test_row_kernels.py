@@ -217,3 +217,22 @@ def test_norm_of_wide_rows(hidden, waves):
         # one rounding of the result; the sum and its root in FP32
         assert ((got[:: max(1, rows // 20)].cpu().double() - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs()).all()
     ops.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,hidden,top_k", [(319, 2056, 1), (320, 2056, 1), (330, 1032, 2), (320, 520, 3), (400, 4104, 4), (511, 2056, 6), (512, 2056, 6), (600, 1032, 16)])
+def test_expert_rows_of_many_rows_combined(rows, hidden, top_k):
+    """A CTA per row and several: the weighted sum of a row's choices, some of them served elsewhere, vectors left over behind the last round."""
+    from flyingfish_b200 import ops
+    from flyingfish_b200.ops import moe_cuda
+    g = torch.Generator().manual_seed(rows)
+    ids = torch.stack([torch.randperm(40, generator=g)[:top_k] for _ in range(rows)]).to(torch.int32)
+    pos = torch.randperm(rows * top_k, generator=g).to(torch.int32)
+    pos[torch.rand(rows * top_k, generator=g) < 0.2] = -1
+    w, y = torch.rand(rows, top_k, generator=g), torch.randn(rows * top_k, hidden, generator=g).to(BF16)
+    got = moe_cuda.combine(y.cuda(), pos.cuda(), ids.cuda(), w.cuda(), rows, hidden).cpu().double()
+    ops.check_status()
+    terms = y.double()[pos.long().clamp_min(0)].view(rows, top_k, hidden) * (w.double() * (pos >= 0).view(rows, top_k))[..., None]
+    want, size = terms.sum(1), terms.abs().sum(1)
+    # one rounding of the result, a rounding of FP32 per addition
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + (top_k + 1) * 2.0 ** -23 * size).all()
