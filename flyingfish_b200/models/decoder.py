@@ -110,7 +110,9 @@ class DecoderModel:
         if self._chain_ok(b):
             return self._hidden_states_chain(b, kv, inputs_embeds)
         if b.positions.is_cuda and self.d == 128 and not s.qk_norm and \
-                (b.positions.shape[0] <= ops.SKINNY_MAX_M or type(self)._attention is DecoderModel._attention):
+                (b.positions.shape[0] <= ops.SKINNY_MAX_M or
+                 (type(self)._attention is DecoderModel._attention and type(w.layers[0].wqkv) is torch.Tensor and
+                  ops.rope_in_product(b.positions.shape[0], *w.layers[0].wqkv.shape))):
             # one cos/sin table per step for the fused QKV + rotary + KV-write kernels of all layers
             self._rope_cs = ops.rope_table(b.positions, self.d, s.rope_theta)
         if inputs_embeds is None:

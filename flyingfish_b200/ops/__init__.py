@@ -470,6 +470,12 @@ def rope_table(positions: torch.Tensor, rot_dim: int, theta: float, inv_freq: to
     return out
 
 
+def rope_in_product(rows: int, n: int, k: int) -> bool:
+    """Whether :func:`linear_rope_kv` over so many rows turns and caches heads of 128 in the product's epilogue: always in the decode product, above its
+    rows where that is the quicker form."""
+    return rows <= SKINNY_MAX_M or bool(kernels().ff_gemm_bf16_rope_in_product(rows, n, k))
+
+
 def linear_rope_kv(x: torch.Tensor, wqkv: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor,
                    kcache: torch.Tensor, vcache: torch.Tensor, hq: int, hkv: int, dim: int, theta: float,
                    rot_dim: int | None = None, inv_freq: torch.Tensor | None = None,
@@ -477,14 +483,14 @@ def linear_rope_kv(x: torch.Tensor, wqkv: torch.Tensor, positions: torch.Tensor,
     """Fused QKV projection + rotary embedding + paged KV write: ``qkv = x @ wqkv.T`` with Q and K
     rotated and K/V stored at ``slots``. 128-dim heads run as one kernel (the
     rotation and the cache write are the GEMM's epilogue; ``cos_sin`` from :func:`rope_table` is
-    reused across layers); everything else as GEMM + rope kernel."""
+    reused across layers) where :func:`rope_in_product` says so; everything else as GEMM + rope kernel."""
     m = x.shape[0]
     n = wqkv.shape[0]
     fused = (FUSE_ROPE and _is_cuda(x) and dim == 128 and n == (hq + 2 * hkv) * 128 and x.dtype == BF16
              and kcache.dim() == 4 and kcache.is_contiguous() and vcache.is_contiguous())
     if m > SKINNY_MAX_M and fused:                       # what the two kernels take and the one does not
         fused = (type(wqkv) is torch.Tensor and wqkv.dtype == kcache.dtype == vcache.dtype == BF16 and wqkv.shape[1] == x.shape[1] and
-                 (kcache.data_ptr() | vcache.data_ptr()) % 16 == 0)
+                 (kcache.data_ptr() | vcache.data_ptr()) % 16 == 0 and rope_in_product(m, n, x.shape[1]))
     if not fused:
         qkv = linear(x, wqkv)
         rope_kv_paged(qkv, positions, slots, kcache, vcache, hq, hkv, dim, theta, rot_dim, inv_freq)

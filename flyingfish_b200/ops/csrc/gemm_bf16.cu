@@ -189,30 +189,53 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
       }
     }
   } else if (epi == 3) {
-    // The values are rounded to BF16 and turned in BF16 arithmetic, as the rotation kernel turns the stored rows: the bits are the same. A pass
-    // over the rows of its own took 72 us of a layer at 8121 rows (32 + 16 heads) and 11 at 1000; here it runs under the next tile's main loop.
+    // The values are rounded to BF16 and turned in BF16 arithmetic, as the rotation kernel turns the stored rows: the bits are the same. It
+    // runs under the next tile's main loop, and a pass over the rows of its own falls away: product and rotation apart / in one, us: 8191 rows of 32 + 16 heads,
+    // K = 4096 317 / 281 (292 with the angles read again for every head, 8 bytes at a time), of 64 + 8 heads 476 / 416, of 8 + 4, K = 1024 50 / 44 (60);
+    // the last tile's is not hidden, see rope_in_product.
+    const int heads = tail.hq + 2 * tail.hkv, head0 = col0 >> 7;
+    int blk = -1, off = 0;                                // this row's place in the cache; a negative slot is a padding row, nothing cached
+    if (live && head0 + (width >> 7) > tail.hq) {
+      const int slot = tail.slots[row];
+      if (slot >= 0) { blk = slot / tail.block_size; off = slot - blk * tail.block_size; }
+      if (blk >= tail.num_blocks) { if (part == 0) set_status(status, KID_ROPE_KV, FF_ERR_BOUNDS, row, slot); blk = -1; }
+    }
+    const float2* angles = tail.cos_sin + (size_t)row * tail.rhalf;
+    const bool pairs = tail.rhalf % 2 == 0;               // two angles are 16 aligned bytes
 #pragma unroll 1
-    for (int h0 = 0; h0 < width; h0 += 128) {
-      const int head = (col0 + h0) >> 7;
-      if (head >= tail.hq + 2 * tail.hkv) break;
-      const bool is_v = head >= tail.hq + tail.hkv;
-      __nv_bfloat16* cached = nullptr;
-      if (live && head >= tail.hq) {
-        const int slot = tail.slots[row], blk = slot / tail.block_size, kvh = is_v ? head - tail.hq - tail.hkv : head - tail.hq;
-        if (slot >= 0 && blk >= tail.num_blocks) { if (part == 0) set_status(status, KID_ROPE_KV, FF_ERR_BOUNDS, row, slot); }
-        else if (slot >= 0) {                             // a negative slot: a padding row, nothing cached
-          if (part == 0) dbg_write_once(status, KID_ROPE_KV, is_v ? DBG_KV_V : DBG_KV_K, (long long)slot * tail.hkv + kvh);
-          cached = (is_v ? tail.vcache : tail.kcache) + (((size_t)blk * tail.hkv + kvh) * tail.block_size + (slot - blk * tail.block_size)) * 128;
+    for (int c = 16 * part; c < 64; c += 16 * PARTS) {
+      // The angles of 16 columns, once for the heads of a tile and in front of the tile's values: next to the ring there is hardly a first-level
+      // cache that would hold them.
+      float4 t[8];
+      const bool turned = live && head0 < tail.hq + tail.hkv && c < tail.rhalf;
+      if (turned) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int i = c + 2 * j;
+          if (pairs && i < tail.rhalf) t[j] = __ldg(reinterpret_cast<const float4*>(angles + i));
+          else {
+            const float2 t0 = i < tail.rhalf ? __ldg(angles + i) : make_float2(1.f, 0.f), t1 = i + 1 < tail.rhalf ? __ldg(angles + i + 1) : make_float2(1.f, 0.f);
+            t[j] = make_float4(t0.x, t0.y, t1.x, t1.y);
+          }
         }
       }
-      __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + col0 + h0;
 #pragma unroll 1
-      for (int c = 16 * part; c < 64; c += 16 * PARTS) {
+      for (int h0 = 0; h0 < width; h0 += 128) {
+        const int head = head0 + (h0 >> 7);
+        if (head >= heads) break;
+        const bool is_v = head >= tail.hq + tail.hkv;
         uint32_t a[16], b[16];
         tmem_ld_x16(taddr + h0 + c, a);
         tmem_ld_x16(taddr + h0 + c + 64, b);
         tmem_ld_wait();
         if (live) {
+          __nv_bfloat16* cached = nullptr;
+          if (blk >= 0 && head >= tail.hq) {
+            const int kvh = is_v ? head - tail.hq - tail.hkv : head - tail.hq;
+            if (c == 0) dbg_write_once(status, KID_ROPE_KV, is_v ? DBG_KV_V : DBG_KV_K, ((long long)blk * tail.block_size + off) * tail.hkv + kvh);
+            cached = (is_v ? tail.vcache : tail.kcache) + (((size_t)blk * tail.hkv + kvh) * tail.block_size + off) * 128;
+          }
+          __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(Cout) + (size_t)row * ldc + col0 + h0;
           auto r = [](float x) { return __bfloat162float(__float2bfloat16(x)); };
           uint32_t lo[8], hi[8];
 #pragma unroll
@@ -222,11 +245,10 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
             for (int e = 0; e < 2; ++e) {
               x[e] = r(__uint_as_float(a[2 * j + e]));
               y[e] = r(__uint_as_float(b[2 * j + e]));
-              if (!is_v && c + 2 * j + e < tail.rhalf) {
-                const float2 t = __ldg(tail.cos_sin + (size_t)row * tail.rhalf + c + 2 * j + e);
-                const float u = x[e], v = y[e];
-                x[e] = r(u * t.x) - r(v * t.y);
-                y[e] = r(v * t.x) + r(u * t.y);
+              if (turned && !is_v && c + 2 * j + e < tail.rhalf) {
+                const float cs = e ? t[j].z : t[j].x, sn = e ? t[j].w : t[j].y, u = x[e], v = y[e];
+                x[e] = r(u * cs) - r(v * sn);
+                y[e] = r(v * cs) + r(u * sn);
               }
             }
             lo[j] = pack_bf16x2(x[0], x[1]);
@@ -802,6 +824,37 @@ static float pair_plan(int M, int N, int epi, int pairs, PairTiles& best) {
   return least;
 }
 
+// Tiles of one CTA where they finish in clearly fewer waves: 256-row tiles of pairs pad rows more, and at short K a pair's set-up and its
+// epilogue take what its main loop saves. A wave of one-CTA tiles is charged 1 / 0.86 of a pair's; with a SwiGLU epilogue 1 / 0.79, at K up to 2048
+// 1 / 0.97; 1 / 1.05 at K up to 512, and at K up to 1024 for a single wave or a SwiGLU epilogue (tanh-GELU, which computes more: 4096 x 8192 x
+// 1024 53 / 47 us). Both forms in turn at 736 sizes (24 shapes of 512 x 512 to
+// 65536 x 2048, 129 to 8191 rows): that is the quicker form within 2 % at all but 6, within 3.3 % at those. One-CTA / pair tiles: 1100 x 4096 x 14336
+// 95 / 104 us, 1100 x 8192 x 1024 21 / 23, 4096 x 32768 x 512 152 / 180, 600 x 36864 x 7168 251 / 263.
+// K is walked in the same order: the bits are the same.
+// pt: the pairs' tiles; waves: of 256-wide pair tiles, the time the launch is reckoned to take.
+static bool one_cta_tiles(int M, int N, int K, int epi, bool gated, PairTiles& pt, float& waves) {
+  const int ctas = sm_count(), waves1 = (((M + BM - 1) / BM) * ((N + 255) / 256) + ctas - 1) / ctas;
+  const float share = K <= 512 || (K <= 1024 && (waves1 == 1 || (epi == 1 && !gated))) ? 1.05f : epi != 1 ? 0.86f : K <= 2048 ? 0.97f : 0.79f;
+  const float pair_waves = pair_plan(M, N, epi, ctas / 2, pt) / pair_cost(256);
+  const bool one = waves1 < share * pair_waves;
+  waves = one ? waves1 / share : pair_waves;
+  return one;
+}
+
+// Whether rotation and cache write go into a QKV product's epilogue (host only). Heads want tiles of whole 128 columns, which fill a last wave less well, and
+// the last tile's epilogue is not hidden; a pass of its own costs a launch and its bytes. Fitted to both, timed at 53 sizes (7 shapes of 896 x 640 to
+// 10240 x 8192, 129 to 8191 rows): the quicker within 1 % at all but two, within 4 % at those. Apart / in one, us: 300 rows of 32 + 16 heads, K = 4096
+// 31.7 / 37.1, 1000 rows 50.8 / 48.8; 300 rows of 64 + 8 heads 41.6 / 38.5; 512 rows of 8 + 4, K = 1024 13.5 / 14.8, 1000 rows 17.3 / 15.0.
+static bool rope_in_product(int M, int N, int K) {
+  PairTiles pt;
+  float apart, in;
+  one_cta_tiles(M, N, K, 0, false, pt, apart);
+  one_cta_tiles(M, N, K, 3, false, pt, in);
+  const float wave_us = 552.0f / 1900.0f * K / BK;
+  return in * wave_us < apart * wave_us - 0.5f + 0.25e-6f * 2.0f * M * N;
+}
+FF_EXPORT int ff_gemm_bf16_rope_in_product(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && N % 128 == 0 && rope_in_product(M, N, K) ? 1 : 0; }
+
 // the plan as {w1, wide, w2} (host only)
 FF_EXPORT int ff_gemm_bf16_pair_tiles(int M, int N, int epi, int pairs, int* tiles) {
   if (M <= 0 || N <= 0 || pairs <= 0 || epi < 0 || epi > 3) return FF_HOST_BAD_SHAPE;
@@ -843,26 +896,16 @@ static int gemm_bf16_launch(const void* X, const void* W, void* Y, int M, int N,
   if (reinterpret_cast<uintptr_t>(Y) & 15) return FF_HOST_BAD_ALIGN;
   CUtensorMap tmA;
   if (int e = make_tmap_2d(&tmA, X, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, (uint64_t)ldx * 2, BK, BM)) return e;
-  const int pairs = sm_count() / 2;
   PairTiles pt;
-  const float pair_waves = pair_plan(M, N, epi, pairs, pt) / pair_cost(256);
-  // Tiles of one CTA where they finish in clearly fewer waves: 256-row tiles of pairs pad rows more, and at short K a pair's set-up and its
-  // epilogue take what its main loop saves. A wave of one-CTA tiles is charged 1 / 0.86 of a pair's; with a SwiGLU epilogue 1 / 0.79, at K up to 2048
-  // 1 / 0.97; 1 / 1.05 at K up to 512, and at K up to 1024 for a single wave or a SwiGLU epilogue (tanh-GELU, which computes more: 4096 x 8192 x
-  // 1024 53 / 47 us). Both forms in turn at 736 sizes (24 shapes of 512 x 512 to
-  // 65536 x 2048, 129 to 8191 rows): that is the quicker form within 2 % at all but 6, within 3.3 % at those. One-CTA / pair tiles: 1100 x 4096 x 14336
-  // 95 / 104 us, 1100 x 8192 x 1024 21 / 23, 4096 x 32768 x 512 152 / 180, 600 x 36864 x 7168 251 / 263.
-  // K is walked in the same order: the bits are the same.
-  const int ctas = sm_count(), waves1 = (((M + BM - 1) / BM) * ((N + 255) / 256) + ctas - 1) / ctas;
-  const float share = K <= 512 || (K <= 1024 && (waves1 == 1 || (epi == 1 && tail.gate == 0))) ? 1.05f : epi != 1 ? 0.86f : K <= 2048 ? 0.97f : 0.79f;
-  if (waves1 < share * pair_waves) {
+  float waves;
+  if (one_cta_tiles(M, N, K, epi, tail.gate != 0, pt, waves)) {
     constexpr int BN = 256, STAGES = 4;
     CUtensorMap tmB;
     if (int e = make_tmap_2d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, N, (uint64_t)ldw * 2, BK, BN)) return e;
     const int smem = STAGES * (BM + BN) * BK * 2 + 1024, tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     auto kern = gemm_bf16_kernel<BN, STAGES, 0>;
     if (int e = opt_in_smem(kern, smem)) return e;
-    kern<<<tiles < ctas ? tiles : ctas, 320, smem, stream>>>(tmA, tmA, tmA, tmB, Y, M, N, K, ldy, epi, status, CommArgs{}, GroupArgs{}, tail);
+    kern<<<tiles < sm_count() ? tiles : sm_count(), 320, smem, stream>>>(tmA, tmA, tmA, tmB, Y, M, N, K, ldy, epi, status, CommArgs{}, GroupArgs{}, tail);
     return launch_result();
   }
   return pair_launch(tmA, W, Y, M, N, K, ldw, ldy, epi, pt, tail, status, stream);

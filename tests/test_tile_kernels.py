@@ -426,9 +426,10 @@ def test_merge_of_many_splits(ctx):
 @pytest.mark.gpu
 @pytest.mark.parametrize("m", [129, 300, 1000])
 @pytest.mark.parametrize("hq,hkv,k,rot", [(8, 2, 1024, 128), (32, 8, 256, 128), (5, 1, 520, 64)])      # tiles of pairs and of single CTAs, a part turned
-def test_rotation_in_the_product_of_prompts(m, hq, hkv, k, rot):
+def test_rotation_in_the_product_of_prompts(m, hq, hkv, k, rot, monkeypatch):
     """The bits of the product followed by the rotation kernel, in the rows and in the cache; padding rows are not cached."""
     from flyingfish_b200 import ops
+    monkeypatch.setattr(ops, "rope_in_product", lambda *a: True)           # also at sizes where the kernels apart are quicker
     n, blocks = (hq + 2 * hkv) * 128, 20
     x, w = _rand((m, k), 1).cuda(), (_rand((n, k), 2) * 0.1).cuda()
     g = torch.Generator().manual_seed(m)
@@ -444,6 +445,19 @@ def test_rotation_in_the_product_of_prompts(m, hq, hkv, k, rot):
     torch.cuda.synchronize()
     ops.check_status()
     assert torch.equal(got, want) and torch.equal(k0, k1) and torch.equal(v0, v1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rot", [2, 66, 94, 96])                 # an odd number of angles, which lie on 8 bytes; ends inside a group of columns
+def test_part_rotation_in_the_product_of_prompts(rot, monkeypatch):
+    test_rotation_in_the_product_of_prompts(300, 6, 3, 512, rot, monkeypatch)
+
+
+def test_rotation_joins_the_products_that_hide_it():
+    from flyingfish_b200 import ops
+    shapes = [((hq + 2 * hkv) * 128, k) for hq, hkv, k in ((32, 8, 4096), (8, 2, 1024), (64, 8, 8192), (16, 16, 2048))]
+    assert all(ops.rope_in_product(m, n, k) for n, k in shapes for m in (1, 128, 4096, 8191))
+    assert not any(ops.rope_in_product(m, n, k) for n, k in shapes for m in (129, 512))
 
 
 @pytest.mark.gpu
