@@ -519,6 +519,29 @@ def test_splits_share_the_pages_evenly(lens, hq, hkv, nq):
     assert torch.equal(full, wide)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[5, 64, 66, 300, 1000], [70] * 40])         # one split with keys, several, two of which one has pages
+@pytest.mark.parametrize("nq", [3, 8])
+def test_splits_of_draft_trees(lens, nq):
+    """Rows of a draft tree see the context and their ancestors, wherever the last pages fall among the splits."""
+    from flyingfish_b200 import ops
+    hq, hkv, d, blocks, pool = 8, 2, 128, 32, 30
+    lens = [max(n, nq) for n in lens]
+    b, g = len(lens), torch.Generator().manual_seed(nq)
+    masks = torch.zeros(b, nq, dtype=torch.int64)
+    for i in range(nq):                                      # a parent among the rows before, and the row itself
+        masks[:, i] = 1 << i
+        if i:
+            masks[:, i] |= masks.gather(1, torch.randint(0, i, (b, 1), generator=g))[:, 0]
+    q, k, v = _rand((b * nq, hq * d), 1), _rand((pool, hkv, 64, d), 2), _rand((pool, hkv, 64, d), 3)
+    table = torch.randint(0, pool, (b, blocks), generator=g).to(torch.int32)
+    ctx = torch.tensor(lens, dtype=torch.int32)
+    got = ops.attn_decode(q.cuda(), k.cuda(), v.cuda(), table.cuda(), ctx.cuda(), hq, hkv, d, d ** -0.5, nq=nq, tree_mask=masks.view(-1).cuda(), max_ctx=blocks * 64)
+    ops.check_status()
+    want = ops.attn_decode(q, k, v, table, ctx, hq, hkv, d, d ** -0.5, nq=nq, tree_mask=masks.view(-1), max_ctx=blocks * 64).float()
+    assert ((got.cpu().float() - want).abs() <= 1e-2 + 1e-2 * want.abs()).all()      # BF16 weights and result
+
+
 @pytest.mark.parametrize("n,k", [(7168, 18432), (7168, 2560), (4096, 7168), (6144, 4096), (34048, 512), (33920, 512), (576, 2560), (128, 128)])
 def test_fp8_split_does_not_depend_on_the_rows(n, k):
     import ctypes
