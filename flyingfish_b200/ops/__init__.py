@@ -490,7 +490,9 @@ def linear_rope_kv(x: torch.Tensor, wqkv: torch.Tensor, positions: torch.Tensor,
              and kcache.dim() == 4 and kcache.is_contiguous() and vcache.is_contiguous())
     if m > SKINNY_MAX_M and fused:                       # what the two kernels take and the one does not
         fused = (type(wqkv) is torch.Tensor and wqkv.dtype == kcache.dtype == vcache.dtype == BF16 and wqkv.shape[1] == x.shape[1] and
-                 (kcache.data_ptr() | vcache.data_ptr()) % 16 == 0 and rope_in_product(m, n, x.shape[1]))
+                 (kcache.data_ptr() | vcache.data_ptr()) % 16 == 0 and (cos_sin is None or (
+                     cos_sin.dtype == torch.float32 and cos_sin.shape == (m, (rot_dim or dim) // 2, 2) and cos_sin.is_contiguous() and cos_sin.data_ptr() % 8 == 0))
+                 and rope_in_product(m, n, x.shape[1]))
     if not fused:
         qkv = linear(x, wqkv)
         rope_kv_paged(qkv, positions, slots, kcache, vcache, hq, hkv, dim, theta, rot_dim, inv_freq)

@@ -201,7 +201,7 @@ __device__ __forceinline__ void store_tile_row(uint32_t taddr, void* __restrict_
       if (blk >= tail.num_blocks) { if (part == 0) set_status(status, KID_ROPE_KV, FF_ERR_BOUNDS, row, slot); blk = -1; }
     }
     const float2* angles = tail.cos_sin + (size_t)row * tail.rhalf;
-    const bool pairs = tail.rhalf % 2 == 0;               // two angles are 16 aligned bytes
+    const bool pairs = tail.rhalf % 2 == 0 && (reinterpret_cast<uintptr_t>(tail.cos_sin) & 15) == 0;     // two angles are 16 aligned bytes
 #pragma unroll 1
     for (int c = 16 * part; c < 64; c += 16 * PARTS) {
       // The angles of 16 columns, once for the heads of a tile and in front of the tile's values: next to the ring there is hardly a first-level
@@ -936,7 +936,7 @@ FF_EXPORT int ff_gemm_bf16_rope_kv(const void* X, const void* W, void* Y, int M,
                                    const int* slots, void* kcache, void* vcache, int hq, int hkv, int rot_dim, int block_size, int num_blocks,
                                    int* status, cudaStream_t stream) {
   if (hq <= 0 || hkv <= 0 || N != (hq + 2 * hkv) * 128 || rot_dim <= 0 || rot_dim > 128 || rot_dim % 2 || block_size <= 0 || num_blocks <= 0) return FF_HOST_BAD_SHAPE;
-  if (cos_sin == nullptr || slots == nullptr || ((reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15)) return FF_HOST_BAD_ALIGN;
+  if (cos_sin == nullptr || slots == nullptr || (reinterpret_cast<uintptr_t>(cos_sin) & 7) || ((reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15)) return FF_HOST_BAD_ALIGN;
   LinTail tail = {};
   tail.cos_sin = reinterpret_cast<const float2*>(cos_sin); tail.slots = slots;
   tail.kcache = static_cast<__nv_bfloat16*>(kcache); tail.vcache = static_cast<__nv_bfloat16*>(vcache);

@@ -453,6 +453,26 @@ def test_part_rotation_in_the_product_of_prompts(rot, monkeypatch):
     test_rotation_in_the_product_of_prompts(300, 6, 3, 512, rot, monkeypatch)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])                 # floats in front of the table: 16, 4 and 8 byte boundaries
+def test_rotation_in_the_product_takes_any_table(offset, monkeypatch):
+    from flyingfish_b200 import ops
+    monkeypatch.setattr(ops, "rope_in_product", lambda *a: True)
+    m, hq, hkv, k, blocks = 140, 4, 2, 256, 3
+    x, w = _rand((m, k), 1).cuda(), (_rand(((hq + 2 * hkv) * 128, k), 2) * 0.1).cuda()
+    pos = torch.arange(m, dtype=torch.int32).cuda()
+    table = ops.rope_table(pos, 128, 5e5)
+    moved = torch.cat([torch.zeros(offset, device="cuda"), table.view(-1)])[offset:].view(table.shape)
+    assert moved.data_ptr() % 16 == 4 * offset
+    out = []
+    for t in (None, moved):
+        kc, vc = (torch.zeros(blocks, hkv, 64, 128, dtype=BF16, device="cuda") for _ in range(2))
+        out.append((ops.linear_rope_kv(x, w, pos, pos, kc, vc, hq, hkv, 128, 5e5, cos_sin=t), kc, vc))
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
 def test_rotation_joins_the_products_that_hide_it():
     from flyingfish_b200 import ops
     shapes = [((hq + 2 * hkv) * 128, k) for hq, hkv, k in ((32, 8, 4096), (8, 2, 1024), (64, 8, 8192), (16, 16, 2048))]
