@@ -800,7 +800,7 @@ class Engine:
     def _read_ids(self, ids: torch.Tensor) -> list[int]:
         """The step's ids on the host, and its device status looked at: both behind one wait."""
         n, read = ids.numel(), self.prefill_batch.results
-        if not ids.is_cuda or ids.dtype != torch.int32 or not ids.is_contiguous() or n + 4 > read.numel():
+        if not ids.is_cuda or ids.dim() != 1 or ids.dtype != torch.int32 or not ids.is_contiguous() or n + 4 > read.numel():
             toks = [int(t) for t in ids.cpu().tolist()]
             self._after_sync()
             return toks
