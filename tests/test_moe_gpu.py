@@ -138,6 +138,78 @@ def test_model_with_packed_nvfp4_experts():
     ops.check_status()
 
 
+def _decode64(w, spec, tokens, k64, v64):
+    """A decode step of one sequence in 64 bits (``k64``, ``v64``: its cached rows of every layer): logits, and the smallest distance, in standard
+    deviations of a layer's router logits, between a chosen expert and one that is not."""
+    d, hq, hkv, moe = spec.head_dim, spec.heads, spec.kv_heads, spec.moe
+    norm = lambda x, g: x * torch.rsqrt(x.square().mean(-1, keepdim=True) + spec.rms_eps) * g.double()
+    pos = k64[0].shape[0]
+    ang = pos * spec.rope_theta ** (-torch.arange(0, d, 2, dtype=torch.float64, device="cuda") / d)
+    turn = lambda x: torch.cat([x[..., : d // 2] * ang.cos() - x[..., d // 2:] * ang.sin(), x[..., d // 2:] * ang.cos() + x[..., : d // 2] * ang.sin()], -1)
+    x, clear = w.embed[tokens].double(), float("inf")
+    for lw, k, v in zip(w.layers, k64, v64):
+        q, kn, vn = (norm(x, lw.input_ln) @ lw.wqkv.double().t()).view(-1, d).split([hq, hkv, hkv])
+        q = turn(norm(q, lw.q_norm)).view(hkv, -1, d)
+        k, v = torch.cat([k, turn(norm(kn, lw.k_norm))[None]]), torch.cat([v, vn[None]])
+        o = torch.einsum("hgt,thd->hgd", torch.softmax(torch.einsum("hgd,thd->hgt", q, k) * d ** -0.5, -1), v)
+        x = x + o.reshape(-1) @ lw.wo.double().t()
+        n = norm(x, lw.post_ln)
+        scores = n @ lw.router.double().t()
+        top = scores.topk(moe.top_k + 1)
+        clear = min(clear, float((top.values[-2] - top.values[-1]) / scores.std()))
+        ids, share = top.indices[:-1], torch.softmax(top.values[:-1], -1)
+        gu, dn = lw.extra["experts64"]
+        for e, s in zip(ids.tolist(), share):
+            gate, up = (n @ gu[e].t()).chunk(2)
+            x = x + s * ((gate * torch.sigmoid(gate) * up) @ dn[e].t())
+    return norm(x, w.final_norm) @ w.lm_head.double().t(), clear
+
+
+def test_decode_steps_of_packed_experts_near_64_bits():
+    """Decode steps over seeds and context lengths, most of them cut into several splits: a row whose experts are chosen by a clear distance stays near
+    64 bits, and rows whose rounding may turn a choice are the fewer."""
+    from flyingfish_b200.api import Model
+    from flyingfish_b200.config import Settings
+    from flyingfish_b200.engine.engine import bucket_for
+    from flyingfish_b200.ops.moe_cuda import interleave64
+    from flyingfish_b200.ops.quant_ops import dequant_nvfp4
+    batch, page = 24, 64
+    m = Model.load("qwen3-moe-fp4-tiny", Settings(capacity=1024, max_batch=32), device="cuda", seed=0)
+    eng, spec, w = m.engine, m.engine.spec, m.engine.model.w
+    for lw in w.layers:
+        gu, dn = ([dequant_nvfp4(s.codes[e], s.scales[e], s.global_scale[e]).double() for e in range(s.experts)] for s in lw.extra["experts_fp4"])
+        back = interleave64(torch.arange(gu[0].shape[0], device="cuda").view(1, -1, 1)).view(-1).argsort()
+        lw.extra["experts64"] = ([t[back] for t in gu], dn)
+    logits = eng.capture(bucket_for(batch)).logits
+    errors = []
+    for seed in range(6):
+        g = torch.Generator().manual_seed(seed)
+        lens, tokens = torch.randint(1, 900, (batch,), generator=g).tolist(), torch.randint(0, spec.vocab, (batch,), generator=g).tolist()
+        eng.reset()
+        seqs, used = [], []
+        for n, tok in zip(lens, tokens):
+            s = eng.add_sequence([0] * n)
+            eng.kv.reserve(s.seq_id, n)
+            eng.kv.commit(s.seq_id, n)
+            s.prefilled, s.pending = n, tok
+            seqs.append(s)
+            used.append(torch.tensor(list(eng.kv.seqs[s.seq_id].blocks)[: (n + page - 1) // page], device="cuda"))
+        for t in eng.kv.k + eng.kv.v:
+            t.copy_(torch.randn(t.shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda"))
+        cached = lambda pools, i: [t[used[i]].transpose(1, 2).reshape(-1, spec.kv_heads, spec.head_dim)[: lens[i]].double() for t in pools]
+        context = [(cached(eng.kv.k, i), cached(eng.kv.v, i)) for i in range(batch)]
+        eng.decode(seqs)
+        got = logits[:batch].double()
+        for i in range(batch):
+            want, clear = _decode64(w, spec, tokens[i], *context[i])
+            errors.append((float((got[i] - want).norm() / want.norm()), clear))
+    ops.check_status()
+    sure = [e for e, clear in errors if clear > 0.05]
+    print(f"{len(sure)} of {len(errors)} rows: worst {max(sure):.4f}, mean {sum(sure) / len(sure):.4f}; of all: worst {max(e for e, _ in errors):.4f}")
+    assert len(sure) > len(errors) / 2
+    assert max(sure) < 0.03                                  # BF16 roundings of two layers
+
+
 @pytest.mark.parametrize("name", ["qwen3-moe-tiny", "qwen3-moe-fp4-tiny"])
 def test_tiered_provider_gpu_half_resident(name):
     """Half of the experts in GPU slots (BF16 slots, or packed NVFP4 slots for an NVFP4-expert model), the rest served
